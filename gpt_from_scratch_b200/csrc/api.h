@@ -1,0 +1,36 @@
+// C entry points of the library that are also called from inside it (model.cu strings them into
+// whole passes over a stack of transformer blocks). The definitions document the arguments.
+#pragma once
+#include <stddef.h>
+
+extern "C" {
+int gfs_gemm_bf16_rope(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb,
+                       int ldc, int ldr, int a_mn_major, int b_mn_major, int add, void* ws, size_t ws_bytes,
+                       int force_split, const void* rope_cos, const void* rope_sin, int rope_cols, int rope_d,
+                       int rope_b, void* stream);
+int gfs_gemm2_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,
+                   int ldr, int a_mn_major, int b_mn_major, const void* rope_cos, const void* rope_sin, int rope_cols,
+                   int rope_d, int rope_b, void* stream);
+int gfs_gemm_bf16_swiglu(int mode, const void* a, const void* b, void* c, void* extra, int M, int I, int K, int lda,
+                         int ldb, int ldc, int ld_extra, void* stream);
+int gfs_gemm2_bf16_swiglu(int mode, const void* a, const void* b, void* c, void* extra, int M, int I, int K, int lda,
+                          int ldb, int ldc, int ld_extra, void* stream);
+int gfs_gemm2_wgrad_grouped(int n, const unsigned long long* A, const unsigned long long* B,
+                            const unsigned long long* C, const int* M, const int* N, const int* K, const int* lda,
+                            const int* ldb, const int* ldc, const int* accumulate, void* stream);
+int gfs_gemm_bf16_launches(int M, int N, int K, size_t ws_bytes);
+int gfs_rmsnorm_fwd(const void* x, const void* w, void* y, void* rstd, int rows, int H, float eps, void* stream);
+int gfs_rmsnorm_bwd_parts(int rows);
+int gfs_rmsnorm_bwd(const void* dy, const void* x, const void* w, const void* rstd, const void* dres, void* dx,
+                    void* dw, void* partial, int rows, int H, int accumulate_dw, void* stream);
+int gfs_rmsnorm_dw_reduce_multi(int n, const unsigned long long* partial, const unsigned long long* dw,
+                                const int* parts, const int* accumulate, int H, void* stream);
+int gfs_dropout_residual(const void* x, const void* residual, void* out, long long n, float p, unsigned long long seed,
+                         int backward, void* stream);
+int gfs_swiglu_bwd(const void* dact, const void* gu, void* dgu, int M, int I, void* stream);
+int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int S, int B, int nh, int D,
+                  const long long* strides, float scale, int causal, void* stream);
+int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dO, const void* lse,
+                  void* dvec, void* dq, void* dk, void* dv, int S, int B, int nh, int D, const long long* strides,
+                  float scale, int causal, const void* rope_cos, const void* rope_sin, void* stream);
+}

@@ -81,18 +81,27 @@ struct Key2DHash {
   }
 };
 
+// The caches are bounded: a full one is emptied (maps are cheap to rebuild). Callers still hold the
+// pointers they were given for the launch in progress, so those maps are only freed when the cache has
+// filled up once more.
+template <typename Cache>
+static void retire_maps(Cache& cache, std::vector<CUtensorMap*>& retired) {
+  for (CUtensorMap* m : retired) delete m;
+  retired.clear();
+  for (auto& kv : cache) retired.push_back(kv.second);
+  cache.clear();
+}
+
 const CUtensorMap* tmap_2d_cached(const void* base, uint64_t rows, uint64_t cols, uint64_t ld_elems,
                                   uint32_t box_rows, uint32_t box_cols) {
   static std::mutex mu;
   static std::unordered_map<Key2D, CUtensorMap*, Key2DHash> cache;
+  static std::vector<CUtensorMap*> retired;
   Key2D key{base, rows, cols, ld_elems, box_rows, box_cols};
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find(key);
   if (it != cache.end()) return it->second;
-  if (cache.size() > 8192) {  // bounded: drop everything, maps are cheap to rebuild
-    for (auto& kv : cache) delete kv.second;
-    cache.clear();
-  }
+  if (cache.size() > 8192) retire_maps(cache, retired);
   CUtensorMap* m = new CUtensorMap;
   uint64_t dims[2] = {cols, rows};
   uint64_t strides[2] = {2, ld_elems * 2};
@@ -127,6 +136,7 @@ const CUtensorMap* tmap_nd_cached(const void* base, int rank, const uint64_t* di
                                   const uint32_t* box) {
   static std::mutex mu;
   static std::unordered_map<KeyND, CUtensorMap*, KeyNDHash> cache;
+  static std::vector<CUtensorMap*> retired;
   KeyND key;
   memset(&key, 0, sizeof(key));
   key.base = base;
@@ -139,10 +149,7 @@ const CUtensorMap* tmap_nd_cached(const void* base, int rank, const uint64_t* di
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find(key);
   if (it != cache.end()) return it->second;
-  if (cache.size() > 8192) {
-    for (auto& kv : cache) delete kv.second;
-    cache.clear();
-  }
+  if (cache.size() > 8192) retire_maps(cache, retired);
   CUtensorMap* m = new CUtensorMap;
   if (encode_tmap_bf16(m, base, rank, dims, strides_bytes, box) != 0) {
     delete m;

@@ -344,3 +344,50 @@ def test_cuda_graph_step_matches_eager(cuda_device):
     t = batches[0][:4]
     loss = float(eng.train_step(t[:, :-1].contiguous().cuda(), t[:, 1:].contiguous().cuda()))   # other shape: eager
     assert loss == loss and eng.optimizer._step_count == 9
+
+
+@pytest.mark.parametrize("H,heads,I,layers,V,B,S,dropout", [
+    (256, 4, 512, 2, 512, 4, 128, 0.0),       # tiles that divide everything
+    (128, 2, 200, 1, 264, 3, 33, 0.0),        # one block, ragged rows and columns
+    (256, 2, 520, 3, 1032, 2, 77, 0.0),       # head_dim 128
+    (768, 12, 2048, 2, 1024, 8, 512, 0.0),    # CTA pairs and grouped weight gradients
+    (256, 4, 512, 2, 512, 3, 50, 0.1),
+])
+def test_native_model_pass_matches_module_path(cuda_device, H, heads, I, layers, V, B, S, dropout):
+    """The whole-model native pass against the module-by-module path it replaces (a forward hook keeps a
+    model on the latter): the same kernels in the same order, so the same bits; with dropout the module
+    path rounds the two gradients of a residual branch one by one."""
+    from gpt_from_scratch_b200.config import GPTConfig
+    from gpt_from_scratch_b200.engine import TrainEngine
+    from gpt_from_scratch_b200.models import native
+    from gpt_from_scratch_b200.parallel import parallel_state as ps
+    ps.set_device(cuda_device)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_parallel_state(1)
+    cfg = GPTConfig(vocab_size=V, hidden_size=H, num_layers=layers, num_attention_heads=heads,
+                    max_position_embeddings=S, intermediate_size=I, dropout_prob=dropout)
+    g = torch.Generator().manual_seed(3)
+    batches = [torch.randint(0, V, (B, S + 1), generator=g) for _ in range(3)]
+    runs = []
+    for modules in (False, True):
+        torch.manual_seed(11)
+        eng = TrainEngine(cfg, lr=1e-3, seed=5)
+        if modules:
+            eng.model.layers[-1].mlp.register_forward_hook(lambda *a: None)
+        assert (native.plan_for(eng.model, batches[0].cuda()) is None) == modules
+        losses = []
+        for t in batches:
+            x, y = t[:, :-1].contiguous().cuda(), t[:, 1:].contiguous().cuda()
+            losses.append(eng.train_step(x, y).item())
+        with torch.no_grad():
+            logits = eng.model(x)
+        runs.append((losses, logits, eng.optimizer.grad_buffer.clone(), eng.optimizer.fp32_master_shard.clone()))
+    if dropout == 0.0:
+        assert runs[0][0] == runs[1][0]
+        for a, b in zip(runs[0][1:], runs[1][1:]):
+            assert torch.equal(a, b)
+        return
+    # one bf16 rounding (2^-9) per residual gradient, amplified over three steps at lr 1e-3
+    assert all(abs(a - b) < 1e-2 for a, b in zip(runs[0][0], runs[1][0])), (runs[0][0], runs[1][0])
+    rel = (runs[0][3] - runs[1][3]).norm() / runs[1][3].norm()
+    assert rel < 1e-2, rel
