@@ -112,7 +112,7 @@ class TrainEngine:
         system), undo its host-side effects, say so once and keep the eager loop."""
         import sys
         from .ops import gemm as gemm_ops
-        from .ops import rmsnorm as rmsnorm_ops
+        from .ops.rmsnorm import _dw_queue
         steps_before = self.optimizer._step_count
         try:
             self._capture(inputs, labels)
@@ -123,7 +123,7 @@ class TrainEngine:
             symm.abort_graph_capture()
             gemm_ops._wgrad_queue.items.clear()          # parked work refers to tensors of the failed capture
             gemm_ops._wgrad_queue.tiles = 0
-            rmsnorm_ops._dw_queue.items.clear()
+            _dw_queue.items.clear()
             if self.optimizer._step_count != steps_before:   # the captured step never ran on the GPU
                 self.optimizer._step_count = steps_before
                 st = self.optimizer._adam_state()
