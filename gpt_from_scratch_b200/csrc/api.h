@@ -28,6 +28,21 @@ int gfs_rmsnorm_dw_reduce_multi(int n, const unsigned long long* partial, const 
 int gfs_dropout_residual(const void* x, const void* residual, void* out, long long n, float p, unsigned long long seed,
                          int backward, void* stream);
 int gfs_swiglu_bwd(const void* dact, const void* gu, void* dgu, int M, int I, void* stream);
+int gfs_embedding_fwd(const void* ids, const void* W, void* out, int B, int S, int H, int v0, int v1, int s0,
+                      int s_count, void* stream);
+int gfs_embedding_sort_keys(const void* ids_bs, void* keys, int B, int S, int v0, int v1, void* stream);
+int gfs_embedding_bwd_keys(const void* keys, const void* dout, void* dW, int n, int H, int shift, void* stream);
+int gfs_gemm2_ce_parts(int N);
+int gfs_gemm2_bf16_ce(const void* A, const void* B, void* C, void* partials, int M, int N, int K, int lda, int ldb,
+                      int ldc, void* stream);
+int gfs_ce_fwd(const void* logits, const void* target, void* stats, void* lse, void* loss, int M, int Vp, long ld,
+               int v0, int single_rank, int target_batch, void* stream);
+int gfs_ce_from_partials(const void* partials, const void* logits, const void* target, void* stats, void* lse,
+                         void* loss, int parts, int M, int Vp, long ld, int v0, int single_rank, int target_batch,
+                         void* stream);
+int gfs_ce_bwd(void* logits, const void* lse, const void* target, const void* grad_rows, float grad_all, int M, int Vp,
+               long ld, int v0, int target_batch, void* stream);
+int gfs_mean_f32(const void* x, void* out, int n, void* stream);
 int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int S, int B, int nh, int D,
                   const long long* strides, float scale, int causal, void* stream);
 int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dO, const void* lse,

@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "api.h"
 #include "common.cuh"
 
 using namespace gfs;

@@ -6,6 +6,7 @@
 // (RoPE), core/mlp.py:25-28 (SwiGLU), core/tensor_parallel/layers.py:117-134 (embedding).
 #include <algorithm>
 
+#include "api.h"
 #include "common.cuh"
 
 using namespace gfs;

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstdio>
 
+#include "api.h"
 #include "common.cuh"
 
 using namespace gfs;
@@ -623,11 +624,6 @@ extern "C" {
 // ws/ws_bytes: fp32 workspace for split-K (may be null: split-K is then disabled).
 // force_split: 0 = automatic, >0 = use exactly that many splits (tests).
 // Returns 0 on success, a negative value if the arguments cannot be served.
-int gfs_gemm_bf16_rope(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb,
-                       int ldc, int ldr, int a_mn_major, int b_mn_major, int add, void* ws, size_t ws_bytes,
-                       int force_split, const void* rope_cos, const void* rope_sin, int rope_cols, int rope_d,
-                       int rope_b, void* stream_);
-
 int gfs_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,
                   int ldr, int a_mn_major, int b_mn_major, int add, void* ws, size_t ws_bytes, int force_split,
                   void* stream_) {

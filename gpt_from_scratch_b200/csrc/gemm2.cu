@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cstdio>
 
+#include "api.h"
 #include "common.cuh"
 
 using namespace gfs;

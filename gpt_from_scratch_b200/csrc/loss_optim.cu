@@ -7,6 +7,7 @@
 // compare, scale, AdamW, cast become two kernels with the clip decided on the device).
 #include <algorithm>
 
+#include "api.h"
 #include "common.cuh"
 
 using namespace gfs;
@@ -29,13 +30,19 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 
 constexpr int CE_THREADS = 256;
 
+// Target id of logits row `row` (rows are [S, B]): from a [S, B] array (tb = 0) or straight from the
+// caller's [B, S] labels (tb = B), which saves the transposing copy.
+__device__ __forceinline__ long long target_of(const long long* __restrict__ target, int row, int M, int tb) {
+  return tb == 0 ? target[row] : target[static_cast<size_t>(row % tb) * (M / tb) + row / tb];
+}
+
 // One CTA per row of the local logits [M, Vp] (pitch ld). Online max / sum-exp in a
 // single pass. stats[row] = {local max, sum exp(z - max), z[target] or 0 if the target
 // id is outside [v0, v0+Vp)}. With single_rank != 0 also writes lse and loss.
 __global__ void __launch_bounds__(CE_THREADS)
 ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
               float* __restrict__ stats, float* __restrict__ lse, float* __restrict__ loss, int Vp, long ld, int v0,
-              int single_rank) {
+              int single_rank, int tb) {
   const int row = blockIdx.x;
   const __nv_bfloat16* z = logits + static_cast<size_t>(row) * ld;
   const int nvec = Vp >> 3;
@@ -68,7 +75,7 @@ ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restr
     for (int i = 1; i < CE_THREADS / 32; ++i) gm = fmaxf(gm, sm_m[i]);
     float gs = 0.f;
     for (int i = 0; i < CE_THREADS / 32; ++i) gs += (sm_m[i] == -INFINITY) ? 0.f : sm_s[i] * __expf(sm_m[i] - gm);
-    const long long t = target[row];
+    const long long t = target_of(target, row, gridDim.x, tb);
     float tz = 0.f;
     if (t >= v0 && t < v0 + Vp) tz = __bfloat162float(z[t - v0]);
     stats[3 * row + 0] = gm;
@@ -97,7 +104,7 @@ __device__ __forceinline__ void ce_merge(float& gm, float& gs, float2 ms) {
 __global__ void __launch_bounds__(32 * CE_PW)
 ce_from_partials_kernel(const float2* __restrict__ partials, const __nv_bfloat16* __restrict__ logits,
                         const long long* __restrict__ target, float* __restrict__ stats, float* __restrict__ lse,
-                        float* __restrict__ loss, int parts, int M, int Vp, long ld, int v0, int single_rank) {
+                        float* __restrict__ loss, int parts, int M, int Vp, long ld, int v0, int single_rank, int tb) {
   __shared__ float2 part_res[CE_PW][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * 32 + lane;
@@ -122,7 +129,7 @@ ce_from_partials_kernel(const float2* __restrict__ partials, const __nv_bfloat16
   gs = 0.f;
 #pragma unroll
   for (int w = 0; w < CE_PW; ++w) ce_merge(gm, gs, part_res[w][lane]);
-  const long long t = target[row];
+  const long long t = target_of(target, row, M, tb);
   float tz = 0.f;
   if (t >= v0 && t < v0 + Vp) tz = __bfloat162float(logits[static_cast<size_t>(row) * ld + (t - v0)]);
   stats[3 * row + 0] = gm;
@@ -153,11 +160,11 @@ __global__ void ce_combine_kernel(const float* __restrict__ stats_all, float* __
   loss[row] = l - tz;
 }
 
-// In place: z <- (exp(z - lse) - [col == target - v0]) * g[row]. Grid: x covers the vectors of
-// a row, y strides over rows.
+// In place: z <- (exp(z - lse) - [col == target - v0]) * g[row] (one g for all rows when grad_rows is
+// null). Grid: x covers the vectors of a row, y strides over rows.
 __global__ void ce_bwd_kernel(__nv_bfloat16* __restrict__ logits, const float* __restrict__ lse,
-                              const long long* __restrict__ target, const float* __restrict__ grad_rows, int M, int Vp,
-                              long ld, int v0) {
+                              const long long* __restrict__ target, const float* __restrict__ grad_rows, float grad_all,
+                              int M, int Vp, long ld, int v0, int tb) {
   const int nvec = Vp >> 3;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nvec) return;
@@ -175,8 +182,8 @@ __global__ void ce_bwd_kernel(__nv_bfloat16* __restrict__ logits, const float* _
       if (row < M) {
         raw[u] = *reinterpret_cast<const uint4*>(logits + static_cast<size_t>(row) * ld + c);
         l[u] = lse[row];
-        g[u] = grad_rows[row];
-        t[u] = target[row] - v0;
+        g[u] = grad_rows != nullptr ? grad_rows[row] : grad_all;
+        t[u] = target_of(target, row, M, tb) - v0;
       }
     }
 #pragma unroll
@@ -319,6 +326,20 @@ __global__ void adamw_kernel(const __nv_bfloat16* __restrict__ grad, float* __re
   }
 }
 
+// Mean of n floats by one CTA, in a fixed order.
+__global__ void __launch_bounds__(1024) mean_f32_kernel(const float* __restrict__ x, float* __restrict__ out, int n) {
+  __shared__ float sm[32];
+  float s = 0.f;
+  for (int i = threadIdx.x; i < n; i += 1024) s += x[i];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = warp_sum(sm[threadIdx.x]);
+    if (threadIdx.x == 0) *out = s / static_cast<float>(n);
+  }
+}
+
 // A wait that nothing satisfies: used to exercise the bounded-wait path on one GPU.
 __global__ void wait_probe_kernel(const unsigned int* flag, unsigned long long limit_ns, uint32_t* status) {
   const uint64_t t0 = globaltimer_ns();
@@ -335,23 +356,27 @@ __global__ void wait_probe_kernel(const unsigned int* flag, unsigned long long l
 
 extern "C" {
 
+// target_batch: 0 = target is [M] in row order; B = target is the [B, M/B] label array of a batch whose
+// logits rows are [M/B, B].
 int gfs_ce_fwd(const void* logits, const void* target, void* stats, void* lse, void* loss, int M, int Vp, long ld,
-               int v0, int single_rank, void* stream) {
-  if ((Vp & 7) || (ld & 7)) return -1;
+               int v0, int single_rank, int target_batch, void* stream) {
+  if ((Vp & 7) || (ld & 7) || target_batch < 0 || (target_batch > 0 && M % target_batch != 0)) return -1;
   if (M == 0) return 0;
   ce_fwd_kernel<<<M, CE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(logits), static_cast<const long long*>(target), static_cast<float*>(stats),
-      static_cast<float*>(lse), static_cast<float*>(loss), Vp, ld, v0, single_rank);
+      static_cast<float*>(lse), static_cast<float*>(loss), Vp, ld, v0, single_rank, target_batch);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 int gfs_ce_from_partials(const void* partials, const void* logits, const void* target, void* stats, void* lse,
-                         void* loss, int parts, int M, int Vp, long ld, int v0, int single_rank, void* stream) {
+                         void* loss, int parts, int M, int Vp, long ld, int v0, int single_rank, int target_batch,
+                         void* stream) {
   if (M == 0) return 0;
+  if (target_batch < 0 || (target_batch > 0 && M % target_batch != 0)) return -1;
   ce_from_partials_kernel<<<(M + 31) / 32, 32 * CE_PW, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const float2*>(partials), static_cast<const __nv_bfloat16*>(logits),
       static_cast<const long long*>(target), static_cast<float*>(stats), static_cast<float*>(lse),
-      static_cast<float*>(loss), parts, M, Vp, ld, v0, single_rank);
+      static_cast<float*>(loss), parts, M, Vp, ld, v0, single_rank, target_batch);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -362,14 +387,21 @@ int gfs_ce_combine(const void* stats_all, void* lse, void* loss, int M, int worl
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
-int gfs_ce_bwd(void* logits, const void* lse, const void* target, const void* grad_rows, int M, int Vp, long ld,
-               int v0, void* stream) {
-  if ((Vp & 7) || (ld & 7)) return -1;
+int gfs_ce_bwd(void* logits, const void* lse, const void* target, const void* grad_rows, float grad_all, int M, int Vp,
+               long ld, int v0, int target_batch, void* stream) {
+  if ((Vp & 7) || (ld & 7) || target_batch < 0 || (target_batch > 0 && M % target_batch != 0)) return -1;
   if (M == 0 || Vp == 0) return 0;
   const dim3 grid(((Vp >> 3) + 255) / 256, std::min((M + 3) / 4, 1024));
   ce_bwd_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<__nv_bfloat16*>(logits), static_cast<const float*>(lse), static_cast<const long long*>(target),
-      static_cast<const float*>(grad_rows), M, Vp, ld, v0);
+      static_cast<const float*>(grad_rows), grad_all, M, Vp, ld, v0, target_batch);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+int gfs_mean_f32(const void* x, void* out, int n, void* stream) {
+  if (n <= 0) return -1;
+  mean_f32_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const float*>(x),
+                                                                     static_cast<float*>(out), n);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -1,4 +1,5 @@
-// Whole passes over a stack of transformer blocks (forward, backward) as ONE host call each.
+// Whole passes of the model as ONE host call each: the stack of transformer blocks forward and
+// backward, and a training step's forward, loss and backward.
 //
 // A block is eight forward and about thirteen backward kernels of 2-300 us. Launched one by one from
 // Python through autograd, a block costs the host about 0.3 ms forward and 0.5 ms backward, more
@@ -345,6 +346,150 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
     dout = dnext;
   }
   return flush_norms();
+}
+
+// ---------------------------------------------------------------------------
+// Forward, mean loss and backward of one micro-batch.
+// ---------------------------------------------------------------------------
+struct GfsModelTop {
+  const void *w_emb, *w_final, *w_out;   // [V, H], [H], [V, H]
+  void *g_emb, *g_final, *g_out;
+  int acc_emb, acc_final, acc_out;       // add to the gradient instead of overwriting it
+  int V;
+};
+
+}  // extern "C"
+
+namespace {
+
+// Buffers of a step besides the blocks' activations. The logits are dead when the blocks' backward
+// begins, so its scratch lies in the same place.
+struct StepLayout {
+  size_t acts, x0, y_final, rstd_final, keys, loss_rows, stats, lse, dy, dx0, logits, partials, scratch, total;
+  StepLayout(const GfsBlockDims& d, const GfsModelTop& t, const ActLayout& a) {
+    const size_t T = static_cast<size_t>(d.S) * d.B, H = d.H, V = t.V;
+    size_t o = 0;
+    auto take = [&](size_t bytes) {
+      const size_t at = o;
+      o += align256(bytes);
+      return at;
+    };
+    acts = take(a.total * d.n_layers);
+    x0 = take(2 * T * H);
+    y_final = take(2 * T * H);
+    rstd_final = take(4 * T);
+    keys = take(4 * T);
+    loss_rows = take(4 * T);
+    stats = take(12 * T);
+    lse = take(4 * T);
+    dy = take(2 * T * H);
+    dx0 = take(2 * T * H);
+    scratch = o;   // also the dropout's temporary in the forward
+    logits = take(2 * T * V);
+    partials = take(8 * T * static_cast<size_t>(gfs_gemm2_ce_parts(t.V)));
+    total = std::max(o, scratch + std::max(BwdLayout(d).total, align256(2 * T * H)));
+  }
+};
+
+// The id sort of the embedding backward needs only the ids: it runs beside the forward on a stream of
+// its own (one per thread and device, so that neither threads nor captures meet in its events).
+struct SideStream {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+SideStream* side_stream() {
+  static thread_local SideStream per_dev[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  SideStream& s = per_dev[dev];
+  if (s.join == nullptr) {
+    if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) != cudaSuccess)
+      return nullptr;
+  }
+  return &s;
+}
+
+}  // namespace
+
+extern "C" {
+
+size_t gfs_model_step_bytes(const GfsBlockDims* d, const GfsModelTop* t) {
+  return StepLayout(*d, *t, ActLayout(*d)).total;
+}
+
+// One micro-batch: ids, labels int64 [B, S] -> *loss (fp32, mean over all tokens) and all weight
+// gradients. arena: gfs_model_step_bytes bytes. Returns -20 (nothing launched) when the batch does not
+// fit the single-CTA id sort of the embedding backward.
+int gfs_model_step(const GfsBlockDims* dp, const GfsBlockParams* layers, const GfsModelTop* tp, const void* ids,
+                   const void* labels, void* arena, void* loss, int* launches, void* stream) {
+  const GfsBlockDims& d = *dp;
+  const GfsModelTop& t = *tp;
+  if (!dims_ok(d) || (t.V & 7)) return -1;
+  const ActLayout a(d);
+  const StepLayout lay(d, t, a);
+  const int T = d.S * d.B, H = d.H, V = t.V;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  char* m = static_cast<char*>(arena);
+  void *x0 = m + lay.x0, *y = m + lay.y_final, *rstd = m + lay.rstd_final, *keys = m + lay.keys,
+       *rows = m + lay.loss_rows, *stats = m + lay.stats, *lse = m + lay.lse, *dy = m + lay.dy, *dx0 = m + lay.dx0,
+       *logits = m + lay.logits, *partials = m + lay.partials, *scratch = m + lay.scratch;
+
+  SideStream* side = side_stream();
+  if (side == nullptr) return -10;
+  if (T > 32768) return -20;
+  if (cudaEventRecord(side->fork, st) != cudaSuccess || cudaStreamWaitEvent(side->stream, side->fork, 0) != cudaSuccess)
+    return -11;
+  const int shift = gfs_embedding_sort_keys(ids, keys, d.B, d.S, 0, V, side->stream);
+  if (cudaEventRecord(side->join, side->stream) != cudaSuccess) return -11;
+  if (shift <= 0) {
+    cudaStreamWaitEvent(st, side->join, 0);   // a capture must not end with the fork open
+    return shift == 0 ? -1 : shift;
+  }
+  ++*launches;
+
+  GFS_TRY(gfs_embedding_fwd(ids, t.w_emb, x0, d.B, d.S, H, 0, V, 0, d.S, stream));
+  constexpr int MAX_LAYERS = 512;
+  if (d.n_layers > MAX_LAYERS) return -1;
+  u64 act[MAX_LAYERS];
+  for (int l = 0; l < d.n_layers; ++l) act[l] = reinterpret_cast<u64>(m + lay.acts + a.total * l);
+  int rc = gfs_blocks_forward(dp, layers, t.w_final, x0, act, scratch, y, rstd, launches, stream);
+  if (rc != 0) return rc;
+
+  // LM head and loss
+  const float g_row = 1.0f / static_cast<float>(T);
+  rc = -20;
+  if (H >= 256 && use_pair(d, tiles256(T, V))) {
+    rc = gfs_gemm2_bf16_ce(y, t.w_out, logits, partials, T, V, H, H, H, V, stream);
+    if (rc == 0) {
+      *launches += 2;
+      rc = gfs_ce_from_partials(partials, logits, labels, stats, lse, rows, gfs_gemm2_ce_parts(V), T, V, V, 0, 1, d.B,
+                                stream);
+    }
+  }
+  if (rc == -20) {
+    GFS_TRY(product(d, y, t.w_out, logits, nullptr, T, V, H, H, H, V, 0, 0, 0, stream));
+    GFS_TRY(gfs_ce_fwd(logits, labels, stats, lse, rows, T, V, V, 0, 1, d.B, stream));
+  } else if (rc != 0) {
+    return rc;
+  }
+  GFS_TRY(gfs_mean_f32(rows, loss, T, stream));
+
+  // backward: the logits become their gradient in place
+  GFS_TRY(gfs_ce_bwd(logits, lse, labels, nullptr, g_row, T, V, V, 0, d.B, stream));
+  GFS_TRY(product(d, logits, t.w_out, dy, nullptr, T, H, V, V, H, H, 0, 1, 0, stream));
+  WgradGroup grp;
+  rc = weight_grad(d, grp, logits, y, t.g_out, t.acc_out, T, V, H, launches, stream);
+  if (rc == 0) rc = grp.flush(launches, stream);
+  if (rc != 0) return rc;
+  rc = gfs_blocks_backward(dp, layers, t.w_final, t.g_final, t.acc_final, x0, act, rstd, dy, scratch, dx0, launches,
+                           stream);
+  if (rc != 0) return rc;
+  if (!t.acc_emb && cudaMemsetAsync(t.g_emb, 0, 2 * static_cast<size_t>(V) * H, st) != cudaSuccess) return -11;
+  if (cudaStreamWaitEvent(st, side->join, 0) != cudaSuccess) return -11;
+  GFS_TRY(gfs_embedding_bwd_keys(keys, dx0, t.g_emb, T, H, shift, stream));
+  return 0;
 }
 
 }  // extern "C"

@@ -19,6 +19,7 @@ import os
 import torch
 
 from .config import GPTConfig
+from .models import native
 from .models.gpt import GPTModel
 from .optimizer import DistributedOptimizer
 from .parallel import parallel_state as ps
@@ -91,8 +92,12 @@ class TrainEngine:
 
     def _eager_step(self, inputs: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
         self.optimizer.zero_grad()
-        loss = self.forward_loss(inputs, labels)
-        loss.backward()
+        loss = None
+        if type(self).forward_loss is TrainEngine.forward_loss:
+            loss = native.train_pass(self.model, inputs, labels)    # forward, loss and backward in one call
+        if loss is None:
+            loss = self.forward_loss(inputs, labels)
+            loss.backward()
         self.optimizer.step()
         return loss.detach()
 

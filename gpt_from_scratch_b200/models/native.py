@@ -45,6 +45,11 @@ class _BlockParams(ctypes.Structure):
                 ("seed", c_ulonglong * 2)]
 
 
+class _Top(ctypes.Structure):
+    """GfsModelTop in csrc/model.cu."""
+    _fields_ = [("w", c_void_p * 3), ("g", c_void_p * 3), ("accumulate", c_int * 3), ("V", c_int)]
+
+
 def _hook_dicts(module: torch.nn.Module):
     return (module._forward_hooks, module._forward_pre_hooks, module._backward_hooks, module._backward_pre_hooks)
 
@@ -72,6 +77,8 @@ class _Plan:
         self.weights: list = []         # per block: its six parameters
         self.hooks: list = []
         self.ptrs: list = []
+        self.step_shape = None          # (S, B, dropout) step_bytes was computed for
+        self.top_args = _Top()
 
     def _bind(self, model) -> bool:
         """Structural checks and everything that depends on the modules only."""
@@ -122,11 +129,14 @@ class _Plan:
                 bp.w[k] = w.data_ptr()
             bp.eps[0], bp.eps[1] = layer.input_norm.eps, layer.post_attention_norm.eps
         self.top = (emb.weight, fin.weight, head.weight)
+        for k, w in enumerate(self.top):
+            self.top_args.w[k] = w.data_ptr()
+        self.top_args.V = head.weight.shape[0]
         self.all_params = [w for ws in self.weights for w in ws] + list(self.top)
         d = self.dims
         d.H, d.nh, d.D = H, layers[0].attention.num_attention_heads, layers[0].attention.head_dim
         d.I, d.n_layers, d.eps_final = layers[0].mlp.intermediate_size, len(layers), fin.eps
-        self.shape = None
+        self.shape = self.step_shape = None
         self.ptrs = self._live_ptrs(model)
         return True
 
@@ -188,6 +198,14 @@ class _Plan:
         self.put_seeds(seeds)
         return seeds
 
+    def put_gradients(self) -> None:
+        """Where the blocks' weight gradients go, and whether they are added to what is there."""
+        for bp, ws in zip(self.params, self.weights):
+            g, acc = bp.g, bp.accumulate
+            for k, w in enumerate(ws):
+                g[k] = w.grad.data_ptr()
+                acc[k] = _consume(w)
+
     def put_seeds(self, seeds: list) -> None:
         for bp, s0, s1 in zip(self.params, seeds[0::2], seeds[1::2]):
             bp.seed[0], bp.seed[1] = s0, s1
@@ -242,10 +260,7 @@ def _stack_forward(plan: _Plan, x: torch.Tensor, keep: bool):
 
 def _stack_backward(plan: _Plan, x, rstd, acts, seeds, dy: torch.Tensor) -> torch.Tensor:
     n = len(plan.layers)
-    for bp, ws in zip(plan.params, plan.weights):
-        for k, w in enumerate(ws):
-            bp.g[k] = w.grad.data_ptr()
-            bp.accumulate[k] = _consume(w)
+    plan.put_gradients()
     if seeds is not None:
         plan.put_seeds(seeds)
     w_fin = plan.top[1]
@@ -325,3 +340,49 @@ def forward(plan: _Plan, inputs: torch.Tensor, ce_stats: bool):
         return gemm_ops.linear_fwd(y, w_out).view(S, B, -1)
     logits, partials = gemm_ops.linear_fwd_ce(y, w_out)
     return logits.view(S, B, -1), partials
+
+
+def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
+    """Forward, mean loss and backward of one micro-batch (``[B, S]`` ids and labels) without autograd:
+    returns the loss (0-dim fp32) with every weight gradient in its sink, or ``None`` if the model has to
+    go through its modules. One call into the library; all intermediates lie in one buffer."""
+    if (not torch.is_grad_enabled() or labels.shape != inputs.shape or not labels.is_cuda or
+            model._forward_hooks or model._forward_pre_hooks or model._backward_hooks or model._backward_pre_hooks):
+        return None
+    plan = plan_for(model, inputs)
+    if plan is None:
+        return None
+    B, S = inputs.shape
+    if B * S > 32768:       # the embedding backward then sorts its ids with the library's sort
+        return None
+    ids, labels = inputs.contiguous(), labels.contiguous()
+    if ids.dtype != torch.int64:
+        ids = ids.long()
+    if labels.dtype != torch.int64:
+        labels = labels.long()
+    dev = plan.top[0].device
+    plan.set_shape(S, B, dev)
+    if plan.dropout > 0.0:
+        plan.draw_seeds()
+    lib, dims, top = _lib.lib(), byref(plan.dims), plan.top_args
+    if plan.step_shape != plan.shape:
+        plan.step_bytes = lib.gfs_model_step_bytes(dims, byref(top))
+        plan.step_shape = plan.shape
+    fresh = [getattr(p, "_grad_fresh", False) for p in plan.all_params]
+    plan.put_gradients()
+    for k, w in enumerate(plan.top):
+        top.g[k] = w.grad.data_ptr()
+        top.accumulate[k] = _consume(w)
+    arena = torch.empty(plan.step_bytes, dtype=torch.uint8, device=dev)
+    loss = torch.empty((), dtype=torch.float32, device=dev)
+    launches = c_int(0)
+    with _lib.nvtx("fused:model_step"):
+        rc = lib.gfs_model_step(dims, plan.params, byref(top), ids.data_ptr(), labels.data_ptr(), arena.data_ptr(),
+                                loss.data_ptr(), byref(launches), _lib.stream_ptr())
+    if rc == -20:           # ids times tokens do not fit the sort's 32-bit keys: nothing was launched
+        for p, f in zip(plan.all_params, fresh):
+            p._grad_fresh = f
+        return None
+    _lib.check(rc, "gfs_model_step")
+    _lib.add_launches(launches.value - 1)
+    return loss

@@ -353,10 +353,11 @@ def test_cuda_graph_step_matches_eager(cuda_device):
     (768, 12, 2048, 2, 1024, 8, 512, 0.0),    # CTA pairs and grouped weight gradients
     (256, 4, 512, 2, 512, 3, 50, 0.1),
 ])
-def test_native_model_pass_matches_module_path(cuda_device, H, heads, I, layers, V, B, S, dropout):
-    """The whole-model native pass against the module-by-module path it replaces (a forward hook keeps a
-    model on the latter): the same kernels in the same order, so the same bits; with dropout the module
-    path rounds the two gradients of a residual branch one by one."""
+def test_native_model_pass_matches_module_path(cuda_device, monkeypatch, H, heads, I, layers, V, B, S, dropout):
+    """The whole-model native passes (the step in one call; forward and backward under autograd) against the
+    module-by-module path they replace (a forward hook keeps a model on the latter): the same kernels in the
+    same order, so the same bits; with dropout the module path rounds the two gradients of a residual branch
+    one by one. The step's own mean of the token losses sums in another order."""
     from gpt_from_scratch_b200.config import GPTConfig
     from gpt_from_scratch_b200.engine import TrainEngine
     from gpt_from_scratch_b200.models import native
@@ -369,9 +370,12 @@ def test_native_model_pass_matches_module_path(cuda_device, H, heads, I, layers,
     g = torch.Generator().manual_seed(3)
     batches = [torch.randint(0, V, (B, S + 1), generator=g) for _ in range(3)]
     runs = []
-    for modules in (False, True):
+    for path in ("step", "autograd", "modules"):
+        modules = path == "modules"
         torch.manual_seed(11)
         eng = TrainEngine(cfg, lr=1e-3, seed=5)
+        if path == "autograd":
+            monkeypatch.setattr(native, "train_pass", lambda *a: None)
         if modules:
             eng.model.layers[-1].mlp.register_forward_hook(lambda *a: None)
         assert (native.plan_for(eng.model, batches[0].cuda()) is None) == modules
@@ -382,12 +386,14 @@ def test_native_model_pass_matches_module_path(cuda_device, H, heads, I, layers,
         with torch.no_grad():
             logits = eng.model(x)
         runs.append((losses, logits, eng.optimizer.grad_buffer.clone(), eng.optimizer.fp32_master_shard.clone()))
-    if dropout == 0.0:
-        assert runs[0][0] == runs[1][0]
-        for a, b in zip(runs[0][1:], runs[1][1:]):
-            assert torch.equal(a, b)
-        return
-    # one bf16 rounding (2^-9) per residual gradient, amplified over three steps at lr 1e-3
-    assert all(abs(a - b) < 1e-2 for a, b in zip(runs[0][0], runs[1][0])), (runs[0][0], runs[1][0])
-    rel = (runs[0][3] - runs[1][3]).norm() / runs[1][3].norm()
-    assert rel < 1e-2, rel
+    for run in runs[:2]:
+        if dropout == 0.0:
+            # fp32 sums of up to 4096 losses of equal size in another order
+            assert all(abs(a - b) < 1e-5 * abs(b) for a, b in zip(run[0], runs[2][0])), (run[0], runs[2][0])
+            for a, b in zip(run[1:], runs[2][1:]):
+                assert torch.equal(a, b)
+        else:
+            # one bf16 rounding (2^-9) per residual gradient, amplified over three steps at lr 1e-3
+            assert all(abs(a - b) < 1e-2 for a, b in zip(run[0], runs[2][0])), (run[0], runs[2][0])
+            rel = (run[3] - runs[2][3]).norm() / runs[2][3].norm()
+            assert rel < 1e-2, rel
