@@ -18,7 +18,20 @@ int gfs_gemm2_bf16_swiglu(int mode, const void* a, const void* b, void* c, void*
 int gfs_gemm2_wgrad_grouped(int n, const unsigned long long* A, const unsigned long long* B,
                             const unsigned long long* C, const int* M, const int* N, const int* K, const int* lda,
                             const int* ldb, const int* ldc, const int* accumulate, void* stream);
-int gfs_gemm_bf16_launches(int M, int N, int K, size_t ws_bytes);
+int gfs_gemm_tile(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,
+                  int ldr, int a_mn_major, int b_mn_major, const void* rope_cos, const void* rope_sin, int rope_cols,
+                  int rope_d, int rope_b, int swi_mode, void* swi_extra, int swi_ld, int bn, int split, void* stream);
+int gfs_gemm_tile_wgrad_grouped(int n, const unsigned long long* A, const unsigned long long* B,
+                                const unsigned long long* C, const int* M, const int* N, const int* K, const int* lda,
+                                const int* ldb, const int* ldc, const int* accumulate, int bn, int split, void* stream);
+int gfs_linear(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,
+               int ldr, int a_mn_major, int b_mn_major, const void* rope_cos, const void* rope_sin, int rope_cols,
+               int rope_d, int rope_b, int pair_min_tiles, void* stream);
+int gfs_linear_swiglu(int mode, const void* a, const void* b, void* c, void* extra, int M, int I, int K, int lda,
+                      int ldb, int ldc, int ld_extra, int pair_min_tiles, void* stream);
+int gfs_wgrad_grouped(int n, const unsigned long long* A, const unsigned long long* B, const unsigned long long* C,
+                      const int* M, const int* N, const int* K, const int* lda, const int* ldb, const int* ldc,
+                      const int* accumulate, void* stream);
 int gfs_rmsnorm_fwd(const void* x, const void* w, void* y, void* rstd, int rows, int H, float eps, void* stream);
 int gfs_rmsnorm_bwd_parts(int rows);
 int gfs_rmsnorm_bwd(const void* dy, const void* x, const void* w, const void* rstd, const void* dres, void* dx,
@@ -44,8 +57,8 @@ int gfs_ce_bwd(void* logits, const void* lse, const void* target, const void* gr
                long ld, int v0, int target_batch, void* stream);
 int gfs_mean_f32(const void* x, void* out, int n, void* stream);
 int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int S, int B, int nh, int D,
-                  const long long* strides, float scale, int causal, void* stream);
+                  const long long* strides, float scale, int causal, int o_f16, void* stream);
 int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dO, const void* lse,
                   void* dvec, void* dq, void* dk, void* dv, int S, int B, int nh, int D, const long long* strides,
-                  float scale, int causal, const void* rope_cos, const void* rope_sin, void* stream);
+                  float scale, int causal, const void* rope_cos, const void* rope_sin, void* do_bf16, void* stream);
 }

@@ -24,6 +24,8 @@
 //
 // Reference counterparts: core/myFlashAttn.py:460-728 (_attn_fwd), :740-790 (pre-pass),
 // :805-1066 (_attn_bwd_LoopQ), :1079-1317 (_attn_bwd_LoopKV).
+#include <cuda_fp16.h>
+
 #include <cstdlib>
 #include <algorithm>
 #include <type_traits>
@@ -154,13 +156,25 @@ __device__ __forceinline__ void store_rows_32x64(uint8_t* stage, const uint32_t 
   __syncwarp();
 }
 
+// Two fp32 values as a 16-bit pair of the output's type. The kernels compute in bf16; tensors of an fp16
+// caller are rounded to bf16 on the way in (cast_qkv_kernel, attn_dvec_kernel) and results leave as fp16
+// straight from fp32, so an fp16 call costs one launch more than a bf16 one and no pass over its results.
+__device__ __forceinline__ uint32_t pack_out(float lo, float hi, int f16) {
+  if (f16) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return pack_bf16x2(lo, hi);
+}
+
 // ---------------------------------------------------------------------------
 // Forward
 // ---------------------------------------------------------------------------
 struct FwdParams {
-  __nv_bfloat16* O;
+  __nv_bfloat16* O;            // 16-bit elements; fp16 when o_f16 is set
   long long o_ss, o_bs, o_hs;  // element strides: sequence, batch, head
-  float* lse;                  // [B, nh, S_pad]
+  float* lse;                  // [B, nh, S_pad], log2 of the row's sum of exponentials (base e scores)
+  int o_f16;
   int S, S_pad, B, nh;
   float scale;
   int causal;
@@ -438,13 +452,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       for (int hf = 0; hf < D / 64; ++hf) {
         uint32_t ow[32];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) ow[e] = pack_bf16x2(o[hf * 64 + 2 * e] * inv_l, o[hf * 64 + 2 * e + 1] * inv_l);
+        for (int e = 0; e < 32; ++e) ow[e] = pack_out(o[hf * 64 + 2 * e] * inv_l, o[hf * 64 + 2 * e + 1] * inv_l, p.o_f16);
         store_rows_32x64(stage, ow, lane, g0 + hf * 64, p.o_ss, p.S - row0);
       }
     }
     if (row_g < p.S_pad) {
       const float mm = (m == -INFINITY) ? 0.f : m;
-      p.lse[static_cast<size_t>(bh) * p.S_pad + row_g] = mm * p.scale + logf(fmaxf(l, 1e-37f));
+      p.lse[static_cast<size_t>(bh) * p.S_pad + row_g] = mm * sl2 + log2f(fmaxf(l, 1e-37f));
     }
   }
 
@@ -843,21 +857,21 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 #pragma unroll
             for (int cc = 0; cc < 32; cc += 8) {
               uint4 wv;
-              wv.x = pack_bf16x2(__uint_as_float(wa[cc + 0]) * inv_l, __uint_as_float(wa[cc + 1]) * inv_l);
-              wv.y = pack_bf16x2(__uint_as_float(wa[cc + 2]) * inv_l, __uint_as_float(wa[cc + 3]) * inv_l);
-              wv.z = pack_bf16x2(__uint_as_float(wa[cc + 4]) * inv_l, __uint_as_float(wa[cc + 5]) * inv_l);
-              wv.w = pack_bf16x2(__uint_as_float(wa[cc + 6]) * inv_l, __uint_as_float(wa[cc + 7]) * inv_l);
+              wv.x = pack_out(__uint_as_float(wa[cc + 0]) * inv_l, __uint_as_float(wa[cc + 1]) * inv_l, p.o_f16);
+              wv.y = pack_out(__uint_as_float(wa[cc + 2]) * inv_l, __uint_as_float(wa[cc + 3]) * inv_l, p.o_f16);
+              wv.z = pack_out(__uint_as_float(wa[cc + 4]) * inv_l, __uint_as_float(wa[cc + 5]) * inv_l, p.o_f16);
+              wv.w = pack_out(__uint_as_float(wa[cc + 6]) * inv_l, __uint_as_float(wa[cc + 7]) * inv_l, p.o_f16);
               *reinterpret_cast<uint4*>(dst + cc) = wv;
-              wv.x = pack_bf16x2(__uint_as_float(wb[cc + 0]) * inv_l, __uint_as_float(wb[cc + 1]) * inv_l);
-              wv.y = pack_bf16x2(__uint_as_float(wb[cc + 2]) * inv_l, __uint_as_float(wb[cc + 3]) * inv_l);
-              wv.z = pack_bf16x2(__uint_as_float(wb[cc + 4]) * inv_l, __uint_as_float(wb[cc + 5]) * inv_l);
-              wv.w = pack_bf16x2(__uint_as_float(wb[cc + 6]) * inv_l, __uint_as_float(wb[cc + 7]) * inv_l);
+              wv.x = pack_out(__uint_as_float(wb[cc + 0]) * inv_l, __uint_as_float(wb[cc + 1]) * inv_l, p.o_f16);
+              wv.y = pack_out(__uint_as_float(wb[cc + 2]) * inv_l, __uint_as_float(wb[cc + 3]) * inv_l, p.o_f16);
+              wv.z = pack_out(__uint_as_float(wb[cc + 4]) * inv_l, __uint_as_float(wb[cc + 5]) * inv_l, p.o_f16);
+              wv.w = pack_out(__uint_as_float(wb[cc + 6]) * inv_l, __uint_as_float(wb[cc + 7]) * inv_l, p.o_f16);
               *reinterpret_cast<uint4*>(dst + 32 + cc) = wv;
             }
           }
           if (row_g < p.S_pad) {
             const float mm = (m == -INFINITY) ? 0.f : m;
-            p.lse[static_cast<size_t>(bh) * p.S_pad + row_g] = mm * p.scale + logf(fmaxf(l, 1e-37f));
+            p.lse[static_cast<size_t>(bh) * p.S_pad + row_g] = mm * sl2 + log2f(fmaxf(l, 1e-37f));
           }
         }
         cdone += n_mine;
@@ -872,46 +886,119 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------
-// Backward pre-pass: dvec[b,h,s] = sum_d dO[s,b,h,d] * O[s,b,h,d]; one warp per row. Also writes
-// lse2 = lse * log2(e), the form the backward's exp2 wants (saves a multiply per score there).
+// fp16 callers: q, k, v ([B, nh, S, D] views with any strides) rounded to bf16, contiguous, one launch.
 // ---------------------------------------------------------------------------
-__global__ void attn_dvec_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
-                                 float* __restrict__ dvec, const float* __restrict__ lse, float* __restrict__ lse2,
-                                 int S, int S_pad, int B, int nh, int D, long long do_ss,
-                                 long long do_bs, long long do_hs, long long o_ss, long long o_bs, long long o_hs) {
+struct CastArgs {
+  const __half* src[3];
+  long long ss[3], bs[3], hs[3];   // element strides: sequence, batch, head
+};
+__global__ void cast_qkv_kernel(const CastArgs a, __nv_bfloat16* __restrict__ dst, int S, int B, int nh, int D) {
+  const int vpr = D >> 3;
+  const long long n = static_cast<long long>(B) * nh * S * vpr;
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int c = static_cast<int>(i % vpr) * 8;
+    const long long row = i / vpr;
+    const int s = static_cast<int>(row % S);
+    const long long bh = row / S;
+    const int h = static_cast<int>(bh % nh), b = static_cast<int>(bh / nh);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      const uint4 x = *reinterpret_cast<const uint4*>(a.src[t] + s * a.ss[t] + b * a.bs[t] + h * a.hs[t] + c);
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+        o[e] = pack_bf16x2(f.x, f.y);
+      }
+      *reinterpret_cast<uint4*>(dst + (t * n + i) * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Backward pre-pass: dvec[b,h,s] = sum_d dO[s,b,h,d] * O[s,b,h,d]. F16: dO and O are fp16, and dO is also
+// written rounded to bf16 ([B, nh, S, D] contiguous), the form the gradient products read (and the
+// one the sum uses, so that it matches them).
+//
+// Bound by memory latency, not bandwidth: 50 MB at the GPT-124M shape (batch 16) took 25 us with one row
+// chunk (two 16-byte loads) per thread; four rows per thread with all loads issued first, and
+// no second pass over the LSE (the forward now writes it in the form the backward wants).
+// ---------------------------------------------------------------------------
+constexpr int DVEC_ROWS = 4;
+template <bool F16>
+__global__ void __launch_bounds__(256)
+attn_dvec_kernel(const void* __restrict__ dO_, const void* __restrict__ O_, float* __restrict__ dvec,
+                 __nv_bfloat16* __restrict__ dO_bf16, int S, int S_pad, int B, int nh, int D, long long do_ss,
+                 long long do_bs, long long do_hs, long long o_ss, long long o_bs, long long o_hs, int s_fastest) {
   pdl_wait();
   pdl_trigger();
-  // D/8 threads per (s, b, h) row, 16-byte loads; rows ordered h fastest (memory order of [S,B,nh,D]).
+  const uint16_t* dO = static_cast<const uint16_t*>(dO_);
+  const uint16_t* O = static_cast<const uint16_t*>(O_);
+  // D/8 threads per (s, b, h) row, 16-byte loads; rows in memory order ([S,B,nh,D]: h fastest, [B,nh,S,D]: s fastest)
   const int tpr = D >> 3;                       // 8 or 16 threads per row
-  const int rows_per_block = blockDim.x / tpr;
-  const long long row = blockIdx.x * static_cast<long long>(rows_per_block) + threadIdx.x / tpr;
+  const int rows_per_pass = blockDim.x / tpr;
   const int sub = threadIdx.x % tpr;
-  const long long total = static_cast<long long>(S) * B * nh;
-  float acc = 0.f;
-  int h = 0, b = 0, s = 0;
-  if (row < total) {
-    h = static_cast<int>(row % nh);
-    b = static_cast<int>((row / nh) % B);
-    s = static_cast<int>(row / (static_cast<long long>(nh) * B));
-    const uint4 x = *reinterpret_cast<const uint4*>(dO + s * do_ss + b * do_bs + h * do_hs + sub * 8);
-    const uint4 y = *reinterpret_cast<const uint4*>(O + s * o_ss + b * o_bs + h * o_hs + sub * 8);
-    const float2 x0 = unpack_bf16x2(x.x), x1 = unpack_bf16x2(x.y), x2 = unpack_bf16x2(x.z), x3 = unpack_bf16x2(x.w);
-    const float2 y0 = unpack_bf16x2(y.x), y1 = unpack_bf16x2(y.y), y2 = unpack_bf16x2(y.z), y3 = unpack_bf16x2(y.w);
-    acc = x0.x * y0.x + x0.y * y0.y + x1.x * y1.x + x1.y * y1.y + x2.x * y2.x + x2.y * y2.y + x3.x * y3.x +
-          x3.y * y3.y;
+  const unsigned total = static_cast<unsigned>(S) * B * nh;
+  const unsigned row0 = blockIdx.x * static_cast<unsigned>(rows_per_pass * DVEC_ROWS) + threadIdx.x / tpr;
+  uint4 x[DVEC_ROWS], y[DVEC_ROWS];
+  unsigned at[DVEC_ROWS];                       // b * nh + h, s
+  int sq[DVEC_ROWS];
+#pragma unroll
+  for (int i = 0; i < DVEC_ROWS; ++i) {
+    const unsigned row = row0 + i * rows_per_pass;
+    x[i] = make_uint4(0, 0, 0, 0);
+    y[i] = x[i];
+    unsigned h, b, s;
+    if (s_fastest) {
+      s = row % S;
+      const unsigned bh = row / S;
+      h = bh % nh;
+      b = bh / nh;
+    } else {
+      h = row % nh;
+      const unsigned sb = row / nh;
+      b = sb % B;
+      s = sb / B;
+    }
+    at[i] = b * nh + h;
+    sq[i] = static_cast<int>(s);
+    if (row < total) {
+      x[i] = *reinterpret_cast<const uint4*>(dO + s * do_ss + b * do_bs + h * do_hs + sub * 8);
+      y[i] = *reinterpret_cast<const uint4*>(O + s * o_ss + b * o_bs + h * o_hs + sub * 8);
+    }
   }
-  for (int o = tpr >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (row < total && sub == 0) dvec[(static_cast<size_t>(b) * nh + h) * S_pad + s] = acc;
+#pragma unroll
+  for (int i = 0; i < DVEC_ROWS; ++i) {
+    const unsigned row = row0 + i * rows_per_pass;
+    uint32_t xw[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+    const uint32_t yw[4] = {y[i].x, y[i].y, y[i].z, y[i].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float2 b2;
+      if (F16) {
+        const float2 a2 = __half22float2(*reinterpret_cast<const __half2*>(&xw[e]));
+        xw[e] = pack_bf16x2(a2.x, a2.y);
+        b2 = __half22float2(*reinterpret_cast<const __half2*>(&yw[e]));
+      } else {
+        b2 = unpack_bf16x2(yw[e]);
+      }
+      const float2 a2 = unpack_bf16x2(xw[e]);
+      acc += a2.x * b2.x + a2.y * b2.y;
+    }
+    if (F16 && row < total)
+      *reinterpret_cast<uint4*>(dO_bf16 + (static_cast<size_t>(at[i]) * S + sq[i]) * D + sub * 8) =
+          make_uint4(xw[0], xw[1], xw[2], xw[3]);
+    for (int o = tpr >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (row < total && sub == 0) dvec[static_cast<size_t>(at[i]) * S_pad + sq[i]] = acc;
+  }
   // rows S .. S_pad-1 of every head: zeros (the backward multiplies them by probabilities that are 0)
-  const int pad = S_pad - S;
-  const long long pad_total = static_cast<long long>(pad) * B * nh;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < pad_total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x)
-    dvec[(i / pad) * S_pad + S + (i % pad)] = 0.f;
-  const long long n_lse = static_cast<long long>(S_pad) * B * nh;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n_lse;
-       i += static_cast<long long>(gridDim.x) * blockDim.x)
-    lse2[i] = lse[i] * LOG2E_F;
+  const unsigned pad = S_pad - S;
+  const unsigned pad_total = pad * B * nh;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < pad_total; i += gridDim.x * blockDim.x)
+    dvec[static_cast<size_t>(i / pad) * S_pad + S + (i % pad)] = 0.f;
 }
 
 // ---------------------------------------------------------------------------
@@ -922,7 +1009,7 @@ struct BwdParams {
   __nv_bfloat16* out2;  // mode 0: dV
   long long o1_ss, o1_bs, o1_hs;
   long long o2_ss, o2_bs, o2_hs;
-  const float* lse;   // [B, nh, S_pad], already multiplied by log2(e)
+  const float* lse;   // [B, nh, S_pad], base 2
   const float* dvec;  // [B, nh, S_pad]
   int S, S_pad, B, nh;
   float scale;
@@ -931,6 +1018,7 @@ struct BwdParams {
   // optional: inverse rotary embedding applied to dQ and dK rows before they are stored
   const float* rope_cos;
   const float* rope_sin;
+  int out_f16;        // dQ, dK, dV are stored as fp16
 };
 
 // CW = number of compute warps (4 or 8). With 8, every accumulator row is shared by two
@@ -1382,17 +1470,17 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
           f[4] = a4 * cs.z + a5 * sn.z; f[5] = a5 * cs.z - a4 * sn.z;
           f[6] = a6 * cs.w + a7 * sn.w; f[7] = a7 * cs.w - a6 * sn.w;
         }
-        w[4 * q4 + 0] = pack_bf16x2(f[0], f[1]);
-        w[4 * q4 + 1] = pack_bf16x2(f[2], f[3]);
-        w[4 * q4 + 2] = pack_bf16x2(f[4], f[5]);
-        w[4 * q4 + 3] = pack_bf16x2(f[6], f[7]);
+        w[4 * q4 + 0] = pack_out(f[0], f[1], p.out_f16);
+        w[4 * q4 + 1] = pack_out(f[2], f[3], p.out_f16);
+        w[4 * q4 + 2] = pack_out(f[4], f[5], p.out_f16);
+        w[4 * q4 + 3] = pack_out(f[6], f[7], p.out_f16);
       }
       store_rows_32x32(stage, w, lane, g1 + c, p.o1_ss, p.S - row0);
       if (MODE == 0) {
         tmem_ld_32x32(tmem_base + lane_base + ACC1 + c, v);
         tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 16; ++e) w[e] = pack_bf16x2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
+        for (int e = 0; e < 16; ++e) w[e] = pack_out(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]), p.out_f16);
         store_rows_32x32(stage, w, lane, g2 + c, p.o2_ss, p.S - row0);
       }
     }
@@ -1434,10 +1522,33 @@ bool strides_ok(const long long* st, int n) {
 
 extern "C" {
 
-// strides: 12 element strides {q_seq,q_batch,q_head, k_.., v_.., o_..}. lse: fp32 [B, nh, S_pad],
-// S_pad = S rounded up to a multiple of 128.
+// fp16 q, k, v -> bf16 copies in dst (3 x [B, nh, S, D], contiguous). strides: 9 element strides
+// {q_seq, q_batch, q_head, k_.., v_..}.
+int gfs_attn_cast_qkv(const void* q, const void* k, const void* v, void* dst, int S, int B, int nh, int D,
+                      const long long* strides, void* stream_) {
+  if (D & 7) return -1;
+  if (!strides_ok(strides, 9)) return -1;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+       reinterpret_cast<uintptr_t>(dst)) & 15)
+    return -2;
+  const long long n = static_cast<long long>(B) * nh * S * (D >> 3);
+  if (n <= 0) return 0;
+  CastArgs a;
+  const void* src[3] = {q, k, v};
+  for (int t = 0; t < 3; ++t) {
+    a.src[t] = static_cast<const __half*>(src[t]);
+    a.ss[t] = strides[3 * t]; a.bs[t] = strides[3 * t + 1]; a.hs[t] = strides[3 * t + 2];
+  }
+  const int blocks = static_cast<int>(std::min<long long>((n + 255) / 256, gfs_host::sm_count() * 16));
+  cast_qkv_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream_)>>>(a, static_cast<__nv_bfloat16*>(dst), S, B, nh,
+                                                                          D);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+// strides: 12 element strides {q_seq,q_batch,q_head, k_.., v_.., o_..}. lse: fp32 [B, nh, S_pad] (base 2),
+// S_pad = S rounded up to a multiple of 128. o_f16: store the output as fp16.
 int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int S, int B, int nh, int D,
-                  const long long* strides, float scale, int causal, void* stream_) {
+                  const long long* strides, float scale, int causal, int o_f16, void* stream_) {
   if (D != 64 && D != 128) return -1;
   if (!strides_ok(strides, 12)) return -1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
@@ -1454,7 +1565,7 @@ int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* ls
   p.o_ss = strides[9]; p.o_bs = strides[10]; p.o_hs = strides[11];
   p.lse = static_cast<float*>(lse);
   p.S = S; p.S_pad = ((S + 127) / 128) * 128; p.B = B; p.nh = nh;
-  p.scale = scale; p.causal = causal;
+  p.scale = scale; p.causal = causal; p.o_f16 = o_f16;
   p.status = gfs_host::status_words();
   const dim3 grid((S + 127) / 128, B * nh);
   static bool set64 = false, set128 = false;
@@ -1477,36 +1588,46 @@ int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* ls
 }
 
 // strides: 24 element strides for {q, k, v, o, do, dq, dk, dv} x {seq, batch, head}.
-// lse, dvec: fp32 [B, nh, S_pad]; dvec is scratch written by the pre-pass.
+// lse (from the forward), dvec: fp32 [B, nh, S_pad]; dvec is scratch written by the pre-pass.
 // rope_cos / rope_sin (optional, fp32 [>=S, D/2]): when given, dq and dk are rotated back
 // (inverse rotary embedding) as they are written, i.e. they are gradients w.r.t. the
 // un-rotated projections.
+// do_bf16: null for bf16 tensors; otherwise o, dO, dq, dk and dv are fp16 (q, k, v stay bf16) and this is
+// scratch for a contiguous bf16 [B, nh, S, D] copy of dO.
 int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dO, const void* lse,
                   void* dvec, void* dq, void* dk, void* dv, int S, int B, int nh, int D, const long long* strides,
-                  float scale, int causal, const void* rope_cos, const void* rope_sin, void* stream_) {
+                  float scale, int causal, const void* rope_cos, const void* rope_sin, void* do_bf16, void* stream_) {
   if (D != 64 && D != 128) return -1;
   if (!strides_ok(strides, 24)) return -1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
-       reinterpret_cast<uintptr_t>(dO) | reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) |
-       reinterpret_cast<uintptr_t>(dv)) & 15)
+       reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dO) | reinterpret_cast<uintptr_t>(dq) |
+       reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv) | reinterpret_cast<uintptr_t>(do_bf16)) & 15)
     return -2;
   if (S <= 0 || B <= 0 || nh <= 0) return 0;
+  if (static_cast<long long>(S) * B * nh > 0x3fffffffll) return -1;   // 32-bit row numbers in the pre-pass
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const int S_pad = ((S + 127) / 128) * 128;
   const long long *sq = strides, *sk = strides + 3, *sv = strides + 6, *so = strides + 9, *sdo = strides + 12,
                   *sdq = strides + 15, *sdk = strides + 18, *sdv = strides + 21;
-  // second half of the dvec buffer: lse * log2(e)
-  float* lse2 = static_cast<float*>(dvec) + static_cast<size_t>(S_pad) * B * nh;
+  long long sdo16[3];
   {
     const long long rows = static_cast<long long>(S) * B * nh;
     const int threads = 256;
-    const int rows_per_block = threads / (D >> 3);
-    gfs_host::launch_pdl(attn_dvec_kernel, dim3(static_cast<unsigned>((rows + rows_per_block - 1) / rows_per_block)),
-                         dim3(threads), 0, stream, static_cast<const __nv_bfloat16*>(dO),
-                         static_cast<const __nv_bfloat16*>(o), static_cast<float*>(dvec),
-                         static_cast<const float*>(lse), lse2, S, S_pad, B, nh, D, sdo[0], sdo[1], sdo[2], so[0],
-                         so[1], so[2]);
+    const int rows_per_block = threads / (D >> 3) * DVEC_ROWS;
+    const dim3 grid(static_cast<unsigned>((rows + rows_per_block - 1) / rows_per_block));
+    const int s_fastest = so[0] < so[2] ? 1 : 0;
+    auto kern = do_bf16 != nullptr ? attn_dvec_kernel<true> : attn_dvec_kernel<false>;
+    gfs_host::launch_pdl(kern, grid, dim3(threads), 0, stream, dO, o, static_cast<float*>(dvec),
+                         static_cast<__nv_bfloat16*>(do_bf16), S, S_pad, B, nh, D, sdo[0], sdo[1], sdo[2], so[0], so[1],
+                         so[2], s_fastest);
     if (cudaGetLastError() != cudaSuccess) return -11;
+    if (do_bf16 != nullptr) {
+      dO = do_bf16;
+      sdo16[0] = D;
+      sdo16[2] = static_cast<long long>(S) * D;
+      sdo16[1] = nh * sdo16[2];
+      sdo = sdo16;
+    }
   }
   const CUtensorMap* q128 = make_map(q, D, S, nh, B, sq, 128);
   const CUtensorMap* k128 = make_map(k, D, S, nh, B, sk, 128);
@@ -1518,7 +1639,8 @@ int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, co
   const CUtensorMap* do64 = make_map(dO, D, S, nh, B, sdo, 64);
   if (!q128 || !k128 || !v128 || !do128 || !q64 || !k64 || !v64 || !do64) return -3;
   BwdParams p;
-  p.lse = lse2;
+  p.lse = static_cast<const float*>(lse);
+  p.out_f16 = do_bf16 != nullptr ? 1 : 0;
   p.dvec = static_cast<const float*>(dvec);
   p.S = S; p.S_pad = S_pad; p.B = B; p.nh = nh; p.scale = scale; p.causal = causal;
   p.status = gfs_host::status_words();

@@ -34,13 +34,10 @@ struct GfsBlockDims {
   int n_layers;
   int pair_min_tiles;      // 256 x 256 tiles from which a product runs on CTA pairs; < 0: never
   int grouped_wgrad;       // small weight gradients of a block share a launch
-  int swiglu_bwd_min_h;    // hidden size from which the single-CTA GEMM fuses the SwiGLU backward
   float dropout_p;         // 0: residual adds run in the GEMM epilogues
   float eps_final;
   const void* cos_table;   // fp32 [>= S, D/2]
   const void* sin_table;
-  void* gemm_ws;           // fp32 workspace of split-K products
-  size_t gemm_ws_bytes;
 };
 
 struct GfsBlockParams {
@@ -87,7 +84,7 @@ struct ActLayout {
 // Scratch of the backward pass. Reused by every block (stream order), except the column partials of
 // the norm weight gradients, which wait for one reduction launch at the end.
 struct BwdLayout {
-  size_t dgu, dact, dy, dx1, dattn, dqkv, dvec, dmask, dx[2], partial, partial_stride, total;
+  size_t dgu, dy, dx1, dattn, dqkv, dvec, dmask, dx[2], partial, partial_stride, total;
   explicit BwdLayout(const GfsBlockDims& d) {
     const size_t T = static_cast<size_t>(d.S) * d.B, H = d.H, I = d.I;
     const size_t s_pad = (static_cast<size_t>(d.S) + 127) / 128 * 128;
@@ -98,12 +95,11 @@ struct BwdLayout {
       return at;
     };
     dgu = take(2 * T * 2 * I);
-    dact = take(2 * T * I);
     dy = take(2 * T * H);
     dx1 = take(2 * T * H);
     dattn = take(2 * T * H);
     dqkv = take(2 * T * 3 * H);
-    dvec = take(2 * 4 * d.B * d.nh * s_pad);
+    dvec = take(4 * d.B * d.nh * s_pad);
     dmask = d.dropout_p > 0.f ? take(2 * 2 * T * H) : 0;
     dx[0] = take(2 * T * H);
     dx[1] = take(2 * T * H);
@@ -117,16 +113,12 @@ int tiles256(int m, int n) { return ((m + 255) / 256) * ((n + 255) / 256); }
 
 bool use_pair(const GfsBlockDims& d, int tiles) { return d.pair_min_tiles >= 0 && tiles >= d.pair_min_tiles; }
 
-// C[M,N] = op(A) op(B) (+ R), choosing the kernel by the rule of ops/gemm.py (gemm_bf16).
+// C[M,N] = op(A) op(B) (+ R), R with the pitch of C
 int product(const GfsBlockDims& d, const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda,
             int ldb, int ldc, int a_mn, int b_mn, int rope_cols, void* stream) {
-  const void* cosp = rope_cols > 0 ? d.cos_table : nullptr;
-  const void* sinp = rope_cols > 0 ? d.sin_table : nullptr;
-  const int ldr = R != nullptr ? ldc : 0;
-  if (K >= 256 && use_pair(d, tiles256(M, N)))
-    return gfs_gemm2_bf16(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, cosp, sinp, rope_cols, d.D, d.B, stream);
-  return gfs_gemm_bf16_rope(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, R != nullptr ? 1 : 0, d.gemm_ws,
-                            d.gemm_ws_bytes, 0, cosp, sinp, rope_cols, d.D, d.B, stream);
+  return gfs_linear(A, B, C, R, M, N, K, lda, ldb, ldc, R != nullptr ? ldc : 0, a_mn, b_mn,
+                    rope_cols > 0 ? d.cos_table : nullptr, rope_cols > 0 ? d.sin_table : nullptr, rope_cols, d.D, d.B,
+                    d.pair_min_tiles, stream);
 }
 
 // The weight gradients of one block that are too small to fill the chip alone share a launch.
@@ -137,7 +129,7 @@ struct WgradGroup {
   int n = 0, tiles = 0;
   int flush(int* launches, void* stream) {
     if (n == 0) return 0;
-    const int rc = gfs_gemm2_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, acc, stream);
+    const int rc = gfs_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, acc, stream);
     n = tiles = 0;
     ++*launches;
     return rc;
@@ -148,7 +140,7 @@ struct WgradGroup {
 int weight_grad(const GfsBlockDims& d, WgradGroup& grp, const void* dY, const void* X, void* dW, int accumulate, int T,
                 int n_out, int n_in, int* launches, void* stream) {
   const int tiles = tiles256(n_out, n_in);
-  if (d.grouped_wgrad && d.pair_min_tiles >= 0 && tiles < d.pair_min_tiles && T >= 256) {
+  if (d.grouped_wgrad && d.pair_min_tiles >= 0 && tiles < d.pair_min_tiles) {
     const int i = grp.n++;
     grp.A[i] = reinterpret_cast<u64>(dY);
     grp.B[i] = reinterpret_cast<u64>(X);
@@ -213,7 +205,7 @@ int gfs_blocks_forward(const GfsBlockDims* dp, const GfsBlockParams* layers, con
     GFS_TRY(gfs_rmsnorm_fwd(x, p.w[W_NORM1], y1, rstd1, T, H, p.eps[0], stream));
     GFS_TRY(product(d, y1, p.w[W_QKV], qkv, nullptr, T, 3 * H, H, H, H, 3 * H, 0, 0, 2 * H, stream));
     GFS_TRY(gfs_flash_fwd(qkv, qkv + 2 * static_cast<size_t>(H), qkv + 4 * static_cast<size_t>(H), attn, lse, d.S, d.B,
-                          d.nh, d.D, st, scale, 1, stream));
+                          d.nh, d.D, st, scale, 1, 0, stream));
     if (!drop) {
       GFS_TRY(product(d, attn, p.w[W_OUT], x1, x, T, H, H, H, H, H, 0, 0, 0, stream));
     } else {
@@ -221,10 +213,7 @@ int gfs_blocks_forward(const GfsBlockDims* dp, const GfsBlockParams* layers, con
       GFS_TRY(gfs_dropout_residual(tmp, x, x1, n_el, d.dropout_p, p.seed[0], 0, stream));
     }
     GFS_TRY(gfs_rmsnorm_fwd(x1, p.w[W_NORM2], y2, rstd2, T, H, p.eps[1], stream));
-    if (use_pair(d, ((T + 255) / 256) * ((I + 127) / 128)))
-      GFS_TRY(gfs_gemm2_bf16_swiglu(1, y2, p.w[W_GATE_UP], gu, ac, T, I, H, H, H, 2 * I, I, stream));
-    else
-      GFS_TRY(gfs_gemm_bf16_swiglu(1, y2, p.w[W_GATE_UP], gu, ac, T, I, H, H, H, 2 * I, I, stream));
+    GFS_TRY(gfs_linear_swiglu(1, y2, p.w[W_GATE_UP], gu, ac, T, I, H, H, H, 2 * I, I, d.pair_min_tiles, stream));
     if (!drop) {
       GFS_TRY(product(d, ac, p.w[W_DOWN], x2, x1, T, H, I, I, I, H, 0, 0, 0, stream));
     } else {
@@ -260,7 +249,7 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
     st[9 + i] = st[12 + i] = o3[i];
   }
   char* s = static_cast<char*>(scratch);
-  void *dgu = s + b.dgu, *dact = s + b.dact, *dy = s + b.dy, *dx1 = s + b.dx1, *dattn = s + b.dattn, *dvec = s + b.dvec;
+  void *dgu = s + b.dgu, *dy = s + b.dy, *dx1 = s + b.dx1, *dattn = s + b.dattn, *dvec = s + b.dvec;
   char* dqkv = s + b.dqkv;
 
   // one batched reduction of the norm weight gradients at the end
@@ -306,16 +295,8 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
       GFS_TRY(gfs_dropout_residual(dout, nullptr, s + b.dmask, n_el, d.dropout_p, p.seed[1], 1, stream));
       dm = s + b.dmask;
     }
-    const bool pair_swi = use_pair(d, tiles256(T, I));
-    if (pair_swi) {
-      GFS_TRY(gfs_gemm2_bf16_swiglu(2, dm, p.w[W_DOWN], dgu, const_cast<void*>(gu), T, I, H, H, I, 2 * I, 2 * I, stream));
-    } else if (H >= d.swiglu_bwd_min_h) {
-      GFS_TRY(gfs_gemm_bf16_swiglu(2, dm, p.w[W_DOWN], dgu, const_cast<void*>(gu), T, I, H, H, I, 2 * I, 2 * I, stream));
-    } else {
-      // short contraction: the plain dgrad product and the SwiGLU backward kernel are faster
-      GFS_TRY(product(d, dm, p.w[W_DOWN], dact, nullptr, T, I, H, H, I, I, 0, 1, 0, stream));
-      GFS_TRY(gfs_swiglu_bwd(dact, gu, dgu, T, I, stream));
-    }
+    GFS_TRY(gfs_linear_swiglu(2, dm, p.w[W_DOWN], dgu, const_cast<void*>(gu), T, I, H, H, I, 2 * I, 2 * I,
+                              d.pair_min_tiles, stream));
     int rc = weight_grad(d, grp, dm, ac, p.g[W_DOWN], p.accumulate[W_DOWN], T, H, I, launches, stream);
     if (rc != 0) return rc;
     GFS_TRY(product(d, dgu, p.w[W_GATE_UP], dy, nullptr, T, H, 2 * I, 2 * I, H, H, 0, 1, 0, stream));
@@ -334,7 +315,7 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
     if (rc != 0) return rc;
     const size_t h2 = 2 * static_cast<size_t>(H);
     GFS_TRY(gfs_flash_bwd(qkv, qkv + h2, qkv + 2 * h2, attn, dattn, lse, dvec, dqkv, dqkv + h2, dqkv + 2 * h2, d.S, d.B,
-                          d.nh, d.D, st, scale, 1, d.cos_table, d.sin_table, stream));
+                          d.nh, d.D, st, scale, 1, d.cos_table, d.sin_table, nullptr, stream));
     *launches += 2;   // a pre-pass and two main kernels
     GFS_TRY(product(d, dqkv, p.w[W_QKV], dy, nullptr, T, H, 3 * H, 3 * H, H, H, 0, 1, 0, stream));
     rc = weight_grad(d, grp, dqkv, y1, p.g[W_QKV], p.accumulate[W_QKV], T, 3 * H, H, launches, stream);

@@ -1,0 +1,159 @@
+// Which GEMM kernel serves a product, for every caller (ops/gemm.py, ops/mlp_fused.py, model.cu).
+//
+//   persistent pairs   gemm2.cu   256 x 256 per CTA pair, epilogue of one tile behind the next tile's K loop
+//   persistent CTAs    gemm.cu    128 x 256 per CTA
+//   one tile per CTA   gemm3.cu   128 x 64, 128 x 128 or 256 x 256 (pair), K split over a cluster
+//
+// From `pair_min_tiles` (60) tiles of 256 x 256 on, the persistent pairs always win. Below, a product is one
+// wave of whatever kernel runs it, and its time is a constant (launch, first TMA, epilogue) plus the K blocks
+// one CTA works through. The constants below were fitted to 110 measured (shape, kernel) pairs on B200: M 103 to
+// 4096, N 256 to 50304, K 103 to 50304, every layout, back to back in a CUDA graph; the fits are within 15 %.
+// us per launch, before (persistent kernels, K split through a workspace and a second launch) -> with this rule:
+// 512 x 768 x 256 with rotary epilogue 16.5 -> 5.5, 130 x 768 x 3072 with addend 18.6 -> 7.7,
+// 2048 x 768 x 2304 21.4 -> 16.3, weight gradient 768 x 768 x 2331 20.8 -> 9.8.
+#include <algorithm>
+
+#include "api.h"
+#include "common.cuh"
+
+namespace {
+
+struct Choice {
+  enum Kernel { PERSISTENT_CTA, PERSISTENT_PAIR, TILE } kernel;
+  int bn, split;
+};
+
+// Most CTAs that are resident together when they come in clusters of `c` (148 SMs in GPCs of unequal
+// size; counted by where a second wave shows in the measured times).
+int wave_of_clusters(int c) {
+  switch (c) {
+    case 1: return 148;
+    case 2: return 148;
+    case 3: return 135;
+    case 4: return 132;
+    case 6: return 108;
+    default: return 96;
+  }
+}
+
+struct TileShape {
+  int bn;               // columns of the tile
+  int cluster;          // CTAs per tile without a split
+  float base, per_kblock, split_cost;
+};
+constexpr TileShape kShapes[3] = {
+    {64, 1, 4.2f, 0.21f, 0.4f},     // 96 cycles per MMA (A and B read for 64 columns), 64-column epilogue
+    {128, 1, 6.3f, 0.265f, 0.7f},   // 128 cycles per MMA: shared-memory reads
+    {256, 2, 8.2f, 0.29f, 2.6f},    // tensor-bound, but 256 columns per row in the epilogue
+};
+
+// Best one-wave tile for `tiles(bn)` tiles of 128 (bn = 256: 256) rows. us, or a huge number if none fits.
+template <typename Tiles>
+float best_tile(Tiles tiles, int kblocks, bool pairs, Choice* c) {
+  float best = 1e30f;
+  for (const TileShape& s : kShapes) {
+    if (s.bn == 256 && !pairs) continue;
+    const int n = tiles(s.bn);
+    for (int split : {1, 2, 3, 4, 8}) {
+      if (split > (s.bn == 256 ? 4 : 8)) break;
+      const int per = (kblocks + split - 1) / split;
+      if (per * (split - 1) >= kblocks) break;              // a CTA without K blocks
+      const int cluster = s.cluster * split;
+      if (n * cluster > wave_of_clusters(cluster)) break;
+      const float t = s.base + s.per_kblock * per + (split > 1 ? s.split_cost : 0.f);
+      if (t < best) {
+        best = t;
+        *c = Choice{Choice::TILE, s.bn, split};
+      }
+    }
+  }
+  return best;
+}
+
+int ceil_div(int a, int b) { return (a + b - 1) / b; }
+
+// cols(bn): output columns covered by a tile of bn accumulator columns.
+Choice choose(int M, int N, int K, int swi_mode, bool add, bool rope, int pair_min_tiles) {
+  auto tiles = [&](int bn) {
+    const int cols = swi_mode == 1 ? bn / 2 : bn;
+    return ceil_div(M, bn == 256 ? 256 : 128) * ceil_div(N, cols);
+  };
+  const int kb = ceil_div(K, 64);
+  const bool pairs = pair_min_tiles >= 0;
+  if (pairs && (K >= 256 || swi_mode != 0) && tiles(256) >= pair_min_tiles) return Choice{Choice::PERSISTENT_PAIR, 256, 1};
+  Choice c{Choice::PERSISTENT_CTA, 256, 1};
+  const float t_tile = best_tile(tiles, kb, pairs, &c);
+  // persistent CTAs: 128 x 256 tiles in waves; the addend, the rotation and the SwiGLU gradient are serial
+  // loads in its epilogue
+  const int waves = ceil_div(ceil_div(M, 128) * ceil_div(N, swi_mode == 1 ? 128 : 256), 148);
+  const float t_cta = 5.2f + 0.3f * kb * waves + 3.8f * (waves - 1) + (add ? 3.3f : 0.f) + (rope ? 9.5f : 0.f) +
+                      (swi_mode == 1 ? 2.0f : 0.f) + (swi_mode == 2 ? 6.0f : 0.f);
+  if (t_cta < t_tile) c = Choice{Choice::PERSISTENT_CTA, 256, 1};
+  return c;
+}
+
+}  // namespace
+
+extern "C" {
+
+// C[M,N] = op(A) op(B) (+ R); arguments as gfs_gemm_bf16_rope (R null: no addend). pair_min_tiles: number of
+// 256 x 256 tiles from which the persistent pair kernel is used; < 0: no kernel on CTA pairs.
+int gfs_linear(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,
+               int ldr, int a_mn_major, int b_mn_major, const void* rope_cos, const void* rope_sin, int rope_cols,
+               int rope_d, int rope_b, int pair_min_tiles, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const Choice c = choose(M, N, K, 0, R != nullptr, rope_cos != nullptr, pair_min_tiles);
+  switch (c.kernel) {
+    case Choice::PERSISTENT_PAIR:
+      return gfs_gemm2_bf16(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn_major, b_mn_major, rope_cos, rope_sin,
+                            rope_cols, rope_d, rope_b, stream);
+    case Choice::TILE:
+      return gfs_gemm_tile(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn_major, b_mn_major, rope_cos, rope_sin,
+                           rope_cols, rope_d, rope_b, 0, nullptr, 0, c.bn, c.split, stream);
+    default:
+      return gfs_gemm_bf16_rope(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn_major, b_mn_major, R != nullptr, nullptr,
+                                0, 1, rope_cos, rope_sin, rope_cols, rope_d, rope_b, stream);
+  }
+}
+
+// The SwiGLU-fused products of the MLP; arguments as gfs_gemm_bf16_swiglu.
+int gfs_linear_swiglu(int mode, const void* a, const void* b, void* c, void* extra, int M, int I, int K, int lda,
+                      int ldb, int ldc, int ld_extra, int pair_min_tiles, void* stream) {
+  if (mode != 1 && mode != 2) return -1;
+  if (M <= 0 || I <= 0 || K <= 0) return 0;
+  const Choice ch = choose(M, I, K, mode, false, false, pair_min_tiles);
+  switch (ch.kernel) {
+    case Choice::PERSISTENT_PAIR:
+      return gfs_gemm2_bf16_swiglu(mode, a, b, c, extra, M, I, K, lda, ldb, ldc, ld_extra, stream);
+    case Choice::TILE:
+      return gfs_gemm_tile(a, b, c, nullptr, M, I, K, lda, ldb, ldc, 0, 0, mode == 2, nullptr, nullptr, 0, 0, 1, mode,
+                           extra, ld_extra, ch.bn, ch.split, stream);
+    default:
+      return gfs_gemm_bf16_swiglu(mode, a, b, c, extra, M, I, K, lda, ldb, ldc, ld_extra, stream);
+  }
+}
+
+// Grouped weight gradients; arguments as gfs_gemm2_wgrad_grouped.
+int gfs_wgrad_grouped(int n, const unsigned long long* A, const unsigned long long* B, const unsigned long long* C,
+                      const int* M, const int* N, const int* K, const int* lda, const int* ldb, const int* ldc,
+                      const int* accumulate, void* stream) {
+  if (n <= 0) return 0;
+  int kb = 0, kb_min = 1 << 30;
+  for (int i = 0; i < n; ++i) {
+    kb = std::max(kb, ceil_div(K[i], 64));
+    kb_min = std::min(kb_min, ceil_div(K[i], 64));
+  }
+  auto tiles = [&](int bn) {
+    int t = 0;
+    for (int i = 0; i < n; ++i) t += ceil_div(M[i], bn == 256 ? 256 : 128) * ceil_div(N[i], bn);
+    return t;
+  };
+  Choice c{Choice::PERSISTENT_PAIR, 256, 1};
+  // the persistent grouped kernel: one wave of pairs, an epilogue of four warps
+  const float t_pair = 6.5f + 0.3f * kb * ceil_div(tiles(256), 74);
+  if (kb == kb_min && best_tile(tiles, kb, true, &c) < t_pair && c.kernel == Choice::TILE)
+    return gfs_gemm_tile_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, accumulate, c.bn, c.split, stream);
+  return gfs_gemm2_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, accumulate, stream);
+}
+
+}  // extern "C"

@@ -21,7 +21,6 @@ import torch
 
 from ..ops import _lib
 from ..ops import gemm as gemm_ops
-from ..ops import mlp_fused
 from ..ops.embedding import embedding_bwd_native, embedding_fwd_native, sort_ids_async
 from ..ops.grad_sink import GradSink
 from ..parallel import parallel_state as ps
@@ -35,8 +34,7 @@ class _Dims(ctypes.Structure):
     """GfsBlockDims in csrc/model.cu."""
     _fields_ = [("S", c_int), ("B", c_int), ("H", c_int), ("nh", c_int), ("D", c_int), ("I", c_int),
                 ("n_layers", c_int), ("pair_min_tiles", c_int), ("grouped_wgrad", c_int),
-                ("swiglu_bwd_min_h", c_int), ("dropout_p", c_float), ("eps_final", c_float),
-                ("cos_table", c_void_p), ("sin_table", c_void_p), ("gemm_ws", c_void_p), ("gemm_ws_bytes", c_size_t)]
+                ("dropout_p", c_float), ("eps_final", c_float), ("cos_table", c_void_p), ("sin_table", c_void_p)]
 
 
 class _BlockParams(ctypes.Structure):
@@ -173,16 +171,13 @@ class _Plan:
         self.dropout = self.layers[0].dropout_prob if training else 0.0
         return True
 
-    def set_shape(self, S: int, B: int, device: torch.device) -> None:
+    def set_shape(self, S: int, B: int) -> None:
         d = self.dims
         rot = self.layers[0].attention.rotary_emb
         cos, sin = rot(self.top[0], S)
         d.cos_table, d.sin_table = cos.data_ptr(), sin.data_ptr()
-        d.pair_min_tiles = gemm_ops._PAIR_MIN_TILES if gemm_ops._PAIR_ENABLED else -1
+        d.pair_min_tiles = gemm_ops.pair_threshold()
         d.grouped_wgrad = 1 if gemm_ops._WGRAD_GROUPING else 0
-        d.swiglu_bwd_min_h = mlp_fused.MIN_HIDDEN_FOR_BWD_FUSION
-        ws = gemm_ops._workspace(device)
-        d.gemm_ws, d.gemm_ws_bytes = ws.data_ptr(), ws.numel() * 4
         key = (S, B, self.dropout)
         if key != self.shape:
             d.S, d.B, d.dropout_p = S, B, self.dropout
@@ -307,7 +302,7 @@ class _ModelFn(torch.autograd.Function):
         S, B, dropout = ctx.key
         if ctx.key != plan.shape:       # another pass of the model ran in between
             plan.dropout = dropout
-            plan.set_shape(S, B, x.device)
+            plan.set_shape(S, B)
         w_emb, _, w_out = plan.top
         d2 = dlogits.reshape(S * B, w_out.shape[0])
         if not d2.is_contiguous():
@@ -327,7 +322,7 @@ def forward(plan: _Plan, inputs: torch.Tensor, ce_stats: bool):
         ids = ids.long()
     B, S = ids.shape
     w_emb, _, w_out = plan.top
-    plan.set_shape(S, B, w_emb.device)
+    plan.set_shape(S, B)
     if torch.is_grad_enabled():
         out = _ModelFn.apply(ids, w_emb, plan, ce_stats)
         if not ce_stats:
@@ -361,7 +356,7 @@ def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
     if labels.dtype != torch.int64:
         labels = labels.long()
     dev = plan.top[0].device
-    plan.set_shape(S, B, dev)
+    plan.set_shape(S, B)
     if plan.dropout > 0.0:
         plan.draw_seeds()
     lib, dims, top = _lib.lib(), byref(plan.dims), plan.top_args

@@ -81,8 +81,9 @@ def _declare(lib: ctypes.CDLL) -> None:
         "gfs_adamw_step": ([vp, vp, vp, vp, vp, i64, vp, vp, f, d, d, f, f, f, f, f, f, vp, vp], i),
         "gfs_flag_slots": ([], i),
         "gfs_wait_probe": ([vp, i64, vp], i),
-        "gfs_flash_fwd": ([vp, vp, vp, vp, vp, i, i, i, i, lp, f, i, vp], i),
-        "gfs_flash_bwd": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, lp, f, i, vp, vp, vp], i),
+        "gfs_flash_fwd": ([vp, vp, vp, vp, vp, i, i, i, i, vp, f, i, i, vp], i),
+        "gfs_attn_cast_qkv": ([vp, vp, vp, vp, i, i, i, i, vp, vp], i),
+        "gfs_flash_bwd": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, vp, f, i, vp, vp, vp, vp], i),
         "gfs_gemm_bf16_comm": ([i, vp, i, vp, i, vp, i, vp, i, i, i, i, i, i, i, ulp, ulp, uip, vp, vp, i, i, i,
                                 ctypes.c_longlong, vp], i),
         "gfs_rmsnorm_dw_reduce_multi": ([i, ulp, ulp, ip, ip, i, vp], i),
@@ -116,6 +117,11 @@ def _declare(lib: ctypes.CDLL) -> None:
         "gfs_blocks_backward": ([vp, vp, vp, vp, i, vp, vp, vp, vp, vp, vp, vp, vp], i),
         "gfs_model_step_bytes": ([vp, vp], sz),
         "gfs_model_step": ([vp, vp, vp, vp, vp, vp, vp, vp, vp], i),
+        "gfs_linear": ([vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, vp, vp, i, i, i, i, vp], i),
+        "gfs_linear_swiglu": ([i, vp, vp, vp, vp, i, i, i, i, i, i, i, i, vp], i),
+        "gfs_wgrad_grouped": ([i, ulp, ulp, ulp, ip, ip, ip, ip, ip, ip, ip, vp], i),
+        "gfs_gemm_tile": ([vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, vp, vp, i, i, i, i, vp, i, i, i, vp], i),
+        "gfs_gemm_tile_wgrad_grouped": ([i, ulp, ulp, ulp, ip, ip, ip, ip, ip, ip, ip, i, i, vp], i),
         "gfs_gemm_bf16_rope": ([vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, i, vp, sz, i, vp, vp, i, i, i, vp], i),
     }
     for name, (argtypes, restype) in sigs.items():

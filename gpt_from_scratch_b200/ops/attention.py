@@ -14,6 +14,7 @@ Two entry points:
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 
 import torch
@@ -37,8 +38,20 @@ def attention_reference(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causa
 
 
 def _strides3(t: torch.Tensor) -> tuple[int, int, int]:
-    assert t.dim() == 4 and t.stride(3) == 1, "need a [S,B,nh,D] view with contiguous head_dim"
-    return t.stride(0), t.stride(1), t.stride(2)
+    """Element strides (sequence, batch, head) of a ``[S, B, nh, D]`` view."""
+    s, b, h, d = t.stride()
+    assert d == 1, "need a [S,B,nh,D] view with contiguous head_dim"
+    return s, b, h
+
+
+def _strides_bhsd(t: torch.Tensor) -> tuple[int, int, int]:
+    """The same of a ``[B, nh, S, D]`` tensor."""
+    b, h, s, d = t.stride()
+    assert d == 1, "need contiguous head_dim"
+    return s, b, h
+
+
+_Strides12, _Strides24 = ctypes.c_longlong * 12, ctypes.c_longlong * 24
 
 
 def _pad128(S: int) -> int:
@@ -46,13 +59,14 @@ def _pad128(S: int) -> int:
 
 
 def flash_fwd_native(q, k, v, out, causal: bool, scale: float) -> torch.Tensor:
-    """q, k, v, out: logical ``[S, B, nh, D]`` views (any strides, head_dim contiguous). Returns LSE."""
+    """q, k, v, out: logical ``[S, B, nh, D]`` views (any strides, head_dim contiguous). Returns the LSE
+    (base 2), the form the backward wants it in."""
     S, B, nh, D = q.shape
     lse = torch.empty((B, nh, _pad128(S)), dtype=torch.float32, device=q.device)
-    st = (ctypes.c_longlong * 12)(*_strides3(q), *_strides3(k), *_strides3(v), *_strides3(out))
+    st = _Strides12(*_strides3(q), *_strides3(k), *_strides3(v), *_strides3(out))
     with _lib.nvtx("flash_attention_fwd"):
         rc = _lib.lib().gfs_flash_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
-                                      S, B, nh, D, st, scale, 1 if causal else 0, _lib.stream_ptr())
+                                      S, B, nh, D, st, scale, 1 if causal else 0, 0, _lib.stream_ptr())
     _lib.check(rc, "gfs_flash_fwd")
     return lse
 
@@ -60,61 +74,104 @@ def flash_fwd_native(q, k, v, out, causal: bool, scale: float) -> torch.Tensor:
 def flash_bwd_native(q, k, v, out, dout, lse, dq, dk, dv, causal: bool, scale: float, rope=None) -> None:
     """``rope = (cos, sin)``: dq and dk are rotated back (inverse RoPE) as they are written."""
     S, B, nh, D = q.shape
-    # scratch of the pre-pass: dvec = rowsum(dO * O), then a copy of lse scaled by log2(e)
-    dvec = torch.empty((2,) + tuple(lse.shape), dtype=torch.float32, device=lse.device)
-    st = (ctypes.c_longlong * 24)(*_strides3(q), *_strides3(k), *_strides3(v), *_strides3(out), *_strides3(dout),
-                                  *_strides3(dq), *_strides3(dk), *_strides3(dv))
+    dvec = torch.empty_like(lse)      # scratch of the pre-pass: rowsum(dO * O)
+    st = _Strides24(*_strides3(q), *_strides3(k), *_strides3(v), *_strides3(out), *_strides3(dout),
+                    *_strides3(dq), *_strides3(dk), *_strides3(dv))
     rc = _lib.lib().gfs_flash_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
                                   lse.data_ptr(), dvec.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                                   S, B, nh, D, st, scale, 1 if causal else 0,
-                                  rope[0].data_ptr() if rope else 0, rope[1].data_ptr() if rope else 0,
+                                  rope[0].data_ptr() if rope else 0, rope[1].data_ptr() if rope else 0, 0,
                                   _lib.stream_ptr())
     _lib.check(rc, "gfs_flash_bwd")
     _lib.add_launches(2)  # pre-pass + two main kernels
 
 
-def _native_ok(*ts: torch.Tensor) -> bool:
-    return all(t.is_cuda and t.dtype == torch.bfloat16 for t in ts) and ts[0].shape[-1] in (64, 128)
+@functools.lru_cache(maxsize=256)
+def _contiguous_strides(n: int, B: int, nh: int, S: int, D: int):
+    """ctypes array of the strides of ``n`` contiguous ``[B, nh, S, D]`` tensors."""
+    return (ctypes.c_longlong * (3 * n))(*([D, nh * S * D, S * D] * n))
+
+
+def _stride_array(*ts: torch.Tensor):
+    for t in ts:
+        if not t.is_contiguous():
+            return (ctypes.c_longlong * (3 * len(ts)))(*[x for t in ts for x in _strides_bhsd(t)])
+    return _contiguous_strides(len(ts), *ts[0].shape)
 
 
 class _FlashAttnBHSD(torch.autograd.Function):
-    """[B, nh, S, D] API on the native kernels."""
+    """[B, nh, S, D] API on the native kernels, for bf16 tensors and for fp16 ones: the kernels are bf16, so
+    fp16 inputs (the dtype of the reference's self-test, core/myFlashAttn.py:28-32) are rounded to bf16, which
+    keeps 8 of their 11 significand bits, within the self-test's tolerances; results are stored as fp16."""
 
     @staticmethod
     def forward(ctx, q, k, v, causal, scale):
-        qv, kv, vv = (t.permute(2, 0, 1, 3) for t in (q, k, v))
+        B, nh, S, D = q.shape
+        lib, stream = _lib.lib(), _lib.stream_ptr()
         out = torch.empty_like(q)
-        lse = flash_fwd_native(qv, kv, vv, out.permute(2, 0, 1, 3), causal, scale)
-        ctx.save_for_backward(q, k, v, out, lse)
-        ctx.causal, ctx.scale = causal, scale
+        lse = torch.empty((B, nh, _pad128(S)), dtype=torch.float32, device=q.device)
+        pq, pk, pv = q.data_ptr(), k.data_ptr(), v.data_ptr()
+        if q.dtype == torch.float16:
+            qkv = torch.empty((3, B, nh, S, D), dtype=torch.bfloat16, device=q.device)
+            src, n = (pq, pk, pv), 2 * B * nh * S * D
+            pq = qkv.data_ptr()
+            pk, pv = pq + n, pq + 2 * n
+            _lib.check(lib.gfs_attn_cast_qkv(*src, pq, S, B, nh, D, _stride_array(q, k, v), stream),
+                       "gfs_attn_cast_qkv")
+            st = _stride_array(qkv[0], qkv[1], qkv[2], out) if not out.is_contiguous() else \
+                _contiguous_strides(4, B, nh, S, D)
+            ctx.save_for_backward(qkv, out, lse)
+        else:
+            st = _stride_array(q, k, v, out)
+            ctx.save_for_backward(q, k, v, out, lse)
+        rc = lib.gfs_flash_fwd(pq, pk, pv, out.data_ptr(), lse.data_ptr(), S, B, nh, D, st, scale, causal,
+                               q.dtype == torch.float16, stream)
+        _lib.check(rc, "gfs_flash_fwd")
+        ctx.args = (causal, scale)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        q, k, v, out, lse = ctx.saved_tensors
-        if dout.stride(-1) != 1:
-            dout = dout.contiguous()
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        pm = lambda t: t.permute(2, 0, 1, 3)  # noqa: E731
-        flash_bwd_native(pm(q), pm(k), pm(v), pm(out), pm(dout), lse, pm(dq), pm(dk), pm(dv), ctx.causal, ctx.scale)
+        *qkv, out, lse = ctx.saved_tensors
+        causal, scale = ctx.args
+        B, nh, S, D = out.shape
+        dout = _tma_ready(dout)
+        f16 = len(qkv) == 1
+        dob = 0
+        if f16:
+            qkv = qkv[0].unbind(0)
+            copy = torch.empty_like(qkv[0])     # dout rounded to bf16, written by the pre-pass
+            dob = copy.data_ptr()
+        q, k, v = qkv
+        dq, dk, dv = (torch.empty_like(t, dtype=out.dtype) for t in qkv)
+        dvec = torch.empty_like(lse)
+        rc = _lib.lib().gfs_flash_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
+                                      lse.data_ptr(), dvec.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                      S, B, nh, D, _stride_array(q, k, v, out, dout, dq, dk, dv), scale, causal, 0, 0,
+                                      dob, _lib.stream_ptr())
+        _lib.check(rc, "gfs_flash_bwd")
+        _lib.add_launches(2)  # pre-pass + two main kernels
         return dq, dk, dv, None, None
+
+
+def _tma_ready(t: torch.Tensor) -> torch.Tensor:
+    """``t`` itself if the kernels can read its layout, else a contiguous copy."""
+    b, h, s, d = t.stride()
+    if d == 1 and not ((b | h | s) & 7) and not t.data_ptr() & 15:
+        return t
+    return t.contiguous()
 
 
 def apply_flash_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal_mask: bool = True) -> torch.Tensor:
     """Flash attention on ``[B, nh, S, D]`` tensors (reference API, core/myFlashAttn.py:1321)."""
-    scale = 1.0 / math.sqrt(q.shape[-1])
-    if (q.is_cuda and q.dtype == k.dtype == v.dtype == torch.float16 and q.shape[-1] in (64, 128)):
-        # the kernels are bf16: fp16 inputs (the dtype of the reference's self-test,
-        # core/myFlashAttn.py:28-32) are rounded to bf16, run natively and the result is cast back;
-        # this keeps 8 of fp16's 11 significand bits, within the self-test's tolerances
-        o = apply_flash_attn(q.to(torch.bfloat16), k.to(torch.bfloat16), v.to(torch.bfloat16), causal_mask)
-        return o.to(torch.float16)
-    if q.is_cuda and q.dtype in (torch.float16, torch.bfloat16) and q.shape[-1] not in (64, 128):
-        raise ValueError(f"apply_flash_attn: head_dim {q.shape[-1]} has no native kernel (64 and 128 do); "
-                         "use attention_reference for other sizes")
-    if _native_ok(q, k, v):
-        fix = lambda t: t if t.stride(-1) == 1 else t.contiguous()  # noqa: E731
-        return _FlashAttnBHSD.apply(fix(q), fix(k), fix(v), bool(causal_mask), scale)
+    D = q.shape[-1]
+    scale = 1.0 / math.sqrt(D)
+    if q.is_cuda and q.dtype in (torch.float16, torch.bfloat16):
+        if D not in (64, 128):
+            raise ValueError(f"apply_flash_attn: head_dim {D} has no native kernel (64 and 128 do); "
+                             "use attention_reference for other sizes")
+        if k.is_cuda and v.is_cuda and q.dtype == k.dtype == v.dtype:
+            return _FlashAttnBHSD.apply(_tma_ready(q), _tma_ready(k), _tma_ready(v), 1 if causal_mask else 0, scale)
     return attention_reference(q, k, v, causal_mask, scale)
 
 

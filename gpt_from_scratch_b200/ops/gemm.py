@@ -1,6 +1,6 @@
 """bf16 GEMMs of a linear layer (forward, dgrad, wgrad) on the tcgen05 kernel.
 
-On CUDA bf16 tensors the three products run on ``gfs_gemm_bf16`` (csrc/gemm.cu);
+On CUDA bf16 tensors the three products run on the library's kernels (csrc/select.cu chooses);
 on any other device/dtype they are plain ``torch.matmul`` calls so the same model
 code runs in fp32 on CPU.
 
@@ -45,6 +45,12 @@ class pair_min_tiles:
         return False
 
 
+def pair_threshold() -> int:
+    """Number of 256 x 256 tiles from which the persistent CTA-pair kernel serves a product; -1: no kernel
+    on CTA pairs. csrc/select.cu chooses by it."""
+    return _PAIR_MIN_TILES if _PAIR_ENABLED else -1
+
+
 def _workspace(device: torch.device) -> torch.Tensor:
     idx = device.index if device.index is not None else torch.cuda.current_device()
     ws = _workspaces.get(idx)
@@ -75,7 +81,8 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_m
     (K-major) or ``[K,N]`` (``b_mn_major``). ``addend`` may alias ``out``.
     ``rope = (cos, sin, rope_cols, head_dim, batch)`` rotates the first ``rope_cols`` output
     columns in the epilogue (fp32 tables ``[positions, head_dim/2]``; row ``r`` is position
-    ``r // batch``).
+    ``r // batch``). ``pair`` / ``force_split`` pick the persistent CTA-pair / single-CTA kernel (the latter
+    with that many K splits) instead of the rule in csrc/select.cu.
     """
     a = _rowmajor_2d(a)
     b = _rowmajor_2d(b)
@@ -91,40 +98,24 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_m
     if out is None:
         out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
     assert out.shape == (M, N) and out.stride(1) == 1
-    if pair is None:
-        pair = (_PAIR_ENABLED and force_split == 0 and K >= 256 and
-                ((M + 255) // 256) * ((N + 255) // 256) >= _PAIR_MIN_TILES)
+    cos, sin, rope_cols, head_dim, batch = rope if rope is not None else (None, None, 0, 0, 1)
+    if rope is not None:
+        assert cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+        assert cos.shape[1] == head_dim // 2 and cos.shape[0] * batch >= M
+    args = (a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(addend), M, N, K, a.stride(0), b.stride(0),
+            out.stride(0), addend.stride(0) if addend is not None else 0, 1 if a_mn_major else 0, 1 if b_mn_major else 0)
+    rargs = (_lib.ptr(cos), _lib.ptr(sin), rope_cols, head_dim, batch)
+    if pair is None and force_split == 0:
+        rc = _lib.lib().gfs_linear(*args, *rargs, pair_threshold(), _lib.stream_ptr())
+        _lib.check(rc, "gfs_linear")
+        return out
     if pair:
-        if rope is not None:
-            cos, sin, rope_cols, head_dim, batch = rope
-            rargs = (cos.data_ptr(), sin.data_ptr(), rope_cols, head_dim, batch)
-        else:
-            rargs = (0, 0, 0, 0, 1)
-        rc = _lib.lib().gfs_gemm2_bf16(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(addend), M, N, K, a.stride(0), b.stride(0),
-            out.stride(0), addend.stride(0) if addend is not None else 0,
-            1 if a_mn_major else 0, 1 if b_mn_major else 0, *rargs, _lib.stream_ptr())
+        rc = _lib.lib().gfs_gemm2_bf16(*args, *rargs, _lib.stream_ptr())
         _lib.check(rc, "gfs_gemm2_bf16")
         return out
     ws = _workspace(a.device)
-    if rope is None:
-        rc = _lib.lib().gfs_gemm_bf16(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(addend),
-            M, N, K, a.stride(0), b.stride(0), out.stride(0),
-            addend.stride(0) if addend is not None else 0,
-            1 if a_mn_major else 0, 1 if b_mn_major else 0, 1 if addend is not None else 0,
-            ws.data_ptr(), ws.numel() * 4, force_split, _lib.stream_ptr())
-    else:
-        cos, sin, rope_cols, head_dim, batch = rope
-        assert cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
-        assert cos.shape[1] == head_dim // 2 and cos.shape[0] * batch >= M
-        rc = _lib.lib().gfs_gemm_bf16_rope(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(addend),
-            M, N, K, a.stride(0), b.stride(0), out.stride(0),
-            addend.stride(0) if addend is not None else 0,
-            1 if a_mn_major else 0, 1 if b_mn_major else 0, 1 if addend is not None else 0,
-            ws.data_ptr(), ws.numel() * 4, force_split, cos.data_ptr(), sin.data_ptr(), rope_cols, head_dim, batch,
-            _lib.stream_ptr())
+    rc = _lib.lib().gfs_gemm_bf16_rope(*args, 1 if addend is not None else 0, ws.data_ptr(), ws.numel() * 4, force_split,
+                                       *rargs, _lib.stream_ptr())
     _lib.check(rc, "gfs_gemm_bf16")
     return out
 
@@ -183,7 +174,7 @@ class _WgradQueue:
 
     A layer's weight gradients are ``[out, in] = dY^T X`` with K = tokens: few output tiles,
     very deep. One at a time they occupy a fraction of the SMs (or need split-K and a
-    reduction pass); several of them in ONE grouped launch (``gfs_gemm2_wgrad_grouped``) fill
+    reduction pass); several of them in ONE grouped launch (``gfs_wgrad_grouped``) fill
     a wave of CTA pairs. A weight gradient is only needed at the optimizer step, so problems
     that write into a gradient sink are parked here (holding references to their operands)
     and launched when enough tiles have accumulated, at the end of the backward pass that
@@ -232,7 +223,7 @@ class _WgradQueue:
         n = len(items)
         with _lib.nvtx("fused:grouped_wgrad"):
             rc = self._launch(items, n)
-        _lib.check(rc, "gfs_gemm2_wgrad_grouped")
+        _lib.check(rc, "gfs_wgrad_grouped")
         for it in items:
             if it[4] is not None:
                 it[4]()
@@ -240,7 +231,7 @@ class _WgradQueue:
     @staticmethod
     def _launch(items, n) -> int:
         U, I = ctypes.c_ulonglong * n, ctypes.c_int * n
-        return _lib.lib().gfs_gemm2_wgrad_grouped(
+        return _lib.lib().gfs_wgrad_grouped(
             n, U(*[it[0].data_ptr() for it in items]), U(*[it[1].data_ptr() for it in items]),
             U(*[it[2].data_ptr() for it in items]), I(*[it[0].shape[1] for it in items]),
             I(*[it[1].shape[1] for it in items]), I(*[it[0].shape[0] for it in items]),
@@ -273,8 +264,7 @@ def linear_wgrad_to_sink(dy2d: torch.Tensor, x2d: torch.Tensor, sink) -> None:
     accumulate = sink.consume_accumulate()
     N_out, N_in = dy2d.shape[1], x2d.shape[1]
     if (_WGRAD_GROUPING and _PAIR_ENABLED and use_native(dy2d, x2d, out)
-            and _WgradQueue.tiles_of(N_out, N_in) < _PAIR_MIN_TILES and dy2d.shape[0] >= 256
-            and N_out % 8 == 0 and N_in % 8 == 0 and out.stride(1) == 1 and out.stride(0) % 8 == 0):
+            and _WgradQueue.tiles_of(N_out, N_in) < _PAIR_MIN_TILES and N_out % 8 == 0 and N_in % 8 == 0 and out.stride(1) == 1 and out.stride(0) % 8 == 0):
         _wgrad_queue.push(_rowmajor_2d(dy2d), _rowmajor_2d(x2d), out, accumulate, sink.done)
         if hasattr(sink, "parked"):
             sink.parked()

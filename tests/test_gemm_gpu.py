@@ -150,3 +150,76 @@ def test_grouped_weight_gradients(cuda_device):
             ref = ref + before[off:off + o * i].view(o, i).float()
         _check(sk.t, ref, T)
         off += o * i
+
+
+@pytest.mark.parametrize("bn", [64, 128, 256])
+@pytest.mark.parametrize("split", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+def test_gemm_tile_kernels(cuda_device, bn, split, a_mn, b_mn):
+    """One tile per CTA / CTA pair with K split over the cluster: row, column and K remainders, fewer rows than a
+    tile, addend aliasing the output; tolerance as in _check (one bf16 rounding of fp32 sums)."""
+    from gpt_from_scratch_b200.ops import _lib
+    if bn == 256 and split == 8:
+        pytest.skip("four pairs at most")
+    g = torch.Generator(device="cuda").manual_seed(bn + split)
+    for M, N, K in ((8, 8, 64 * split), (136, 72, 64 * split + 8), (264, 520, 1032)):
+        a = torch.randn((K, M) if a_mn else (M, K), device=cuda_device, generator=g).bfloat16()
+        b = torch.randn((K, N) if b_mn else (N, K), device=cuda_device, generator=g).bfloat16()
+        c = torch.randn(M, N, device=cuda_device, generator=g).bfloat16()
+        ref = _ref(a, b, a_mn, b_mn, c)
+        kb = (K + 63) // 64
+        rc = _lib.lib().gfs_gemm_tile(a.data_ptr(), b.data_ptr(), c.data_ptr(), c.data_ptr(), M, N, K, a.stride(0),
+                                      b.stride(0), N, N, int(a_mn), int(b_mn), 0, 0, 0, 0, 1, 0, 0, 0, bn, split,
+                                      _lib.stream_ptr())
+        if -(-kb // split) * (split - 1) >= kb:
+            assert rc == -1       # a CTA would have no K block
+            continue
+        assert rc == 0
+        _check(c, ref, K)
+
+
+@pytest.mark.parametrize("bn,split", [(64, 1), (64, 3), (128, 2), (256, 1), (256, 2)])
+def test_gemm_tile_epilogues(cuda_device, bn, split):
+    """Rotary and SwiGLU epilogues and the grouped weight gradients of the tile kernels against fp32."""
+    import ctypes
+    from gpt_from_scratch_b200.ops import _lib
+    lib = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(7 * bn + split)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g).bfloat16()  # noqa: E731
+    S, B, nh, D, K, I = 47, 3, 3, 64, 328, 200
+    M = S * B
+    x, w = rnd(M, K), rnd(3 * nh * D, K)
+    ang = torch.rand(S, D // 2, device=cuda_device, generator=g)
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    out = torch.empty(M, 3 * nh * D, device=cuda_device, dtype=torch.bfloat16)
+    assert lib.gfs_gemm_tile(x.data_ptr(), w.data_ptr(), out.data_ptr(), 0, M, 3 * nh * D, K, K, K, out.stride(0), 0, 0, 0,
+                             cos.data_ptr(), sin.data_ptr(), 2 * nh * D, D, B, 0, 0, 0, bn, split, _lib.stream_ptr()) == 0
+    from gpt_from_scratch_b200.ops.rope import rope_reference
+    ref = (x.float() @ w.float().t()).view(S, B, 3 * nh, D)
+    ref[:, :, :2 * nh] = rope_reference(ref[:, :, :2 * nh], cos, sin)
+    _check(out, ref.view(M, -1), K)
+
+    wg, wd, dy = rnd(2 * I, K) * 0.1, rnd(K, I) * 0.1, rnd(M, K)
+    gu, act, dgu = (torch.empty(M, n, device=cuda_device, dtype=torch.bfloat16) for n in (2 * I, I, 2 * I))
+    assert lib.gfs_gemm_tile(x.data_ptr(), wg.data_ptr(), gu.data_ptr(), 0, M, I, K, K, K, 2 * I, 0, 0, 0, 0, 0, 0, 0, 1,
+                             1, act.data_ptr(), I, bn, split, _lib.stream_ptr()) == 0
+    _check(gu, x.float() @ wg.float().t(), K)
+    guf = gu.float().requires_grad_()          # act and the gradient are computed from the bf16 projection
+    act_ref = torch.nn.functional.silu(guf[:, :I]) * guf[:, I:]
+    _check(act, act_ref.detach(), K)
+    assert lib.gfs_gemm_tile(dy.data_ptr(), wd.data_ptr(), dgu.data_ptr(), 0, M, I, K, K, I, 2 * I, 0, 0, 1, 0, 0, 0, 0, 1,
+                             2, gu.data_ptr(), 2 * I, bn, split, _lib.stream_ptr()) == 0
+    act_ref.backward(dy.float() @ wd.float())
+    _check(dgu, guf.grad, K)
+
+    shapes = [(72, 64), (264, 136), (128, 8)]
+    A, X, C = [rnd(K, m) for m, _ in shapes], [rnd(K, n) for _, n in shapes], [rnd(m, n) for m, n in shapes]
+    acc = [0, 1, 1]
+    refs = [a.float().t() @ b.float() + (c.float() if f else 0) for a, b, c, f in zip(A, X, C, acc)]
+    U, I3 = ctypes.c_ulonglong * 3, ctypes.c_int * 3
+    assert lib.gfs_gemm_tile_wgrad_grouped(
+        3, U(*[t.data_ptr() for t in A]), U(*[t.data_ptr() for t in X]), U(*[t.data_ptr() for t in C]),
+        I3(*[m for m, _ in shapes]), I3(*[n for _, n in shapes]), I3(K, K, K), I3(*[m for m, _ in shapes]),
+        I3(*[n for _, n in shapes]), I3(*[n for _, n in shapes]), I3(*acc), bn, split, _lib.stream_ptr()) == 0
+    for c, r in zip(C, refs):
+        _check(c, r, K)

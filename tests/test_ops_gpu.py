@@ -261,3 +261,29 @@ def test_dropout_residual_kernel(cuda_device):
     y2 = dropout_add(x.detach(), res.detach(), p, True, generator=host_gen)
     assert not torch.equal(y2, y.detach())
     assert torch.equal(dropout_add(x.detach(), res.detach(), p, False), res.detach() + x.detach())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,nh,S,D,causal", [(1, 1, 1, 64, True), (3, 5, 333, 64, False), (2, 3, 129, 128, True)])
+def test_flash_attention_api_dtypes_and_layouts(cuda_device, dtype, B, nh, S, D, causal):
+    """bf16 and fp16 tensors (the latter through the cast and fp16-storing variants), contiguous and as
+    transposed views of a [B, S, nh, D] projection, at row counts around the pre-pass' 4-row groups. The
+    bf16 roundings of P, dS and the inputs (2^-9 each) bound the relative error."""
+    from gpt_from_scratch_b200.ops.attention import apply_flash_attn, attention_reference
+    g = torch.Generator(device="cuda").manual_seed(S + D)
+    for transposed in (False, True):
+        shape = (B, S, nh, D) if transposed else (B, nh, S, D)
+        q, k, v, do = (torch.randn(shape, device=cuda_device, generator=g).to(dtype) for _ in range(4))
+        if transposed:
+            q, k, v, do = (t.transpose(1, 2) for t in (q, k, v, do))
+        q, k, v = (t.detach().requires_grad_() for t in (q, k, v))
+        o = apply_flash_attn(q, k, v, causal)
+        grads = torch.autograd.grad(o, (q, k, v), do)
+        qf, kf, vf = (t.detach().float().requires_grad_() for t in (q, k, v))
+        of = attention_reference(qf, kf, vf, causal)
+        refs = torch.autograd.grad(of, (qf, kf, vf), do.float())
+        assert o.dtype == dtype and all(t.dtype == dtype for t in grads)
+        for name, a, b in zip(("O", "dQ", "dK", "dV"), (o, *grads), (of, *refs)):
+            # one token: dQ and dK are exactly zero, what is left is the rounding of dO and V in dP - D
+            err = (a.float() - b).norm()
+            assert err <= 2e-2 * b.norm() + (2e-2 * D ** 0.5 if S == 1 else 0.0), (name, err.item(), b.norm().item())
