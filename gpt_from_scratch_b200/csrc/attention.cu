@@ -14,13 +14,12 @@
 //   double buffered so block j+1's QK^T overlaps block j's softmax.
 //
 // Backward (two kernels from one template, deterministic, no atomics):
-//   mode 0: one CTA per 128 keys   -> dK, dV, streaming 64-query tiles
-//   mode 1: one CTA per 128 queries -> dQ,     streaming 64-key tiles
+//   mode 0: items of 128 keys    -> dK, dV, streaming 64-query tiles
+//   mode 1: items of 128 queries -> dQ,     streaming 64-key tiles
 //   Both recompute P = exp(S*scale - LSE), dS = P * (dP - D) from two score MMAs
-//   (X = R1 T1^T, Y = R2 T2^T), write P / dS (bf16) to shared memory and accumulate
-//   dV += P^T dO, dK += dS^T Q (mode 0) or dQ += dS K (mode 1) in TMEM. The streamed tile
-//   is consumed twice from the same shared-memory bytes: K-major for the score MMA and
-//   MN-major for the gradient MMA.
+//   (X = R1 T1^T, Y = R2 T2^T), write P / dS (bf16) to TMEM and accumulate dV += P^T dO,
+//   dK += dS^T Q (mode 0) or dQ += dS K (mode 1) there. The streamed tile is consumed twice from the same
+//   shared-memory bytes: K-major for the score MMA and MN-major for the gradient MMA.
 //
 // Reference counterparts: core/myFlashAttn.py:460-728 (_attn_fwd), :740-790 (pre-pass),
 // :805-1066 (_attn_bwd_LoopQ), :1079-1317 (_attn_bwd_LoopKV).
@@ -39,10 +38,6 @@ namespace {
 
 constexpr int ATT_THREADS = 192;
 constexpr float LOG2E_F = 1.4426950408889634f;
-
-__device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
-  return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
-}
 
 // A K-major [rows x K] (64-column blocks a_blk bytes apart), B K-major [N x K] (blocks b_blk apart).
 // Classifies a (32-row warp slice) x (column chunk) block of the score matrix against the
@@ -103,15 +98,17 @@ __device__ __forceinline__ void mma_kmn(uint32_t d, uint32_t a, uint32_t a_blk, 
   }
 }
 
-// A in tensor memory (8 columns per 16-wide K step); B MN-major as in mma_kmn.
-template <int KSTEPS>
+// A in tensor memory (8 columns per 16-wide K step; the second half of the K steps starts HALF columns
+// after the first); B MN-major as in mma_kmn.
+template <int KSTEPS, int HALF = KSTEPS * 4>
 __device__ __forceinline__ void mma_tmn(uint32_t d, uint32_t a_tmem, uint32_t b, uint32_t b_blk, uint32_t idesc,
                                         bool accumulate) {
   const uint64_t bd0 = umma_desc_sw128(b, b_blk, 1024);
 #pragma unroll
   for (int ks = 0; ks < KSTEPS; ++ks) {
     const uint64_t bd = bd0 + ((ks * 2048) >> 4);
-    umma_ts_e(d, a_tmem + ks * 8, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
+    const uint32_t a = a_tmem + (ks / (KSTEPS / 2)) * HALF + (ks % (KSTEPS / 2)) * 8;
+    umma_ts_e(d, a, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
   }
 }
 
@@ -1021,48 +1018,53 @@ struct BwdParams {
   int out_f16;        // dQ, dK, dV are stored as fp16
 };
 
-// CW = number of compute warps (4 or 8). With 8, every accumulator row is shared by two
-// threads that each take half of the 64 streamed columns (no exchange is needed: the
-// row/column statistics are inputs), which doubles the warps available to hide latency.
-// TS = stages of the streamed-tile ring. A stage is only released when the gradient MMAs that read
-// it have finished, and the score MMAs run two tiles ahead, so the TMA of a tile has (TS - 2) tile
-// periods to land. head_dim 64 (P / dS in tensor memory, so the shared memory is free) uses 8
-// stages: 214 us against 224 us with 4 for the whole backward at the GPT-124M shape, 217 us with
-// 10; head_dim 128 has room for 3.
-// PP ("ping-pong", needs CW = 8 and NBUF = 2): the two groups of four compute warps take alternate
-// streamed tiles (group = X/Y buffer) with all 64 columns per thread instead of column halves of the
-// same tile, so that one group's barrier tests, tensor-memory loads and stores overlap the other
-// group's arithmetic; and the MMAs are issued by TWO warps (warp 1: scores, warp 2: gradients),
-// because a single issuing warp needs ~ 1,350 cycles per tile in that scheme and the compute warps
-// then wait for scores.
-template <int D, int MODE, int NBUF, int CW, int TS, bool PP>
-__global__ void __launch_bounds__((PP ? 96 : 64) + 32 * CW, NBUF == 1 ? 2 : 1)
+constexpr int BWD_CW = 16;                          // compute warps
+constexpr int BWD_FIRST_CW = 4;                     // warps 0-2: TMA, score MMAs, gradient MMAs; 3: idle
+constexpr int BWD_THREADS = 32 * (BWD_FIRST_CW + BWD_CW);
+
+template <int D, int MODE>
+struct BwdShape {
+  // Stages of the streamed-tile ring. A stage is only released when the gradient MMAs that read it have
+  // finished and the score MMAs run two tiles ahead, so the TMA of a tile has (TS - 2) tile periods to land.
+  static constexpr int TS = D == 64 ? 8 : 4;
+  static constexpr int STAGING = BWD_CW * 2048;     // epilogue: 2 KB per compute warp
+  static constexpr int SMEM = 2 * (D / 64) * 16384 + 2 * TS * (D / 64) * 8192 + STAGING + (MODE == 0 ? TS * 512 : 0) + 256;
+};
+
+// Bound by the chain of a streamed tile in the compute warps (barrier test, tensor-memory loads, ~ 10
+// instructions per score element, tensor-memory store, arrive), not by a unit, so what counts is how many
+// chains are in flight: sixteen compute warps, four per scheduler. Two groups of eight take alternate
+// streamed tiles (group = X/Y buffer); within a group two warps share the 32 rows of a quarter, 32 streamed
+// columns each (no exchange is needed: the row / column statistics are inputs). The MMAs are issued by two
+// warps (1: scores, 2: gradients), so neither order waits for the other. P / dS (bf16) go to the gradient
+// MMAs as their tensor-memory A operand: in columns of their own where there is room, for dK / dV at
+// head_dim 128 in the columns of the scores they were made from (then a score buffer is free again when
+// the gradient MMAs have read it).
+// us per backward (pre-pass, dK / dV, dQ), eight compute warps (at head_dim 128 with P / dS in shared memory)
+// -> this: [16, 12, 1024, 64] causal 211 -> 173, [4, 2, 2048, 128] 92 -> 76, [1, 8, 4096, 128] 166 -> 136.
+template <int D, int MODE>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant__ CUtensorMap tr2,
                  const __grid_constant__ CUtensorMap tt1, const __grid_constant__ CUtensorMap tt2,
                  const BwdParams p, int n_rt, int n_items) {
   constexpr int DB = D / 64;
+  constexpr int TS = BwdShape<D, MODE>::TS;
   constexpr int R_BYTES = DB * 16384;  // resident [128 x D]
   constexpr int T_BYTES = DB * 8192;   // streamed [64 x D]
-  constexpr int M_BYTES = 16384;       // [128 x 64] bf16
-  constexpr uint32_t TMEM_COLS = (NBUF == 1 && D == 64) ? 256 : 512;
-  constexpr uint32_t Y_COL = 64 * NBUF;  // X tiles at [0, 64*NBUF), Y tiles after them
-  constexpr uint32_t ACC1 = 128 * NBUF, ACC2 = 128 * NBUF + D;
-  // head_dim 64 leaves 128 TMEM columns free: P^T / dS^T (bf16, two per column) are handed to the
-  // gradient MMAs through tensor memory instead of shared memory, which halves the shared-memory
-  // traffic of this kernel (its 64-wide MMAs are otherwise bound by operand reads from shared memory)
-  constexpr bool PT = (D == 64 && NBUF == 2);
-  constexpr uint32_t PT_COL = 384;  // [buffer][P 32 cols | dS 32 cols]
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = align1024(smem_raw);
-  uint8_t* R1 = smem;
+  constexpr uint32_t TMEM_COLS = 512;
+  constexpr uint32_t Y_COL = 128;      // X tiles at [0, 128), Y tiles after them
+  constexpr uint32_t ACC1 = 256, ACC2 = 256 + D;
+  constexpr bool OVERLAY = (D == 128 && MODE == 0);   // P over X, dS over Y
+  constexpr uint32_t PT_COL = 384;     // else: [buffer][P 32 cols | dS 32 cols]
+  constexpr int EPI_WARPS = (MODE == 1 && D == 64) ? BWD_CW / 2 : BWD_CW;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* R1 = smem_raw;
   uint8_t* R2 = R1 + R_BYTES;
-  uint8_t* T1 = R2 + R_BYTES;        // 2 stages
+  uint8_t* T1 = R2 + R_BYTES;
   uint8_t* T2 = T1 + TS * T_BYTES;
-  uint8_t* M1 = T2 + TS * T_BYTES;
-  // P / dS through tensor memory: M1 is only the 16 KB staging area of the epilogue, M2 is not used
-  uint8_t* M2 = M1 + (PT ? M_BYTES : NBUF * M_BYTES);
-  float* stats = reinterpret_cast<float*>(M2 + (PT ? 0 : NBUF * M_BYTES));  // mode 0: [TS stages][lse 64 | dvec 64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(stats) + TS * 512);
+  uint8_t* staging = T2 + TS * T_BYTES;
+  float* stats = reinterpret_cast<float*>(staging + BwdShape<D, MODE>::STAGING);  // mode 0: [TS stages][lse 64 | dvec 64]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(stats) + (MODE == 0 ? TS * 512 : 0));
   uint64_t* r_full = bars;
   uint64_t* t_full = bars + 1;             // [TS]
   uint64_t* t_empty = t_full + TS;         // [TS]
@@ -1078,6 +1080,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  if (smem_u32(smem_raw) & 1023u) {
+    if (threadIdx.x == 0) record_status(p.status, STATUS_BAD_ARGUMENT, 0x5a13u);
+    return;
+  }
   const int n_small = (p.S + 63) >> 6;  // number of 64-row streamed tiles in the sequence
   const int BH = p.B * p.nh;
   // Persistent: a CTA walks work items (resident tile, batch*head), heaviest resident tiles
@@ -1088,7 +1094,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
   auto snake = [&](int rnd) {
     return rnd * G + ((rnd & 1) ? G - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x));
   };
-  // resident tile index and range of streamed tiles of work item w
+  // resident tile index and range of streamed tiles of work item w (at least one tile)
   auto decode = [&](int w, int& rt, int& bh, int& t_begin, int& n_t) {
     const int level = w / BH;
     bh = w % BH;
@@ -1113,12 +1119,12 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&xy_full[i], 1);
-      mbar_init(&xy_empty[i], PP ? 4 : CW);
-      mbar_init(&m_full[i], PP ? 4 : CW);
+      mbar_init(&xy_empty[i], BWD_CW / 2);
+      mbar_init(&m_full[i], BWD_CW / 2);
       mbar_init(&m_empty[i], 1);
     }
     mbar_init(acc_full, 1);
-    mbar_init(acc_empty, CW);
+    mbar_init(acc_empty, EPI_WARPS);
     mbar_init(r_empty, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -1149,345 +1155,257 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
         decode(w, rt, bh, t_begin, n_t);
         const int b = bh / p.nh, h = bh % p.nh;
         mbar_wait(r_empty, (it & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);  // previous item's score MMAs done
-      mbar_arrive_expect_tx(r_full, 2 * R_BYTES);
-#pragma unroll
-      for (int db = 0; db < DB; ++db) {
-        tma_load_4d(R1 + db * 16384, &tr1, r_full, db * 64, rt * 128, h, b);
-        tma_load_4d(R2 + db * 16384, &tr2, r_full, db * 64, rt * 128, h, b);
-      }
-      for (int t = 0; t < n_t; ++t, ++g) {
-        const int st = g % TS;
-        const int ti = t_begin + t;
-        mbar_wait(&t_empty[st], ((g / TS) & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
-        mbar_arrive_expect_tx(&t_full[st], 2 * T_BYTES + (MODE == 0 ? 512 : 0));
+        mbar_arrive_expect_tx(r_full, 2 * R_BYTES);
 #pragma unroll
         for (int db = 0; db < DB; ++db) {
-          tma_load_4d(T1 + st * T_BYTES + db * 8192, &tt1, &t_full[st], db * 64, ti * 64, h, b);
-          tma_load_4d(T2 + st * T_BYTES + db * 8192, &tt2, &t_full[st], db * 64, ti * 64, h, b);
+          tma_load_4d(R1 + db * 16384, &tr1, r_full, db * 64, rt * 128, h, b);
+          tma_load_4d(R2 + db * 16384, &tr2, r_full, db * 64, rt * 128, h, b);
         }
-        if (MODE == 0) {
-          const size_t off = static_cast<size_t>(bh) * p.S_pad + ti * 64;
-          bulk_load_1d(stats + st * 128, p.lse + off, 256, &t_full[st]);
-          bulk_load_1d(stats + st * 128 + 64, p.dvec + off, 256, &t_full[st]);
+        for (int t = 0; t < n_t; ++t, ++g) {
+          const int st = g % TS;
+          const int ti = t_begin + t;
+          mbar_wait(&t_empty[st], ((g / TS) & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
+          mbar_arrive_expect_tx(&t_full[st], 2 * T_BYTES + (MODE == 0 ? 512 : 0));
+#pragma unroll
+          for (int db = 0; db < DB; ++db) {
+            tma_load_4d(T1 + st * T_BYTES + db * 8192, &tt1, &t_full[st], db * 64, ti * 64, h, b);
+            tma_load_4d(T2 + st * T_BYTES + db * 8192, &tt2, &t_full[st], db * 64, ti * 64, h, b);
+          }
+          if (MODE == 0) {
+            const size_t off = static_cast<size_t>(bh) * p.S_pad + ti * 64;
+            bulk_load_1d(stats + st * 128, p.lse + off, 256, &t_full[st]);
+            bulk_load_1d(stats + st * 128 + 64, p.dvec + off, 256, &t_full[st]);
+          }
         }
-      }
       }
       if (*abort_flag) {
         for (int i = 0; i < 64; ++i) __nanosleep(1000);
       }
     }
-  } else if (warp == 1 || (PP && warp == 2)) {
-    {  // whole warp, converged: the MMA / commit helpers elect the issuing lane
-      static_assert(!PP || (CW == 8 && NBUF == 2), "ping-pong needs two warp groups and two X/Y buffers");
-      const bool do_xy = !PP || warp == 1;      // this warp issues the score MMAs
-      constexpr uint32_t idesc_xy = umma_idesc_bf16(128, 64, 0, 0);
-      constexpr uint32_t idesc_acc = umma_idesc_bf16(128, D, 0, 1);
-      const uint32_t r1 = smem_u32(R1), r2 = smem_u32(R2);
-      int g0 = 0;  // ring position of the item's first streamed tile
-      for (int it = 0; it * G < n_items; ++it) {
-        const int w = snake(it);
-        if (w >= n_items) break;
-        int rt, bh, t_begin, n_t;
-        decode(w, rt, bh, t_begin, n_t);
-      if (do_xy) mbar_wait(r_full, it & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
-      auto issue_xy = [&](int t) {
-        const int g = g0 + t;
-        const int st = g % TS;                      // streamed-tile stage
-        const uint32_t par = (g / TS) & 1;
-        const int sb = (NBUF == 2) ? (g & 1) : 0;   // X / Y / P / dS buffer
-        const uint32_t spar = (NBUF == 2) ? ((g >> 1) & 1) : (g & 1);
-        mbar_wait(&t_full[st], par, wctx, STATUS_TIMEOUT_PIPE_FULL);
-        mbar_wait(&xy_empty[sb], spar ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
+  } else if (warp == 1) {
+    // Score MMAs (whole warp, converged: the MMA / commit helpers elect the issuing lane); runs ahead as
+    // far as the X/Y buffers and the streamed-tile ring allow.
+    constexpr uint32_t idesc_xy = umma_idesc_bf16(128, 64, 0, 0);
+    const uint32_t r1 = smem_u32(R1), r2 = smem_u32(R2);
+    int g = 0;
+    for (int it = 0; it * G < n_items; ++it) {
+      const int w = snake(it);
+      if (w >= n_items) break;
+      int rt, bh, t_begin, n_t;
+      decode(w, rt, bh, t_begin, n_t);
+      mbar_wait(r_full, it & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+      for (int t = 0; t < n_t; ++t, ++g) {
+        const int st = g % TS, sb = g & 1;
+        mbar_wait(&t_full[st], (g / TS) & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+        mbar_wait(OVERLAY ? &m_empty[sb] : &xy_empty[sb], ((g >> 1) & 1) ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
         tc_fence_after();
         mma_kk<D / 16>(tmem_base + sb * 64, r1, 16384, smem_u32(T1 + st * T_BYTES), 8192, idesc_xy, false);
         mma_kk<D / 16>(tmem_base + Y_COL + sb * 64, r2, 16384, smem_u32(T2 + st * T_BYTES), 8192, idesc_xy, false);
         umma_commit_e(&xy_full[sb]);
-      };
-      // Score MMAs run LA blocks ahead of the gradient MMAs. With two X/Y buffers and a ring
-      // deep enough (LA = 2), block t+2's scores are issued as soon as the compute warps have
-      // pulled block t's X/Y into registers (xy_empty is signalled right after those loads),
-      // i.e. while they are still doing block t's math, so they never wait for scores.
-      constexpr int LA = (NBUF == 2 && TS >= 4) ? 2 : 1;
-      if (PP && do_xy) {
-        // score warp: runs ahead as far as the X/Y buffers and the streamed-tile ring allow
-        for (int t = 0; t < n_t; ++t) issue_xy(t);
-        umma_commit_e(r_empty);
-        g0 += n_t;
-        continue;
       }
-      if (!PP) {
-        for (int t = 0; t < LA && t < n_t; ++t) issue_xy(t);
-        if (n_t <= LA) umma_commit_e(r_empty);
-      }
-      for (int t = 0; t < n_t; ++t) {
-        if (!PP && t + LA < n_t) {
-          issue_xy(t + LA);
-          if (t + LA + 1 == n_t) umma_commit_e(r_empty);  // the item's last score MMAs are issued
-        }
-        const int g = g0 + t;
-        const int st = g % TS;
-        const int sb = (NBUF == 2) ? (g & 1) : 0;
-        mbar_wait(&m_full[sb], (NBUF == 2) ? ((g >> 1) & 1) : (g & 1), wctx, STATUS_TIMEOUT_SOFTMAX);
+      umma_commit_e(r_empty);
+    }
+  } else if (warp == 2) {
+    // gradient MMAs
+    constexpr uint32_t idesc_acc = umma_idesc_bf16(128, D, 0, 1);
+    int g = 0;
+    for (int it = 0; it * G < n_items; ++it) {
+      const int w = snake(it);
+      if (w >= n_items) break;
+      int rt, bh, t_begin, n_t;
+      decode(w, rt, bh, t_begin, n_t);
+      for (int t = 0; t < n_t; ++t, ++g) {
+        const int st = g % TS, sb = g & 1;
+        mbar_wait(&m_full[sb], (g >> 1) & 1, wctx, STATUS_TIMEOUT_SOFTMAX);
         if (t == 0) mbar_wait(acc_empty, (it & 1) ^ 1u, wctx, STATUS_TIMEOUT_TMEM_EMPTY);  // previous epilogue done
         tc_fence_after();
-        if (PT) {
-          const uint32_t pt = tmem_base + PT_COL + sb * 64;
-          if (MODE == 0) {
-            mma_tmn<4>(tmem_base + ACC1, pt, smem_u32(T2 + st * T_BYTES), 8192, idesc_acc, t > 0);        // dV += P^T dO
-            mma_tmn<4>(tmem_base + ACC2, pt + 32, smem_u32(T1 + st * T_BYTES), 8192, idesc_acc, t > 0);   // dK += dS^T Q
-          } else {
-            mma_tmn<4>(tmem_base + ACC1, pt + 32, smem_u32(T1 + st * T_BYTES), 8192, idesc_acc, t > 0);   // dQ += dS K
-          }
-        } else if (MODE == 0) {
-          // dV += P^T dO ; dK += dS^T Q
-          mma_kmn<4>(tmem_base + ACC1, smem_u32(M1 + sb * M_BYTES), 0, smem_u32(T2 + st * T_BYTES), 8192, idesc_acc,
-                     t > 0);
-          mma_kmn<4>(tmem_base + ACC2, smem_u32(M2 + sb * M_BYTES), 0, smem_u32(T1 + st * T_BYTES), 8192, idesc_acc,
-                     t > 0);
+        const uint32_t pt = tmem_base + (OVERLAY ? sb * 64 : PT_COL + sb * 64);
+        const uint32_t ds = OVERLAY ? pt + Y_COL : pt + 32;
+        constexpr int HALF = OVERLAY ? 32 : 16;   // columns from the first to the second half of P / dS
+        if (MODE == 0) {
+          mma_tmn<4, HALF>(tmem_base + ACC1, pt, smem_u32(T2 + st * T_BYTES), 8192, idesc_acc, t > 0);   // dV += P^T dO
+          mma_tmn<4, HALF>(tmem_base + ACC2, ds, smem_u32(T1 + st * T_BYTES), 8192, idesc_acc, t > 0);   // dK += dS^T Q
         } else {
-          // dQ += dS K
-          mma_kmn<4>(tmem_base + ACC1, smem_u32(M1 + sb * M_BYTES), 0, smem_u32(T1 + st * T_BYTES), 8192, idesc_acc,
-                     t > 0);
+          mma_tmn<4, HALF>(tmem_base + ACC1, ds, smem_u32(T1 + st * T_BYTES), 8192, idesc_acc, t > 0);   // dQ += dS K
         }
         umma_commit_e(&t_empty[st]);
         umma_commit_e(&m_empty[sb]);
       }
       umma_commit_e(acc_full);
-      g0 += n_t;
-      }
     }
-  } else {
+  } else if (warp >= BWD_FIRST_CW) {
+    const int cw = warp - BWD_FIRST_CW;
     const int quarter = warp & 3;
-    constexpr int FIRST_CW = PP ? 3 : 2;            // first compute warp
-    constexpr int COLS = PP ? 64 : 64 / (CW / 4);   // streamed columns handled by this thread
-    const int chalf = (CW == 8) ? ((warp - FIRST_CW) >> 2) : 0;   // warp group: epilogue column half; tile parity (PP) or column half of the math
-    const int cbase = PP ? 0 : chalf * COLS;
+    const int half = (cw >> 2) & 1;     // 32 of the 64 streamed columns
+    const int group = cw >> 3;          // parity of the streamed tiles of this warp
     const int r = quarter * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     const float sl2 = p.scale * LOG2E_F;
+    const uint64_t neg_sl2 = pack_f32x2(-sl2, -sl2), neg_one = pack_f32x2(-1.f, -1.f);
+    const uint32_t x_addr = tmem_base + lane_base + group * 64 + half * 32;
+    const uint32_t y_addr = x_addr + Y_COL;
+    const uint32_t p_addr = OVERLAY ? x_addr : tmem_base + lane_base + PT_COL + group * 64 + half * 16;
+    const uint32_t ds_addr = OVERLAY ? y_addr : p_addr + 32;
+    uint8_t* stage = staging + cw * 2048;
+    bool acc_pending = false;           // the previous item's acc_full phase has not been waited for
     int g0 = 0;
     for (int it = 0; it * G < n_items; ++it) {
-    const int w = snake(it);
-    if (w >= n_items) break;
-    int rt, bh, t_begin, n_t;
-    decode(w, rt, bh, t_begin, n_t);
-    const int b = bh / p.nh, h = bh % p.nh;
-    const int row_g = rt * 128 + r;  // mode 0: key position, mode 1: query position
-    float row_lse = 0.f, row_dvec = 0.f;
-    if (MODE == 1 && row_g < p.S_pad) {
-      row_lse = p.lse[static_cast<size_t>(bh) * p.S_pad + row_g];
-      row_dvec = p.dvec[static_cast<size_t>(bh) * p.S_pad + row_g];
-    }
-    for (int t = 0; t < n_t; ++t) {
-      const int g = g0 + t;
-      const int st = g % TS;                      // streamed-tile stage (for the column statistics)
-      const int sb = (NBUF == 2) ? (g & 1) : 0;   // X / Y / P / dS buffer
-      const uint32_t par = (NBUF == 2) ? ((g >> 1) & 1) : (g & 1);
-      if (PP && sb != chalf) continue;            // the other warp group's tile
-      const int ti = t_begin + t;
-      bool need_mask;
-      if (MODE == 0) need_mask = (p.causal && ti < 2 * rt + 2) || ((ti + 1) * 64 > p.S);
-      else need_mask = (p.causal && ti >= 2 * rt) || ((ti + 1) * 64 > p.S);
-      mbar_wait(&xy_full[sb], par, wctx, STATUS_TIMEOUT_SOFTMAX);
-      mbar_wait(&m_empty[sb], par ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
-      tc_fence_after();
-      const float* st_lse = stats + st * 128;
-      const float* st_dv = st_lse + 64;
-      uint8_t* m1row = M1 + sb * M_BYTES + r * 128;
-      uint8_t* m2row = M2 + sb * M_BYTES + r * 128;
-      uint32_t xa[32], ya[32], xb[32], yb[32];
-      // Masked tiles (the diagonal, the sequence tail) turn their dead scores into -inf in the
-      // registers, which makes both P and dS exact zeros (dvec and dP are finite everywhere, the
-      // padding rows of dvec are written as zeros), and then run the same code as every other tile.
-      auto grad_chunk_impl = [&](uint32_t (&xv)[32], const uint32_t (&yv)[32], int c) {
-        if (need_mask) {
-          const int col0 = ti * 64 + c;
-          const int hi = p.S - col0;                                   // first column past the sequence
-          if (MODE == 0) {                                             // col = query, row = key
-            const int lo = p.causal ? row_g - col0 : -0x7fffffff;      // queries before the key are dead
-#pragma unroll
-            for (int e = 0; e < 32; ++e) xv[e] = (e < lo || e >= hi) ? 0xff800000u : xv[e];
-          } else {                                                     // col = key, row = query
-            const int lim = min(p.causal ? row_g - col0 : 0x7fffffff, hi - 1);
-#pragma unroll
-            for (int e = 0; e < 32; ++e) xv[e] = (e > lim) ? 0xff800000u : xv[e];
-          }
-        }
-        uint32_t pp[16], dd[16];
-#pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          float ls[4], dv[4];
-          if (MODE == 0) {   // per-column statistics of the streamed query tile (same address in all lanes)
-            const float4 l4 = *reinterpret_cast<const float4*>(st_lse + c + e);
-            const float4 d4 = *reinterpret_cast<const float4*>(st_dv + c + e);
-            ls[0] = l4.x; ls[1] = l4.y; ls[2] = l4.z; ls[3] = l4.w;
-            dv[0] = d4.x; dv[1] = d4.y; dv[2] = d4.z; dv[3] = d4.w;
-          } else {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              ls[u] = row_lse;
-              dv[u] = row_dvec;
-            }
-          }
-          float pe[4], de[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            pe[u] = fast_exp2(fmaf(__uint_as_float(xv[e + u]), sl2, -ls[u]));
-            de[u] = pe[u] * (__uint_as_float(yv[e + u]) - dv[u]);
-          }
-          if (MODE == 0) {
-            pp[e >> 1] = pack_bf16x2(pe[0], pe[1]);
-            pp[(e >> 1) + 1] = pack_bf16x2(pe[2], pe[3]);
-          }
-          dd[e >> 1] = pack_bf16x2(de[0], de[1]);
-          dd[(e >> 1) + 1] = pack_bf16x2(de[2], de[3]);
-        }
-        if (PT) {
-          // columns c .. c+31 of this row -> 16 packed columns of the P / dS tensor-memory tiles
-          const uint32_t pt = tmem_base + lane_base + PT_COL + sb * 64 + (c >> 1);
-          if (MODE == 0) tmem_st_32x16(pt, pp);
-          tmem_st_32x16(pt + 32, dd);
-          return;
-        }
-        const int chunk0 = c >> 3;
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const int off = (((chunk0 + q4) ^ (r & 7)) & 7) << 4;
-          if (MODE == 0) {
-            *reinterpret_cast<uint4*>(m1row + off) = make_uint4(pp[4 * q4], pp[4 * q4 + 1], pp[4 * q4 + 2],
-                                                                 pp[4 * q4 + 3]);
-          }
-          *reinterpret_cast<uint4*>((MODE == 0 ? m2row : m1row) + off) =
-              make_uint4(dd[4 * q4], dd[4 * q4 + 1], dd[4 * q4 + 2], dd[4 * q4 + 3]);
-        }
-      };
-      auto grad_chunk = [&](uint32_t (&xv)[32], const uint32_t (&yv)[32], int c) {
+      const int w = snake(it);
+      if (w >= n_items) break;
+      int rt, bh, t_begin, n_t;
+      decode(w, rt, bh, t_begin, n_t);
+      const int b = bh / p.nh, h = bh % p.nh;
+      const int row_g = rt * 128 + r;  // mode 0: key position, mode 1: query position
+      float row_lse = 0.f, row_dvec = 0.f;
+      if (MODE == 1 && row_g < p.S_pad) {
+        row_lse = p.lse[static_cast<size_t>(bh) * p.S_pad + row_g];
+        row_dvec = p.dvec[static_cast<size_t>(bh) * p.S_pad + row_g];
+      }
+      for (int t = (g0 + group) & 1; t < n_t; t += 2) {
+        const int g = g0 + t;
+        const int st = g % TS;                      // streamed-tile stage (for the column statistics)
+        const uint32_t par = (g >> 1) & 1;
+        const int ti = t_begin + t;
+        const int col0 = ti * 64 + half * 32;       // position of this warp's first column
+        bool need_mask;
+        if (MODE == 0) need_mask = (p.causal && ti < 2 * rt + 2) || ((ti + 1) * 64 > p.S);
+        else need_mask = (p.causal && ti >= 2 * rt) || ((ti + 1) * 64 > p.S);
         // alive / mixed / dead for this warp's 32 rows x 32 columns; a dead chunk costs no math
         const int row_lo = rt * 128 + quarter * 32;
-        const int kind = need_mask ? mask_class<MODE == 0>(row_lo, row_lo + 31, ti * 64 + c, ti * 64 + c + 31,
-                                                           p.causal != 0, p.S)
-                                   : 0;
-        if (kind == 2 && PT) {
-          uint32_t zeros[16];
+        const int kind = need_mask ? mask_class<MODE == 0>(row_lo, row_lo + 31, col0, col0 + 31, p.causal != 0, p.S) : 0;
+        mbar_wait(&xy_full[group], par, wctx, STATUS_TIMEOUT_SOFTMAX);
+        tc_fence_after();
+        uint32_t pp[16], dd[16];
+        if (kind == 2) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) zeros[e] = 0u;
-          const uint32_t pt = tmem_base + lane_base + PT_COL + sb * 64 + (c >> 1);
-          if (MODE == 0) tmem_st_32x16(pt, zeros);
-          tmem_st_32x16(pt + 32, zeros);
+          for (int e = 0; e < 16; ++e) pp[e] = dd[e] = 0u;
+          if (!OVERLAY && lane == 0) mbar_arrive(&xy_empty[group]);
         } else {
-          grad_chunk_impl(xv, yv, c);
+          uint32_t xv[32], yv[32];
+          tmem_ld_32x32(x_addr, xv);
+          tmem_ld_32x32(y_addr, yv);
+          tmem_ld_wait_for(xv);
+          tmem_ld_wait_for(yv);
+          if (!OVERLAY) {
+            // X / Y are in registers: hand the buffer back now so the next scores can be computed
+            // into it while this block's math runs
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&xy_empty[group]);
+          }
+          // Masked tiles (the diagonal, the sequence tail) turn their dead scores into -inf in the
+          // registers, which makes both P and dS exact zeros (dvec and dP are finite everywhere, the
+          // padding rows of dvec are written as zeros), and then run the same code as every other tile.
+          if (kind == 1) {
+            const int hi = p.S - col0;                                   // first column past the sequence
+            if (MODE == 0) {                                             // col = query, row = key
+              const int lo = p.causal ? row_g - col0 : -0x7fffffff;      // queries before the key are dead
+#pragma unroll
+              for (int e = 0; e < 32; ++e) xv[e] = (e < lo || e >= hi) ? 0xff800000u : xv[e];
+            } else {                                                     // col = key, row = query
+              const int lim = min(p.causal ? row_g - col0 : 0x7fffffff, hi - 1);
+#pragma unroll
+              for (int e = 0; e < 32; ++e) xv[e] = (e > lim) ? 0xff800000u : xv[e];
+            }
+          }
+          const float* st_lse = stats + st * 128 + half * 32;
+          const float* st_dv = st_lse + 64;
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            uint64_t ls[2], dv[2];
+            if (MODE == 0) {   // per-column statistics of the streamed query tile (same address in all lanes)
+              const float4 l4 = *reinterpret_cast<const float4*>(st_lse + e);
+              const float4 d4 = *reinterpret_cast<const float4*>(st_dv + e);
+              ls[0] = pack_f32x2(l4.x, l4.y); ls[1] = pack_f32x2(l4.z, l4.w);
+              dv[0] = pack_f32x2(d4.x, d4.y); dv[1] = pack_f32x2(d4.z, d4.w);
+            } else {
+              ls[0] = ls[1] = pack_f32x2(row_lse, row_lse);
+              dv[0] = dv[1] = pack_f32x2(row_dvec, row_dvec);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              // P = 2^(x scale log2(e) - lse), dS = P (y - dvec), two columns per instruction. The first
+              // sum is formed negated; the exponential turns the sign back.
+              const float2 a = unpack_f32x2(fma_f32x2(pack_u32x2(xv[e + 2 * u], xv[e + 2 * u + 1]), neg_sl2, ls[u]));
+              const float p0 = fast_exp2(-a.x), p1 = fast_exp2(-a.y);
+              const uint64_t dy = fma_f32x2(dv[u], neg_one, pack_u32x2(yv[e + 2 * u], yv[e + 2 * u + 1]));
+              const float2 d = unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), dy));
+              if (MODE == 0) pp[(e >> 1) + u] = pack_bf16x2(p0, p1);
+              dd[(e >> 1) + u] = pack_bf16x2(d.x, d.y);
+            }
+          }
         }
-      };
-      const uint32_t x_addr = tmem_base + lane_base + sb * 64;
-      const uint32_t y_addr = tmem_base + lane_base + Y_COL + sb * 64;
-      if (PP) {
-        // one 32-column half at a time in the same registers (all 64 columns at once would not fit
-        // the 168 registers of a thread); the X/Y buffer goes back once the second half is loaded
-        tmem_ld_32x32(x_addr, xa);
-        tmem_ld_32x32(y_addr, ya);
-        tmem_ld_wait_for(xa);
-        tmem_ld_wait_for(ya);
-        grad_chunk(xa, ya, 0);
-        tmem_ld_32x32(x_addr + 32, xa);
-        tmem_ld_32x32(y_addr + 32, ya);
-        tmem_ld_wait_for(xa);
-        tmem_ld_wait_for(ya);
+        // columns of this row -> 16 packed columns of the P / dS tensor-memory tiles
+        if (!OVERLAY) {
+          mbar_wait(&m_empty[group], par ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
+          tc_fence_after();
+        }
+        if (MODE == 0) tmem_st_32x16(p_addr, pp);
+        tmem_st_32x16(ds_addr, dd);
+        if (acc_pending) {   // before the arrival that lets the next phase of acc_full complete
+          mbar_wait(acc_full, (it - 1) & 1, wctx, STATUS_TIMEOUT_TMEM_FULL);
+          acc_pending = false;
+        }
+        tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&xy_empty[sb]);
-        grad_chunk(xa, ya, 32);
-      } else {
-        tmem_ld_32x32(x_addr + cbase, xa);
-        tmem_ld_32x32(y_addr + cbase, ya);
-        if (COLS == 64) {
-          tmem_ld_32x32(x_addr + 32, xb);
-          tmem_ld_32x32(y_addr + 32, yb);
+        if (lane == 0) mbar_arrive(&m_full[group]);
+      }
+      g0 += n_t;
+      // Epilogue: accumulators -> global. dK / dV: one group of warps each, a half of the columns per warp.
+      // dQ: a quarter of the columns per warp at head_dim 128; at head_dim 64 the group that does not own
+      // the next item's first tile does it all and the other one goes on.
+      if (EPI_WARPS != BWD_CW && group == (g0 & 1)) {
+        acc_pending = true;
+        continue;
+      }
+      constexpr int NC = (MODE == 0) ? D / 64 : 1;    // 32-column chunks per warp
+      const int c0 = (MODE == 0) ? half * (D / 2) : (D == 128 ? group * 64 + half * 32 : half * 32);
+      const bool is_dv = MODE == 0 && group == 1;
+      const bool rope_on = !is_dv && p.rope_cos != nullptr && row_g < p.S;
+      const float out_scale = is_dv ? 1.f : p.scale;
+      const int row0 = rt * 128 + quarter * 32;
+      const long long o_ss = is_dv ? p.o2_ss : p.o1_ss;
+      __nv_bfloat16* out = is_dv ? p.out2 + row0 * p.o2_ss + b * p.o2_bs + h * p.o2_hs
+                                 : p.out1 + row0 * p.o1_ss + b * p.o1_bs + h * p.o1_hs;
+      const uint32_t acc = tmem_base + lane_base + (MODE == 0 && !is_dv ? ACC2 : ACC1);
+#pragma unroll
+      for (int ci = 0; ci < NC; ++ci) {
+        const int c = c0 + 32 * ci;
+        if (ci == 0) {
+          mbar_wait(acc_full, it & 1, wctx, STATUS_TIMEOUT_TMEM_FULL);
+          tc_fence_after();
         }
-        tmem_ld_wait_for(xa);
-        tmem_ld_wait_for(ya);
-        if (COLS == 64) {
-          tmem_ld_wait_for(xb);
-          tmem_ld_wait_for(yb);
+        uint32_t v[32], wv[16];
+        tmem_ld_32x32(acc + c, v);
+        tmem_ld_wait_for(v);
+        if (ci == NC - 1) {      // the accumulators may be overwritten by the next item
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty);
         }
-        // X / Y are in registers: hand the buffer back now so the next scores can be computed
-        // into it while this block's math runs
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&xy_empty[sb]);
-        grad_chunk(xa, ya, cbase);
-        if (COLS == 64) grad_chunk(xb, yb, 32);
-      }
-      if (PT) tmem_st_wait();
-      tc_fence_before();
-      if (!PT) fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&m_full[sb]);
-    }
-    // epilogue: accumulators -> global
-    g0 += n_t;
-    // the rotary table entries of this thread's row and columns are fetched while the item's last
-    // gradient MMAs finish (their global-memory latency would otherwise sit between the
-    // accumulator load and the stores)
-    constexpr int EC = D / (CW / 4);   // accumulator columns per thread
-    float4 rope_c[EC / 8], rope_s[EC / 8];
-    const bool rope_on = p.rope_cos != nullptr && row_g < p.S;
-    if (rope_on) {
 #pragma unroll
-      for (int i = 0; i < EC / 8; ++i) {
-        const size_t ti = static_cast<size_t>(row_g) * (D / 2) + ((chalf * EC + 8 * i) >> 1);
-        rope_c[i] = *reinterpret_cast<const float4*>(p.rope_cos + ti);
-        rope_s[i] = *reinterpret_cast<const float4*>(p.rope_sin + ti);
-      }
-    }
-    mbar_wait(acc_full, it & 1, wctx, STATUS_TIMEOUT_TMEM_FULL);
-    tc_fence_after();
-    // The accumulators leave through a staging area in the M1 buffer (nothing reads it any more:
-    // acc_full covers the item's last gradient MMAs): rows [32 * quarter, +32) of M1 are only ever
-    // written by the two warps of this quarter, which meet at a named barrier before either of them
-    // goes on to the next item's first block.
-    const int row0 = rt * 128 + quarter * 32;
-    uint8_t* stage = M1 + quarter * 4096 + chalf * 2048;
-    __nv_bfloat16* g1 = p.out1 + row0 * p.o1_ss + b * p.o1_bs + h * p.o1_hs;
-    __nv_bfloat16* g2 = (MODE == 0) ? p.out2 + row0 * p.o2_ss + b * p.o2_bs + h * p.o2_hs : nullptr;
+        for (int q4 = 0; q4 < 4; ++q4) {
+          float f[8];
 #pragma unroll
-    for (int ci = 0; ci < EC / 32; ++ci) {
-      const int c = chalf * EC + 32 * ci;
-      uint32_t v[32], w[16];
-      // mode 0: ACC2 holds dK (scaled), ACC1 holds dV; mode 1: ACC1 holds dQ (scaled)
-      tmem_ld_32x32(tmem_base + lane_base + (MODE == 0 ? ACC2 : ACC1) + c, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) {
-        float f[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[8 * q4 + e]) * p.scale;
-        if (rope_on) {  // inverse rotation: sin -> -sin
-          const float4 cs = rope_c[4 * ci + q4];
-          const float4 sn = rope_s[4 * ci + q4];
-          const float a0 = f[0], a1 = f[1], a2 = f[2], a3 = f[3], a4 = f[4], a5 = f[5], a6 = f[6], a7 = f[7];
-          f[0] = a0 * cs.x + a1 * sn.x; f[1] = a1 * cs.x - a0 * sn.x;
-          f[2] = a2 * cs.y + a3 * sn.y; f[3] = a3 * cs.y - a2 * sn.y;
-          f[4] = a4 * cs.z + a5 * sn.z; f[5] = a5 * cs.z - a4 * sn.z;
-          f[6] = a6 * cs.w + a7 * sn.w; f[7] = a7 * cs.w - a6 * sn.w;
+          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[8 * q4 + e]) * out_scale;
+          if (rope_on) {  // inverse rotation: sin -> -sin
+            const size_t at = static_cast<size_t>(row_g) * (D / 2) + ((c + 8 * q4) >> 1);
+            const float4 cs = *reinterpret_cast<const float4*>(p.rope_cos + at);
+            const float4 sn = *reinterpret_cast<const float4*>(p.rope_sin + at);
+            const float a0 = f[0], a1 = f[1], a2 = f[2], a3 = f[3], a4 = f[4], a5 = f[5], a6 = f[6], a7 = f[7];
+            f[0] = a0 * cs.x + a1 * sn.x; f[1] = a1 * cs.x - a0 * sn.x;
+            f[2] = a2 * cs.y + a3 * sn.y; f[3] = a3 * cs.y - a2 * sn.y;
+            f[4] = a4 * cs.z + a5 * sn.z; f[5] = a5 * cs.z - a4 * sn.z;
+            f[6] = a6 * cs.w + a7 * sn.w; f[7] = a7 * cs.w - a6 * sn.w;
+          }
+          wv[4 * q4 + 0] = pack_out(f[0], f[1], p.out_f16);
+          wv[4 * q4 + 1] = pack_out(f[2], f[3], p.out_f16);
+          wv[4 * q4 + 2] = pack_out(f[4], f[5], p.out_f16);
+          wv[4 * q4 + 3] = pack_out(f[6], f[7], p.out_f16);
         }
-        w[4 * q4 + 0] = pack_out(f[0], f[1], p.out_f16);
-        w[4 * q4 + 1] = pack_out(f[2], f[3], p.out_f16);
-        w[4 * q4 + 2] = pack_out(f[4], f[5], p.out_f16);
-        w[4 * q4 + 3] = pack_out(f[6], f[7], p.out_f16);
+        store_rows_32x32(stage, wv, lane, out + c, o_ss, p.S - row0);
       }
-      store_rows_32x32(stage, w, lane, g1 + c, p.o1_ss, p.S - row0);
-      if (MODE == 0) {
-        tmem_ld_32x32(tmem_base + lane_base + ACC1 + c, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int e = 0; e < 16; ++e) w[e] = pack_out(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]), p.out_f16);
-        store_rows_32x32(stage, w, lane, g2 + c, p.o2_ss, p.S - row0);
-      }
-    }
-    if (CW == 8) named_barrier_sync(8 + quarter, 64);
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(acc_empty);  // the accumulators may be overwritten by the next item
     }
   }
 
@@ -1649,11 +1567,6 @@ int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, co
   const int n_rt = (S + 127) / 128;
   const int n_items = n_rt * B * nh;
   const int ctas = std::min(n_items, gfs_host::sm_count());
-  const int nbuf = 2;
-  const int bwd_threads = ((D == 64) ? 96 : 64) + 32 * 8;   // head_dim 64: a second MMA-issuing warp
-  const int ts = (D == 64) ? 8 : 3;
-  const int m_bytes = (D == 64) ? 16384 : 2 * nbuf * 16384;   // head_dim 64: epilogue staging only
-  const int smem = 2 * (D / 64) * 16384 + 2 * ts * (D / 64) * 8192 + m_bytes + ts * 512 + 512 + 1024;
   static bool set_done[4] = {false, false, false, false};
   // mode 0: dK, dV
   BwdParams p0 = p;
@@ -1663,20 +1576,24 @@ int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, co
   p1.out1 = static_cast<__nv_bfloat16*>(dq); p1.o1_ss = sdq[0]; p1.o1_bs = sdq[1]; p1.o1_hs = sdq[2];
   p1.out2 = nullptr; p1.o2_ss = p1.o2_bs = p1.o2_hs = 0;
   if (D == 64) {
-    if (!set_done[0]) { if (set_smem(flash_bwd_kernel<64, 0, 2, 8, 8, true>, smem)) return -10; set_done[0] = true; }
-    if (!set_done[1]) { if (set_smem(flash_bwd_kernel<64, 1, 2, 8, 8, true>, smem)) return -10; set_done[1] = true; }
-    gfs_host::launch_pdl(flash_bwd_kernel<64, 0, 2, 8, 8, true>, dim3(ctas), dim3(bwd_threads), smem, stream, *k128, *v128,
+    constexpr int smem0 = BwdShape<64, 0>::SMEM;
+    if (!set_done[0]) { if (set_smem(flash_bwd_kernel<64, 0>, smem0)) return -10; set_done[0] = true; }
+    gfs_host::launch_pdl(flash_bwd_kernel<64, 0>, dim3(ctas), dim3(BWD_THREADS), smem0, stream, *k128, *v128,
                          *q64, *do64, p0, n_rt, n_items);
     if (cudaGetLastError() != cudaSuccess) return -12;
-    gfs_host::launch_pdl(flash_bwd_kernel<64, 1, 2, 8, 8, true>, dim3(ctas), dim3(bwd_threads), smem, stream, *q128, *do128,
+    constexpr int smem1 = BwdShape<64, 1>::SMEM;
+    if (!set_done[1]) { if (set_smem(flash_bwd_kernel<64, 1>, smem1)) return -10; set_done[1] = true; }
+    gfs_host::launch_pdl(flash_bwd_kernel<64, 1>, dim3(ctas), dim3(BWD_THREADS), smem1, stream, *q128, *do128,
                          *k64, *v64, p1, n_rt, n_items);
   } else {
-    if (!set_done[2]) { if (set_smem(flash_bwd_kernel<128, 0, 2, 8, 3, false>, smem)) return -10; set_done[2] = true; }
-    if (!set_done[3]) { if (set_smem(flash_bwd_kernel<128, 1, 2, 8, 3, false>, smem)) return -10; set_done[3] = true; }
-    gfs_host::launch_pdl(flash_bwd_kernel<128, 0, 2, 8, 3, false>, dim3(ctas), dim3(bwd_threads), smem, stream, *k128, *v128,
+    constexpr int smem0 = BwdShape<128, 0>::SMEM;
+    if (!set_done[2]) { if (set_smem(flash_bwd_kernel<128, 0>, smem0)) return -10; set_done[2] = true; }
+    gfs_host::launch_pdl(flash_bwd_kernel<128, 0>, dim3(ctas), dim3(BWD_THREADS), smem0, stream, *k128, *v128,
                          *q64, *do64, p0, n_rt, n_items);
     if (cudaGetLastError() != cudaSuccess) return -12;
-    gfs_host::launch_pdl(flash_bwd_kernel<128, 1, 2, 8, 3, false>, dim3(ctas), dim3(bwd_threads), smem, stream, *q128, *do128,
+    constexpr int smem1 = BwdShape<128, 1>::SMEM;
+    if (!set_done[3]) { if (set_smem(flash_bwd_kernel<128, 1>, smem1)) return -10; set_done[3] = true; }
+    gfs_host::launch_pdl(flash_bwd_kernel<128, 1>, dim3(ctas), dim3(BWD_THREADS), smem1, stream, *q128, *do128,
                          *k64, *v64, p1, n_rt, n_items);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -13;

@@ -92,6 +92,30 @@ def test_flash_attention_growing_scores(cuda_device, causal, D):
         assert rel < 3e-2, f"{name}: relative error {rel:.4g}"
 
 
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,nh,S", [(1, 1, 1), (2, 1, 33), (1, 2, 63), (1, 1, 65), (2, 3, 127), (1, 2, 129), (3, 1, 193),
+                                    (1, 3, 385), (3, 51, 257)])
+def test_flash_attention_tile_edges(cuda_device, B, nh, S, D, causal):
+    """Lengths around the tiles' edges (64 streamed rows, 32-row warp slices, 128-row items), and more items
+    than pipelines. Tolerance: P and dS are rounded to bf16 (2^-9 relative), like the results."""
+    from gpt_from_scratch_b200.ops.attention import apply_flash_attn, attention_reference
+    g = torch.Generator(device="cuda").manual_seed(S * 2 + D)
+    q, k, v = (torch.randn(B, nh, S, D, device=cuda_device, generator=g).bfloat16().requires_grad_() for _ in range(3))
+    do = torch.randn(B, nh, S, D, device=cuda_device, generator=g).bfloat16()
+    o = apply_flash_attn(q, k, v, causal)
+    o.backward(do)
+    qf, kf, vf = (t.detach().double().requires_grad_() for t in (q, k, v))
+    of = attention_reference(qf, kf, vf, causal)
+    of.backward(do.double())
+    for name, a, b in (("O", o, of), ("dQ", q.grad, qf.grad), ("dK", k.grad, kf.grad), ("dV", v.grad, vf.grad)):
+        if S == 1 and name in ("dQ", "dK"):     # a single key: zero up to fp32 sums in two orders
+            assert a.float().abs().max() < 1e-3
+            continue
+        rel = (a.double() - b).norm() / b.norm()
+        assert rel < 1e-2, f"{name}: relative error {rel:.4g}"
+
+
 def test_flash_attention_noncausal_and_ragged(cuda_device):
     from gpt_from_scratch_b200.ops.attention import apply_flash_attn, attention_reference
     g = torch.Generator(device="cuda").manual_seed(3)
