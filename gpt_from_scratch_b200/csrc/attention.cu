@@ -5,13 +5,10 @@
 // [S,B,3,nh,D] qkv buffer, so no permute/contiguous copies exist), and the output is
 // written directly in [S,B,nh*D] layout.
 //
-// Forward (one CTA per 128 query rows of one (batch, head); 6 warps):
-//   warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 softmax (one thread per query row).
-//   Per 128-key block: S = Q K^T -> TMEM; softmax threads read their row with tcgen05.ld,
-//   keep the running max / sum, write P (bf16) into 128B-swizzled shared memory; the MMA
-//   warp then computes P V into a second TMEM tile that the softmax threads fold into
-//   their register-resident output row (rescaled by exp(m_old - m_new)). S, P and PV are
-//   double buffered so block j+1's QK^T overlaps block j's softmax.
+// Forward (persistent; head_dim 64: pairs of 128-row query tiles, 128: two pipelines of 128-row items): per
+//   128-key block S = Q K^T -> TMEM; the softmax threads read their row (128: half row) with tcgen05.ld, keep
+//   the running max / sum and store P (bf16) in TMEM, from where the MMA warp adds P V to the output
+//   accumulator, which stays in TMEM for the whole item.
 //
 // Backward (two kernels from one template, deterministic, no atomics):
 //   mode 0: items of 128 keys    -> dK, dV, streaming 64-query tiles
@@ -36,7 +33,6 @@ using namespace gfs;
 
 namespace {
 
-constexpr int ATT_THREADS = 192;
 constexpr float LOG2E_F = 1.4426950408889634f;
 
 // A K-major [rows x K] (64-column blocks a_blk bytes apart), B K-major [N x K] (blocks b_blk apart).
@@ -136,23 +132,6 @@ __device__ __forceinline__ void store_rows_32x32(uint8_t* stage, const uint32_t 
   __syncwarp();
 }
 
-// 32 rows x 64 bf16 columns; w = this lane's row (32 packed words); stage: 4 KB of this warp.
-__device__ __forceinline__ void store_rows_32x64(uint8_t* stage, const uint32_t (&w)[32], int lane,
-                                                 __nv_bfloat16* g0, long long row_stride, int rows_valid) {
-#pragma unroll
-  for (int ch = 0; ch < 8; ++ch)
-    *reinterpret_cast<uint4*>(stage + lane * 128 + ((ch ^ (lane & 7)) << 4)) =
-        make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int row = (lane >> 3) + 4 * i;
-    const uint4 v = *reinterpret_cast<const uint4*>(stage + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
-    if (row < rows_valid) *reinterpret_cast<uint4*>(g0 + row * row_stride + (lane & 7) * 8) = v;
-  }
-  __syncwarp();
-}
-
 // Two fp32 values as a 16-bit pair of the output's type. The kernels compute in bf16; tensors of an fp16
 // caller are rounded to bf16 on the way in (cast_qkv_kernel, attn_dvec_kernel) and results leave as fp16
 // straight from fp32, so an fp16 call costs one launch more than a bf16 one and no pass over its results.
@@ -178,65 +157,72 @@ struct FwdParams {
   uint32_t* status;
 };
 
-// NBUF = 2: S / P / PV tiles double buffered, one CTA per SM (head_dim 128).
-// NBUF = 1: single buffers, half the shared memory and TMEM, so two CTAs share an SM and
-//           hide each other's softmax / MMA latencies (head_dim 64).
-template <int D, int NBUF>
-__global__ void __launch_bounds__(ATT_THREADS, NBUF == 1 ? 2 : 1)
-flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
-                 const __grid_constant__ CUtensorMap tv, const FwdParams p) {
-  constexpr int DB = D / 64;
-  constexpr int TILE_BYTES = DB * 16384;  // [128 x D] bf16 as DB swizzled blocks
-  constexpr int P_BYTES = 32768;          // [128 x 128] bf16 as 2 swizzled blocks
-  constexpr uint32_t TMEM_COLS = (NBUF == 2) ? 512 : 256;
-  constexpr uint32_t OP_COL = NBUF * 128;  // PV tiles start after the S tiles
+constexpr int FWD128_CW = 8;                           // softmax warps of a pipeline
+constexpr int FWD128_FIRST_CW = 4;                     // warps 0, 1: TMA; 2, 3: MMAs (one each per pipeline)
+constexpr int FWD128_THREADS = 32 * (FWD128_FIRST_CW + 2 * FWD128_CW);
+
+constexpr int FWD128_TILE = 128 * 256;              // [128 x 128] bf16
+constexpr int FWD128_PIPE = 3 * FWD128_TILE;        // Q, K, V of a pipeline
+constexpr int FWD128_XCH = 2 * 2 * 2 * 128 * 4;     // [pipeline][parity][half][row] fp32
+constexpr int FWD128_SMEM = 2 * FWD128_PIPE + FWD128_XCH + 512;
+
+// head_dim 128: two independent pipelines per CTA, each with its own work items (128 query rows of one (batch, head)),
+// TMA warp, MMA warp, eight softmax warps and half of the tensor memory: S | O. What one pipeline loses
+// while it waits for its MMAs and at an item's end the other one's exponentials fill. Two warps share the 32
+// rows of a quarter, 64 of a block's 128 keys each, and exchange their row maxima through shared memory.
+// There are no columns left for P: it overwrites the scores it was made from, and the next block's scores
+// wait for its P V.
+//
+// The output accumulates in tensor memory, and the running maximum is only raised when it grows by more
+// than 2^8 (any consistent offset gives the same softmax; the stale one keeps exp2 arguments <= 8).
+// Raising it rescales the accumulator in tensor memory, which after the first blocks is rare.
+//
+// Persistent: items are dealt heaviest first in a snake (left to right, then right to left), which evens
+// out the totals; all barrier parities run on counters that continue across items.
+//
+// us, one CTA per 128 rows with P through shared memory and the output folded into registers -> this:
+// [1, 8, 4096, 128] causal 103 -> 84, [4, 2, 2048, 128] 42 -> 41. At head_dim 64, where a block's products are
+// half as long, the kernel below is the faster one (75 against 78 us at [16, 12, 1024, 64]): its two tiles share
+// the K and V loads.
+__global__ void __launch_bounds__(FWD128_THREADS, 1)
+flash_fwd128_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
+                 const __grid_constant__ CUtensorMap tv, const FwdParams p, int nb, int n_items) {
+  constexpr int D = 128, DB = D / 64, TILE = FWD128_TILE;
+  constexpr uint32_t O_COL = 128;
+  constexpr uint32_t P_HALF = 64;                   // columns from the first to the second half of P (over S)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = smem_raw;  // the launcher requests exactly the bytes used; the base must be 1024-aligned
-  uint8_t* Qs = smem;
-  uint8_t* Ks = Qs + TILE_BYTES;
-  uint8_t* Vs = Ks + 2 * TILE_BYTES;
-  uint8_t* Ps = Vs + 2 * TILE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(Ps + NBUF * P_BYTES);
-  uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;
-  uint64_t* k_empty = bars + 3;
-  uint64_t* v_full = bars + 5;
-  uint64_t* v_empty = bars + 7;
-  uint64_t* s_full = bars + 9;
-  uint64_t* s_empty = bars + 11;
-  uint64_t* p_full = bars + 13;
-  uint64_t* p_empty = bars + 15;
-  uint64_t* o_full = bars + 17;
-  uint64_t* o_empty = bars + 19;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
+  float* xch = reinterpret_cast<float*>(smem_raw + 2 * FWD128_PIPE);
+  uint64_t* bars0 = reinterpret_cast<uint64_t*>(smem_raw + 2 * FWD128_PIPE + FWD128_XCH);
+  constexpr int N_BARS = 10;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars0 + 2 * N_BARS);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  if (smem_u32(smem_raw) & 1023u) {  // swizzled tiles need a 1024-byte aligned base
-    if (threadIdx.x == 0) record_status(p.status, STATUS_BAD_ARGUMENT, 0x5a11u);
+  if (smem_u32(smem_raw) & 1023u) {
+    if (threadIdx.x == 0) record_status(p.status, STATUS_BAD_ARGUMENT, 0x5a12u);
     return;
   }
-  const int qt = gridDim.x - 1 - blockIdx.x;  // heaviest (most key blocks) first
-  const int bh = blockIdx.y;
-  const int b = bh / p.nh;
-  const int h = bh % p.nh;
-  const int n_blocks_all = (p.S + 127) >> 7;
-  const int n_kv = p.causal ? min(qt + 1, n_blocks_all) : n_blocks_all;
+  const int BH = p.B * p.nh;
+  const int x = warp < FWD128_FIRST_CW ? (warp & 1) : (warp - FWD128_FIRST_CW) / FWD128_CW;   // this warp's pipeline
+  uint8_t* Qs = smem_raw + x * FWD128_PIPE;   // [128 x D], 64-column blocks
+  uint8_t* Ks = Qs + TILE;
+  uint8_t* Vs = Ks + TILE;
+  uint64_t* q_full = bars0 + x * N_BARS;
+  uint64_t* q_empty = q_full + 1;
+  uint64_t* k_full = q_full + 2;
+  uint64_t* k_empty = q_full + 3;
+  uint64_t* v_full = q_full + 4;
+  uint64_t* v_empty = q_full + 5;
+  uint64_t* s_full = q_full + 6;
+  uint64_t* o_full = q_full + 7;
+  uint64_t* p_full = q_full + 8;
+  uint64_t* o_empty = q_full + 9;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
-      mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], 4);
-      mbar_init(&p_full[i], 4);
-      mbar_init(&p_empty[i], 1);
-      mbar_init(&o_full[i], 1);
-      mbar_init(&o_empty[i], 4);
+    for (int pipe = 0; pipe < 2; ++pipe) {
+      uint64_t* b = bars0 + pipe * N_BARS;
+      for (int i = 0; i < N_BARS; ++i) mbar_init(&b[i], i < 8 ? 1 : FWD128_CW);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -244,8 +230,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     tma_prefetch_desc(&tk);
     tma_prefetch_desc(&tv);
   }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
+  if (warp == 2) {
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -253,216 +239,246 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   tc_fence_after();
   pdl_wait();       // set-up above may overlap the tail of the preceding kernel (programmatic launch)
   pdl_trigger();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = *tmem_slot + x * 256;
   WaitCtx wctx{abort_flag, p.status, GFS_WAIT_LIMIT_NS};
 
-  if (warp == 0) {
+  // pipeline 1 of a CTA comes after pipeline 0 of all CTAs: with few items every SM has one
+  const int W = 2 * static_cast<int>(gridDim.x);
+  const int wk = x * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
+  auto snake = [&](int rnd) { return rnd * W + ((rnd & 1) ? W - 1 - wk : wk); };
+  // query tile, batch * head and number of key blocks (at least one) of work item w
+  auto decode = [&](int w, int& qt, int& bh, int& n) {
+    qt = nb - 1 - w / BH;
+    bh = w % BH;
+    n = p.causal ? qt + 1 : nb;
+  };
+
+  if (warp < 2) {
     if (lane == 0) {
-      mbar_arrive_expect_tx(q_full, TILE_BYTES);
+      // in the order of the MMAs: K of block g + 1, then V of block g
+      auto load = [&](uint8_t* dst, const CUtensorMap& map, uint64_t* full, uint64_t* empty, int n_loaded, int row,
+                      int bh) {
+        mbar_wait(empty, (n_loaded & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
+        mbar_arrive_expect_tx(full, TILE);
 #pragma unroll
-      for (int db = 0; db < DB; ++db) tma_load_4d(Qs + db * 16384, &tq, q_full, db * 64, qt * 128, h, b);
-      for (int j = 0; j < n_kv; ++j) {
-        const int st = j & 1;
-        const uint32_t par = ((j >> 1) & 1) ^ 1u;
-        mbar_wait(&k_empty[st], par, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
-        mbar_arrive_expect_tx(&k_full[st], TILE_BYTES);
-#pragma unroll
-        for (int db = 0; db < DB; ++db)
-          tma_load_4d(Ks + st * TILE_BYTES + db * 16384, &tk, &k_full[st], db * 64, j * 128, h, b);
-        mbar_wait(&v_empty[st], par, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
-        mbar_arrive_expect_tx(&v_full[st], TILE_BYTES);
-#pragma unroll
-        for (int db = 0; db < DB; ++db)
-          tma_load_4d(Vs + st * TILE_BYTES + db * 16384, &tv, &v_full[st], db * 64, j * 128, h, b);
+        for (int db = 0; db < DB; ++db)    // rows past S: zeros
+          tma_load_4d(dst + db * 16384, &map, full, db * 64, row, bh % p.nh, bh / p.nh);
+      };
+      int v_prev = -1, bh_prev = 0;        // the V block that is still to be loaded
+      int gk = 0, gv = 0;
+      for (int rnd = 0; rnd * W < n_items; ++rnd) {
+        const int w = snake(rnd);
+        if (w >= n_items) break;
+        int qt, bh, n;
+        decode(w, qt, bh, n);
+        for (int j = 0; j < n; ++j) {
+          if (j == 0) load(Qs, tq, q_full, q_empty, rnd, qt * 128, bh);
+          load(Ks, tk, k_full, k_empty, gk++, j * 128, bh);
+          if (v_prev >= 0) load(Vs, tv, v_full, v_empty, gv++, v_prev * 128, bh_prev);
+          v_prev = j;
+          bh_prev = bh;
+        }
       }
+      if (v_prev >= 0) load(Vs, tv, v_full, v_empty, gv++, v_prev * 128, bh_prev);
       if (*abort_flag) {
         for (int i = 0; i < 64; ++i) __nanosleep(1000);
       }
     }
-  } else if (warp == 1) {
-    {  // whole warp, converged: the MMA / commit helpers elect the issuing lane
-      constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
-      constexpr uint32_t idesc_o = umma_idesc_bf16(128, D, 0, 1);
-      const uint32_t q_addr = smem_u32(Qs);
-      mbar_wait(q_full, 0, wctx, STATUS_TIMEOUT_PIPE_FULL);
-      auto issue_s = [&](int j) {
-        const int st = j & 1;                       // K/V stage
-        const uint32_t par = (j >> 1) & 1;
-        const int sb = (NBUF == 2) ? (j & 1) : 0;   // S / P / PV buffer
-        const uint32_t spar = (NBUF == 2) ? ((j >> 1) & 1) : (j & 1);
-        mbar_wait(&k_full[st], par, wctx, STATUS_TIMEOUT_PIPE_FULL);
-        mbar_wait(&s_empty[sb], spar ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
+  } else if (warp < FWD128_FIRST_CW) {
+    // whole warp, converged: the MMA / commit helpers elect the issuing lane. The blocks of all items are one
+    // sequence g = 0, 1, ...: P V of block g, then, when it has read P, the scores of block g + 1.
+    constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
+    constexpr uint32_t idesc_o = umma_idesc_bf16(128, D, 0, 1);
+    int s_rnd = 0, s_j = 0, s_n = 0, s_g = 0;     // next block whose scores are issued
+    auto open_item = [&]() {
+      s_n = 0;
+      s_j = 0;
+      if (s_rnd * W < n_items) {
+        const int w = snake(s_rnd);
+        int qt, bh;
+        if (w < n_items) decode(w, qt, bh, s_n);
+      }
+    };
+    open_item();
+    auto issue_s = [&]() {
+      if (s_n == 0) return;
+      if (s_j == 0) mbar_wait(q_full, s_rnd & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+      mbar_wait(k_full, s_g & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+      tc_fence_after();
+      mma_kk<D / 16>(tmem_base, smem_u32(Qs), 16384, smem_u32(Ks), 16384, idesc_s, false);
+      umma_commit_e(s_full);
+      umma_commit_e(k_empty);
+      ++s_g;
+      if (++s_j == s_n) {
+        umma_commit_e(q_empty);
+        ++s_rnd;
+        open_item();
+      }
+    };
+    issue_s();
+    int g = 0;
+    for (int rnd = 0; rnd * W < n_items; ++rnd) {
+      const int w = snake(rnd);
+      if (w >= n_items) break;
+      int qt, bh, n;
+      decode(w, qt, bh, n);
+      for (int j = 0; j < n; ++j, ++g) {
+        mbar_wait(v_full, g & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+        mbar_wait(p_full, g & 1, wctx, STATUS_TIMEOUT_SOFTMAX);
+        // the accumulator is overwritten once per item: the previous item's result has been read out of it
+        if (j == 0) mbar_wait(o_empty, (rnd & 1) ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
         tc_fence_after();
-        mma_kk<D / 16>(tmem_base + sb * 128, q_addr, 16384, smem_u32(Ks + st * TILE_BYTES), 16384, idesc_s, false);
-        umma_commit_e(&s_full[sb]);
-        umma_commit_e(&k_empty[st]);
-      };
-      issue_s(0);
-      for (int j = 0; j < n_kv; ++j) {
-        if (j + 1 < n_kv) issue_s(j + 1);
-        const int st = j & 1;
-        const uint32_t par = (j >> 1) & 1;
-        const int sb = (NBUF == 2) ? (j & 1) : 0;
-        const uint32_t spar = (NBUF == 2) ? ((j >> 1) & 1) : (j & 1);
-        mbar_wait(&p_full[sb], spar, wctx, STATUS_TIMEOUT_SOFTMAX);
-        mbar_wait(&v_full[st], par, wctx, STATUS_TIMEOUT_PIPE_FULL);
-        mbar_wait(&o_empty[sb], spar ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
-        tc_fence_after();
-        mma_kmn<8>(tmem_base + OP_COL + sb * D, smem_u32(Ps + sb * P_BYTES), 16384, smem_u32(Vs + st * TILE_BYTES),
-                   16384, idesc_o, false);
-        umma_commit_e(&o_full[sb]);
-        umma_commit_e(&v_empty[st]);
-        umma_commit_e(&p_empty[sb]);
+        mma_tmn<8, P_HALF>(tmem_base + O_COL, tmem_base, smem_u32(Vs), 16384, idesc_o, j > 0);
+        umma_commit_e(o_full);
+        umma_commit_e(v_empty);
+        if (s_n > 0) mbar_wait(o_full, g & 1, wctx, STATUS_TIMEOUT_TMEM_FULL);
+        issue_s();
       }
     }
   } else {
+    const int half = ((warp - FWD128_FIRST_CW) >> 2) & 1;   // keys [64 half, + 64) of every block
     const int quarter = warp & 3;
-    const int r = quarter * 32 + lane;       // row inside the query tile
-    const int row_g = qt * 128 + r;          // query position
+    const int r = quarter * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t s_addr = tmem_base + lane_base + half * 64;
+    const uint32_t o_addr = tmem_base + lane_base + O_COL + half * (D / 2);
+    const uint32_t p_addr = tmem_base + lane_base + half * P_HALF;
+    const int bar_id = 1 + x * 4 + quarter;              // the two warps that share these rows
+    float* const xch_own = xch + x * 512 + half * 128 + r;          // + 256 * parity
+    const float* const xch_other = xch + x * 512 + (half ^ 1) * 128 + r;
     const float sl2 = p.scale * LOG2E_F;
-    float m = -INFINITY, l = 0.f, alpha_prev = 0.f;
-    float o[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) o[i] = 0.f;
-
-    auto fold_pv = [&](int j, float alpha) {
-      const int st = (NBUF == 2) ? (j & 1) : 0;
-      mbar_wait(&o_full[st], (NBUF == 2) ? ((j >> 1) & 1) : (j & 1), wctx, STATUS_TIMEOUT_SOFTMAX);
-      tc_fence_after();
-      const uint32_t o_addr = tmem_base + lane_base + OP_COL + st * D;
-      uint32_t wa[32], wb[32];
-      tmem_ld_32x32(o_addr, wa);
-#pragma unroll
-      for (int c = 0; c < D; c += 64) {
-        tmem_ld_wait_for(wa);
-        tmem_ld_32x32(o_addr + c + 32, wb);
-#pragma unroll
-        for (int e = 0; e < 32; ++e) o[c + e] = fmaf(o[c + e], alpha, __uint_as_float(wa[e]));
-        tmem_ld_wait_for(wb);
-        if (c + 64 < D) tmem_ld_32x32(o_addr + c + 64, wa);
-#pragma unroll
-        for (int e = 0; e < 32; ++e) o[c + 32 + e] = fmaf(o[c + 32 + e], alpha, __uint_as_float(wb[e]));
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&o_empty[st]);
+    const uint64_t sl2_2 = pack_f32x2(sl2, sl2);
+    int g = 0;
+    uint32_t xpar = 0;                                   // parity of the exchange buffer
+    auto exchange = [&](float v) {
+      xch_own[xpar * 256] = v;
+      named_barrier_sync(bar_id, 64);
+      const float o = xch_other[xpar * 256];
+      xpar ^= 1u;
+      return o;
     };
-
-    for (int j = 0; j < n_kv; ++j) {
-      const int st = (NBUF == 2) ? (j & 1) : 0;
-      const uint32_t par = (NBUF == 2) ? ((j >> 1) & 1) : (j & 1);
-      const bool need_mask = (p.causal && j == qt) || ((j + 1) * 128 > p.S);
-      mbar_wait(&s_full[st], par, wctx, STATUS_TIMEOUT_SOFTMAX);
-      tc_fence_after();
-      const uint32_t s_addr = tmem_base + lane_base + st * 128;
-      // pass 1: row maximum (TMEM loads double buffered against the arithmetic)
-      float mx = -INFINITY;
-      uint32_t va[32], vb[32];
-      // Diagonal / tail block: dead scores become -inf in the registers and the block runs the same
-      // max / exponential code as every other block (a separate masked copy of that code executes
-      // once per CTA from a cold instruction cache and cost more than two unmasked blocks).
-      auto mask_chunk = [&](uint32_t (&v)[32], int c) {
+    for (int rnd = 0; rnd * W < n_items; ++rnd) {
+      const int w = snake(rnd);
+      if (w >= n_items) break;
+      int qt, bh, n;
+      decode(w, qt, bh, n);
+      const int b = bh / p.nh, h = bh % p.nh;
+      const int row_g = qt * 128 + r;
+      float m = -INFINITY;
+      uint64_t l2 = 0;                                   // two partial sums of this thread's exponentials
+      for (int j = 0; j < n; ++j, ++g) {
+        const int col0 = j * 128 + half * 64;
+        const bool need_mask = (p.causal && j == qt) || ((j + 1) * 128 > p.S);
+        mbar_wait(s_full, g & 1, wctx, STATUS_TIMEOUT_SOFTMAX);
+        tc_fence_after();
+        uint32_t v[2][32];
+        float mx0 = -INFINITY, mx1 = -INFINITY;
+        tmem_ld_32x32(s_addr, v[0]);
+        tmem_ld_32x32(s_addr + 32, v[1]);
+        tmem_ld_wait_for(v[0]);
+        tmem_ld_wait_for(v[1]);
         if (need_mask) {
-          const int lim_c = p.causal ? row_g - j * 128 - c : 0x7fffffff;   // last live column of the chunk
-          const int lim = min(lim_c, p.S - 1 - j * 128 - c);
+          // Diagonal block (causal) or the block that crosses the end of the sequence: dead scores
+          // become -inf in the registers, then the block takes the same code as every other one
+          // (exp2(-inf) = 0, max ignores -inf).
+          const int lim = min(p.causal ? row_g - col0 : 0x7fffffff, p.S - 1 - col0);   // last live column
 #pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] = (e > lim) ? 0xff800000u : v[e];
+          for (int e = 0; e < 64; ++e) v[e >> 5][e & 31] = (e > lim) ? 0xff800000u : v[e >> 5][e & 31];
         }
-      };
-      auto max_chunk = [&](uint32_t (&v)[32], int c) {
-        mask_chunk(v, c);
-#pragma unroll
-        for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(v[e]));
-      };
-      tmem_ld_32x32(s_addr + 0, va);
-      tmem_ld_wait_for(va);
-      tmem_ld_32x32(s_addr + 32, vb);
-      max_chunk(va, 0);
-      tmem_ld_wait_for(vb);
-      tmem_ld_32x32(s_addr + 64, va);
-      max_chunk(vb, 32);
-      tmem_ld_wait_for(va);
-      tmem_ld_32x32(s_addr + 96, vb);
-      max_chunk(va, 64);
-      tmem_ld_wait_for(vb);
-      tmem_ld_32x32(s_addr + 0, va);  // first chunk of pass 2
-      max_chunk(vb, 96);
-      const float m_new = fmaxf(m, mx);
-      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;  // row with no live key so far
-      const float alpha = fast_exp2((m - m_use) * sl2);
-      const float moff = m_use * sl2;
-      mbar_wait(&p_empty[st], par ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
-      // pass 2: probabilities -> shared memory (bf16, swizzled K-major), row sum
-      float rs = 0.f;
-      uint8_t* prow = Ps + st * P_BYTES + r * 128;
-      auto prob_chunk = [&](uint32_t (&v)[32], int c) {
-        mask_chunk(v, c);
-        uint32_t packed[16];
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
-          const float x0 = fast_exp2(fmaf(__uint_as_float(v[e]), sl2, -moff));
-          const float x1 = fast_exp2(fmaf(__uint_as_float(v[e + 1]), sl2, -moff));
-          rs += x0 + x1;
-          packed[e >> 1] = pack_bf16x2(x0, x1);
+          mx0 = fmax3(mx0, __uint_as_float(v[0][e]), __uint_as_float(v[0][e + 1]));
+          mx1 = fmax3(mx1, __uint_as_float(v[1][e]), __uint_as_float(v[1][e + 1]));
         }
-        uint8_t* blk = prow + (c >> 6) * 16384;
-        const int chunk0 = (c & 63) >> 3;
+        const float mx = fmaxf(mx0, mx1);
+        const float m_new = fmax3(m, mx, exchange(mx));
+        // raise the running maximum only when it grew by more than 2^8 (or was still -inf); both threads of
+        // a row decide alike
+        bool grow = false;
+        float alpha = 1.f;
+        if (m_new > m && (m == -INFINITY || (m_new - m) * sl2 > 8.f)) {
+          grow = true;
+          alpha = (m == -INFINITY) ? 0.f : fast_exp2((m - m_new) * sl2);
+        }
+        if (j > 0 && __any_sync(0xffffffffu, grow)) {
+          // rescale this warp's 32 accumulator rows in tensor memory (warp-collective accesses; rows whose
+          // maximum stays get factor 1), its half of the columns. P V of the previous block must be done.
+          mbar_wait(o_full, (g - 1) & 1, wctx, STATUS_TIMEOUT_SOFTMAX);
+          tc_fence_after();
+#pragma unroll 1
+          for (int cc = 0; cc < D / 2; cc += 16) {
+            uint32_t wv[16];
+            tmem_ld_32x16(o_addr + cc, wv);
+            tmem_ld_wait_for16(wv);
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const uint4 w = make_uint4(packed[4 * q4], packed[4 * q4 + 1], packed[4 * q4 + 2], packed[4 * q4 + 3]);
-          *reinterpret_cast<uint4*>(blk + ((((chunk0 + q4) ^ (r & 7)) & 7) << 4)) = w;
+            for (int e = 0; e < 16; ++e) wv[e] = __float_as_uint(__uint_as_float(wv[e]) * alpha);
+            tmem_st_32x16(o_addr + cc, wv);
+          }
+          tmem_st_wait();
         }
-      };
-      tmem_ld_wait_for(va);
-      tmem_ld_32x32(s_addr + 32, vb);
-      prob_chunk(va, 0);
-      tmem_ld_wait_for(vb);
-      tmem_ld_32x32(s_addr + 64, va);
-      prob_chunk(vb, 32);
-      tmem_ld_wait_for(va);
-      tmem_ld_32x32(s_addr + 96, vb);
-      prob_chunk(va, 64);
-      tmem_ld_wait_for(vb);
-      prob_chunk(vb, 96);
-      l = l * alpha + rs;
-      m = m_new;
+        if (grow) {
+          l2 = mul_f32x2(l2, pack_f32x2(alpha, alpha));
+          m = m_new;
+        }
+        const float moff = ((m == -INFINITY) ? 0.f : m) * sl2;
+        const uint64_t moff2 = pack_f32x2(-moff, -moff);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            const float2 a = unpack_f32x2(fma_f32x2(pack_u32x2(v[c][e], v[c][e + 1]), sl2_2, moff2));
+            const float p0 = fast_exp2(a.x), p1 = fast_exp2(a.y);
+            l2 = add_f32x2(l2, pack_f32x2(p0, p1));
+            pk[e >> 1] = pack_bf16x2(p0, p1);
+          }
+          tmem_st_32x16(p_addr + 16 * c, pk);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      }
+      const float2 lp = unpack_f32x2(l2);
+      float l = lp.x + lp.y;
+      l += exchange(l);
+      const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
+      mbar_wait(o_full, (g - 1) & 1, wctx, STATUS_TIMEOUT_SOFTMAX);
+      tc_fence_after();
+      __nv_bfloat16* dst = p.O + row_g * p.o_ss + b * p.o_bs + h * p.o_hs + half * (D / 2);
+      uint32_t o[D / 64][32];
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) tmem_ld_32x32(o_addr + 32 * c, o[c]);
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) tmem_ld_wait_for(o[c]);
       tc_fence_before();
-      fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&s_empty[st]);
-        mbar_arrive(&p_full[st]);
-      }
-      if (j > 0) fold_pv(j - 1, alpha_prev);
-      alpha_prev = alpha;
-    }
-    fold_pv(n_kv - 1, alpha_prev);
-
-    const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
-    {
-      // every P V MMA has completed (the last fold waited for it): the P buffer serves as staging
-      uint8_t* stage = Ps + (r >> 5) * 4096;
-      const int row0 = row_g - lane;
-      __nv_bfloat16* g0 = p.O + row0 * p.o_ss + b * p.o_bs + h * p.o_hs;
+      if (lane == 0) mbar_arrive(o_empty);   // the next item's first P V may overwrite the accumulator
+      if (row_g < p.S) {
 #pragma unroll
-      for (int hf = 0; hf < D / 64; ++hf) {
-        uint32_t ow[32];
+        for (int c = 0; c < D / 64; ++c) {
 #pragma unroll
-        for (int e = 0; e < 32; ++e) ow[e] = pack_out(o[hf * 64 + 2 * e] * inv_l, o[hf * 64 + 2 * e + 1] * inv_l, p.o_f16);
-        store_rows_32x64(stage, ow, lane, g0 + hf * 64, p.o_ss, p.S - row0);
+          for (int e = 0; e < 32; e += 8) {
+            uint4 wv;
+            wv.x = pack_out(__uint_as_float(o[c][e + 0]) * inv_l, __uint_as_float(o[c][e + 1]) * inv_l, p.o_f16);
+            wv.y = pack_out(__uint_as_float(o[c][e + 2]) * inv_l, __uint_as_float(o[c][e + 3]) * inv_l, p.o_f16);
+            wv.z = pack_out(__uint_as_float(o[c][e + 4]) * inv_l, __uint_as_float(o[c][e + 5]) * inv_l, p.o_f16);
+            wv.w = pack_out(__uint_as_float(o[c][e + 6]) * inv_l, __uint_as_float(o[c][e + 7]) * inv_l, p.o_f16);
+            *reinterpret_cast<uint4*>(dst + 32 * c + e) = wv;
+          }
+        }
       }
-    }
-    if (row_g < p.S_pad) {
-      const float mm = (m == -INFINITY) ? 0.f : m;
-      p.lse[static_cast<size_t>(bh) * p.S_pad + row_g] = mm * sl2 + log2f(fmaxf(l, 1e-37f));
+      if (half == 0 && row_g < p.S_pad) {
+        const float mm = (m == -INFINITY) ? 0.f : m;
+        p.lse[static_cast<size_t>(bh) * p.S_pad + row_g] = mm * sl2 + log2f(fmaxf(l, 1e-37f));
+      }
     }
   }
 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+  if (warp == 2) tmem_dealloc(*tmem_slot, 512);
 }
 
 // ---------------------------------------------------------------------------
@@ -1485,22 +1501,21 @@ int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* ls
   p.S = S; p.S_pad = ((S + 127) / 128) * 128; p.B = B; p.nh = nh;
   p.scale = scale; p.causal = causal; p.o_f16 = o_f16;
   p.status = gfs_host::status_words();
-  const dim3 grid((S + 127) / 128, B * nh);
+  const int nb = (S + 127) / 128;
   static bool set64 = false, set128 = false;
   if (D == 64) {
-    if (!set64) {
-      if (set_smem(flash_fwd64_kernel, FWD64_SMEM)) return -10;
-      set64 = true;
-    }
-    const int n_pairs = (static_cast<int>(grid.x) + 1) / 2;
+    if (!set64) { if (set_smem(flash_fwd64_kernel, FWD64_SMEM)) return -10; set64 = true; }
+    const int n_pairs = (nb + 1) / 2;
     const int n_items = n_pairs * B * nh;
     const int ctas = std::min(n_items, gfs_host::sm_count());
     gfs_host::launch_pdl(flash_fwd64_kernel, dim3(ctas), dim3(FWD64_THREADS), FWD64_SMEM, stream, *tq, *tk, *tv, p,
                          n_pairs, n_items);
   } else {
-    const int smem = 32768 * 5 + 2 * 32768 + 256;
-    if (!set128) { if (set_smem(flash_fwd_kernel<128, 2>, smem)) return -10; set128 = true; }
-    gfs_host::launch_pdl(flash_fwd_kernel<128, 2>, grid, dim3(ATT_THREADS), smem, stream, *tq, *tk, *tv, p);
+    if (!set128) { if (set_smem(flash_fwd128_kernel, FWD128_SMEM)) return -10; set128 = true; }
+    const int n_items = nb * B * nh;
+    const int ctas = std::min(n_items, gfs_host::sm_count());
+    gfs_host::launch_pdl(flash_fwd128_kernel, dim3(ctas), dim3(FWD128_THREADS), FWD128_SMEM, stream, *tq, *tk, *tv, p, nb,
+                         n_items);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
