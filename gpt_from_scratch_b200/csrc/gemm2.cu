@@ -63,6 +63,20 @@ constexpr int EPI_BYTES = 8 * 4096;     // one [32 rows x 128 B] transpose buffe
 __host__ __device__ constexpr int epi_warps(int comm) { return 8 + 0 * comm; }
 __host__ __device__ constexpr int threads2(int comm) { return 64 + 32 * epi_warps(comm) + (comm != 0 ? 64 : 0); }
 constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + 256 + 1024;
+// SWI == 4: the SwiGLU backward epilogue reads gate | up and writes their gradients with TMA, through two
+// [gate | up] slots of [32 rows x 64 columns] each per warp, paid for with half of the ring's stages. With a short K
+// loop what bounds that product is the 512 KB that a tile reads and writes there: loads by the epilogue's own threads
+// leave their latency (once per 64 columns) and the transposes exposed. With a long one the ring counts more.
+// us, loads by the threads -> TMA, [16384, K] x [K, 3072]: K 256 127 -> 109, 768 133 -> 121, 1024 139 -> 137,
+// 1280 141 -> 154, 2048 159 -> 209; [8192, K] x [K, 5632]: 512 121 -> 104, 1024 127 -> 127, 1536 133 -> 162.
+// (The forward's epilogue only writes; the same scheme there, with four ring stages, took 161 us instead of 151.)
+constexpr int SWI_TMA_MAX_K = 1024;
+__host__ __device__ constexpr bool epi_tma(int comm, int swi) { return comm == COMM_NONE && swi == 4; }
+__host__ __device__ constexpr int stages2(int comm, int swi) { return epi_tma(comm, swi) ? 3 : STAGES; }
+__host__ __device__ constexpr int epi_bytes2(int comm, int swi) { return epi_tma(comm, swi) ? 8 * 16384 : EPI_BYTES; }
+__host__ __device__ constexpr int smem2(int comm, int swi) {
+  return stages2(comm, swi) * STAGE_BYTES + epi_bytes2(comm, swi) + 512 + 1024;
+}
 
 struct Params2 {
   int M, N, K;
@@ -83,6 +97,7 @@ struct Params2 {
   int swi_I, swi_ld;
   __nv_bfloat16* swi_act;
   const __nv_bfloat16* swi_gu;
+  // SWI == 4: as 2, gate | up and their gradients through shared memory with TMA.
   // SWI == 3 (LM head): besides storing the logits, every epilogue warp writes the online-softmax
   // statistics (max, sum exp(x - max)) of its 128 columns of each row, computed from the
   // bf16-rounded logits: ce_partials[(tile_n * 2 + column half) * M + row]. A small kernel
@@ -197,7 +212,11 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_addr) {
 template <bool A_MN, bool B_MN, int COMM, int SWI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads2(COMM), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-             const __grid_constant__ CUtensorMap tmap_a_local, const Params2 p) {
+             const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y, const Params2 p) {
+  // tmap_x, tmap_y: all-gather: the local shard of A, unused; EPI_TMA: gate | up, d_gate | d_up
+  constexpr bool EPI_TMA = epi_tma(COMM, SWI);
+  constexpr int STAGES = stages2(COMM, SWI);
+  constexpr int EPI_BYTES = epi_bytes2(COMM, SWI);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* tiles = smem;
@@ -210,6 +229,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
   uint32_t* rs_sent = tmem_slot + 2;   // [MAX_PEERS] reduce-scatter: (warp, tile) units stored for each peer
+  uint64_t* epi_full = reinterpret_cast<uint64_t*>(rs_sent + MAX_PEERS);   // [8 warps][2 slots], EPI_TMA
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -228,11 +248,16 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       mbar_init(&tmem_full[b], 1);
       mbar_init(&tmem_empty[b], 2 * epi_warps(COMM));
     }
+    if (EPI_TMA) {
+      for (int i = 0; i < 16; ++i) mbar_init(&epi_full[i], 1);
+      tma_prefetch_desc(&tmap_x);
+      tma_prefetch_desc(&tmap_y);
+    }
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
-    if (COMM == COMM_ALLGATHER) tma_prefetch_desc(&tmap_a_local);
+    if (COMM == COMM_ALLGATHER) tma_prefetch_desc(&tmap_x);
   }
   __syncthreads();
   if (warp == 1) {
@@ -268,7 +293,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         decode_tile2<COMM>(p, t, m0, n0, chunk);
         m0 += static_cast<int>(rank) * BM;
         n0 += static_cast<int>(rank) * BNH;
-        // all-gather: this rank's own chunk is read straight from its shard (tmap_a_local), so the
+        // all-gather: this rank's own chunk is read straight from its shard (tmap_x), so the
         // first tiles start at once; only the peers' chunks wait for their arrival in the gathered buffer
         const bool local_chunk = (COMM == COMM_ALLGATHER) && chunk == p.comm.rank;
         if (COMM == COMM_ALLGATHER && !local_chunk && !((chunk_ready >> chunk) & 1u)) {
@@ -290,7 +315,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           const uint32_t bar = mapa_u32(smem_u32(&full_bar[stage]), 0);
           const int k0 = kb * BK;
           if (!A_MN) {
-            if (local_chunk) tma_load_2d_pair(sa, &tmap_a_local, bar, k0, m0 - chunk * p.comm.rows_per_rank);
+            if (local_chunk) tma_load_2d_pair(sa, &tmap_x, bar, k0, m0 - chunk * p.comm.rows_per_rank);
             else tma_load_2d_pair(sa, &tmap_a, bar, k0, m0);
           } else {
 #pragma unroll
@@ -376,7 +401,34 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     uint8_t* ebuf = epi_smem + (warp - 2) * 4096;
     const int rrow = lane >> 3;
     const int rch = lane & 7;
-    const bool has_add = (p.R != nullptr);
+    const bool has_add = !EPI_TMA && (p.R != nullptr);
+    // EPI_TMA: this warp's slots, and the loads of gate | up, one 64-column chunk ahead of the math
+    uint8_t* const slots = epi_smem + (warp - 2) * (EPI_BYTES / 8);
+    uint32_t n_chunk = 0;                   // chunks this warp has worked through (slot = parity)
+    int pf_t = pair, pf_c = c_begin - 64;   // the last chunk asked for
+    auto prefetch_chunk = [&](uint32_t n) { // the next chunk with anything in range, as the warp's n-th
+      while (true) {
+        pf_c += 64;
+        if (pf_c >= c_begin + BN / 2) {
+          pf_c = c_begin;
+          pf_t += num_pairs;
+        }
+        if (pf_t >= total_tiles) return;
+        const int row0 = (pf_t / p.tiles_n) * 256 + static_cast<int>(rank) * BM + q * 32;
+        const int col0 = (pf_t % p.tiles_n) * BN + pf_c;
+        if (row0 >= p.M || col0 >= p.N) continue;
+        if (lane == 0) {
+          uint64_t* bar = &epi_full[(warp - 2) * 2 + (n & 1)];
+          uint8_t* slot = slots + (n & 1) * 8192;
+          bulk_wait_read_all();             // the slot's previous results have left it
+          mbar_arrive_expect_tx(bar, 8192);
+          tma_load_3d(slot, &tmap_x, bar, col0, 0, row0);
+          tma_load_3d(slot + 4096, &tmap_x, bar, col0, 1, row0);
+        }
+        return;
+      }
+    };
+    if (EPI_TMA) prefetch_chunk(0);
     // The addend of a 64-column chunk is fetched one chunk ahead (across tile boundaries too), so
     // its global-memory latency is covered by the previous chunk's work instead of stalling this one.
     uint4 pre[8];
@@ -403,7 +455,57 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       if (t == pair && warp == 2 && lane == 0) trace_stamp(p, TRACE_EPI_BEGIN);
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-      if (SWI == 1) {
+      if (EPI_TMA) {
+        // A thread owns a row: the tiles' 16-byte chunks are swizzled (128-byte rows), so its accesses are free of
+        // bank conflicts, and rows and columns past the end are clipped by the tensor maps. gate | up are
+        // [row][half][column] to the maps, so the last gate columns cannot run into up.
+        const int row0 = m0 + q * 32;
+        const uint32_t sw = lane & 7;
+#pragma unroll 1
+        for (int c = c_begin; c < c_begin + BN / 2; c += 64) {
+          const int col0 = n0 + c;
+          if (row0 >= p.M || col0 >= p.N) break;
+          uint8_t* slot = slots + (n_chunk & 1) * 8192;
+          uint8_t* row = slot + lane * 128;
+          mbar_wait(&epi_full[(warp - 2) * 2 + (n_chunk & 1)], (n_chunk >> 1) & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+          ++n_chunk;
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
+            uint32_t vd[32];
+            tmem_ld_32x32(t_row + c + 32 * h, vd);
+            // half way, when the previous chunk's results will have left the slot that the next one takes
+            if (h == 1) prefetch_chunk(n_chunk);
+            __syncwarp();
+            tmem_ld_wait_for(vd);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint8_t* at = row + (((4 * h + j) ^ sw) << 4);
+              uint4 g4 = *reinterpret_cast<const uint4*>(at), u4 = *reinterpret_cast<const uint4*>(at + 4096);
+              uint32_t *gp = &g4.x, *up = &u4.x;
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                // d_act rounded to bf16, as when it is a tensor of its own
+                const float2 d2 = unpack_bf16x2(
+                    pack_bf16x2(__uint_as_float(vd[8 * j + 2 * e]), __uint_as_float(vd[8 * j + 2 * e + 1])));
+                const float2 g2 = unpack_bf16x2(gp[e]), u2 = unpack_bf16x2(up[e]);
+                const float sg0 = sigmoid_f(g2.x), sg1 = sigmoid_f(g2.y);
+                gp[e] = pack_bf16x2(d2.x * u2.x * sg0 * (1.f + g2.x * (1.f - sg0)),
+                                    d2.y * u2.y * sg1 * (1.f + g2.y * (1.f - sg1)));
+                up[e] = pack_bf16x2(d2.x * g2.x * sg0, d2.y * g2.y * sg1);
+              }
+              *reinterpret_cast<uint4*>(at) = g4;
+              *reinterpret_cast<uint4*>(at + 4096) = u4;
+            }
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&tmap_y, slot, col0, 0, row0);
+            tma_store_3d(&tmap_y, slot + 4096, col0, 1, row0);
+            bulk_commit();
+          }
+        }
+      } else if (SWI == 1) {
         // accumulator columns [0,128) are gate, [128,256) the matching up columns
         const int g0 = n0 >> 1;  // first gate column of the tile
         const int sc_begin = (EW == 8) ? ((warp - 2) >> 2) * 64 : 0;
@@ -664,6 +766,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         acc_phase ^= 1u;
       }
     }
+    if (EPI_TMA && lane == 0) bulk_wait_all();
     if (COMM == COMM_REDUCE_SCATTER) {
       if (!rs_handed_over) named_barrier_arrive(2, 32 * EW + COMM_THREADS);   // CTAs without local tiles
       // tiles done: join the reduction of this rank's row chunk (second share of the vectors)
@@ -969,22 +1072,23 @@ static unsigned long long* g_trace = nullptr;
 
 template <bool A_MN, bool B_MN, int COMM = COMM_NONE, int SWI = 0>
 int launch2(const CUtensorMap* ta, const CUtensorMap* tb, const Params2& p, int grid, cudaStream_t stream,
-            const CUtensorMap* ta_local = nullptr) {
+            const CUtensorMap* tx = nullptr, const CUtensorMap* ty = nullptr) {
   auto kern = gemm2_kernel<A_MN, B_MN, COMM, SWI>;
+  constexpr int smem = smem2(COMM, SWI);
   static bool attr_set = false;
   static int attr_dev = -1;
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set || attr_dev != dev) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL) != cudaSuccess)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return -10;
     attr_set = true;
     attr_dev = dev;
   }
   Params2 pt = p;
   pt.trace = g_trace;
-  if (gfs_host::launch_pdl(kern, dim3(grid), dim3(threads2(COMM)), SMEM_TOTAL, stream, *ta, *tb,
-                           ta_local ? *ta_local : *ta, pt) != cudaSuccess)
+  if (gfs_host::launch_pdl(kern, dim3(grid), dim3(threads2(COMM)), smem, stream, *ta, *tb, tx ? *tx : *ta,
+                           ty ? *ty : *ta, pt) != cudaSuccess)
     return -11;
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
@@ -1100,8 +1204,19 @@ int gfs_gemm2_bf16_swiglu(int mode, const void* a, const void* b, void* c, void*
                                       : gfs_host::tmap_2d_cached(b, K, I, ldb, 64, 64);
   if (ta == nullptr || tb == nullptr) return -3;
   const int pairs = std::min(p.tiles_m * p.tiles_n, gfs_host::sm_count() / 2);
-  return (mode == 1) ? launch2<false, false, COMM_NONE, 1>(ta, tb, p, 2 * pairs, stream)
-                     : launch2<false, true, COMM_NONE, 2>(ta, tb, p, 2 * pairs, stream);
+  if (mode == 1) return launch2<false, false, COMM_NONE, 1>(ta, tb, p, 2 * pairs, stream);
+  if (K > SWI_TMA_MAX_K) return launch2<false, true, COMM_NONE, 2>(ta, tb, p, 2 * pairs, stream);
+  // gate | up as [row][half][column], in boxes of one warp's 32 rows x 64 columns
+  auto epi_map = [&](const void* base, int ld) {
+    const uint64_t dims[3] = {static_cast<uint64_t>(I), 2, static_cast<uint64_t>(M)};
+    const uint64_t strides[3] = {2, static_cast<uint64_t>(I) * 2, static_cast<uint64_t>(ld) * 2};
+    const uint32_t box[3] = {64, 1, 32};
+    return gfs_host::tmap_nd_cached(base, 3, dims, strides, box);
+  };
+  const CUtensorMap* tx = epi_map(extra, ld_extra);
+  const CUtensorMap* ty = epi_map(c, ldc);
+  if (tx == nullptr || ty == nullptr) return -3;
+  return launch2<false, true, COMM_NONE, 4>(ta, tb, p, 2 * pairs, stream, tx, ty);
 }
 
 // Fused collective + GEMM on CTA pairs; same contract as gfs_gemm_bf16_comm (gemm.cu) with the

@@ -223,3 +223,29 @@ def test_gemm_tile_epilogues(cuda_device, bn, split):
         I3(*[n for _, n in shapes]), I3(*[n for _, n in shapes]), I3(*acc), bn, split, _lib.stream_ptr()) == 0
     for c, r in zip(C, refs):
         _check(c, r, K)
+
+
+@pytest.mark.parametrize("M,I,K", [(1, 8, 8), (33, 72, 64), (300, 200, 768), (1000, 1408, 1024), (777, 3080, 256),
+                                   (520, 264, 1032), (20000, 136, 192)])
+def test_swiglu_backward_on_pairs(cuda_device, M, I, K):
+    """Rows and columns that end inside a warp's 32 x 64 box (the last gate columns lie next to the first up
+    columns), more chunks than slots, and both sides of the line at K = 1024. Nothing outside the result is
+    written. Tolerance: d_act is rounded to bf16 before the epilogue and the result after it."""
+    from gpt_from_scratch_b200.ops import _lib
+    g = torch.Generator(device="cuda").manual_seed(M + I + K)
+    dy = torch.randn(M, K, device=cuda_device, generator=g).bfloat16()
+    w = (torch.randn(K, I, device=cuda_device, generator=g) / K ** 0.5).bfloat16()
+    gu = torch.randn(M, 2 * I + 16, device=cuda_device, generator=g).bfloat16()
+    out = torch.full((M + 1, 2 * I + 8), 7.0, device=cuda_device, dtype=torch.bfloat16)
+    rc = _lib.lib().gfs_gemm2_bf16_swiglu(2, dy.data_ptr(), w.data_ptr(), out.data_ptr(), gu.data_ptr(), M, I, K, K, I,
+                                          out.stride(0), gu.stride(0), _lib.stream_ptr())
+    assert rc == 0
+    torch.cuda.synchronize()
+    _lib.raise_on_status()
+    gate, up = gu[:, :I].double(), gu[:, I:2 * I].double()
+    d = (dy.double() @ w.double()).bfloat16().double()
+    s = torch.sigmoid(gate)
+    ref = torch.cat([d * up * s * (1 + gate * (1 - s)), d * gate * s], dim=1)
+    assert (out[M] == 7.0).all() and (out[:, 2 * I:] == 7.0).all()
+    rel = (out[:M, :2 * I].double() - ref).norm() / ref.norm()
+    assert rel < 5e-3, rel
