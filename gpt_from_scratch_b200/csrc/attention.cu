@@ -1042,8 +1042,11 @@ template <int D, int MODE>
 struct BwdShape {
   // Stages of the streamed-tile ring. A stage is only released when the gradient MMAs that read it have
   // finished and the score MMAs run two tiles ahead, so the TMA of a tile has (TS - 2) tile periods to land.
-  static constexpr int TS = D == 64 ? 8 : 4;
-  static constexpr int STAGING = BWD_CW * 2048;     // epilogue: 2 KB per compute warp
+  static constexpr int TS = D == 64 ? 7 : 4;
+  // epilogue, per compute warp: 2 KB to transpose through; at head_dim 64 the rotary table's entries before that
+  static constexpr bool ROPE_STAGED = D == 64;
+  static constexpr int STAGE_BYTES = ROPE_STAGED ? 4096 : 2048;
+  static constexpr int STAGING = BWD_CW * STAGE_BYTES;
   static constexpr int SMEM = 2 * (D / 64) * 16384 + 2 * TS * (D / 64) * 8192 + STAGING + (MODE == 0 ? TS * 512 : 0) + 256;
 };
 
@@ -1262,7 +1265,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
     const uint32_t y_addr = x_addr + Y_COL;
     const uint32_t p_addr = OVERLAY ? x_addr : tmem_base + lane_base + PT_COL + group * 64 + half * 16;
     const uint32_t ds_addr = OVERLAY ? y_addr : p_addr + 32;
-    uint8_t* stage = staging + cw * 2048;
+    uint8_t* stage = staging + cw * BwdShape<D, MODE>::STAGE_BYTES;
     bool acc_pending = false;           // the previous item's acc_full phase has not been waited for
     int g0 = 0;
     for (int it = 0; it * G < n_items; ++it) {
@@ -1385,6 +1388,22 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
       __nv_bfloat16* out = is_dv ? p.out2 + row0 * p.o2_ss + b * p.o2_bs + h * p.o2_hs
                                  : p.out1 + row0 * p.o1_ss + b * p.o1_bs + h * p.o1_hs;
       const uint32_t acc = tmem_base + lane_base + (MODE == 0 && !is_dv ? ACC2 : ACC1);
+      constexpr bool ROPE_STAGED = BwdShape<D, MODE>::ROPE_STAGED;
+      if (ROPE_STAGED && p.rope_cos != nullptr && !is_dv) {
+        // The rotary table's entries of the 32 rows come into shared memory as whole 64-byte segments while the
+        // item's last gradient MMAs finish: read by their rows' threads they would be 256 passes through the
+        // load / store unit after the wait.
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = (lane >> 2) + 8 * i, ch = lane & 3;
+          if (row0 + row < p.S) {
+            const size_t at = static_cast<size_t>(row0 + row) * (D / 2) + (c0 >> 1) + ch * 4;
+            uint8_t* dst = stage + row * 64 + ((ch ^ ((row >> 1) & 3)) << 4);
+            cp_async_16(dst, p.rope_cos + at);
+            cp_async_16(dst + 2048, p.rope_sin + at);
+          }
+        }
+      }
 #pragma unroll
       for (int ci = 0; ci < NC; ++ci) {
         const int c = c0 + 32 * ci;
@@ -1400,15 +1419,26 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
           __syncwarp();
           if (lane == 0) mbar_arrive(acc_empty);
         }
+        if (ROPE_STAGED) {
+          cp_async_wait_all();
+          __syncwarp();
+        }
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[8 * q4 + e]) * out_scale;
           if (rope_on) {  // inverse rotation: sin -> -sin
-            const size_t at = static_cast<size_t>(row_g) * (D / 2) + ((c + 8 * q4) >> 1);
-            const float4 cs = *reinterpret_cast<const float4*>(p.rope_cos + at);
-            const float4 sn = *reinterpret_cast<const float4*>(p.rope_sin + at);
+            float4 cs, sn;
+            if (ROPE_STAGED) {
+              const uint8_t* src = stage + lane * 64 + ((q4 ^ ((lane >> 1) & 3)) << 4);
+              cs = *reinterpret_cast<const float4*>(src);
+              sn = *reinterpret_cast<const float4*>(src + 2048);
+            } else {
+              const size_t at = static_cast<size_t>(row_g) * (D / 2) + ((c + 8 * q4) >> 1);
+              cs = *reinterpret_cast<const float4*>(p.rope_cos + at);
+              sn = *reinterpret_cast<const float4*>(p.rope_sin + at);
+            }
             const float a0 = f[0], a1 = f[1], a2 = f[2], a3 = f[3], a4 = f[4], a5 = f[5], a6 = f[6], a7 = f[7];
             f[0] = a0 * cs.x + a1 * sn.x; f[1] = a1 * cs.x - a0 * sn.x;
             f[2] = a2 * cs.y + a3 * sn.y; f[3] = a3 * cs.y - a2 * sn.y;
@@ -1420,6 +1450,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
           wv[4 * q4 + 2] = pack_out(f[4], f[5], p.out_f16);
           wv[4 * q4 + 3] = pack_out(f[6], f[7], p.out_f16);
         }
+        if (ROPE_STAGED) __syncwarp();   // every row's entries have been read
         store_rows_32x32(stage, wv, lane, out + c, o_ss, p.S - row0);
       }
     }
