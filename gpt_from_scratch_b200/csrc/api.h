@@ -49,12 +49,12 @@ int gfs_gemm2_ce_parts(int N);
 int gfs_gemm2_bf16_ce(const void* A, const void* B, void* C, void* partials, int M, int N, int K, int lda, int ldb,
                       int ldc, void* stream);
 int gfs_ce_fwd(const void* logits, const void* target, void* stats, void* lse, void* loss, int M, int Vp, long ld,
-               int v0, int single_rank, int target_batch, void* stream);
+               int v0, int single_rank, int target_batch, void* rows_target, void* stream);
 int gfs_ce_from_partials(const void* partials, const void* logits, const void* target, void* stats, void* lse,
                          void* loss, int parts, int M, int Vp, long ld, int v0, int single_rank, int target_batch,
-                         void* stream);
+                         void* rows_target, void* stream);
 int gfs_ce_bwd(void* logits, const void* lse, const void* target, const void* grad_rows, float grad_all, int M, int Vp,
-               long ld, int v0, int target_batch, void* stream);
+               long ld, int v0, void* stream);
 int gfs_mean_f32(const void* x, void* out, int n, void* stream);
 int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int S, int B, int nh, int D,
                   const long long* strides, float scale, int causal, int o_f16, void* stream);

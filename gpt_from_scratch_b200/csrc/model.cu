@@ -346,7 +346,7 @@ namespace {
 // Buffers of a step besides the blocks' activations. The logits are dead when the blocks' backward
 // begins, so its scratch lies in the same place.
 struct StepLayout {
-  size_t acts, x0, y_final, rstd_final, keys, loss_rows, stats, lse, dy, dx0, logits, partials, scratch, total;
+  size_t acts, x0, y_final, rstd_final, keys, targets, loss_rows, stats, lse, dy, dx0, logits, partials, scratch, total;
   StepLayout(const GfsBlockDims& d, const GfsModelTop& t, const ActLayout& a) {
     const size_t T = static_cast<size_t>(d.S) * d.B, H = d.H, V = t.V;
     size_t o = 0;
@@ -360,6 +360,7 @@ struct StepLayout {
     y_final = take(2 * T * H);
     rstd_final = take(4 * T);
     keys = take(4 * T);
+    targets = take(8 * T);
     loss_rows = take(4 * T);
     stats = take(12 * T);
     lse = take(4 * T);
@@ -413,7 +414,7 @@ int gfs_model_step(const GfsBlockDims* dp, const GfsBlockParams* layers, const G
   const int T = d.S * d.B, H = d.H, V = t.V;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   char* m = static_cast<char*>(arena);
-  void *x0 = m + lay.x0, *y = m + lay.y_final, *rstd = m + lay.rstd_final, *keys = m + lay.keys,
+  void *x0 = m + lay.x0, *y = m + lay.y_final, *rstd = m + lay.rstd_final, *keys = m + lay.keys, *targets = m + lay.targets,
        *rows = m + lay.loss_rows, *stats = m + lay.stats, *lse = m + lay.lse, *dy = m + lay.dy, *dx0 = m + lay.dx0,
        *logits = m + lay.logits, *partials = m + lay.partials, *scratch = m + lay.scratch;
 
@@ -446,19 +447,19 @@ int gfs_model_step(const GfsBlockDims* dp, const GfsBlockParams* layers, const G
     if (rc == 0) {
       *launches += 2;
       rc = gfs_ce_from_partials(partials, logits, labels, stats, lse, rows, gfs_gemm2_ce_parts(V), T, V, V, 0, 1, d.B,
-                                stream);
+                                targets, stream);
     }
   }
   if (rc == -20) {
     GFS_TRY(product(d, y, t.w_out, logits, nullptr, T, V, H, H, H, V, 0, 0, 0, stream));
-    GFS_TRY(gfs_ce_fwd(logits, labels, stats, lse, rows, T, V, V, 0, 1, d.B, stream));
+    GFS_TRY(gfs_ce_fwd(logits, labels, stats, lse, rows, T, V, V, 0, 1, d.B, targets, stream));
   } else if (rc != 0) {
     return rc;
   }
   GFS_TRY(gfs_mean_f32(rows, loss, T, stream));
 
   // backward: the logits become their gradient in place
-  GFS_TRY(gfs_ce_bwd(logits, lse, labels, nullptr, g_row, T, V, V, 0, d.B, stream));
+  GFS_TRY(gfs_ce_bwd(logits, lse, targets, nullptr, g_row, T, V, V, 0, stream));
   GFS_TRY(product(d, logits, t.w_out, dy, nullptr, T, H, V, V, H, H, 0, 1, 0, stream));
   WgradGroup grp;
   rc = weight_grad(d, grp, logits, y, t.g_out, t.acc_out, T, V, H, launches, stream);

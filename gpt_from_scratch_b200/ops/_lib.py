@@ -73,9 +73,9 @@ def _declare(lib: ctypes.CDLL) -> None:
         "gfs_embedding_bwd": ([vp, vp, vp, vp, i, i, i, i, vp], i),
         "gfs_embedding_sort_keys": ([vp, vp, i, i, i, i, vp], i),
         "gfs_embedding_bwd_keys": ([vp, vp, vp, i, i, i, vp], i),
-        "gfs_ce_fwd": ([vp, vp, vp, vp, vp, i, i, cl, i, i, i, vp], i),
+        "gfs_ce_fwd": ([vp, vp, vp, vp, vp, i, i, cl, i, i, i, vp, vp], i),
         "gfs_ce_combine": ([vp, vp, vp, i, i, vp], i),
-        "gfs_ce_bwd": ([vp, vp, vp, vp, f, i, i, cl, i, i, vp], i),
+        "gfs_ce_bwd": ([vp, vp, vp, vp, f, i, i, cl, i, vp], i),
         "gfs_sumsq_scratch_bytes": ([], i),
         "gfs_sumsq_bf16": ([vp, i64, vp, vp, vp], i),
         "gfs_adamw_step": ([vp, vp, vp, vp, vp, i64, vp, vp, f, d, d, f, f, f, f, f, f, vp, vp], i),
@@ -90,7 +90,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "gfs_dropout_residual": ([vp, vp, vp, ctypes.c_longlong, f, ctypes.c_ulonglong, i, vp], i),
         "gfs_gemm2_ce_parts": ([i], i),
         "gfs_gemm2_bf16_ce": ([vp, vp, vp, vp, i, i, i, i, i, i, vp], i),
-        "gfs_ce_from_partials": ([vp, vp, vp, vp, vp, vp, i, i, i, cl, i, i, i, vp], i),
+        "gfs_ce_from_partials": ([vp, vp, vp, vp, vp, vp, i, i, i, cl, i, i, i, vp, vp], i),
         "gfs_gemm2_wgrad_grouped": ([i, ulp, ulp, ulp, ip, ip, ip, ip, ip, ip, ip, vp], i),
         "gfs_gemm2_bf16_comm": ([i, vp, i, vp, i, vp, i, vp, i, i, i, i, i, i, i, ulp, ulp, uip, vp, vp, i, i, i,
                                  ctypes.c_longlong, vp], i),

@@ -21,7 +21,7 @@ def ce_local_stats(logits2d: torch.Tensor, target: torch.Tensor, vocab_start: in
     loss = torch.empty(M, dtype=torch.float32, device=dev)
     rc = _lib.lib().gfs_ce_fwd(logits2d.data_ptr(), target.data_ptr(), stats.data_ptr(), lse.data_ptr(),
                                loss.data_ptr(), M, Vp, logits2d.stride(0), vocab_start, 1 if single_rank else 0, 0,
-                               _lib.stream_ptr())
+                               None, _lib.stream_ptr())
     _lib.check(rc, "gfs_ce_fwd")
     return stats, lse, loss
 
@@ -37,7 +37,8 @@ def ce_stats_from_partials(partials: torch.Tensor, logits2d: torch.Tensor, targe
     loss = torch.empty(M, dtype=torch.float32, device=dev)
     rc = _lib.lib().gfs_ce_from_partials(partials.data_ptr(), logits2d.data_ptr(), target.data_ptr(), stats.data_ptr(),
                                          lse.data_ptr(), loss.data_ptr(), partials.shape[0], M, Vp,
-                                         logits2d.stride(0), vocab_start, 1 if single_rank else 0, 0, _lib.stream_ptr())
+                                         logits2d.stride(0), vocab_start, 1 if single_rank else 0, 0, None,
+                                         _lib.stream_ptr())
     _lib.check(rc, "gfs_ce_from_partials")
     return stats, lse, loss
 
@@ -57,6 +58,6 @@ def ce_backward_inplace(logits2d: torch.Tensor, lse: torch.Tensor, target: torch
                         vocab_start: int) -> torch.Tensor:
     M, Vp = logits2d.shape
     rc = _lib.lib().gfs_ce_bwd(logits2d.data_ptr(), lse.data_ptr(), target.data_ptr(), grad_rows.data_ptr(), 0.0, M, Vp,
-                               logits2d.stride(0), vocab_start, 0, _lib.stream_ptr())
+                               logits2d.stride(0), vocab_start, _lib.stream_ptr())
     _lib.check(rc, "gfs_ce_bwd")
     return logits2d
