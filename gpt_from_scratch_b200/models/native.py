@@ -131,6 +131,10 @@ class _Plan:
             self.top_args.w[k] = w.data_ptr()
         self.top_args.V = head.weight.shape[0]
         self.all_params = [w for ws in self.weights for w in ws] + list(self.top)
+        # A shared parameter (a tied head, a block that occurs twice) needs its overwrite-or-add flag taken where
+        # each kernel runs, and its uses in one launch kept apart: the modules do both.
+        if len({id(w) for w in self.all_params}) != len(self.all_params):
+            return False
         d = self.dims
         d.H, d.nh, d.D = H, layers[0].attention.num_attention_heads, layers[0].attention.head_dim
         d.I, d.n_layers, d.eps_final = layers[0].mlp.intermediate_size, len(layers), fin.eps
@@ -214,7 +218,7 @@ _plans: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 def plan_for(model, inputs: torch.Tensor):
     """The model's plan if this pass can run natively, else ``None``."""
     w = model.embedding.weight
-    if not (w.is_cuda and w.dtype == torch.bfloat16 and inputs.dim() == 2 and inputs.is_cuda and inputs.numel() > 0):
+    if not (_native_weight(w) and inputs.dim() == 2 and inputs.device == w.device and inputs.numel() > 0):
         return None
     if ps.get_tensor_model_parallel_world_size() != 1:
         return None
@@ -225,10 +229,14 @@ def plan_for(model, inputs: torch.Tensor):
     if not plan.refresh(model):
         return None
     if torch.is_grad_enabled():
+        slices = set()
         for p in plan.all_params:
-            # every gradient goes to its slice of the optimizer's buffer and nobody waits for single ones
+            # every gradient goes to a slice of its own in the optimizer's buffer and nobody waits for single ones
             if not p.requires_grad or GradSink.of(p) is None or getattr(p, "_grad_ready_cb", None) is not None:
                 return None
+            slices.add(p.grad.data_ptr())
+        if len(slices) != len(plan.all_params):
+            return None
     return plan
 
 

@@ -392,3 +392,50 @@ def test_native_model_pass_matches_module_path(cuda_device, monkeypatch, H, head
         for name, a, b in zip(("logits", "gradients", "master"), run[1:], runs[2][1:]):
             rel = (a.float() - b.float()).norm() / b.float().norm()
             assert rel < (1e-2 if dropout else 2e-3), (name, rel)
+
+
+def _shared_gradients(share, H, layers, V, steps=2):
+    """Gradients by name after ``steps`` optimizer steps of a model that ``share`` changes and of one with equal
+    weights in its place; the latter's are summed over ``share``'s pairs (kept name, name it stands for)."""
+    from gpt_from_scratch_b200.config import GPTConfig
+    from gpt_from_scratch_b200.engine import TrainEngine
+    cfg = GPTConfig(vocab_size=V, hidden_size=H, num_layers=layers, num_attention_heads=H // 64,
+                    max_position_embeddings=64, intermediate_size=2 * H)
+    g = torch.Generator().manual_seed(4)
+    batches = [torch.randint(0, V, (4, 65), generator=g) for _ in range(steps)]
+    out = []
+    for shared in (True, False):
+        eng = TrainEngine(cfg, lr=1e-9, seed=9)
+        with torch.no_grad():
+            pairs = share(eng.model, shared)
+        for t in batches:
+            eng.train_step(t[:, :-1].contiguous().cuda(), t[:, 1:].contiguous().cuda())
+        grads = {n: p.grad.double() for n, p in eng.model.named_parameters()}
+        if not shared:
+            for keep, other in pairs:
+                grads[keep] = grads[keep] + grads.pop(other)
+        out.append(grads)
+    assert set(out[0]) == set(out[1])
+    return out
+
+
+def _tie_head(m, shared):
+    if shared:
+        m.output.weight = m.embedding.weight
+    else:
+        m.output.weight.copy_(m.embedding.weight)
+    return [("embedding.weight", "output.weight")]
+
+
+@pytest.mark.parametrize("V", [16384])
+def test_tied_head_gets_both_gradients(cuda_device, V):
+    """A head that shares the embedding's weight: its gradient is the sum of the two uses, of this step only. The sum
+    is rounded to bf16 twice (2^-9 each) on rows that cancel, the uses themselves once."""
+    from gpt_from_scratch_b200.parallel import parallel_state as ps
+    ps.set_device(cuda_device)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_parallel_state(1)
+    tied, apart = _shared_gradients(_tie_head, 256, 2, V)
+    for name, g in tied.items():
+        rel = (g - apart[name]).norm() / apart[name].norm()
+        assert rel < 1e-2, (name, rel)
