@@ -36,8 +36,6 @@ struct GfsBlockDims {
   int grouped_wgrad;       // small weight gradients of a block share a launch
   float dropout_p;         // 0: residual adds run in the GEMM epilogues
   float eps_final;
-  const void* cos_table;   // fp32 [>= S, D/2]
-  const void* sin_table;
 };
 
 struct GfsBlockParams {
@@ -45,6 +43,8 @@ struct GfsBlockParams {
   void* g[W_COUNT];        // their gradients (bf16)
   int accumulate[W_COUNT]; // add to the gradient instead of overwriting it
   float eps[2];            // norm1, norm2
+  const void* cos_table;   // fp32 [>= S, D/2]
+  const void* sin_table;
   u64 seed[2];             // dropout after the attention, after the MLP
 };
 
@@ -115,10 +115,9 @@ bool use_pair(const GfsBlockDims& d, int tiles) { return d.pair_min_tiles >= 0 &
 
 // C[M,N] = op(A) op(B) (+ R), R with the pitch of C
 int product(const GfsBlockDims& d, const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda,
-            int ldb, int ldc, int a_mn, int b_mn, int rope_cols, void* stream) {
-  return gfs_linear(A, B, C, R, M, N, K, lda, ldb, ldc, R != nullptr ? ldc : 0, a_mn, b_mn,
-                    rope_cols > 0 ? d.cos_table : nullptr, rope_cols > 0 ? d.sin_table : nullptr, rope_cols, d.D, d.B,
-                    d.pair_min_tiles, stream);
+            int ldb, int ldc, int a_mn, int b_mn, void* stream) {
+  return gfs_linear(A, B, C, R, M, N, K, lda, ldb, ldc, R != nullptr ? ldc : 0, a_mn, b_mn, nullptr, nullptr, 0, d.D,
+                    d.B, d.pair_min_tiles, stream);
 }
 
 // The weight gradients of one block that are too small to fill the chip alone share a launch.
@@ -153,7 +152,7 @@ int weight_grad(const GfsBlockDims& d, WgradGroup& grp, const void* dY, const vo
     return 0;
   }
   ++*launches;
-  return product(d, dY, X, dW, accumulate ? dW : nullptr, n_out, n_in, T, n_out, n_in, n_in, 1, 1, 0, stream);
+  return product(d, dY, X, dW, accumulate ? dW : nullptr, n_out, n_in, T, n_out, n_in, n_in, 1, 1, stream);
 }
 
 bool dims_ok(const GfsBlockDims& d) {
@@ -203,21 +202,22 @@ int gfs_blocks_forward(const GfsBlockDims* dp, const GfsBlockParams* layers, con
          *y2 = base + a.y2, *rstd2 = base + a.rstd2, *gu = base + a.gu, *ac = base + a.act, *x2 = base + a.x2;
     char* qkv = base + a.qkv;
     GFS_TRY(gfs_rmsnorm_fwd(x, p.w[W_NORM1], y1, rstd1, T, H, p.eps[0], stream));
-    GFS_TRY(product(d, y1, p.w[W_QKV], qkv, nullptr, T, 3 * H, H, H, H, 3 * H, 0, 0, 2 * H, stream));
+    GFS_TRY(gfs_linear(y1, p.w[W_QKV], qkv, nullptr, T, 3 * H, H, H, H, 3 * H, 0, 0, 0, p.cos_table, p.sin_table, 2 * H,
+                       d.D, d.B, d.pair_min_tiles, stream));   // q and k leave rotated
     GFS_TRY(gfs_flash_fwd(qkv, qkv + 2 * static_cast<size_t>(H), qkv + 4 * static_cast<size_t>(H), attn, lse, d.S, d.B,
                           d.nh, d.D, st, scale, 1, 0, stream));
     if (!drop) {
-      GFS_TRY(product(d, attn, p.w[W_OUT], x1, x, T, H, H, H, H, H, 0, 0, 0, stream));
+      GFS_TRY(product(d, attn, p.w[W_OUT], x1, x, T, H, H, H, H, H, 0, 0, stream));
     } else {
-      GFS_TRY(product(d, attn, p.w[W_OUT], tmp, nullptr, T, H, H, H, H, H, 0, 0, 0, stream));
+      GFS_TRY(product(d, attn, p.w[W_OUT], tmp, nullptr, T, H, H, H, H, H, 0, 0, stream));
       GFS_TRY(gfs_dropout_residual(tmp, x, x1, n_el, d.dropout_p, p.seed[0], 0, stream));
     }
     GFS_TRY(gfs_rmsnorm_fwd(x1, p.w[W_NORM2], y2, rstd2, T, H, p.eps[1], stream));
     GFS_TRY(gfs_linear_swiglu(1, y2, p.w[W_GATE_UP], gu, ac, T, I, H, H, H, 2 * I, I, d.pair_min_tiles, stream));
     if (!drop) {
-      GFS_TRY(product(d, ac, p.w[W_DOWN], x2, x1, T, H, I, I, I, H, 0, 0, 0, stream));
+      GFS_TRY(product(d, ac, p.w[W_DOWN], x2, x1, T, H, I, I, I, H, 0, 0, stream));
     } else {
-      GFS_TRY(product(d, ac, p.w[W_DOWN], tmp, nullptr, T, H, I, I, I, H, 0, 0, 0, stream));
+      GFS_TRY(product(d, ac, p.w[W_DOWN], tmp, nullptr, T, H, I, I, I, H, 0, 0, stream));
       GFS_TRY(gfs_dropout_residual(tmp, x1, x2, n_el, d.dropout_p, p.seed[1], 0, stream));
     }
     x = x2;
@@ -299,7 +299,7 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
                               d.pair_min_tiles, stream));
     int rc = weight_grad(d, grp, dm, ac, p.g[W_DOWN], p.accumulate[W_DOWN], T, H, I, launches, stream);
     if (rc != 0) return rc;
-    GFS_TRY(product(d, dgu, p.w[W_GATE_UP], dy, nullptr, T, H, 2 * I, 2 * I, H, H, 0, 1, 0, stream));
+    GFS_TRY(product(d, dgu, p.w[W_GATE_UP], dy, nullptr, T, H, 2 * I, 2 * I, H, H, 0, 1, stream));
     rc = weight_grad(d, grp, dgu, y2, p.g[W_GATE_UP], p.accumulate[W_GATE_UP], T, 2 * I, H, launches, stream);
     if (rc != 0) return rc;
     GFS_TRY(norm_bwd(dy, x1, p.w[W_NORM2], rstd2, dout, dx1, p.g[W_NORM2], p.accumulate[W_NORM2]));
@@ -310,14 +310,14 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
       GFS_TRY(gfs_dropout_residual(dx1, nullptr, m, n_el, d.dropout_p, p.seed[0], 1, stream));
       da = m;
     }
-    GFS_TRY(product(d, da, p.w[W_OUT], dattn, nullptr, T, H, H, H, H, H, 0, 1, 0, stream));
+    GFS_TRY(product(d, da, p.w[W_OUT], dattn, nullptr, T, H, H, H, H, H, 0, 1, stream));
     rc = weight_grad(d, grp, da, attn, p.g[W_OUT], p.accumulate[W_OUT], T, H, H, launches, stream);
     if (rc != 0) return rc;
     const size_t h2 = 2 * static_cast<size_t>(H);
     GFS_TRY(gfs_flash_bwd(qkv, qkv + h2, qkv + 2 * h2, attn, dattn, lse, dvec, dqkv, dqkv + h2, dqkv + 2 * h2, d.S, d.B,
-                          d.nh, d.D, st, scale, 1, d.cos_table, d.sin_table, nullptr, stream));
+                          d.nh, d.D, st, scale, 1, p.cos_table, p.sin_table, nullptr, stream));
     *launches += 2;   // a pre-pass and two main kernels
-    GFS_TRY(product(d, dqkv, p.w[W_QKV], dy, nullptr, T, H, 3 * H, 3 * H, H, H, 0, 1, 0, stream));
+    GFS_TRY(product(d, dqkv, p.w[W_QKV], dy, nullptr, T, H, 3 * H, 3 * H, H, H, 0, 1, stream));
     rc = weight_grad(d, grp, dqkv, y1, p.g[W_QKV], p.accumulate[W_QKV], T, 3 * H, H, launches, stream);
     if (rc != 0) return rc;
     rc = grp.flush(launches, stream);   // its operands are overwritten by the next block
@@ -451,7 +451,7 @@ int gfs_model_step(const GfsBlockDims* dp, const GfsBlockParams* layers, const G
     }
   }
   if (rc == -20) {
-    GFS_TRY(product(d, y, t.w_out, logits, nullptr, T, V, H, H, H, V, 0, 0, 0, stream));
+    GFS_TRY(product(d, y, t.w_out, logits, nullptr, T, V, H, H, H, V, 0, 0, stream));
     GFS_TRY(gfs_ce_fwd(logits, labels, stats, lse, rows, T, V, V, 0, 1, d.B, targets, stream));
   } else if (rc != 0) {
     return rc;
@@ -460,7 +460,7 @@ int gfs_model_step(const GfsBlockDims* dp, const GfsBlockParams* layers, const G
 
   // backward: the logits become their gradient in place
   GFS_TRY(gfs_ce_bwd(logits, lse, targets, nullptr, g_row, T, V, V, 0, stream));
-  GFS_TRY(product(d, logits, t.w_out, dy, nullptr, T, H, V, V, H, H, 0, 1, 0, stream));
+  GFS_TRY(product(d, logits, t.w_out, dy, nullptr, T, H, V, V, H, H, 0, 1, stream));
   WgradGroup grp;
   rc = weight_grad(d, grp, logits, y, t.g_out, t.acc_out, T, V, H, launches, stream);
   if (rc == 0) rc = grp.flush(launches, stream);

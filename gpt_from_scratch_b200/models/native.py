@@ -7,15 +7,18 @@ the module-by-module path: the stack of blocks with the final norm is ONE call i
 direction (csrc/model.cu), and autograd sees one function for the model. Same kernels, same order, same
 results.
 
-The modules stay the owners of the parameters and every condition is looked up again in each pass
-(``_Plan.refresh``), so replacing a module or a parameter, registering a hook, freezing a weight or
-switching a module to another implementation sends the next pass down the module path.
+The modules stay the owners of the parameters, and each pass compares what it is about to use with what they
+hold: modules and their types, weights, biases, rotary tables, norm constants, dropout, hooks, ``forward`` methods
+replaced on an instance or a class (``_Plan.current``, ``_Plan.plain_modules``). A change within what the native
+passes compute is followed; any other one, a frozen weight included, sends the pass down the module path.
 """
 from __future__ import annotations
 
 import ctypes
 import weakref
 from ctypes import byref, c_float, c_int, c_size_t, c_ulonglong, c_void_p
+from itertools import repeat
+from operator import contains, getitem, is_
 
 import torch
 
@@ -28,19 +31,20 @@ from ..parallel.layers import ColumnParallelLinear, RowParallelLinear, VocabPara
 from .mlp import ParallelMLP
 from .normalization import RMSNorm
 from .position_embeddings import RotaryEmbedding
+from .transformer_layer import ParallelAttention, TransformerLayer
 
 
 class _Dims(ctypes.Structure):
     """GfsBlockDims in csrc/model.cu."""
     _fields_ = [("S", c_int), ("B", c_int), ("H", c_int), ("nh", c_int), ("D", c_int), ("I", c_int),
                 ("n_layers", c_int), ("pair_min_tiles", c_int), ("grouped_wgrad", c_int),
-                ("dropout_p", c_float), ("eps_final", c_float), ("cos_table", c_void_p), ("sin_table", c_void_p)]
+                ("dropout_p", c_float), ("eps_final", c_float)]
 
 
 class _BlockParams(ctypes.Structure):
     """GfsBlockParams in csrc/model.cu."""
     _fields_ = [("w", c_void_p * 6), ("g", c_void_p * 6), ("accumulate", c_int * 6), ("eps", c_float * 2),
-                ("seed", c_ulonglong * 2)]
+                ("cos_table", c_void_p), ("sin_table", c_void_p), ("seed", c_ulonglong * 2)]
 
 
 class _Top(ctypes.Structure):
@@ -48,12 +52,8 @@ class _Top(ctypes.Structure):
     _fields_ = [("w", c_void_p * 3), ("g", c_void_p * 3), ("accumulate", c_int * 3), ("V", c_int)]
 
 
-def _hook_dicts(module: torch.nn.Module):
-    return (module._forward_hooks, module._forward_pre_hooks, module._backward_hooks, module._backward_pre_hooks)
-
-
-def _native_weight(w) -> bool:
-    return w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 16 == 0
+def _native_tensor(t: torch.Tensor, dtype: torch.dtype) -> bool:
+    return t.is_cuda and t.dtype == dtype and t.is_contiguous() and t.data_ptr() % 16 == 0
 
 
 def _consume(p: torch.nn.Parameter) -> int:
@@ -63,123 +63,166 @@ def _consume(p: torch.nn.Parameter) -> int:
     return 0 if fresh else 1
 
 
+# The methods whose work the native passes do: a class that has been given another one is asked.
+_FORWARDS = tuple((c, c.forward) for c in (
+    VocabParallelEmbedding, TransformerLayer, RMSNorm, ParallelAttention, RotaryEmbedding, ParallelMLP,
+    ColumnParallelLinear, RowParallelLinear))
+
+
+class _Unsupported(Exception):
+    """The modules compute something that the native passes do not."""
+
+
+def _require(ok: bool) -> None:
+    if not ok:
+        raise _Unsupported
+
+
 class _Plan:
-    """What a pass of one model needs, kept between passes; ``refresh`` brings it up to date."""
+    """What the passes of one model need, and everything it was derived from: the modules in their places, their
+    weights, tables and settings (``dicts[i][keys[i]] is values[i]``) and what each tensor looked like. Built anew
+    when any of it has changed (:meth:`current`)."""
 
-    def __init__(self, layer_type, attention_type):
-        self.layer_type, self.attention_type = layer_type, attention_type
-        self.layers: list = []          # the blocks the arrays below were built for
-        self.shape = None               # (S, B) the workspace sizes were computed for
-        self.dims = _Dims()
-        self.params = None              # ctypes array of _BlockParams
-        self.weights: list = []         # per block: its six parameters
-        self.hooks: list = []
-        self.ptrs: list = []
-        self.step_shape = None          # (S, B, dropout) step_bytes was computed for
-        self.top_args = _Top()
+    def __init__(self, model):
+        self.dicts, self.keys, self.values = [], [], []
+        self.modules, self.tensors = [], []
 
-    def _bind(self, model) -> bool:
-        """Structural checks and everything that depends on the modules only."""
-        self.ptrs = []
-        layers = list(model.layers)
-        head, emb, fin = model.output, model.embedding, model.final_norm
-        if (type(head) is not ColumnParallelLinear or head.bias is not None or
-                type(emb) is not VocabParallelEmbedding or type(fin) is not RMSNorm):
-            return False
-        modules = [emb, fin, head]
-        for layer in layers:
-            a, m = layer.attention, layer.mlp
-            if (type(layer) is not self.layer_type or type(a) is not self.attention_type or
-                    type(m) is not ParallelMLP or type(layer.input_norm) is not RMSNorm or
-                    type(layer.post_attention_norm) is not RMSNorm or
-                    type(a.qkv_proj) is not ColumnParallelLinear or type(a.out_proj) is not RowParallelLinear or
-                    type(m.gate_up_proj) is not ColumnParallelLinear or type(m.down_proj) is not RowParallelLinear or
-                    type(a.rotary_emb) is not RotaryEmbedding):
-                return False
-            if any(x.bias is not None for x in (a.qkv_proj, a.out_proj, m.gate_up_proj, m.down_proj)):
-                return False
-            modules += [layer, a, m, layer.input_norm, layer.post_attention_norm, a.qkv_proj, a.out_proj,
-                        m.gate_up_proj, m.down_proj, a.rotary_emb]
-        H = fin.weight.shape[0]
-        for layer in layers:
-            a, m = layer.attention, layer.mlp
-            if (a.hidden_size != H or a.head_dim not in (64, 128) or a.num_heads_per_partition * a.head_dim != H or
-                    a.head_dim != layers[0].attention.head_dim or a.qkv_proj.weight.shape != (3 * H, H) or
-                    a.out_proj.weight.shape != (H, H) or m.down_proj.weight.shape != (H, m.intermediate_size) or
-                    m.gate_up_proj.weight.shape != (2 * m.intermediate_size, H) or
-                    m.intermediate_size != layers[0].mlp.intermediate_size or m.intermediate_size % 8):
-                return False
-            r, r0 = a.rotary_emb, layers[0].attention.rotary_emb
-            if (layer.dropout_prob != layers[0].dropout_prob or
-                    (r.base, r.head_dim, r.round_to_activation_dtype) !=
-                    (r0.base, r0.head_dim, r0.round_to_activation_dtype)):
-                return False
-        if not layers or H % 8 or head.weight.shape[1] != H or emb.weight.shape[1] != H or head.weight.shape[0] % 8:
-            return False
-        if any(not _native_weight(p) for p in model.parameters()):
-            return False
-        self.layers = layers
-        self.hooks = [d for x in modules for d in _hook_dicts(x)]
-        self.params = (_BlockParams * len(layers))()
-        self.weights = [self._weights_of(layer) for layer in layers]
-        for bp, layer, ws in zip(self.params, layers, self.weights):
+        def read(place: dict, key: str):
+            value = place[key]
+            self.dicts.append(place)
+            self.keys.append(key)
+            self.values.append(value)
+            return value
+
+        def child(parent, name: str, cls):
+            m = read(parent._modules, name)
+            _require(type(m) is cls)
+            self.modules.append(m)
+            return m
+
+        def tensor(place: dict, name: str, dtype: torch.dtype, shape=None):
+            t = read(place, name)
+            _require(_native_tensor(t, dtype) and (shape is None or tuple(t.shape) == shape))
+            self.tensors.append(t)
+            return t
+
+        def weight(m, *shape):
+            return tensor(m._parameters, "weight", torch.bfloat16, shape or None)
+
+        def linear(parent, name: str, cls, *shape):
+            m = child(parent, name, cls)
+            _require(read(m._parameters, "bias") is None)
+            return weight(m, *shape)
+
+        def norm(parent, name: str):
+            m = child(parent, name, RMSNorm)
+            eps = read(m.__dict__, "eps")
+            _require(type(eps) in (int, float))
+            return weight(m, H), eps
+
+        emb = child(model, "embedding", VocabParallelEmbedding)
+        w_emb = weight(emb)
+        V, H = w_emb.shape
+        _require(read(emb.__dict__, "vocab_start_index") == 0 and read(emb.__dict__, "vocab_end_index") == V)
+        w_fin, eps_final = norm(model, "final_norm")
+        w_out = linear(model, "output", ColumnParallelLinear)
+        _require(w_out.shape[1] == H and w_out.shape[0] % 8 == 0 and H % 8 == 0)
+        self.stack = read(model._modules, "layers")
+        _require(type(self.stack) is torch.nn.ModuleList and len(self.stack) > 0)
+        self.layers = list(self.stack)
+        self.rotaries, self.weights, self.settings = [], [], set()
+        self.table_rows = None
+        self.params = (_BlockParams * len(self.layers))()
+        for name, bp in zip(self.stack._modules, self.params):
+            layer = child(self.stack, name, TransformerLayer)
+            w1, eps1 = norm(layer, "input_norm")
+            w2, eps2 = norm(layer, "post_attention_norm")
+            a, m = child(layer, "attention", ParallelAttention), child(layer, "mlp", ParallelMLP)
+            nh, D = read(a.__dict__, "num_heads_per_partition"), read(a.__dict__, "head_dim")
+            _require(read(a.__dict__, "attention_impl") == "fused" and D in (64, 128) and nh * D == H)
+            ws = (w1, linear(a, "qkv_proj", ColumnParallelLinear, 3 * H, H),
+                  linear(a, "out_proj", RowParallelLinear, H, H), w2,
+                  linear(m, "gate_up_proj", ColumnParallelLinear), linear(m, "down_proj", RowParallelLinear))
+            I = ws[5].shape[1]
+            _require(ws[4].shape == (2 * I, H) and ws[5].shape == (H, I) and I % 8 == 0)
+            rot = child(a, "rotary_emb", RotaryEmbedding)
+            cos, sin = (tensor(rot._buffers, k, torch.float32) for k in ("cos_cached", "sin_cached"))
+            _require(cos.shape == sin.shape and cos.dim() == 2 and cos.shape[1] == D // 2)
+            self.table_rows = min(self.table_rows or cos.shape[0], cos.shape[0])
+            self.settings.add((nh, D, I, read(layer.__dict__, "dropout_prob")))
+            self.rotaries.append(rot)
+            self.weights.append(ws)
             for k, w in enumerate(ws):
                 bp.w[k] = w.data_ptr()
-            bp.eps[0], bp.eps[1] = layer.input_norm.eps, layer.post_attention_norm.eps
-        self.top = (emb.weight, fin.weight, head.weight)
-        for k, w in enumerate(self.top):
-            self.top_args.w[k] = w.data_ptr()
-        self.top_args.V = head.weight.shape[0]
+            bp.eps[0], bp.eps[1] = eps1, eps2
+            bp.cos_table, bp.sin_table = cos.data_ptr(), sin.data_ptr()
+        _require(len(self.settings) == 1)
+        nh, D, I, self.dropout_prob = self.settings.pop()
+        _require(0.0 <= self.dropout_prob < 1.0)
+        self.top = (w_emb, w_fin, w_out)
         self.all_params = [w for ws in self.weights for w in ws] + list(self.top)
         # A shared parameter (a tied head, a block that occurs twice) needs its overwrite-or-add flag taken where
         # each kernel runs, and its uses in one launch kept apart: the modules do both.
-        if len({id(w) for w in self.all_params}) != len(self.all_params):
-            return False
-        d = self.dims
-        d.H, d.nh, d.D = H, layers[0].attention.num_attention_heads, layers[0].attention.head_dim
-        d.I, d.n_layers, d.eps_final = layers[0].mlp.intermediate_size, len(layers), fin.eps
-        self.shape = self.step_shape = None
-        self.ptrs = self._live_ptrs(model)
-        return True
+        _require(len({id(w) for w in self.all_params}) == len(self.all_params))
+        self.types = [type(m) for m in self.modules]
+        self.module_dicts = [m.__dict__ for m in self.modules]
+        self.layer_dicts = [layer.__dict__ for layer in self.layers]
+        self.hooks = [d for m in self.modules for d in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks,
+                                                        m._backward_pre_hooks)]
+        self.looks = self._looks()
+        self.dims = _Dims(H=H, nh=nh, D=D, I=I, n_layers=len(self.layers), eps_final=eps_final)
+        self.top_args = _Top(V=w_out.shape[0])
+        for k, w in enumerate(self.top):
+            self.top_args.w[k] = w.data_ptr()
+        self.shape = self.step_shape = None   # (S, B, dropout) the workspace sizes were computed for
 
-    @staticmethod
-    def _weights_of(layer) -> tuple:
-        m = layer._modules
-        a, f = m["attention"]._modules, m["mlp"]._modules
-        return (m["input_norm"]._parameters["weight"], a["qkv_proj"]._parameters["weight"],
-                a["out_proj"]._parameters["weight"], m["post_attention_norm"]._parameters["weight"],
-                f["gate_up_proj"]._parameters["weight"], f["down_proj"]._parameters["weight"])
-
-    def _live_ptrs(self, model) -> list:
-        """Identity of every parameter and address of its data as the modules hold them now."""
-        top = model._modules
-        ws = [w for layer in top["layers"]._modules.values() for w in self._weights_of(layer)]
-        ws += [top["embedding"]._parameters["weight"], top["final_norm"]._parameters["weight"],
-               top["output"]._parameters["weight"]]
-        return [(id(w), w.data_ptr()) for w in ws]
-
-    def refresh(self, model) -> bool:
-        """True if this pass can run natively."""
+    @classmethod
+    def of(cls, model) -> "_Plan | None":
         try:
-            current = self._live_ptrs(model)
-        except (KeyError, AttributeError):     # modules replaced by others
-            return False
-        if current != self.ptrs and not self._bind(model):
-            return False
-        if any(self.hooks) or torch.nn.modules.module._has_any_global_hook():
-            return False
-        training = self.layers[0].training
-        for layer in self.layers:
-            if layer.training != training or layer._modules["attention"].attention_impl != "fused":
+            return cls(model)
+        except (_Unsupported, KeyError, AttributeError, TypeError, ValueError):   # others in our modules' places
+            return None
+
+    def _looks(self) -> tuple:
+        ts = self.tensors
+        return ([t.data_ptr() for t in ts], [t.shape for t in ts], [t.dtype for t in ts],
+                [t.is_contiguous() for t in ts])
+
+    def current(self) -> bool:
+        """True if nothing that the plan was built from has changed. (Loops in C: 60 us for 12 blocks.)"""
+        try:
+            if not all(map(is_, map(getitem, self.dicts, self.keys), self.values)):
                 return False
-        self.dropout = self.layers[0].dropout_prob if training else 0.0
+        except KeyError:
+            return False
+        return (all(map(is_, map(type, self.modules), self.types)) and list(self.stack._modules.values()) == self.layers
+                and self._looks() == self.looks)
+
+    def plain_modules(self) -> bool:
+        """No hook, no replaced method: calling a module is calling its class's ``forward``."""
+        return not (any(self.hooks) or torch.nn.modules.module._has_any_global_hook() or
+                    any(map(contains, self.module_dicts, repeat("forward"))) or
+                    any(c.forward is not f for c, f in _FORWARDS))
+
+    def grow_tables(self, S: int) -> bool:
+        """Have the rotary modules make their tables for S positions, as they do when called."""
+        grown = False
+        for r in self.rotaries:
+            if S > r.max_seq_len_cached or (r.round_to_activation_dtype and r._rounded_for is not torch.bfloat16):
+                r(self.top[0], S)
+                grown = True
+        return grown
+
+    def set_mode(self) -> bool:
+        """Take the dropout probability of this pass; False if the blocks differ in it."""
+        training = self.layer_dicts[0]["training"]
+        if self.dropout_prob != 0.0 and any(d["training"] != training for d in self.layer_dicts):
+            return False
+        self.dropout = self.dropout_prob if training else 0.0
         return True
 
     def set_shape(self, S: int, B: int) -> None:
         d = self.dims
-        rot = self.layers[0].attention.rotary_emb
-        cos, sin = rot(self.top[0], S)
-        d.cos_table, d.sin_table = cos.data_ptr(), sin.data_ptr()
         d.pair_min_tiles = gemm_ops.pair_threshold()
         d.grouped_wgrad = 1 if gemm_ops._WGRAD_GROUPING else 0
         key = (S, B, self.dropout)
@@ -217,16 +260,21 @@ _plans: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 
 def plan_for(model, inputs: torch.Tensor):
     """The model's plan if this pass can run natively, else ``None``."""
-    w = model.embedding.weight
-    if not (_native_weight(w) and inputs.dim() == 2 and inputs.device == w.device and inputs.numel() > 0):
+    if not (inputs.dim() == 2 and inputs.numel() > 0) or ps.get_tensor_model_parallel_world_size() != 1:
         return None
-    if ps.get_tensor_model_parallel_world_size() != 1:
-        return None
+    S = inputs.shape[1]
     plan = _plans.get(model)
+    if plan is None or not plan.current():
+        plan = _Plan.of(model)
+    if plan is not None and not plan.plain_modules():
+        return None
+    if plan is not None and plan.grow_tables(S):
+        plan = _Plan.of(model)
     if plan is None:
-        from .transformer_layer import ParallelAttention, TransformerLayer
-        plan = _plans[model] = _Plan(TransformerLayer, ParallelAttention)
-    if not plan.refresh(model):
+        _plans.pop(model, None)
+        return None
+    _plans[model] = plan
+    if inputs.device != plan.top[0].device or S > plan.table_rows or not plan.set_mode():
         return None
     if torch.is_grad_enabled():
         slices = set()

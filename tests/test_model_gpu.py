@@ -439,3 +439,43 @@ def test_tied_head_gets_both_gradients(cuda_device, V):
     for name, g in tied.items():
         rel = (g - apart[name]).norm() / apart[name].norm()
         assert rel < 1e-2, (name, rel)
+
+
+def test_native_pass_follows_changed_modules(cuda_device):
+    """After a first native pass: one block's rotary table, a norm's constant, a module with its own ``forward``. The
+    logits are those of the module path, which a hook selects; the two run the same kernels forward."""
+    import types
+    from gpt_from_scratch_b200.config import GPTConfig
+    from gpt_from_scratch_b200.engine import TrainEngine
+    from gpt_from_scratch_b200.models import native
+    from gpt_from_scratch_b200.parallel import parallel_state as ps
+    ps.set_device(cuda_device)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_parallel_state(1)
+    cfg = GPTConfig(vocab_size=512, hidden_size=256, num_layers=3, num_attention_heads=4,
+                    max_position_embeddings=64, intermediate_size=512)
+    model = TrainEngine(cfg, seed=5).model
+    ids = torch.randint(0, 512, (2, 64), generator=torch.Generator().manual_seed(1)).cuda()
+
+    def by_modules():
+        hook = model.layers[0].register_forward_hook(lambda *a: None)
+        try:
+            return model(ids)
+        finally:
+            hook.remove()
+
+    with torch.no_grad():
+        seen = [model(ids)]
+        assert torch.equal(seen[0], by_modules())
+        rot = model.layers[1].attention.rotary_emb
+        rot.cos_cached, rot.sin_cached = rot.sin_cached.clone(), rot.cos_cached.clone()
+        seen.append(model(ids))
+        model.layers[2].input_norm.eps = 0.7
+        seen.append(model(ids))
+        assert native.plan_for(model, ids) is not None
+        assert torch.equal(seen[-1], by_modules())
+        mlp = model.layers[0].mlp
+        mlp.forward = types.MethodType(lambda self, x, residual=None: residual, mlp)
+        seen.append(model(ids))
+        assert torch.equal(seen[-1], by_modules())
+    assert all(not torch.equal(a, b) for a, b in zip(seen, seen[1:]))

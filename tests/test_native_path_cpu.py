@@ -1,6 +1,8 @@
 """When the whole-model native passes may serve a model, on the CPU: the device checks are stubbed out, nothing
 is launched. A pass that the native path cannot serve has to go through the modules, also when an earlier pass of the
 same model ran natively."""
+import types
+
 import pytest
 import torch
 
@@ -23,7 +25,7 @@ def _cpu_state():
 
 @pytest.fixture
 def model(monkeypatch):
-    monkeypatch.setattr(native, "_native_weight", lambda w: True)
+    monkeypatch.setattr(native, "_native_tensor", lambda t, dtype: t.is_contiguous())
     m = GPTModel(GPTConfig(vocab_size=64, hidden_size=128, num_layers=3, num_attention_heads=2,
                            max_position_embeddings=16, intermediate_size=64))
     for p in m.parameters():
@@ -53,3 +55,117 @@ def _share_gradient(m):
 def test_shared_parameters_take_the_module_path(model, share):
     share(model)
     assert native.plan_for(model, IDS) is None
+
+
+class _OtherLinear(torch.nn.Module):
+    bias = None
+
+    def __init__(self, weight):
+        super().__init__()
+        self.weight = weight
+
+
+def _subclass_linear(m):
+    a = m.layers[1].attention
+    new = type("Scaled", (type(a.out_proj),), {})(128, 128, bias=False)
+    new.weight = a.out_proj.weight
+    a.out_proj = new
+
+
+def _other_linear(m):
+    m.layers[1].mlp.down_proj = _OtherLinear(m.layers[1].mlp.down_proj.weight)
+
+
+def _retype(m):
+    m.layers[2].__class__ = type("Block", (type(m.layers[2]),), {})
+
+
+def _own_forward(m):
+    m.layers[0].mlp.forward = types.MethodType(lambda self, x, residual=None: x, m.layers[0].mlp)
+
+
+def _attach_bias(m):
+    m.layers[2].attention.qkv_proj.bias = torch.nn.Parameter(torch.zeros(384))
+
+
+def _head_bias(m):
+    m.output.bias = torch.nn.Parameter(torch.zeros(64))
+
+
+def _other_impl(m):
+    m.layers[1].attention.attention_impl = "reference"
+
+
+def _hook(m):
+    m.layers[1].attention.rotary_emb.register_forward_hook(lambda *a: None)
+
+
+def _uneven_dropout(m):
+    m.layers[1].dropout_prob = 0.25
+
+
+def _vocabulary_slice(m):
+    m.embedding.vocab_start_index = 8
+
+
+def _other_stack(m):
+    m.layers = torch.nn.Sequential(*m.layers)
+
+
+def _view_of_weight(m):
+    w = m.layers[1].attention.out_proj.weight        # same parameter, same address, other strides
+    w.data = w.data.t()
+
+
+def _shorter_table(m):
+    r = m.layers[1].attention.rotary_emb
+    r.cos_cached, r.sin_cached = r.cos_cached[:4], r.sin_cached[:4]
+
+
+def _wrapped_embedding(m):
+    m.embedding = torch.nn.Sequential(m.embedding)
+
+
+def _freeze(m):
+    m.layers[0].mlp.gate_up_proj.weight.requires_grad_(False)
+
+
+@pytest.mark.parametrize("change", [
+    _subclass_linear, _other_linear, _retype, _own_forward, _attach_bias, _head_bias, _other_impl, _hook, _uneven_dropout,
+    _vocabulary_slice, _other_stack, _view_of_weight, _shorter_table, _wrapped_embedding, _freeze])
+def test_changes_after_a_native_pass_take_the_module_path(model, change):
+    change(model)
+    assert native.plan_for(model, IDS) is None
+
+
+@pytest.mark.parametrize("cls", ["RMSNorm", "TransformerLayer", "RotaryEmbedding"])
+def test_replaced_class_method_takes_the_module_path(model, monkeypatch, cls):
+    monkeypatch.setattr(getattr(native, cls), "forward", lambda self, *a, **k: None)
+    assert native.plan_for(model, IDS) is None
+
+
+def test_changed_settings_are_followed(model):
+    """Values that the modules read in each pass, tables and weights that are exchanged for others."""
+    model.layers[1].post_attention_norm.eps = 0.5
+    model.final_norm.eps = 0.25
+    for layer in model.layers:
+        layer.dropout_prob = 0.125
+    table = model.layers[2].attention.rotary_emb
+    table.cos_cached = table.cos_cached * 0.5
+    old = model.layers[0].mlp.down_proj.weight
+    model.layers[0].mlp.down_proj.weight = new = torch.nn.Parameter(old.detach().clone())
+    new.grad, new._grad_sink_ok = torch.zeros_like(new), True
+    plan = native.plan_for(model, IDS)
+    assert plan.params[1].eps[1] == 0.5 and plan.dims.eps_final == 0.25 and plan.dropout == 0.125
+    assert plan.params[2].cos_table == table.cos_cached.data_ptr() != plan.params[1].cos_table
+    assert plan.params[0].w[5] == new.data_ptr()
+    model.eval()
+    assert native.plan_for(model, IDS).dropout == 0.0
+
+
+def test_tables_grow_with_the_sequence(model):
+    """Positions past max_position_embeddings, as through the modules: every block's own table grows."""
+    plan = native.plan_for(model, torch.zeros(1, 40, dtype=torch.int64))
+    for bp, layer in zip(plan.params, model.layers):
+        cos = layer.attention.rotary_emb.cos_cached
+        assert cos.shape[0] == 40 and bp.cos_table == cos.data_ptr()
