@@ -28,9 +28,9 @@ class GPTModel(nn.Module):
     def forward(self, inputs, return_ce_stats: bool = False):
         """``return_ce_stats=True`` returns ``(logits, partials)``: the LM head's GEMM epilogue also
         emits the softmax statistics the loss needs (``None`` on paths without that epilogue)."""
-        plan = native.plan_for(self, inputs)
-        if plan is not None:                       # one tensor-parallel rank, bf16: a few native calls
-            return native.forward(plan, inputs, return_ce_stats)
+        run = native.plan_for(self, inputs)
+        if run is not None:                        # one tensor-parallel rank, bf16: a few native calls
+            return native.forward(run, inputs, return_ce_stats)
         hidden = self.embedding(inputs)            # [S/P, B, H]
         for layer in self.layers:
             hidden = layer(hidden)

@@ -174,7 +174,6 @@ class _Plan:
         self.top_args = _Top(V=w_out.shape[0])
         for k, w in enumerate(self.top):
             self.top_args.w[k] = w.data_ptr()
-        self.shape = self.step_shape = None   # (S, B, dropout) the workspace sizes were computed for
 
     @classmethod
     def of(cls, model) -> "_Plan | None":
@@ -213,44 +212,58 @@ class _Plan:
                 grown = True
         return grown
 
-    def set_mode(self) -> bool:
-        """Take the dropout probability of this pass; False if the blocks differ in it."""
+    def dropout_now(self) -> float | None:
+        """The dropout probability of a pass that starts now; ``None`` if the blocks differ in it."""
         training = self.layer_dicts[0]["training"]
         if self.dropout_prob != 0.0 and any(d["training"] != training for d in self.layer_dicts):
-            return False
-        self.dropout = self.dropout_prob if training else 0.0
-        return True
+            return None
+        return self.dropout_prob if training else 0.0
 
-    def set_shape(self, S: int, B: int) -> None:
-        d = self.dims
+
+class _Pass:
+    """The arguments of one pass: copies of its own, because the library reads them without the interpreter lock
+    while other threads start passes of the same model, and because a backward may come long after its forward."""
+    __slots__ = ("plan", "S", "B", "dropout", "dims", "params")
+
+    def __init__(self, plan: _Plan, S: int, B: int, dropout: float):
+        self.plan, self.S, self.B, self.dropout = plan, S, B, dropout     # the plan also keeps the tables alive
+        d = self.dims = _Dims.from_buffer_copy(plan.dims)
+        d.S, d.B, d.dropout_p = S, B, dropout
         d.pair_min_tiles = gemm_ops.pair_threshold()
         d.grouped_wgrad = 1 if gemm_ops._WGRAD_GROUPING else 0
-        key = (S, B, self.dropout)
-        if key != self.shape:
-            d.S, d.B, d.dropout_p = S, B, self.dropout
-            out_off = c_size_t()
-            lib = _lib.lib()
-            self.act_bytes = lib.gfs_blocks_act_bytes(byref(d), byref(out_off))
-            self.bwd_bytes = lib.gfs_blocks_bwd_bytes(byref(d))
-            self.shape = key
+        self.params = type(plan.params).from_buffer_copy(plan.params)
 
-    def draw_seeds(self) -> list:
+    def act_bytes(self) -> int:
+        return _lib.lib().gfs_blocks_act_bytes(byref(self.dims), byref(c_size_t()))
+
+    def bwd_bytes(self) -> int:
+        return _lib.lib().gfs_blocks_bwd_bytes(byref(self.dims))
+
+    def draw_seeds(self) -> None:
         """Two dropout seeds per block, in the order the modules would draw them."""
-        seeds = torch.randint(0, 2 ** 62, (2 * len(self.layers),)).tolist()   # host generator: no device sync
-        self.put_seeds(seeds)
-        return seeds
+        seeds = torch.randint(0, 2 ** 62, (2 * len(self.params),)).tolist()   # host generator: no device sync
+        for bp, s0, s1 in zip(self.params, seeds[0::2], seeds[1::2]):
+            bp.seed[0], bp.seed[1] = s0, s1
 
-    def put_gradients(self) -> None:
+    def put_gradients(self, params) -> None:
         """Where the blocks' weight gradients go, and whether they are added to what is there."""
-        for bp, ws in zip(self.params, self.weights):
+        for bp, ws in zip(params, self.plan.weights):
             g, acc = bp.g, bp.accumulate
             for k, w in enumerate(ws):
                 g[k] = w.grad.data_ptr()
                 acc[k] = _consume(w)
 
-    def put_seeds(self, seeds: list) -> None:
-        for bp, s0, s1 in zip(self.params, seeds[0::2], seeds[1::2]):
-            bp.seed[0], bp.seed[1] = s0, s1
+    def for_backward(self, weights):
+        """The blocks' arguments with ``weights`` (as autograd returns them) and their gradients."""
+        params = type(self.params).from_buffer_copy(self.params)
+        it = iter(weights)
+        for bp, ws in zip(params, self.plan.weights):
+            for k, w in enumerate(ws):
+                t = next(it)
+                assert t.shape == w.shape and _native_tensor(t, torch.bfloat16), "a weight changed since the forward"
+                bp.w[k] = t.data_ptr()
+        self.put_gradients(params)
+        return params
 
 
 # beside the modules, not in them: a plan holds raw addresses, which must not travel with a model that
@@ -258,23 +271,31 @@ class _Plan:
 _plans: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 
 
-def plan_for(model, inputs: torch.Tensor):
-    """The model's plan if this pass can run natively, else ``None``."""
+def _renew(model) -> _Plan | None:
+    plan = _Plan.of(model)
+    if plan is None:
+        _plans.pop(model, None)
+    else:
+        _plans[model] = plan
+    return plan
+
+
+def plan_for(model, inputs: torch.Tensor) -> _Pass | None:
+    """The arguments of a pass over ``inputs`` if it can run natively, else ``None``."""
     if not (inputs.dim() == 2 and inputs.numel() > 0) or ps.get_tensor_model_parallel_world_size() != 1:
         return None
     S = inputs.shape[1]
     plan = _plans.get(model)
     if plan is None or not plan.current():
-        plan = _Plan.of(model)
-    if plan is not None and not plan.plain_modules():
+        plan = _renew(model)
+    if plan is None or not plan.plain_modules():
         return None
-    if plan is not None and plan.grow_tables(S):
-        plan = _Plan.of(model)
-    if plan is None:
-        _plans.pop(model, None)
-        return None
-    _plans[model] = plan
-    if inputs.device != plan.top[0].device or S > plan.table_rows or not plan.set_mode():
+    if plan.grow_tables(S):
+        plan = _renew(model)
+        if plan is None:
+            return None
+    dropout = plan.dropout_now()
+    if inputs.device != plan.top[0].device or S > plan.table_rows or dropout is None:
         return None
     if torch.is_grad_enabled():
         slices = set()
@@ -285,43 +306,44 @@ def plan_for(model, inputs: torch.Tensor):
             slices.add(p.grad.data_ptr())
         if len(slices) != len(plan.all_params):
             return None
-    return plan
+    return _Pass(plan, S, inputs.shape[0], dropout)
 
 
-def _stack_forward(plan: _Plan, x: torch.Tensor, keep: bool):
+def _stack_forward(run: _Pass, x: torch.Tensor, keep: bool):
     """Blocks + final norm on ``x [S, B, H]`` -> (y [S*B, H], what the backward needs)."""
     S, B, H = x.shape
     dev = x.device
-    n = len(plan.layers)
-    seeds = plan.draw_seeds() if plan.dropout > 0.0 else None
-    acts = [torch.empty(plan.act_bytes, dtype=torch.uint8, device=dev) for _ in range(n if keep else 1)]
+    n = len(run.params)
+    drop = run.dropout > 0.0
+    act_bytes = run.act_bytes()
+    acts = [torch.empty(act_bytes, dtype=torch.uint8, device=dev) for _ in range(n if keep else 1)]
     addr = (c_ulonglong * n)(*[(acts[i] if keep else acts[0]).data_ptr() for i in range(n)])
     y = torch.empty((S * B, H), dtype=torch.bfloat16, device=dev)
     rstd = torch.empty(S * B, dtype=torch.float32, device=dev)
-    tmp = torch.empty_like(y) if seeds is not None else None
+    tmp = torch.empty_like(y) if drop else None
+    if drop:
+        run.draw_seeds()
     launches = c_int(0)
     with _lib.nvtx("fused:blocks_fwd"):
-        rc = _lib.lib().gfs_blocks_forward(byref(plan.dims), plan.params, plan.top[1].data_ptr(), x.data_ptr(), addr,
+        rc = _lib.lib().gfs_blocks_forward(byref(run.dims), run.params, run.plan.top[1].data_ptr(), x.data_ptr(), addr,
                                            _lib.ptr(tmp), y.data_ptr(), rstd.data_ptr(), byref(launches),
                                            _lib.stream_ptr())
     _lib.check(rc, "gfs_blocks_forward")
     _lib.add_launches(launches.value - 1)
-    return y, (x, rstd, acts, seeds)
+    return y, rstd, acts
 
 
-def _stack_backward(plan: _Plan, x, rstd, acts, seeds, dy: torch.Tensor) -> torch.Tensor:
-    n = len(plan.layers)
-    plan.put_gradients()
-    if seeds is not None:
-        plan.put_seeds(seeds)
-    w_fin = plan.top[1]
+def _stack_backward(run: _Pass, weights, w_fin, x, rstd, acts, dy: torch.Tensor) -> torch.Tensor:
+    n = len(run.params)
     addr = (c_ulonglong * n)(*[t.data_ptr() for t in acts])
-    scratch = torch.empty(plan.bwd_bytes, dtype=torch.uint8, device=x.device)
+    scratch = torch.empty(run.bwd_bytes(), dtype=torch.uint8, device=x.device)
     dx = torch.empty_like(x)
+    p_fin = run.plan.top[1]
+    params = run.for_backward(weights)
     launches = c_int(0)
     with _lib.nvtx("fused:blocks_bwd"):
-        rc = _lib.lib().gfs_blocks_backward(byref(plan.dims), plan.params, w_fin.data_ptr(), w_fin.grad.data_ptr(),
-                                            _consume(w_fin), x.data_ptr(), addr, rstd.data_ptr(), dy.data_ptr(),
+        rc = _lib.lib().gfs_blocks_backward(byref(run.dims), params, w_fin.data_ptr(), p_fin.grad.data_ptr(),
+                                            _consume(p_fin), x.data_ptr(), addr, rstd.data_ptr(), dy.data_ptr(),
                                             scratch.data_ptr(), dx.data_ptr(), byref(launches), _lib.stream_ptr())
     _lib.check(rc, "gfs_blocks_backward")
     _lib.add_launches(launches.value - 1)
@@ -331,18 +353,19 @@ def _stack_backward(plan: _Plan, x, rstd, acts, seeds, dy: torch.Tensor) -> torc
 class _ModelFn(torch.autograd.Function):
     """logits ``[S, B, V]`` (and, for the loss, the LM head's softmax statistics) from token ids. The
     embedding weight is an input so that the result requires a gradient; all weight gradients go
-    to their sinks."""
+    to their sinks. The other weights are saved like the modules save theirs: autograd notices one that is
+    written to before the backward."""
 
     @staticmethod
-    def forward(ctx, ids, w_emb, plan, ce_stats):
+    def forward(ctx, ids, w_emb, run, ce_stats):
         B, S = ids.shape
         x = embedding_fwd_native(ids, w_emb, 0, w_emb.shape[0])
         ctx.sorted_ids = sort_ids_async(ids, 0, w_emb.shape[0])   # needed by the backward; side stream
-        y, (x, rstd, acts, seeds) = _stack_forward(plan, x, keep=True)
-        w_out = plan.top[2]
+        y, rstd, acts = _stack_forward(run, x, keep=True)
+        w_out = run.plan.top[2]
         logits, partials = gemm_ops.linear_fwd_ce(y, w_out) if ce_stats else (gemm_ops.linear_fwd(y, w_out), None)
-        ctx.save_for_backward(ids, x, y, rstd, *acts)
-        ctx.plan, ctx.seeds, ctx.key = plan, seeds, (S, B, plan.dropout)
+        ctx.save_for_backward(ids, x, y, rstd, *acts, *run.plan.all_params[:-3], *run.plan.top[1:])
+        ctx.run = run
         logits = logits.view(S, B, -1)
         if not ce_stats:
             return logits
@@ -353,44 +376,40 @@ class _ModelFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dlogits, _dpartials=None):
-        plan = ctx.plan
-        ids, x, y, rstd, *acts = ctx.saved_tensors
-        S, B, dropout = ctx.key
-        if ctx.key != plan.shape:       # another pass of the model ran in between
-            plan.dropout = dropout
-            plan.set_shape(S, B)
-        w_emb, _, w_out = plan.top
-        d2 = dlogits.reshape(S * B, w_out.shape[0])
+        run = ctx.run
+        n = len(run.params)
+        ids, x, y, rstd, *saved = ctx.saved_tensors
+        acts, weights, (w_fin, w_out) = saved[:n], saved[n:-2], saved[-2:]
+        p_emb, _, p_out = run.plan.top
+        d2 = dlogits.reshape(run.S * run.B, w_out.shape[0])
         if not d2.is_contiguous():
             d2 = d2.contiguous()
         dy = gemm_ops.linear_dgrad(d2, w_out)
-        gemm_ops.linear_wgrad_to_sink(d2, y, GradSink(w_out))
-        dx = _stack_backward(plan, x, rstd, acts, ctx.seeds, dy)
-        embedding_bwd_native(ids, dx, w_emb.grad, 0, w_emb.shape[0], accumulate=bool(_consume(w_emb)),
+        gemm_ops.linear_wgrad_to_sink(d2, y, GradSink(p_out))
+        dx = _stack_backward(run, weights, w_fin, x, rstd, acts, dy)
+        embedding_bwd_native(ids, dx, p_emb.grad, 0, p_emb.shape[0], accumulate=bool(_consume(p_emb)),
                              sorted_ids=ctx.sorted_ids)
         return None, None, None, None
 
 
-def forward(plan: _Plan, inputs: torch.Tensor, ce_stats: bool):
+def forward(run: _Pass, inputs: torch.Tensor, ce_stats: bool):
     """The model's forward on the native path: ``logits`` or ``(logits, partials or None)``."""
     ids = inputs.contiguous()
     if ids.dtype != torch.int64:
         ids = ids.long()
-    B, S = ids.shape
-    w_emb, _, w_out = plan.top
-    plan.set_shape(S, B)
+    w_emb, _, w_out = run.plan.top
     if torch.is_grad_enabled():
-        out = _ModelFn.apply(ids, w_emb, plan, ce_stats)
+        out = _ModelFn.apply(ids, w_emb, run, ce_stats)
         if not ce_stats:
             return out
         logits, partials = out
         return logits, (partials if partials.numel() else None)
     x = embedding_fwd_native(ids, w_emb, 0, w_emb.shape[0])
-    y, _ = _stack_forward(plan, x, keep=False)
+    y, _, _ = _stack_forward(run, x, keep=False)
     if not ce_stats:
-        return gemm_ops.linear_fwd(y, w_out).view(S, B, -1)
+        return gemm_ops.linear_fwd(y, w_out).view(run.S, run.B, -1)
     logits, partials = gemm_ops.linear_fwd_ce(y, w_out)
-    return logits.view(S, B, -1), partials
+    return logits.view(run.S, run.B, -1), partials
 
 
 def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
@@ -400,35 +419,31 @@ def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
     if (not torch.is_grad_enabled() or labels.shape != inputs.shape or not labels.is_cuda or
             model._forward_hooks or model._forward_pre_hooks or model._backward_hooks or model._backward_pre_hooks):
         return None
-    plan = plan_for(model, inputs)
-    if plan is None:
+    run = plan_for(model, inputs)
+    if run is None:
         return None
-    B, S = inputs.shape
-    if B * S > 32768:       # the embedding backward then sorts its ids with the library's sort
+    if run.B * run.S > 32768:       # the embedding backward then sorts its ids with the library's sort
         return None
+    plan = run.plan
     ids, labels = inputs.contiguous(), labels.contiguous()
     if ids.dtype != torch.int64:
         ids = ids.long()
     if labels.dtype != torch.int64:
         labels = labels.long()
+    lib, dims, top = _lib.lib(), byref(run.dims), _Top.from_buffer_copy(plan.top_args)
     dev = plan.top[0].device
-    plan.set_shape(S, B)
-    if plan.dropout > 0.0:
-        plan.draw_seeds()
-    lib, dims, top = _lib.lib(), byref(plan.dims), plan.top_args
-    if plan.step_shape != plan.shape:
-        plan.step_bytes = lib.gfs_model_step_bytes(dims, byref(top))
-        plan.step_shape = plan.shape
+    arena = torch.empty(lib.gfs_model_step_bytes(dims, byref(top)), dtype=torch.uint8, device=dev)
+    loss = torch.empty((), dtype=torch.float32, device=dev)
+    if run.dropout > 0.0:
+        run.draw_seeds()
     fresh = [getattr(p, "_grad_fresh", False) for p in plan.all_params]
-    plan.put_gradients()
+    run.put_gradients(run.params)
     for k, w in enumerate(plan.top):
         top.g[k] = w.grad.data_ptr()
         top.accumulate[k] = _consume(w)
-    arena = torch.empty(plan.step_bytes, dtype=torch.uint8, device=dev)
-    loss = torch.empty((), dtype=torch.float32, device=dev)
     launches = c_int(0)
     with _lib.nvtx("fused:model_step"):
-        rc = lib.gfs_model_step(dims, plan.params, byref(top), ids.data_ptr(), labels.data_ptr(), arena.data_ptr(),
+        rc = lib.gfs_model_step(dims, run.params, byref(top), ids.data_ptr(), labels.data_ptr(), arena.data_ptr(),
                                 loss.data_ptr(), byref(launches), _lib.stream_ptr())
     if rc == -20:           # ids times tokens do not fit the sort's 32-bit keys: nothing was launched
         for p, f in zip(plan.all_params, fresh):

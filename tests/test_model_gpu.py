@@ -479,3 +479,55 @@ def test_native_pass_follows_changed_modules(cuda_device):
         seen.append(model(ids))
         assert torch.equal(seen[-1], by_modules())
     assert all(not torch.equal(a, b) for a, b in zip(seen, seen[1:]))
+
+
+@pytest.mark.parametrize("dropout", [0.0, 0.1])
+def test_native_passes_overlap_their_backwards(cuda_device, dropout):
+    """Two forwards under autograd, the second of another shape, in another mode and past the rotary tables' length (so
+    that they are made anew), then the backward of each, against the module path. Tolerance as in
+    test_native_model_pass_matches_module_path, for a sum of two gradients."""
+    from gpt_from_scratch_b200.config import GPTConfig
+    from gpt_from_scratch_b200.engine import TrainEngine
+    from gpt_from_scratch_b200.parallel import parallel_state as ps
+    ps.set_device(cuda_device)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_parallel_state(1)
+    cfg = GPTConfig(vocab_size=512, hidden_size=256, num_layers=2, num_attention_heads=4, max_position_embeddings=64,
+                    intermediate_size=512, dropout_prob=dropout)
+    g = torch.Generator().manual_seed(6)
+    a, b = (torch.randint(0, 512, s, generator=g).cuda() for s in ((2, 65), (3, 101)))
+    grads = []
+    for modules in (False, True):
+        eng = TrainEngine(cfg, seed=5)
+        if modules:
+            eng.model.layers[-1].mlp.register_forward_hook(lambda *a: None)
+        torch.manual_seed(11)
+        eng.optimizer.zero_grad()
+        first = eng.forward_loss(a[:, :-1], a[:, 1:])
+        eng.model.eval()
+        second = eng.forward_loss(b[:, :-1], b[:, 1:])
+        del eng.model.layers[0].attention.rotary_emb.cos_cached     # nothing but the passes holds the tables
+        first.backward()
+        second.backward()
+        torch.cuda.synchronize()
+        grads.append(eng.optimizer.grad_buffer.double())
+    rel = (grads[0] - grads[1]).norm() / grads[1].norm()
+    assert rel < (2e-2 if dropout else 4e-3), rel
+
+
+def test_native_pass_notices_weights_written_before_its_backward(cuda_device):
+    from gpt_from_scratch_b200.config import GPTConfig
+    from gpt_from_scratch_b200.engine import TrainEngine
+    from gpt_from_scratch_b200.parallel import parallel_state as ps
+    ps.set_device(cuda_device)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_parallel_state(1)
+    eng = TrainEngine(GPTConfig(vocab_size=512, hidden_size=256, num_layers=2, num_attention_heads=4,
+                                max_position_embeddings=64, intermediate_size=512), seed=5)
+    t = torch.randint(0, 512, (2, 65), generator=torch.Generator().manual_seed(1)).cuda()
+    eng.optimizer.zero_grad()
+    loss = eng.forward_loss(t[:, :-1], t[:, 1:])
+    with torch.no_grad():
+        eng.model.layers[1].mlp.down_proj.weight.mul_(0.5)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        loss.backward()

@@ -1,7 +1,9 @@
 """When the whole-model native passes may serve a model, on the CPU: the device checks are stubbed out, nothing
 is launched. A pass that the native path cannot serve has to go through the modules, also when an earlier pass of the
 same model ran natively."""
+import threading
 import types
+from contextlib import contextmanager
 
 import pytest
 import torch
@@ -169,3 +171,52 @@ def test_tables_grow_with_the_sequence(model):
     for bp, layer in zip(plan.params, model.layers):
         cos = layer.attention.rotary_emb.cos_cached
         assert cos.shape[0] == 40 and bp.cos_table == cos.data_ptr()
+
+
+@contextmanager
+def _fake_library(monkeypatch, **calls):
+    """The native library with some entry points replaced; what runs around them does so on the CPU."""
+    from gpt_from_scratch_b200.ops import _lib
+
+    class Fake:
+        def __getattr__(self, name):
+            return calls.get(name) or getattr(real, name)
+    real, fake = _lib.lib(), Fake()
+    with monkeypatch.context() as m:
+        m.setattr(_lib, "lib", lambda: fake)
+        m.setattr(_lib, "stream_ptr", lambda: 0)
+        m.setattr(native, "embedding_fwd_native", lambda ids, w, v0, v1: torch.zeros(*ids.T.shape, w.shape[1]))
+        m.setattr(native.gemm_ops, "linear_fwd", lambda x, w: torch.zeros(x.shape[0], w.shape[0]))
+        yield
+
+
+def test_passes_of_two_threads_have_their_own_arguments(model, monkeypatch):
+    """The library reads a pass's arguments without the interpreter lock, while another thread starts a pass of
+    another shape (and another dropout mode) on the same model."""
+    for layer in model.layers:
+        layer.dropout_prob = 0.5
+    inside, go_on, seen = threading.Event(), threading.Event(), []
+
+    def blocks_forward(dims, params, *rest):
+        first = not inside.is_set()
+        before = (dims._obj.S, dims._obj.B, dims._obj.dropout_p, [tuple(p.seed) for p in params])
+        if first:
+            inside.set()
+            assert go_on.wait(20)
+        seen.append((before, (dims._obj.S, dims._obj.B, dims._obj.dropout_p, [tuple(p.seed) for p in params])))
+        return 0
+
+    def run(ids, train):
+        with torch.no_grad():
+            model.train(train)
+            model(ids)
+
+    with _fake_library(monkeypatch, gfs_blocks_forward=blocks_forward, gfs_blocks_bwd_bytes=lambda dims: 0):
+        first = threading.Thread(target=run, args=(IDS, True))
+        first.start()
+        assert inside.wait(20)
+        run(torch.zeros(3, 5, dtype=torch.int64), True)
+        go_on.set()
+        first.join()
+    assert [before[:2] for before, _ in seen] == [(5, 3), (8, 2)]
+    assert all(before == after for before, after in seen)
