@@ -38,3 +38,6 @@ class GPTModel(nn.Module):
         if return_ce_stats:
             return self.output(hidden, ce_stats=True)
         return self.output(hidden)                 # [S, B, V/P]
+
+
+native.serve(GPTModel)

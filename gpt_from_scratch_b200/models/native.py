@@ -69,6 +69,15 @@ _FORWARDS = tuple((c, c.forward) for c in (
     ColumnParallelLinear, RowParallelLinear))
 
 
+_model_class = _model_forward = None
+
+
+def serve(model_class) -> None:
+    """``model_class`` is the model that :func:`train_pass` restates (called where the class is defined)."""
+    global _model_class, _model_forward
+    _model_class, _model_forward = model_class, model_class.forward
+
+
 class _Unsupported(Exception):
     """The modules compute something that the native passes do not."""
 
@@ -416,8 +425,12 @@ def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
     """Forward, mean loss and backward of one micro-batch (``[B, S]`` ids and labels) without autograd:
     returns the loss (0-dim fp32) with every weight gradient in its sink, or ``None`` if the model has to
     go through its modules. One call into the library; all intermediates lie in one buffer."""
-    if (not torch.is_grad_enabled() or labels.shape != inputs.shape or not labels.is_cuda or
+    if (type(model) is not _model_class or _model_class.forward is not _model_forward or "forward" in model.__dict__ or
             model._forward_hooks or model._forward_pre_hooks or model._backward_hooks or model._backward_pre_hooks):
+        return None             # the model computes something of its own
+    if not torch.is_grad_enabled():
+        return None
+    if labels.shape != inputs.shape or labels.device != inputs.device:
         return None
     run = plan_for(model, inputs)
     if run is None:

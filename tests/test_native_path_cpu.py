@@ -173,6 +173,56 @@ def test_tables_grow_with_the_sequence(model):
         assert cos.shape[0] == 40 and bp.cos_table == cos.data_ptr()
 
 
+@pytest.fixture
+def step(model, monkeypatch):
+    """``step(model)``: whether the training step in one native call takes the model."""
+    with _fake_library(monkeypatch, gfs_model_step=lambda *a: 0, gfs_model_step_bytes=lambda *a: 1):
+        yield lambda m=model: native.train_pass(m, IDS, IDS) is not None
+
+
+def test_training_step_takes_plain_models_only(model, step, monkeypatch):
+    """A model with a forward of its own (a wrapper, a subclass, a method set on the instance or the class) is called."""
+    assert step()
+
+    class Wrapper(torch.nn.Module):
+        def __init__(self, inner):
+            super().__init__()
+            self.inner = inner
+
+    assert not step(Wrapper(model))
+    model.forward = lambda *a, **k: None
+    assert not step()
+    del model.forward
+    assert step()
+    model.__class__ = type("Sub", (GPTModel,), {})
+    assert not step()
+    model.__class__ = GPTModel
+    monkeypatch.setattr(GPTModel, "forward", lambda *a, **k: None)
+    assert not step()
+
+
+def test_engine_calls_its_own_forward_loss(monkeypatch):
+    """``forward_loss`` replaced in a subclass, on the instance or on the class is what a step runs."""
+    from gpt_from_scratch_b200 import engine as engine_mod
+    cfg = GPTConfig(vocab_size=64, hidden_size=128, num_layers=1, num_attention_heads=2, max_position_embeddings=16,
+                    intermediate_size=64)
+    monkeypatch.setattr(native, "train_pass", lambda *a: torch.tensor(-1.0))
+    base = engine_mod.TrainEngine.forward_loss
+
+    def own(self, x, y):
+        return base(self, x, y) * 0.0 + 7.0
+
+    eng = engine_mod.TrainEngine(cfg, dtype=torch.float32)
+    assert float(eng.train_step(IDS, IDS)) == -1.0
+    eng.forward_loss = types.MethodType(own, eng)
+    assert float(eng.train_step(IDS, IDS)) == 7.0
+    del eng.forward_loss
+    sub = type("Sub", (engine_mod.TrainEngine,), {"forward_loss": own})(cfg, dtype=torch.float32)
+    assert float(sub.train_step(IDS, IDS)) == 7.0
+    monkeypatch.setattr(engine_mod.TrainEngine, "forward_loss", own)
+    assert float(eng.train_step(IDS, IDS)) == 7.0
+
+
 @contextmanager
 def _fake_library(monkeypatch, **calls):
     """The native library with some entry points replaced; what runs around them does so on the CPU."""
