@@ -301,6 +301,7 @@ class DistributedOptimizer:
                 p.grad.zero_()
                 p._grad_fresh = False
             return None
+        hook.clears_slice = True    # no observer of the gradient
         return hook
 
     def _materialise_unwritten(self) -> None:

@@ -223,6 +223,28 @@ def test_engine_calls_its_own_forward_loss(monkeypatch):
     assert float(eng.train_step(IDS, IDS)) == 7.0
 
 
+def test_observers_of_gradients_are_served(model, step):
+    """Who asks to see single gradients or what autograd saves gets a pass under autograd; tangents are refused by
+    the modules, so they must reach them."""
+    w = model.layers[1].mlp.down_proj.weight
+    w.register_hook(lambda g: None).remove()
+    assert step()
+    for register in (w.register_hook, w.register_post_accumulate_grad_hook):
+        handle = register(lambda g: None)
+        assert native.plan_for(model, IDS) is None and not step()
+        handle.remove()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t):
+        assert not step()
+    with torch.autograd.set_detect_anomaly(True):
+        assert not step()
+    with torch.autograd.forward_ad.dual_level(), torch.no_grad():
+        assert native.plan_for(model, IDS) is None
+    w.grad = torch.zeros_like(w.T.contiguous()).T            # of the weight's shape, but strided
+    assert not step()
+    w.grad = torch.zeros_like(w)
+    assert step()
+
+
 @contextmanager
 def _fake_library(monkeypatch, **calls):
     """The native library with some entry points replaced; what runs around them does so on the CPU."""
