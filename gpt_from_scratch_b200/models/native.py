@@ -297,6 +297,11 @@ def _observed(hooks) -> bool:
     return False
 
 
+def _autograd_is_watched() -> bool:
+    """Somebody wants to see what autograd saves (hooks, as for offloading) or every gradient (anomaly mode)."""
+    return torch.is_anomaly_enabled() or torch._C._autograd._top_saved_tensors_default_hooks(False) is not None
+
+
 def plan_for(model, inputs: torch.Tensor) -> _Pass | None:
     """The arguments of a pass over ``inputs`` if it can run natively, else ``None``."""
     if not (inputs.dim() == 2 and inputs.numel() > 0) or ps.get_tensor_model_parallel_world_size() != 1:
@@ -317,6 +322,8 @@ def plan_for(model, inputs: torch.Tensor) -> _Pass | None:
     if inputs.device != plan.top[0].device or S > plan.table_rows or dropout is None:
         return None
     if torch.is_grad_enabled():
+        if _autograd_is_watched():
+            return None
         slices = set()
         for p in plan.all_params:
             # every gradient goes to a slice of its own in the optimizer's buffer and nobody waits for single ones
@@ -435,11 +442,6 @@ def forward(run: _Pass, inputs: torch.Tensor, ce_stats: bool):
     return logits.view(run.S, run.B, -1), partials
 
 
-def _autograd_is_watched() -> bool:
-    """Somebody wants to see what autograd saves (hooks, as for offloading) or every gradient (anomaly mode)."""
-    return torch.is_anomaly_enabled() or torch._C._autograd._top_saved_tensors_default_hooks(False) is not None
-
-
 def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
     """Forward, mean loss and backward of one micro-batch (``[B, S]`` ids and labels) without autograd:
     returns the loss (0-dim fp32) with every weight gradient in its sink, or ``None`` if the model has to
@@ -447,7 +449,7 @@ def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
     if (type(model) is not _model_class or _model_class.forward is not _model_forward or "forward" in model.__dict__ or
             model._forward_hooks or model._forward_pre_hooks or model._backward_hooks or model._backward_pre_hooks):
         return None             # the model computes something of its own
-    if not torch.is_grad_enabled() or _autograd_is_watched() or not gemm_ops._CE_EPILOGUE:
+    if not torch.is_grad_enabled() or not gemm_ops._CE_EPILOGUE:
         return None
     if labels.shape != inputs.shape or labels.device != inputs.device:
         return None
