@@ -43,6 +43,7 @@ int gfs_dropout_residual(const void* x, const void* residual, void* out, long lo
 int gfs_swiglu_bwd(const void* dact, const void* gu, void* dgu, int M, int I, void* stream);
 int gfs_embedding_fwd(const void* ids, const void* W, void* out, int B, int S, int H, int v0, int v1, int s0,
                       int s_count, void* stream);
+int gfs_embedding_sort_shift(long long n, int v);
 int gfs_embedding_sort_keys(const void* ids_bs, void* keys, int B, int S, int v0, int v1, void* stream);
 int gfs_embedding_bwd_keys(const void* keys, const void* dout, void* dW, int n, int H, int shift, void* stream);
 int gfs_gemm2_ce_parts(int N);

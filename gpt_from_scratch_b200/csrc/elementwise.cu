@@ -727,14 +727,20 @@ int gfs_embedding_bwd(const void* sorted_ids, const void* perm, const void* dout
 //                            (n > 32768 or the key does not fit 32 bits: the caller then sorts
 //                            elsewhere and uses gfs_embedding_bwd)
 //   gfs_embedding_bwd_keys   dW [v1 - v0, H] += segmented sum of dout [S, B, H] in key order
-int gfs_embedding_sort_keys(const void* ids_bs, void* keys, int B, int S, int v0, int v1, void* stream_) {
-  const long long n64 = static_cast<long long>(B) * S;
-  if (n64 <= 0) return -1;
-  if (n64 > 32768) return -20;
-  const int n = static_cast<int>(n64);
+//   gfs_embedding_sort_shift what the first one would return for n tokens and a vocabulary of v rows
+int gfs_embedding_sort_shift(long long n, int v) {
+  if (n <= 0 || v < 0) return -1;
+  if (n > 32768) return -20;
   int npow2 = 2, shift = 1;
   while (npow2 < n) { npow2 <<= 1; ++shift; }
-  if ((static_cast<unsigned long long>(v1 - v0) << shift) >= 0xFFFFFFFFull) return -20;
+  return (static_cast<unsigned long long>(v) << shift) >= 0xFFFFFFFFull ? -20 : shift;
+}
+
+int gfs_embedding_sort_keys(const void* ids_bs, void* keys, int B, int S, int v0, int v1, void* stream_) {
+  const long long n64 = static_cast<long long>(B) * S;
+  const int shift = gfs_embedding_sort_shift(n64, v1 - v0);
+  if (shift < 0) return shift;
+  const int n = static_cast<int>(n64), npow2 = 1 << shift;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   static bool attr_set = false;
   if (!attr_set) {

@@ -14,6 +14,8 @@
 // Single tensor-parallel rank only (no collectives).
 #include <algorithm>
 #include <cmath>
+#include <memory>
+#include <new>
 
 #include "api.h"
 #include "common.cuh"
@@ -374,10 +376,16 @@ struct StepLayout {
 };
 
 // The id sort of the embedding backward needs only the ids: it runs beside the forward on a stream of
-// its own (one per thread and device, so that neither threads nor captures meet in its events).
+// its own (one per thread and device, so that neither threads nor captures meet in its events; given back when
+// the thread ends).
 struct SideStream {
   cudaStream_t stream = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
+  ~SideStream() {
+    if (join != nullptr) cudaEventDestroy(join);
+    if (fork != nullptr) cudaEventDestroy(fork);
+    if (stream != nullptr) cudaStreamDestroy(stream);
+  }
 };
 SideStream* side_stream() {
   static thread_local SideStream per_dev[64];
@@ -393,50 +401,16 @@ SideStream* side_stream() {
   return &s;
 }
 
-}  // namespace
-
-extern "C" {
-
-size_t gfs_model_step_bytes(const GfsBlockDims* d, const GfsModelTop* t) {
-  return StepLayout(*d, *t, ActLayout(*d)).total;
-}
-
-// One micro-batch: ids, labels int64 [B, S] -> *loss (fp32, mean over all tokens) and all weight
-// gradients. arena: gfs_model_step_bytes bytes. Returns -20 (nothing launched) when the batch does not
-// fit the single-CTA id sort of the embedding backward.
-int gfs_model_step(const GfsBlockDims* dp, const GfsBlockParams* layers, const GfsModelTop* tp, const void* ids,
-                   const void* labels, void* arena, void* loss, int* launches, void* stream) {
-  const GfsBlockDims& d = *dp;
-  const GfsModelTop& t = *tp;
-  if (!dims_ok(d) || (t.V & 7)) return -1;
-  const ActLayout a(d);
-  const StepLayout lay(d, t, a);
+// The step without the embedding's backward (but with its gradient cleared): logits, loss, and back.
+int step_until_embedding(const GfsBlockDims& d, const GfsBlockParams* layers, const GfsModelTop& t, const void* ids,
+                         const void* labels, char* m, const StepLayout& lay, const u64* act, void* loss, int* launches,
+                         cudaStream_t stream) {
   const int T = d.S * d.B, H = d.H, V = t.V;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  char* m = static_cast<char*>(arena);
-  void *x0 = m + lay.x0, *y = m + lay.y_final, *rstd = m + lay.rstd_final, *keys = m + lay.keys, *targets = m + lay.targets,
+  void *x0 = m + lay.x0, *y = m + lay.y_final, *rstd = m + lay.rstd_final, *targets = m + lay.targets,
        *rows = m + lay.loss_rows, *stats = m + lay.stats, *lse = m + lay.lse, *dy = m + lay.dy, *dx0 = m + lay.dx0,
        *logits = m + lay.logits, *partials = m + lay.partials, *scratch = m + lay.scratch;
-
-  SideStream* side = side_stream();
-  if (side == nullptr) return -10;
-  if (T > 32768) return -20;
-  if (cudaEventRecord(side->fork, st) != cudaSuccess || cudaStreamWaitEvent(side->stream, side->fork, 0) != cudaSuccess)
-    return -11;
-  const int shift = gfs_embedding_sort_keys(ids, keys, d.B, d.S, 0, V, side->stream);
-  if (cudaEventRecord(side->join, side->stream) != cudaSuccess) return -11;
-  if (shift <= 0) {
-    cudaStreamWaitEvent(st, side->join, 0);   // a capture must not end with the fork open
-    return shift == 0 ? -1 : shift;
-  }
-  ++*launches;
-
   GFS_TRY(gfs_embedding_fwd(ids, t.w_emb, x0, d.B, d.S, H, 0, V, 0, d.S, stream));
-  constexpr int MAX_LAYERS = 512;
-  if (d.n_layers > MAX_LAYERS) return -1;
-  u64 act[MAX_LAYERS];
-  for (int l = 0; l < d.n_layers; ++l) act[l] = reinterpret_cast<u64>(m + lay.acts + a.total * l);
-  int rc = gfs_blocks_forward(dp, layers, t.w_final, x0, act, scratch, y, rstd, launches, stream);
+  int rc = gfs_blocks_forward(&d, layers, t.w_final, x0, act, scratch, y, rstd, launches, stream);
   if (rc != 0) return rc;
 
   // LM head and loss
@@ -465,12 +439,51 @@ int gfs_model_step(const GfsBlockDims* dp, const GfsBlockParams* layers, const G
   rc = weight_grad(d, grp, logits, y, t.g_out, t.acc_out, T, V, H, launches, stream);
   if (rc == 0) rc = grp.flush(launches, stream);
   if (rc != 0) return rc;
-  rc = gfs_blocks_backward(dp, layers, t.w_final, t.g_final, t.acc_final, x0, act, rstd, dy, scratch, dx0, launches,
+  rc = gfs_blocks_backward(&d, layers, t.w_final, t.g_final, t.acc_final, x0, act, rstd, dy, scratch, dx0, launches,
                            stream);
   if (rc != 0) return rc;
-  if (!t.acc_emb && cudaMemsetAsync(t.g_emb, 0, 2 * static_cast<size_t>(V) * H, st) != cudaSuccess) return -11;
-  if (cudaStreamWaitEvent(st, side->join, 0) != cudaSuccess) return -11;
-  GFS_TRY(gfs_embedding_bwd_keys(keys, dx0, t.g_emb, T, H, shift, stream));
+  return !t.acc_emb && cudaMemsetAsync(t.g_emb, 0, 2 * static_cast<size_t>(V) * H, stream) != cudaSuccess ? -11 : 0;
+}
+
+}  // namespace
+
+extern "C" {
+
+// 0: the batch does not fit the single-CTA id sort of the embedding backward.
+size_t gfs_model_step_bytes(const GfsBlockDims* d, const GfsModelTop* t) {
+  if (gfs_embedding_sort_shift(static_cast<long long>(d->B) * d->S, t->V) <= 0) return 0;
+  return StepLayout(*d, *t, ActLayout(*d)).total;
+}
+
+// One micro-batch: ids, labels int64 [B, S] -> *loss (fp32, mean over all tokens) and all weight
+// gradients. arena: gfs_model_step_bytes bytes. Arguments that cannot be served are refused before anything is
+// launched; after an error of a launch the caller's stream still waits for the sort, which writes to the arena.
+int gfs_model_step(const GfsBlockDims* dp, const GfsBlockParams* layers, const GfsModelTop* tp, const void* ids,
+                   const void* labels, void* arena, void* loss, int* launches, void* stream) {
+  const GfsBlockDims& d = *dp;
+  const GfsModelTop& t = *tp;
+  if (!dims_ok(d) || (t.V & 7) || gfs_embedding_sort_shift(static_cast<long long>(d.B) * d.S, t.V) <= 0) return -1;
+  const ActLayout a(d);
+  const StepLayout lay(d, t, a);
+  char* m = static_cast<char*>(arena);
+  const std::unique_ptr<u64[]> act(new (std::nothrow) u64[d.n_layers + 1]);
+  if (act == nullptr) return -12;
+  for (int l = 0; l < d.n_layers; ++l) act[l] = reinterpret_cast<u64>(m + lay.acts + a.total * l);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  SideStream* side = side_stream();
+  if (side == nullptr) return -10;
+  if (cudaEventRecord(side->fork, st) != cudaSuccess || cudaStreamWaitEvent(side->stream, side->fork, 0) != cudaSuccess)
+    return -11;
+  const int shift = gfs_embedding_sort_keys(ids, m + lay.keys, d.B, d.S, 0, t.V, side->stream);
+  if (cudaEventRecord(side->join, side->stream) != cudaSuccess) {
+    cudaStreamSynchronize(side->stream);
+    return -11;
+  }
+  ++*launches;
+  int rc = shift < 0 ? shift : step_until_embedding(d, layers, t, ids, labels, m, lay, act.get(), loss, launches, st);
+  if (cudaStreamWaitEvent(st, side->join, 0) != cudaSuccess && rc == 0) rc = -11;
+  if (rc != 0) return rc;
+  GFS_TRY(gfs_embedding_bwd_keys(m + lay.keys, m + lay.dx0, t.g_emb, d.S * d.B, d.H, shift, stream));
   return 0;
 }
 

@@ -456,17 +456,23 @@ def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
     run = plan_for(model, inputs)
     if run is None:
         return None
-    if run.B * run.S > 32768:       # the embedding backward then sorts its ids with the library's sort
-        return None
     plan = run.plan
+    if plan.top[0].shape != plan.top[2].shape:      # a vocabulary for both
+        return None
+    lib, dims, top = _lib.lib(), byref(run.dims), _Top.from_buffer_copy(plan.top_args)
+    step_bytes = lib.gfs_model_step_bytes(dims, byref(top))
+    if step_bytes == 0:             # the embedding backward then sorts its ids with torch.sort
+        return None
     ids, labels = inputs.contiguous(), labels.contiguous()
     if ids.dtype != torch.int64:
         ids = ids.long()
     if labels.dtype != torch.int64:
         labels = labels.long()
-    lib, dims, top = _lib.lib(), byref(run.dims), _Top.from_buffer_copy(plan.top_args)
     dev = plan.top[0].device
-    arena = torch.empty(lib.gfs_model_step_bytes(dims, byref(top)), dtype=torch.uint8, device=dev)
+    try:
+        arena = torch.empty(step_bytes, dtype=torch.uint8, device=dev)
+    except torch.OutOfMemoryError:  # no room in one piece: the modules' smaller tensors may still fit
+        return None
     loss = torch.empty((), dtype=torch.float32, device=dev)
     if run.dropout > 0.0:
         run.draw_seeds()
@@ -479,10 +485,9 @@ def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
     with _lib.nvtx("fused:model_step"):
         rc = lib.gfs_model_step(dims, run.params, byref(top), ids.data_ptr(), labels.data_ptr(), arena.data_ptr(),
                                 loss.data_ptr(), byref(launches), _lib.stream_ptr())
-    if rc == -20:           # ids times tokens do not fit the sort's 32-bit keys: nothing was launched
+    if rc != 0:             # the gradients hold nothing of this step
         for p, f in zip(plan.all_params, fresh):
             p._grad_fresh = f
-        return None
     _lib.check(rc, "gfs_model_step")
     _lib.add_launches(launches.value - 1)
     return loss

@@ -72,6 +72,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "gfs_embedding_fwd": ([vp, vp, vp, i, i, i, i, i, i, i, vp], i),
         "gfs_embedding_bwd": ([vp, vp, vp, vp, i, i, i, i, vp], i),
         "gfs_embedding_sort_keys": ([vp, vp, i, i, i, i, vp], i),
+        "gfs_embedding_sort_shift": ([i64, i], i),
         "gfs_embedding_bwd_keys": ([vp, vp, vp, i, i, i, vp], i),
         "gfs_ce_fwd": ([vp, vp, vp, vp, vp, i, i, cl, i, i, i, vp, vp], i),
         "gfs_ce_combine": ([vp, vp, vp, i, i, vp], i),

@@ -531,3 +531,79 @@ def test_native_pass_notices_weights_written_before_its_backward(cuda_device):
         eng.model.layers[1].mlp.down_proj.weight.mul_(0.5)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         loss.backward()
+
+
+def test_step_of_many_blocks(cuda_device):
+    """More than 512 blocks in one native call, against the module path (a hook selects it): the same kernels but for
+    groups of weight gradients, see test_native_model_pass_matches_module_path."""
+    from gpt_from_scratch_b200.config import GPTConfig
+    from gpt_from_scratch_b200.engine import TrainEngine
+    from gpt_from_scratch_b200.models import native
+    from gpt_from_scratch_b200.parallel import parallel_state as ps
+    ps.set_device(cuda_device)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_parallel_state(1)
+    cfg = GPTConfig(vocab_size=64, hidden_size=64, num_layers=520, num_attention_heads=1, max_position_embeddings=32,
+                    intermediate_size=64)
+    t = torch.randint(0, 64, (2, 33), generator=torch.Generator().manual_seed(1)).cuda()
+    x, y = t[:, :-1].contiguous(), t[:, 1:].contiguous()
+    runs = []
+    for modules in (False, True):
+        eng = TrainEngine(cfg, seed=5)
+        if modules:
+            eng.model.layers[0].register_forward_hook(lambda *a: None)
+        eng.optimizer.zero_grad()
+        loss = native.train_pass(eng.model, x, y)
+        assert (loss is None) == modules
+        if modules:
+            loss = eng.forward_loss(x, y)
+            loss.backward()
+        runs.append((float(loss), eng.optimizer.grad_buffer.double()))
+    assert abs(runs[0][0] - runs[1][0]) < 1e-4
+    assert (runs[0][1] - runs[1][1]).norm() < 2e-3 * runs[1][1].norm()
+
+
+def test_two_threads_train_and_evaluate(cuda_device):
+    """Two threads, each on a stream of its own, run one model on inputs of different shapes; both get what they get
+    alone. The trained gradients and the evaluated logits do not depend on the other thread."""
+    import threading
+    from gpt_from_scratch_b200.config import GPTConfig
+    from gpt_from_scratch_b200.engine import TrainEngine
+    from gpt_from_scratch_b200.models import native
+    from gpt_from_scratch_b200.parallel import parallel_state as ps
+    ps.set_device(cuda_device)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_parallel_state(1)
+    cfg = GPTConfig(vocab_size=512, hidden_size=256, num_layers=4, num_attention_heads=4, max_position_embeddings=160,
+                    intermediate_size=512)
+    eng = TrainEngine(cfg, seed=5)
+    g = torch.Generator().manual_seed(6)
+    t, ids = torch.randint(0, 512, (5, 129), generator=g).cuda(), torch.randint(0, 512, (3, 57), generator=g).cuda()
+    x, y = t[:, :-1].contiguous(), t[:, 1:].contiguous()
+
+    def train(out, n=40):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(n):
+                eng.optimizer.zero_grad()
+                out.append((native.train_pass(eng.model, x, y).clone(), eng.optimizer.grad_buffer.clone()))
+            torch.cuda.current_stream().synchronize()
+
+    def evaluate(out, n=80):
+        with torch.cuda.stream(torch.cuda.Stream()), torch.no_grad():
+            for _ in range(n):
+                out.append(eng.model(ids).clone())
+            torch.cuda.current_stream().synchronize()
+
+    torch.cuda.synchronize()
+    alone, logits_alone = [], []
+    train(alone, 1)
+    evaluate(logits_alone, 1)
+    trained, logits = [], []
+    threads = [threading.Thread(target=train, args=(trained,)), threading.Thread(target=evaluate, args=(logits,))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert len(trained) == 40 and len(logits) == 80
+    assert all(torch.equal(a, alone[0][0]) and torch.equal(b, alone[0][1]) for a, b in trained)
+    assert all(torch.equal(a, logits_alone[0]) for a in logits)

@@ -292,3 +292,51 @@ def test_passes_of_two_threads_have_their_own_arguments(model, monkeypatch):
         first.join()
     assert [before[:2] for before, _ in seen] == [(5, 3), (8, 2)]
     assert all(before == after for before, after in seen)
+
+
+def test_step_refuses_before_it_starts(model):
+    """Batches that the id sort cannot take are refused before anything is launched (on the CPU: before the
+    first CUDA call fails)."""
+    from ctypes import byref, c_int
+    from gpt_from_scratch_b200.ops import _lib
+    lib = _lib.lib()
+    run = native.plan_for(model, IDS)
+    top = native._Top.from_buffer_copy(run.plan.top_args)
+    for S, B, V in ((32769, 1, 64), (256, 129, 64), (16384, 2, 1 << 17)):
+        run.dims.S, run.dims.B, top.V = S, B, V
+        assert lib.gfs_embedding_sort_shift(S * B, V) == -20
+        assert lib.gfs_model_step_bytes(byref(run.dims), byref(top)) == 0
+        launches = c_int(0)
+        assert lib.gfs_model_step(byref(run.dims), run.params, byref(top), 0, 0, 0, 0, byref(launches), 0) == -1
+        assert launches.value == 0
+    assert [lib.gfs_embedding_sort_shift(n, 64) for n in (1, 2, 3, 4, 5, 32768)] == [1, 1, 2, 2, 3, 15]
+
+
+def test_failed_or_refused_step_leaves_no_trace(model, monkeypatch):
+    """Whether gradients are overwritten or added to, and the dropout generator, are as before the call."""
+    for layer in model.layers:
+        layer.dropout_prob = 0.5
+    for i, p in enumerate(model.parameters()):
+        p._grad_fresh = i % 2 == 0
+    before = [p._grad_fresh for p in model.parameters()]
+    rng = torch.get_rng_state()
+    with _fake_library(monkeypatch, gfs_model_step=lambda *a: -13, gfs_model_step_bytes=lambda *a: 8):
+        with pytest.raises(RuntimeError, match="gfs_model_step"):
+            native.train_pass(model, IDS, IDS)
+        assert [p._grad_fresh for p in model.parameters()] == before
+
+        def no_room(*a, **k):
+            raise torch.OutOfMemoryError("no room")
+        with monkeypatch.context() as m:
+            torch.set_rng_state(rng)
+            m.setattr(torch, "empty", no_room)
+            assert native.train_pass(model, IDS, IDS) is None
+    with _fake_library(monkeypatch, gfs_model_step=lambda *a: 0, gfs_model_step_bytes=lambda *a: 0):
+        assert native.train_pass(model, IDS, IDS) is None
+    assert [p._grad_fresh for p in model.parameters()] == before and torch.equal(torch.get_rng_state(), rng)
+
+
+def test_step_wants_one_vocabulary(model, step):
+    head = model.output.weight = torch.nn.Parameter(torch.zeros(72, 128))
+    head.grad, head._grad_sink_ok = torch.zeros_like(head), True
+    assert native.plan_for(model, IDS) is not None and not step()
