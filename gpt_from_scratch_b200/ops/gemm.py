@@ -197,6 +197,8 @@ class _WgradQueue:
         return ((M + 255) // 256) * ((N + 255) // 256)
 
     def push(self, dy2d, x2d, out, accumulate, done_cb) -> None:
+        if any(it[2].data_ptr() == out.data_ptr() for it in self.items):
+            self.flush()       # a weight used twice: the second product adds to the first one's result
         self.items.append((dy2d, x2d, out, accumulate, done_cb))
         self.tiles += self.tiles_of(dy2d.shape[1], x2d.shape[1])
         if not self._callback_pending:
@@ -211,10 +213,10 @@ class _WgradQueue:
             self.flush()
 
     def uses(self, tensor: torch.Tensor) -> bool:
-        """True if a parked problem reads from ``tensor``'s memory."""
+        """True if a parked problem reads from or writes to ``tensor``'s memory."""
         lo = tensor.data_ptr()
         hi = lo + tensor.numel() * tensor.element_size()
-        return any(lo <= it[k].data_ptr() < hi for it in self.items for k in (0, 1))
+        return any(lo <= it[k].data_ptr() < hi for it in self.items for k in (0, 1, 2))
 
     def flush(self) -> None:
         items, self.items, self.tiles = self.items, [], 0
@@ -250,8 +252,8 @@ def flush_wgrad() -> None:
 
 
 def flush_wgrad_if_uses(tensor: torch.Tensor) -> None:
-    """Launch the parked weight-gradient GEMMs if one of them still reads ``tensor`` (call before a
-    reused buffer is overwritten)."""
+    """Launch the parked weight-gradient GEMMs if one of them still reads or writes ``tensor`` (call before a
+    reused buffer is overwritten, or a gradient is written by another kernel)."""
     if _wgrad_queue.items and _wgrad_queue.uses(tensor):
         _wgrad_queue.flush()
 
@@ -264,7 +266,8 @@ def linear_wgrad_to_sink(dy2d: torch.Tensor, x2d: torch.Tensor, sink) -> None:
     accumulate = sink.consume_accumulate()
     N_out, N_in = dy2d.shape[1], x2d.shape[1]
     if (_WGRAD_GROUPING and _PAIR_ENABLED and use_native(dy2d, x2d, out)
-            and _WgradQueue.tiles_of(N_out, N_in) < _PAIR_MIN_TILES and N_out % 8 == 0 and N_in % 8 == 0 and out.stride(1) == 1 and out.stride(0) % 8 == 0):
+            and _WgradQueue.tiles_of(N_out, N_in) < _PAIR_MIN_TILES and N_out % 8 == 0 and N_in % 8 == 0
+            and out.stride(1) == 1 and out.stride(0) % 8 == 0):
         _wgrad_queue.push(_rowmajor_2d(dy2d), _rowmajor_2d(x2d), out, accumulate, sink.done)
         if hasattr(sink, "parked"):
             sink.parked()

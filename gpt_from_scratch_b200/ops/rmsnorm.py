@@ -41,8 +41,8 @@ class _DwReduceQueue:
         self.flush()
 
     def push(self, partial, dw, parts, accumulate, H, done_cb) -> None:
-        if self.items and self.items[0][4] != H:
-            self.flush()
+        if self.items and (self.items[0][4] != H or any(it[1].data_ptr() == dw.data_ptr() for it in self.items)):
+            self.flush()       # one launch has one width, and a norm used twice adds to its first use's result
         self.items.append((partial, dw, parts, accumulate, H, done_cb))
         if len(self.items) == self.MAX:
             self.flush()

@@ -424,6 +424,7 @@ class _EmbeddingReduceScatter(torch.autograd.Function):
         v0, v1, sink, wshape, S, B, H = ctx.meta
         full = allgather_rows(_as2d(dout, B * H), "embb").view(S, B, H)
         if sink is not None:
+            gemm_ops.flush_wgrad_if_uses(sink.target())      # a tied head's gradient may still be parked
             embedding_bwd_native(ids, full, sink.target(), v0, v1, accumulate=sink.consume_accumulate(),
                                  sorted_ids=ctx.sorted_ids)
             sink.done()

@@ -226,6 +226,7 @@ class _EmbeddingFn(torch.autograd.Function):
         v0, v1, sink, wshape = ctx.meta
         dout = dout.contiguous()
         if sink is not None:
+            gemm_ops.flush_wgrad_if_uses(sink.target())      # a tied head's gradient may still be parked
             embedding_bwd_native(ids, dout, sink.target(), v0, v1, accumulate=sink.consume_accumulate(),
                                  sorted_ids=ctx.sorted_ids)
             sink.done()

@@ -427,16 +427,25 @@ def _tie_head(m, shared):
     return [("embedding.weight", "output.weight")]
 
 
-@pytest.mark.parametrize("V", [16384])
-def test_tied_head_gets_both_gradients(cuda_device, V):
-    """A head that shares the embedding's weight: its gradient is the sum of the two uses, of this step only. The sum
+def _repeat_block(m, shared):
+    if shared:
+        m.layers[1] = m.layers[0]
+    else:
+        m.layers[1].load_state_dict(m.layers[0].state_dict())
+    return [(f"layers.0.{n}", f"layers.1.{n}") for n, _ in m.layers[0].named_parameters()]
+
+
+@pytest.mark.parametrize("share,V", [(_tie_head, 16384), (_tie_head, 512), (_repeat_block, 512)])
+def test_shared_weights_get_all_their_gradients(cuda_device, share, V):
+    """A head that shares the embedding's weight (its gradient a launch of its own or parked for a grouped one), a
+    block that occurs twice: the gradient is the sum of the two uses, of this step only. The sum
     is rounded to bf16 twice (2^-9 each) on rows that cancel, the uses themselves once."""
     from gpt_from_scratch_b200.parallel import parallel_state as ps
     ps.set_device(cuda_device)
     if not ps.model_parallel_is_initialized():
         ps.initialize_parallel_state(1)
-    tied, apart = _shared_gradients(_tie_head, 256, 2, V)
-    for name, g in tied.items():
+    together, apart = _shared_gradients(share, 256, 2, V)
+    for name, g in together.items():
         rel = (g - apart[name]).norm() / apart[name].norm()
         assert rel < 1e-2, (name, rel)
 

@@ -405,3 +405,36 @@ def test_pending_flag_counts_are_folded_into_the_base_words():
     finally:
         symm._groups.clear()
         symm._groups.update(saved)
+
+
+def test_parked_gradients_of_a_shared_weight_keep_their_order(monkeypatch):
+    """Two gradients with one destination (a tied head, a block that occurs twice) never share a launch, whose
+    problems run side by side; a kernel that writes to a parked destination finds the parked work done."""
+    from gpt_from_scratch_b200.ops import _lib
+    from gpt_from_scratch_b200.ops import gemm as gemm_ops
+    from gpt_from_scratch_b200.ops.rmsnorm import _DwReduceQueue
+    launched = []
+    monkeypatch.setattr(_lib, "stream_ptr", lambda: 0)
+    q = gemm_ops._WgradQueue()
+    monkeypatch.setattr(q, "_launch", lambda items, n: launched.append([(it[2].data_ptr(), it[3]) for it in items]) or 0)
+    dy, x = torch.zeros(4, 8), torch.zeros(4, 8)
+    a, b = torch.zeros(8, 8), torch.zeros(8, 8)
+    q.push(dy, x, a, False, None)
+    q.push(dy, x, b, False, None)
+    q.push(dy, x, a, True, None)
+    assert launched == [[(a.data_ptr(), False), (b.data_ptr(), False)]]
+    assert q.uses(a) and not q.uses(b)
+    q.flush()
+    assert launched[1:] == [[(a.data_ptr(), True)]]
+
+    class Lib:
+        def gfs_rmsnorm_dw_reduce_multi(self, n, partials, dws, parts, accumulate, H, stream):
+            launched.append([(dws[i], accumulate[i]) for i in range(n)])
+            return 0
+    monkeypatch.setattr(_lib, "lib", Lib)
+    launched.clear()
+    q = _DwReduceQueue()
+    for dw, acc in ((a, False), (b, False), (b, True)):
+        q.push(x, dw, 1, acc, 8, None)
+    q.flush()
+    assert launched == [[(a.data_ptr(), 0), (b.data_ptr(), 0)], [(b.data_ptr(), 1)]]
