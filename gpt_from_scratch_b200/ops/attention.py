@@ -162,6 +162,14 @@ def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     return t.contiguous()
 
 
+def _first_keys(q: torch.Tensor, t: torch.Tensor) -> torch.Tensor:
+    """The rows of a longer k or v that the kernels read: one per query. Anything shorter they would read past."""
+    B, nh, S, D = q.shape
+    if t.dim() != 4 or t.shape[:2] != (B, nh) or t.shape[2] < S or t.shape[3] != D:
+        raise ValueError(f"apply_flash_attn: k and v of shape {tuple(t.shape)} do not cover q of shape {tuple(q.shape)}")
+    return t[:, :, :S]
+
+
 def apply_flash_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal_mask: bool = True) -> torch.Tensor:
     """Flash attention on ``[B, nh, S, D]`` tensors (reference API, core/myFlashAttn.py:1321)."""
     D = q.shape[-1]
@@ -171,6 +179,8 @@ def apply_flash_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal_m
             raise ValueError(f"apply_flash_attn: head_dim {D} has no native kernel (64 and 128 do); "
                              "use attention_reference for other sizes")
         if k.is_cuda and v.is_cuda and q.dtype == k.dtype == v.dtype:
+            if k.shape != q.shape or v.shape != q.shape:
+                k, v = _first_keys(q, k), _first_keys(q, v)
             return _FlashAttnBHSD.apply(_tma_ready(q), _tma_ready(k), _tma_ready(v), 1 if causal_mask else 0, scale)
     return attention_reference(q, k, v, causal_mask, scale)
 

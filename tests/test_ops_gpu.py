@@ -311,3 +311,29 @@ def test_flash_attention_api_dtypes_and_layouts(cuda_device, dtype, B, nh, S, D,
             # one token: dQ and dK are exactly zero, what is left is the rounding of dO and V in dP - D
             err = (a.float() - b).norm()
             assert err <= 2e-2 * b.norm() + (2e-2 * D ** 0.5 if S == 1 else 0.0), (name, err.item(), b.norm().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("Sk,Sv", [(200, 130), (130, 200), (300, 300)])
+def test_flash_attention_longer_keys(cuda_device, dtype, Sk, Sv):
+    """k and v of more rows than q are read with their own strides: the first rows, one per query, also where all
+    tensors are contiguous. The rows past them get no gradient. Shorter ones are refused. Tolerance as in
+    test_flash_attention_api_dtypes_and_layouts."""
+    from gpt_from_scratch_b200.ops.attention import apply_flash_attn, attention_reference
+    B, nh, S, D = 2, 3, 130, 64
+    g = torch.Generator(device="cuda").manual_seed(Sk)
+    q, k, v, do = (torch.randn(B, nh, n, D, device=cuda_device, generator=g).to(dtype).requires_grad_()
+                   for n in (S, Sk, Sv, S))
+    for causal in (True, False):
+        o = apply_flash_attn(q, k, v, causal)
+        grads = torch.autograd.grad(o, (q, k, v), do.detach())
+        qf, kf, vf = (t.detach().float().requires_grad_() for t in (q, k, v))
+        of = attention_reference(qf, kf[:, :, :S], vf[:, :, :S], causal)
+        refs = torch.autograd.grad(of, (qf, kf, vf), do.detach().float())
+        for name, a, b in zip(("O", "dQ", "dK", "dV"), (o, *grads), (of, *refs)):
+            assert a.shape == b.shape and (a.float() - b).norm() <= 2e-2 * b.norm(), name
+    for wrong in (k[:, :, :S - 1], k[:, :1], k[:1], k[..., :32], k[0]):
+        with pytest.raises(ValueError, match="cover q"):
+            apply_flash_attn(q, wrong, v)
+        with pytest.raises(ValueError, match="cover q"):
+            apply_flash_attn(q, k, wrong)

@@ -438,3 +438,13 @@ def test_parked_gradients_of_a_shared_weight_keep_their_order(monkeypatch):
         q.push(x, dw, 1, acc, 8, None)
     q.flush()
     assert launched == [[(a.data_ptr(), 0), (b.data_ptr(), 0)], [(b.data_ptr(), 1)]]
+
+
+def test_flash_attention_key_rows():
+    """The rows of k and v that a kernel of q's shape reads have to exist."""
+    from gpt_from_scratch_b200.ops.attention import _first_keys
+    q, k = torch.zeros(2, 3, 8, 64), torch.arange(2 * 3 * 12 * 64.).view(2, 3, 12, 64)
+    assert torch.equal(_first_keys(q, k), k[:, :, :8]) and _first_keys(q, k).stride() == k.stride()
+    for wrong in (k[:, :, :7], k[:, :1], k[:1], k[..., :32], k[0]):
+        with pytest.raises(ValueError, match="cover q"):
+            _first_keys(q, wrong)
