@@ -159,7 +159,7 @@ def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     b, h, s, d = t.stride()
     if d == 1 and not ((b | h | s) & 7) and not t.data_ptr() & 15:
         return t
-    return t.contiguous()
+    return t.clone(memory_format=torch.contiguous_format)   # a copy also where t is contiguous, but at an odd address
 
 
 def _first_keys(q: torch.Tensor, t: torch.Tensor) -> torch.Tensor:

@@ -337,3 +337,21 @@ def test_flash_attention_longer_keys(cuda_device, dtype, Sk, Sv):
             apply_flash_attn(q, wrong, v)
         with pytest.raises(ValueError, match="cover q"):
             apply_flash_attn(q, k, wrong)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_flash_attention_misaligned_tensors(cuda_device, dtype):
+    """Contiguous q, k, v and gradient at odd addresses give what aligned copies of them give."""
+    from gpt_from_scratch_b200.ops.attention import apply_flash_attn
+    B, nh, S, D = 2, 3, 70, 64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    flat = [torch.randn(1 + B * nh * S * D, device=cuda_device, generator=g).to(dtype) for _ in range(4)]
+    results = []
+    for copy in (True, False):
+        q, k, v, do = (t[1:].view(B, nh, S, D) for t in flat)
+        if copy:
+            q, k, v, do = (t.clone() for t in (q, k, v, do))
+        q, k, v = (t.detach().requires_grad_() for t in (q, k, v))
+        o = apply_flash_attn(q, k, v)
+        results.append((o, *torch.autograd.grad(o, (q, k, v), do)))
+    assert all(torch.equal(a, b) for a, b in zip(*results))

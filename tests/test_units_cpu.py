@@ -448,3 +448,16 @@ def test_flash_attention_key_rows():
     for wrong in (k[:, :, :7], k[:, :1], k[:1], k[..., :32], k[0]):
         with pytest.raises(ValueError, match="cover q"):
             _first_keys(q, wrong)
+
+
+def test_flash_attention_misaligned_tensors_are_copied():
+    """TMA wants 16-byte aligned addresses and strides: everything else is copied, contiguous tensors included."""
+    from gpt_from_scratch_b200.ops.attention import _tma_ready
+    base = torch.arange(2 * 3 * 8 * 72 + 8.).bfloat16()
+    aligned = base[:2 * 3 * 8 * 64].view(2, 3, 8, 64)
+    assert base.data_ptr() % 16 == 0 and _tma_ready(aligned) is aligned
+    for t in (base[1:1 + 2 * 3 * 8 * 64].view(2, 3, 8, 64), base[:2 * 3 * 8 * 68].view(2, 3, 8, 68)[..., :64],
+              aligned.transpose(2, 3), base[:64].expand(2, 3, 8, 64)[..., 1:].contiguous().expand(2, 3, 8, 63)[..., :56]):
+        ready = _tma_ready(t)
+        assert torch.equal(ready, t) and ready.data_ptr() % 16 == 0 and ready.stride(-1) == 1
+        assert all(n % 8 == 0 for n in ready.stride()[:-1])
