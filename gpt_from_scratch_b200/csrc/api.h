@@ -57,8 +57,8 @@ int gfs_ce_from_partials(const void* partials, const void* logits, const void* t
 int gfs_ce_bwd(void* logits, const void* lse, const void* target, const void* grad_rows, float grad_all, int M, int Vp,
                long ld, int v0, void* stream);
 int gfs_mean_f32(const void* x, void* out, int n, void* stream);
-int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int S, int B, int nh, int D,
-                  const long long* strides, float scale, int causal, int o_f16, void* stream);
+int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* o_copy, void* lse, int S, int B, int nh,
+                  int D, const long long* strides, float scale, int causal, int o_f16, void* stream);
 int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dO, const void* lse,
                   void* dvec, void* dq, void* dk, void* dv, int S, int B, int nh, int D, const long long* strides,
                   float scale, int causal, const void* rope_cos, const void* rope_sin, void* do_bf16, void* stream);

@@ -148,6 +148,7 @@ __device__ __forceinline__ uint32_t pack_out(float lo, float hi, int f16) {
 // ---------------------------------------------------------------------------
 struct FwdParams {
   __nv_bfloat16* O;            // 16-bit elements; fp16 when o_f16 is set
+  long long o_copy;            // element offset from O to a second copy of the output; 0: none
   long long o_ss, o_bs, o_hs;  // element strides: sequence, batch, head
   float* lse;                  // [B, nh, S_pad], log2 of the row's sum of exponentials (base e scores)
   int o_f16;
@@ -454,7 +455,9 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(o_empty);   // the next item's first P V may overwrite the accumulator
-      if (row_g < p.S) {
+      // twice when a copy is wanted (rolled: a second store beside the first one cost 12 bytes of spills)
+#pragma unroll 1
+      for (int n_out = row_g >= p.S ? 0 : (p.o_copy != 0 ? 2 : 1); n_out > 0; --n_out, dst += p.o_copy) {
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
 #pragma unroll
@@ -875,11 +878,13 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
               wv.z = pack_out(__uint_as_float(wa[cc + 4]) * inv_l, __uint_as_float(wa[cc + 5]) * inv_l, p.o_f16);
               wv.w = pack_out(__uint_as_float(wa[cc + 6]) * inv_l, __uint_as_float(wa[cc + 7]) * inv_l, p.o_f16);
               *reinterpret_cast<uint4*>(dst + cc) = wv;
+              if (p.o_copy != 0) *reinterpret_cast<uint4*>(dst + p.o_copy + cc) = wv;
               wv.x = pack_out(__uint_as_float(wb[cc + 0]) * inv_l, __uint_as_float(wb[cc + 1]) * inv_l, p.o_f16);
               wv.y = pack_out(__uint_as_float(wb[cc + 2]) * inv_l, __uint_as_float(wb[cc + 3]) * inv_l, p.o_f16);
               wv.z = pack_out(__uint_as_float(wb[cc + 4]) * inv_l, __uint_as_float(wb[cc + 5]) * inv_l, p.o_f16);
               wv.w = pack_out(__uint_as_float(wb[cc + 6]) * inv_l, __uint_as_float(wb[cc + 7]) * inv_l, p.o_f16);
               *reinterpret_cast<uint4*>(dst + 32 + cc) = wv;
+              if (p.o_copy != 0) *reinterpret_cast<uint4*>(dst + p.o_copy + 32 + cc) = wv;
             }
           }
           if (row_g < p.S_pad) {
@@ -1511,13 +1516,14 @@ int gfs_attn_cast_qkv(const void* q, const void* k, const void* v, void* dst, in
 }
 
 // strides: 12 element strides {q_seq,q_batch,q_head, k_.., v_.., o_..}. lse: fp32 [B, nh, S_pad] (base 2),
-// S_pad = S rounded up to a multiple of 128. o_f16: store the output as fp16.
-int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* lse, int S, int B, int nh, int D,
-                  const long long* strides, float scale, int causal, int o_f16, void* stream_) {
+// S_pad = S rounded up to a multiple of 128. o_f16: store the output as fp16. o_copy: null, or where to store the
+// output a second time, with the same strides (for a backward whose caller may write to the first copy).
+int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* o_copy, void* lse, int S, int B, int nh,
+                  int D, const long long* strides, float scale, int causal, int o_f16, void* stream_) {
   if (D != 64 && D != 128) return -1;
   if (!strides_ok(strides, 12)) return -1;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
-       reinterpret_cast<uintptr_t>(o)) & 15)
+       reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(o_copy)) & 15)
     return -2;
   if (S <= 0 || B <= 0 || nh <= 0) return 0;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
@@ -1527,6 +1533,7 @@ int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* ls
   if (!tq || !tk || !tv) return -3;
   FwdParams p;
   p.O = static_cast<__nv_bfloat16*>(o);
+  p.o_copy = o_copy != nullptr ? (static_cast<char*>(o_copy) - static_cast<char*>(o)) / 2 : 0;
   p.o_ss = strides[9]; p.o_bs = strides[10]; p.o_hs = strides[11];
   p.lse = static_cast<float*>(lse);
   p.S = S; p.S_pad = ((S + 127) / 128) * 128; p.B = B; p.nh = nh;

@@ -206,8 +206,8 @@ int gfs_blocks_forward(const GfsBlockDims* dp, const GfsBlockParams* layers, con
     GFS_TRY(gfs_rmsnorm_fwd(x, p.w[W_NORM1], y1, rstd1, T, H, p.eps[0], stream));
     GFS_TRY(gfs_linear(y1, p.w[W_QKV], qkv, nullptr, T, 3 * H, H, H, H, 3 * H, 0, 0, 0, p.cos_table, p.sin_table, 2 * H,
                        d.D, d.B, d.pair_min_tiles, stream));   // q and k leave rotated
-    GFS_TRY(gfs_flash_fwd(qkv, qkv + 2 * static_cast<size_t>(H), qkv + 4 * static_cast<size_t>(H), attn, lse, d.S, d.B,
-                          d.nh, d.D, st, scale, 1, 0, stream));
+    GFS_TRY(gfs_flash_fwd(qkv, qkv + 2 * static_cast<size_t>(H), qkv + 4 * static_cast<size_t>(H), attn, nullptr, lse,
+                          d.S, d.B, d.nh, d.D, st, scale, 1, 0, stream));
     if (!drop) {
       GFS_TRY(product(d, attn, p.w[W_OUT], x1, x, T, H, H, H, H, H, 0, 0, stream));
     } else {

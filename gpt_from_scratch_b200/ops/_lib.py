@@ -82,7 +82,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "gfs_adamw_step": ([vp, vp, vp, vp, vp, i64, vp, vp, f, d, d, f, f, f, f, f, f, vp, vp], i),
         "gfs_flag_slots": ([], i),
         "gfs_wait_probe": ([vp, i64, vp], i),
-        "gfs_flash_fwd": ([vp, vp, vp, vp, vp, i, i, i, i, vp, f, i, i, vp], i),
+        "gfs_flash_fwd": ([vp, vp, vp, vp, vp, vp, i, i, i, i, vp, f, i, i, vp], i),
         "gfs_attn_cast_qkv": ([vp, vp, vp, vp, i, i, i, i, vp, vp], i),
         "gfs_flash_bwd": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, vp, f, i, vp, vp, vp, vp], i),
         "gfs_gemm_bf16_comm": ([i, vp, i, vp, i, vp, i, vp, i, i, i, i, i, i, i, ulp, ulp, uip, vp, vp, i, i, i,

@@ -65,7 +65,7 @@ def flash_fwd_native(q, k, v, out, causal: bool, scale: float) -> torch.Tensor:
     lse = torch.empty((B, nh, _pad128(S)), dtype=torch.float32, device=q.device)
     st = _Strides12(*_strides3(q), *_strides3(k), *_strides3(v), *_strides3(out))
     with _lib.nvtx("flash_attention_fwd"):
-        rc = _lib.lib().gfs_flash_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
+        rc = _lib.lib().gfs_flash_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 0, lse.data_ptr(),
                                       S, B, nh, D, st, scale, 1 if causal else 0, 0, _lib.stream_ptr())
     _lib.check(rc, "gfs_flash_fwd")
     return lse
@@ -111,6 +111,7 @@ class _FlashAttnBHSD(torch.autograd.Function):
         out = torch.empty_like(q)
         lse = torch.empty((B, nh, _pad128(S)), dtype=torch.float32, device=q.device)
         pq, pk, pv = q.data_ptr(), k.data_ptr(), v.data_ptr()
+        copy = None
         if q.dtype == torch.float16:
             qkv = torch.empty((3, B, nh, S, D), dtype=torch.bfloat16, device=q.device)
             src, n = (pq, pk, pv), 2 * B * nh * S * D
@@ -120,11 +121,13 @@ class _FlashAttnBHSD(torch.autograd.Function):
                        "gfs_attn_cast_qkv")
             st = _stride_array(qkv[0], qkv[1], qkv[2], out) if not out.is_contiguous() else \
                 _contiguous_strides(4, B, nh, S, D)
-            ctx.save_for_backward(qkv, out, lse)
+            # the backward reads a copy of the output: the caller may write to his (out += residual)
+            copy = torch.empty_like(out) if any(ctx.needs_input_grad) else None
+            ctx.save_for_backward(qkv, copy, lse)
         else:
             st = _stride_array(q, k, v, out)
             ctx.save_for_backward(q, k, v, out, lse)
-        rc = lib.gfs_flash_fwd(pq, pk, pv, out.data_ptr(), lse.data_ptr(), S, B, nh, D, st, scale, causal,
+        rc = lib.gfs_flash_fwd(pq, pk, pv, out.data_ptr(), _lib.ptr(copy), lse.data_ptr(), S, B, nh, D, st, scale, causal,
                                q.dtype == torch.float16, stream)
         _lib.check(rc, "gfs_flash_fwd")
         ctx.args = (causal, scale)

@@ -355,3 +355,25 @@ def test_flash_attention_misaligned_tensors(cuda_device, dtype):
         o = apply_flash_attn(q, k, v)
         results.append((o, *torch.autograd.grad(o, (q, k, v), do)))
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("B,nh,S,D", [(2, 3, 129, 64), (1, 2, 300, 128)])
+def test_flash_attention_fp16_output_may_be_written_to(cuda_device, B, nh, S, D):
+    """The output of fp16 tensors belongs to the caller: written to in place, the gradients stay what they are. (A bf16
+    output is saved itself, and autograd says so.)"""
+    from gpt_from_scratch_b200.ops.attention import apply_flash_attn
+    g = torch.Generator(device="cuda").manual_seed(1)
+    t = [torch.randn(B, S, nh, D, device=cuda_device, generator=g).half().transpose(1, 2) for _ in range(4)]
+    grads = []
+    for write in (False, True):
+        q, k, v = (x.detach().requires_grad_() for x in t[:3])
+        o = apply_flash_attn(q, k, v)
+        if write:
+            o += 1.0
+        grads.append(torch.autograd.grad(o, (q, k, v), t[3]))
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
+    q, k, v = (x.detach().bfloat16().requires_grad_() for x in t[:3])
+    o = apply_flash_attn(q, k, v)
+    o += 1.0
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        o.sum().backward()
