@@ -593,9 +593,10 @@ int launch_tile(int bn, const TileMaps<NG>& maps, const TileParams<NG>& p, int c
                           stream, set256);
 }
 
+// Splits 5 to 7 round the rows of a CTA up so far that `split` slabs of them exceed the staging area's 129 rows.
 int bad_shape(int bn, int split) {
   if (bn != 64 && bn != 128 && bn != 256) return 1;
-  return split < 1 || split > (bn == 256 ? 4 : 8);
+  return split < 1 || split > (bn == 256 ? 4 : 8) || (BM + split - 1) / split * split > BM + 1;
 }
 
 }  // namespace
@@ -603,7 +604,8 @@ int bad_shape(int bn, int split) {
 extern "C" {
 
 // C[M,N] = op(A) op(B) (+ R) on one tile per CTA (bn = 64, 128: 128 x bn) or per CTA pair (bn = 256: 256 x 256),
-// `split` CTAs (at most 8) or pairs (at most 4) per tile along K, each of which has to get a 64-wide K block. Arguments otherwise as gfs_gemm_bf16_rope;
+// `split` CTAs (1 to 4 or 8) or pairs (1 to 4) per tile along K, each of which has to get a 64-wide K block. Arguments
+// otherwise as gfs_gemm_bf16_rope;
 // swi_mode 1 / 2 with swi_extra as gfs_gemm_bf16_swiglu (then N is I: columns of act, resp. d_act).
 int gfs_gemm_tile(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,
                   int ldr, int a_mn_major, int b_mn_major, const void* rope_cos, const void* rope_sin, int rope_cols,

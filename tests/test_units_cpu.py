@@ -461,3 +461,23 @@ def test_flash_attention_misaligned_tensors_are_copied():
         ready = _tma_ready(t)
         assert torch.equal(ready, t) and ready.data_ptr() % 16 == 0 and ready.stride(-1) == 1
         assert all(n % 8 == 0 for n in ready.stride()[:-1])
+
+
+@pytest.mark.parametrize("bn", [64, 128, 256])
+def test_one_tile_gemm_refuses_splits_past_its_staging_area(bn):
+    """A K split whose rows, rounded up per CTA, need more than the 129 rows of fp32 staging is refused on the host (the
+    addresses here are never read: without a GPU an accepted call ends at its tensor maps)."""
+    import ctypes
+
+    from gpt_from_scratch_b200.ops import _lib
+    lib, p = _lib.lib(), 1 << 20
+    U, I = ctypes.c_ulonglong * 1, ctypes.c_int * 1
+    if torch.cuda.is_available():
+        pytest.skip("addresses are made up")
+    for split in range(1, 10):
+        refused = -(-128 // split) * split > 129 or split > (4 if bn == 256 else 8)
+        K = 64 * split
+        one = lib.gfs_gemm_tile(p, p, p, 0, 128, 128, K, K, K, 128, 0, 0, 0, 0, 0, 0, 0, 1, 0, 0, 0, bn, split, 0)
+        group = lib.gfs_gemm_tile_wgrad_grouped(1, U(p), U(p), U(p), I(128), I(128), I(K), I(128), I(128), I(128), I(0),
+                                                bn, split, 0)
+        assert (one == -1) == refused and (group == -1) == refused, (split, one, group)
