@@ -40,7 +40,6 @@ int gfs_rmsnorm_dw_reduce_multi(int n, const unsigned long long* partial, const 
                                 const int* parts, const int* accumulate, int H, void* stream);
 int gfs_dropout_residual(const void* x, const void* residual, void* out, long long n, float p, unsigned long long seed,
                          int backward, void* stream);
-int gfs_swiglu_bwd(const void* dact, const void* gu, void* dgu, int M, int I, void* stream);
 int gfs_embedding_fwd(const void* ids, const void* W, void* out, int B, int S, int H, int v0, int v1, int s0,
                       int s_count, void* stream);
 int gfs_embedding_sort_shift(long long n, int v);

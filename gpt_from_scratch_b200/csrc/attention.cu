@@ -35,11 +35,6 @@ namespace {
 
 constexpr float LOG2E_F = 1.4426950408889634f;
 
-// A K-major [rows x K] (64-column blocks a_blk bytes apart), B K-major [N x K] (blocks b_blk apart).
-// Classifies a (32-row warp slice) x (column chunk) block of the score matrix against the
-// causal / sequence-end mask: 0 = every element alive, 1 = mixed, 2 = every element dead.
-// KEY_ROWS: rows are key positions and columns are query positions (dead when col < row);
-// otherwise rows are queries and columns are keys (dead when col > row). Warp-uniform.
 // three-input maximum (one instruction on sm_100)
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
@@ -47,6 +42,10 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   return d;
 }
 
+// Classifies a (32-row warp slice) x (column chunk) block of the score matrix against the
+// causal / sequence-end mask: 0 = every element alive, 1 = mixed, 2 = every element dead.
+// KEY_ROWS: rows are key positions and columns are query positions (dead when col < row);
+// otherwise rows are queries and columns are keys (dead when col > row). Warp-uniform.
 template <bool KEY_ROWS>
 __device__ __forceinline__ int mask_class(int row_min, int row_max, int col_min, int col_max, bool causal, int S) {
   if (col_min >= S) return 2;
@@ -63,6 +62,7 @@ __device__ __forceinline__ int mask_class(int row_min, int row_max, int col_min,
   return all_dead ? 2 : (all_alive ? 0 : 1);
 }
 
+// A K-major [rows x K] (64-column blocks a_blk bytes apart), B K-major [N x K] (blocks b_blk apart).
 // The shared-memory descriptors are built once per call and advanced by adding the byte offset
 // (in 16-byte units) to their start-address field: the tiles are 1024-byte aligned and the
 // offsets small, so the 14-bit field never carries. The issuing thread competes with the
@@ -79,23 +79,9 @@ __device__ __forceinline__ void mma_kk(uint32_t d, uint32_t a, uint32_t a_blk, u
     umma_ss_e(d, ad, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
   }
 }
-// A K-major; B MN-major: stored as [K rows x N] in 64-column blocks b_blk bytes apart
-// (each block: K rows of 128 B).
-template <int KSTEPS>
-__device__ __forceinline__ void mma_kmn(uint32_t d, uint32_t a, uint32_t a_blk, uint32_t b, uint32_t b_blk,
-                                        uint32_t idesc, bool accumulate) {
-  const uint64_t ad0 = umma_desc_sw128(a, 16, 1024);
-  const uint64_t bd0 = umma_desc_sw128(b, b_blk, 1024);
-#pragma unroll
-  for (int ks = 0; ks < KSTEPS; ++ks) {
-    const uint64_t ad = ad0 + (((ks >> 2) * a_blk + (ks & 3) * 32) >> 4);
-    const uint64_t bd = bd0 + ((ks * 2048) >> 4);
-    umma_ss_e(d, ad, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
-  }
-}
-
 // A in tensor memory (8 columns per 16-wide K step; the second half of the K steps starts HALF columns
-// after the first); B MN-major as in mma_kmn.
+// after the first); B MN-major: stored as [K rows x N] in 64-column blocks b_blk bytes apart (each block: K
+// rows of 128 B).
 template <int KSTEPS, int HALF = KSTEPS * 4>
 __device__ __forceinline__ void mma_tmn(uint32_t d, uint32_t a_tmem, uint32_t b, uint32_t b_blk, uint32_t idesc,
                                         bool accumulate) {

@@ -14,7 +14,7 @@
 //   dgrad    dX = dY W        : A = dY (K-major),  B = W  (MN-major, contraction over W's rows)
 //   wgrad    dW = dY^T X      : A = dY (MN-major), B = X  (MN-major), contraction over tokens
 //
-// Small outputs (wgrad of the per-layer linears) use deterministic split-K: each split
+// Deterministic split-K where a caller asks for it (force_split, the allocation-free entry point): each split
 // writes an fp32 partial tile to a workspace and a second kernel sums the splits in a
 // fixed order, adds the optional addend and rounds once to bf16.
 //
@@ -597,6 +597,8 @@ int launch_variant(const CUtensorMap* ta, const CUtensorMap* tb, const GemmParam
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
+// K splits of a product that does not fill the chip. For callers that ask for this kernel (gemm_bf16(pair=False), C
+// callers with a workspace); the rule in select.cu gives such products to gemm3.cu's kernels.
 int choose_split(int tiles, int kblocks, int sms, size_t mn_elems, size_t ws_bytes) {
   if (tiles * 10 >= sms * 9 || kblocks < 8) return 1;
   int best = 1;
@@ -837,15 +839,6 @@ int gfs_gemm_bf16_comm(int mode, const void* a, int lda, const void* B, int ldb,
                          : launch_variant<false, false, 128, 6, COMM_REDUCE_SCATTER>(ta, tb, p, grid, stream);
   }
   return rc;
-}
-
-// Number of kernels gfs_gemm_bf16 launches for this problem (1, or 2 with split-K).
-int gfs_gemm_bf16_launches(int M, int N, int K, size_t ws_bytes) {
-  const int BN = (N > 128) ? 256 : 128;
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int kb = (K + BK - 1) / BK;
-  int s = ws_bytes ? choose_split(tiles, kb, gfs_host::sm_count(), static_cast<size_t>(M) * N, ws_bytes) : 1;
-  return s > 1 ? 2 : 1;
 }
 
 }  // extern "C"

@@ -9,8 +9,10 @@
 // one buffer per block for what the backward reads (gfs_blocks_act_bytes) and one scratch for the
 // backward itself (gfs_blocks_bwd_bytes).
 //
-// Nothing here computes: kernels, their selection rules and their order are those of the
-// module-by-module path (models/transformer_layer.py), so both give the same results.
+// Nothing here computes: the kernels and their selection rules are those of the module-by-module path
+// (models/transformer_layer.py). Forward results are its bits. Gradients differ from its by roundings: the weight
+// gradients of a block form other groups, for which other tiles and K splits may be chosen (fp32 sums in another order),
+// and with dropout the modules round the two gradients of a residual branch one by one.
 // Single tensor-parallel rank only (no collectives).
 #include <algorithm>
 #include <cmath>
@@ -173,12 +175,8 @@ bool dims_ok(const GfsBlockDims& d) {
 
 extern "C" {
 
-// Bytes of one block's saved activations, and the byte offset of the block's output in it.
-size_t gfs_blocks_act_bytes(const GfsBlockDims* d, size_t* out_offset) {
-  const ActLayout a(*d);
-  *out_offset = a.x2;
-  return a.total;
-}
+// Bytes of one block's saved activations.
+size_t gfs_blocks_act_bytes(const GfsBlockDims* d) { return ActLayout(*d).total; }
 
 size_t gfs_blocks_bwd_bytes(const GfsBlockDims* d) { return BwdLayout(*d).total; }
 

@@ -98,7 +98,7 @@ def build_cases(dev, small: bool):
     gemm_case("gemm_dgrad_gate_up", M, H, 2 * I, b_mn=True)
     gemm_case("gemm_dgrad_down", M, I, H, b_mn=True)
     gemm_case("gemm_dgrad_lm_head", M, H, V, b_mn=True)
-    gemm_case("gemm_wgrad_qkv_splitk", 3 * H, H, M, a_mn=True, b_mn=True)
+    gemm_case("gemm_wgrad_qkv", 3 * H, H, M, a_mn=True, b_mn=True)
     gemm_case("gemm_wgrad_gate_up", 2 * I, H, M, a_mn=True, b_mn=True)
     gemm_case("gemm_wgrad_lm_head", V, H, M, a_mn=True, b_mn=True)
 

@@ -4,8 +4,8 @@ Module by module, a transformer block costs the host about 0.3 ms forward and 0.
 autograd functions, about twenty launches through ctypes), which is more than its kernels take at small
 and ordinary sizes. ``GPTModel.forward`` therefore hands the whole model to this file when nothing needs
 the module-by-module path: the stack of blocks with the final norm is ONE call into the library per
-direction (csrc/model.cu), and autograd sees one function for the model. Same kernels, same order, same
-results.
+direction (csrc/model.cu), and autograd sees one function for the model. Same kernels and same logits; gradients
+differ by roundings, because the weight gradients are grouped differently (csrc/model.cu says where).
 
 The modules stay the owners of the parameters, and each pass compares what it is about to use with what they
 hold: modules and their types, weights, biases, rotary tables, norm constants, dropout, hooks, ``forward`` methods
@@ -16,7 +16,7 @@ from __future__ import annotations
 
 import ctypes
 import weakref
-from ctypes import byref, c_float, c_int, c_size_t, c_ulonglong, c_void_p
+from ctypes import byref, c_float, c_int, c_ulonglong, c_void_p
 from itertools import repeat
 from operator import contains, getitem, is_
 
@@ -243,7 +243,7 @@ class _Pass:
         self.params = type(plan.params).from_buffer_copy(plan.params)
 
     def act_bytes(self) -> int:
-        return _lib.lib().gfs_blocks_act_bytes(byref(self.dims), byref(c_size_t()))
+        return _lib.lib().gfs_blocks_act_bytes(byref(self.dims))
 
     def bwd_bytes(self) -> int:
         return _lib.lib().gfs_blocks_bwd_bytes(byref(self.dims))

@@ -61,8 +61,6 @@ def _declare(lib: ctypes.CDLL) -> None:
         "gfs_read_status": ([POINTER(c_uint32), i], i),
         "gfs_sm_count": ([], i),
         "gfs_last_cuda_error": ([], c_char_p),
-        "gfs_gemm_bf16": ([vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, i, vp, sz, i, vp], i),
-        "gfs_gemm_bf16_launches": ([i, i, i, sz], i),
         "gfs_rmsnorm_fwd": ([vp, vp, vp, vp, i, i, f, vp], i),
         "gfs_rmsnorm_bwd_parts": ([i], i),
         "gfs_rmsnorm_bwd": ([vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp], i),
@@ -112,7 +110,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "gfs_gemm_bf16_swiglu": ([i, vp, vp, vp, vp, i, i, i, i, i, i, i, vp], i),
         "gfs_gemm2_bf16_swiglu": ([i, vp, vp, vp, vp, i, i, i, i, i, i, i, vp], i),
         "gfs_gemm2_bf16": ([vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, vp, vp, i, i, i, vp], i),
-        "gfs_blocks_act_bytes": ([vp, vp], sz),
+        "gfs_blocks_act_bytes": ([vp], sz),
         "gfs_blocks_bwd_bytes": ([vp], sz),
         "gfs_blocks_forward": ([vp] * 10, i),
         "gfs_blocks_backward": ([vp, vp, vp, vp, i, vp, vp, vp, vp, vp, vp, vp, vp], i),

@@ -173,9 +173,9 @@ class _WgradQueue:
     """Weight-gradient GEMMs waiting to be launched together.
 
     A layer's weight gradients are ``[out, in] = dY^T X`` with K = tokens: few output tiles,
-    very deep. One at a time they occupy a fraction of the SMs (or need split-K and a
-    reduction pass); several of them in ONE grouped launch (``gfs_wgrad_grouped``) fill
-    a wave of CTA pairs. A weight gradient is only needed at the optimizer step, so problems
+    very deep. One at a time they occupy a fraction of the SMs; several of them in ONE grouped
+    launch (``gfs_wgrad_grouped``) fill a wave, of CTA pairs or of single tiles with K split over a cluster
+    (csrc/select.cu). A weight gradient is only needed at the optimizer step, so problems
     that write into a gradient sink are parked here (holding references to their operands)
     and launched when enough tiles have accumulated, at the end of the backward pass that
     parked them (an autograd-engine callback), or when :func:`flush_wgrad` is called.
