@@ -72,25 +72,14 @@ struct Cfg {
   static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING + 256 + 1024;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
 __device__ __forceinline__ void cluster_sync() {
   __syncwarp();   // the aligned barrier wants whole warps
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
+  cluster_sync_all();
 }
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
                : "memory");
 }
-__device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
@@ -215,7 +204,7 @@ __device__ __forceinline__ void stage_row(uint32_t t_row, float* staging, int sl
                                           bool remote, uint32_t owner, int c0, int c1) {
   float* local = staging + (slab * rows_per_cta + row_in_owner) * PITCH;
   uint32_t dst = smem_u32(local);
-  if (remote) dst = mapa(dst, owner);
+  if (remote) dst = mapa_u32(dst, owner);
   uint32_t va[32], vb[32];
 #pragma unroll 1
   for (int c = c0; c < c1; c += 64) {
@@ -258,7 +247,7 @@ gemm_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constan
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int split = p.split;
-  const int rank = split > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int rank = split > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   const int tile = static_cast<int>(blockIdx.x) / split;
   int gi = 0;
   if (NG > 1) {
@@ -382,31 +371,6 @@ constexpr int PAIR_THREADS = 320;   // TMA, MMA, eight warps that drain the accu
 constexpr int PAIR_TOTAL = PAIR_STAGES * PAIR_STAGE_BYTES + 256 + 1024;
 static_assert((BM + 1) * 260 * 4 <= PAIR_STAGES * PAIR_STAGE_BYTES, "staging fits the ring");
 
-__device__ __forceinline__ void tma_load_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], "
-      "[%2];" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(bar_cluster_addr), "r"(x), "r"(y)
-      : "memory");
-}
-__device__ __forceinline__ void umma_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {   // whole warp; one elected lane issues
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void commit_pair(uint32_t cluster_addr) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(cluster_addr)
-      : "memory");
-}
-
 template <bool A_MN, bool B_MN, int NG>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constant__ TileParams<NG> p) {
@@ -425,7 +389,7 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int split = p.split;
-  const uint32_t crank = cluster_rank();
+  const uint32_t crank = cluster_ctarank();
   const int half = static_cast<int>(crank & 1u);     // rows / columns half of this CTA in its pair
   const int z = static_cast<int>(crank >> 1);        // K slice of the pair
   const uint32_t lead = crank & ~1u;
@@ -455,10 +419,8 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
   }
   __syncthreads();
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(static_cast<uint32_t>(BN))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    tmem_alloc_pair(tmem_slot, BN);
+    tmem_relinquish_pair();
   }
   tc_fence_before();
   cluster_sync();   // barriers of all CTAs initialised, TMEM allocated
@@ -479,20 +441,20 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
         uint8_t* sa = tiles + stage * PAIR_STAGE_BYTES;
         uint8_t* sb = sa + 16384;
         if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * PAIR_STAGE_BYTES);   // the bytes of both CTAs
-        const uint32_t bar = mapa(smem_u32(&full_bar[stage]), lead);
+        const uint32_t bar = mapa_u32(smem_u32(&full_bar[stage]), lead);
         const int k0 = kb * BK;
         if (!A_MN) {
-          tma_load_pair(sa, &maps.a[gi], bar, k0, m0);
+          tma_load_2d_pair(sa, &maps.a[gi], bar, k0, m0);
         } else {
 #pragma unroll
-          for (int j = 0; j < 2; ++j) tma_load_pair(sa + j * 8192, &maps.a[gi], bar, m0 + 64 * j, k0);
+          for (int j = 0; j < 2; ++j) tma_load_2d_pair(sa + j * 8192, &maps.a[gi], bar, m0 + 64 * j, k0);
         }
         if (!B_MN) {
           // SwiGLU forward: 128 gate rows for the leader, the matching up rows for the other CTA
-          tma_load_pair(sb, &maps.b[gi], bar, k0, p.swi_mode == 1 ? half * p.swi_I + (n0 >> 1) : nb);
+          tma_load_2d_pair(sb, &maps.b[gi], bar, k0, p.swi_mode == 1 ? half * p.swi_I + (n0 >> 1) : nb);
         } else {
 #pragma unroll
-          for (int j = 0; j < 2; ++j) tma_load_pair(sb + j * 8192, &maps.b[gi], bar, nb + 64 * j, k0);
+          for (int j = 0; j < 2; ++j) tma_load_2d_pair(sb + j * 8192, &maps.b[gi], bar, nb + 64 * j, k0);
         }
       }
       if (*abort_flag) {
@@ -513,13 +475,13 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
         for (int k = 0; k < BK / 16; ++k) {
           const uint64_t adesc = A_MN ? umma_desc_sw128(sa + k * 2048, 8192, 1024) : umma_desc_sw128(sa + k * 32, 16, 1024);
           const uint64_t bdesc = B_MN ? umma_desc_sw128(sb + k * 2048, 8192, 1024) : umma_desc_sw128(sb + k * 32, 16, 1024);
-          umma_pair(tmem_base, adesc, bdesc, idesc, (i > 0 || k > 0) ? 1u : 0u);
+          umma_ss_pair(tmem_base, adesc, bdesc, idesc, (i > 0 || k > 0) ? 1u : 0u);
         }
-        commit_pair(mapa(smem_u32(&empty_bar[stage]), lead));
-        commit_pair(mapa(smem_u32(&empty_bar[stage]), lead | 1u));
+        umma_commit_pair(mapa_u32(smem_u32(&empty_bar[stage]), lead));
+        umma_commit_pair(mapa_u32(smem_u32(&empty_bar[stage]), lead | 1u));
       }
-      commit_pair(mapa(smem_u32(tmem_full), lead));
-      commit_pair(mapa(smem_u32(tmem_full), lead | 1u));
+      umma_commit_pair(mapa_u32(smem_u32(tmem_full), lead));
+      umma_commit_pair(mapa_u32(smem_u32(tmem_full), lead | 1u));
     }
   }
   // every product of this pair is done (both halves of the ring have been read)
@@ -547,9 +509,7 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
   __syncthreads();
   cluster_sync();
   tc_fence_after();
-  if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(static_cast<uint32_t>(BN))
-                 : "memory");
+  if (warp == 1) tmem_dealloc_pair(tmem_base, BN);
 }
 
 // Launch with `cluster` CTAs per cluster (and programmatic stream serialization).
