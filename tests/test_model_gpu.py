@@ -406,9 +406,9 @@ def _shared_gradients(share, H, layers, V, steps=2):
     out = []
     for shared in (True, False):
         eng = TrainEngine(cfg, lr=1e-9, seed=9)
-        with torch.no_grad():
-            pairs = share(eng.model, shared)
         for t in batches:
+            with torch.no_grad():
+                pairs = share(eng.model, shared)      # again: a step restores the weights from their fp32 copies
             eng.train_step(t[:, :-1].contiguous().cuda(), t[:, 1:].contiguous().cuda())
         grads = {n: p.grad.double() for n, p in eng.model.named_parameters()}
         if not shared:
@@ -567,7 +567,7 @@ def test_step_of_many_blocks(cuda_device):
         if modules:
             loss = eng.forward_loss(x, y)
             loss.backward()
-        runs.append((float(loss), eng.optimizer.grad_buffer.double()))
+        runs.append((loss.item(), eng.optimizer.grad_buffer.double()))
     assert abs(runs[0][0] - runs[1][0]) < 1e-4
     assert (runs[0][1] - runs[1][1]).norm() < 2e-3 * runs[1][1].norm()
 
