@@ -8,7 +8,7 @@
 // Forward (persistent; head_dim 64: pairs of 128-row query tiles, 128: two pipelines of 128-row items): per
 //   128-key block S = Q K^T -> TMEM; the softmax threads read their row (128: half row) with tcgen05.ld, keep
 //   the running max / sum and store P (bf16) in TMEM, from where the MMA warp adds P V to the output
-//   accumulator, which stays in TMEM for the whole item.
+//   accumulator, which stays in TMEM for the whole item. (Few items at head_dim 128: a CTA for each.)
 //
 // Backward (two kernels from one template, deterministic, no atomics):
 //   mode 0: items of 128 keys    -> dK, dV, streaming 64-query tiles
@@ -79,9 +79,23 @@ __device__ __forceinline__ void mma_kk(uint32_t d, uint32_t a, uint32_t a_blk, u
     umma_ss_e(d, ad, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
   }
 }
+// A K-major; B MN-major: stored as [K rows x N] in 64-column blocks b_blk bytes apart
+// (each block: K rows of 128 B).
+template <int KSTEPS>
+__device__ __forceinline__ void mma_kmn(uint32_t d, uint32_t a, uint32_t a_blk, uint32_t b, uint32_t b_blk,
+                                        uint32_t idesc, bool accumulate) {
+  const uint64_t ad0 = umma_desc_sw128(a, 16, 1024);
+  const uint64_t bd0 = umma_desc_sw128(b, b_blk, 1024);
+#pragma unroll
+  for (int ks = 0; ks < KSTEPS; ++ks) {
+    const uint64_t ad = ad0 + (((ks >> 2) * a_blk + (ks & 3) * 32) >> 4);
+    const uint64_t bd = bd0 + ((ks * 2048) >> 4);
+    umma_ss_e(d, ad, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
+  }
+}
+
 // A in tensor memory (8 columns per 16-wide K step; the second half of the K steps starts HALF columns
-// after the first); B MN-major: stored as [K rows x N] in 64-column blocks b_blk bytes apart (each block: K
-// rows of 128 B).
+// after the first); B MN-major as in mma_kmn.
 template <int KSTEPS, int HALF = KSTEPS * 4>
 __device__ __forceinline__ void mma_tmn(uint32_t d, uint32_t a_tmem, uint32_t b, uint32_t b_blk, uint32_t idesc,
                                         bool accumulate) {
@@ -118,6 +132,23 @@ __device__ __forceinline__ void store_rows_32x32(uint8_t* stage, const uint32_t 
   __syncwarp();
 }
 
+// 32 rows x 64 bf16 columns; w = this lane's row (32 packed words); stage: 4 KB of this warp.
+__device__ __forceinline__ void store_rows_32x64(uint8_t* stage, const uint32_t (&w)[32], int lane,
+                                                 __nv_bfloat16* g0, long long row_stride, int rows_valid) {
+#pragma unroll
+  for (int ch = 0; ch < 8; ++ch)
+    *reinterpret_cast<uint4*>(stage + lane * 128 + ((ch ^ (lane & 7)) << 4)) =
+        make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = (lane >> 3) + 4 * i;
+    const uint4 v = *reinterpret_cast<const uint4*>(stage + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
+    if (row < rows_valid) *reinterpret_cast<uint4*>(g0 + row * row_stride + (lane & 7) * 8) = v;
+  }
+  __syncwarp();
+}
+
 // Two fp32 values as a 16-bit pair of the output's type. The kernels compute in bf16; tensors of an fp16
 // caller are rounded to bf16 on the way in (cast_qkv_kernel, attn_dvec_kernel) and results leave as fp16
 // straight from fp32, so an fp16 call costs one launch more than a bf16 one and no pass over its results.
@@ -144,6 +175,318 @@ struct FwdParams {
   uint32_t* status;
 };
 
+// ---------------------------------------------------------------------------
+// Forward, head_dim 128, few items: one CTA per 128 query rows, four softmax warps (a row per thread). A lone chain of
+// blocks is what bounds such a problem, and here S, P and P V are double buffered (P through shared memory, the
+// output folded into registers), so the next block's scores are ready when the softmax gets there; the
+// pipelines of the kernel below hide each other's waits instead.
+// ---------------------------------------------------------------------------
+constexpr int FWD128S_THREADS = 192;
+constexpr int FWD128S_SMEM = 5 * 32768 + 2 * 32768 + 256;
+
+// Which of the two serves nb query tiles of B * nh heads. Up to one item per SM, this one: us, here -> two pipelines,
+// [1, 1, 1024, 128] 24 -> 27, [4, 2, 2048] 39 -> 43, [1, 4, 4096] 68 -> 76, [1, 2, 8192] 123 -> 137 (up to 300
+// tokens they are equal). A few more items change nothing as long as they find room behind short causal ones:
+// [1, 5, 4096] 70 -> 80, [1, 6, 4096] 78 -> 84, [1, 3, 8192] 130 -> 152, [1, 10, 2048] 41 -> 47, [1, 12, 2048] 49 -> 50,
+// [1, 19, 1024] 27 -> 31; past that two pipelines per SM win: [1, 7, 4096] 91 -> 86, [1, 13, 2048] 55 -> 51,
+// [1, 20, 1024] 33 -> 31, [1, 40, 512] 25 -> 23, [1, 32, 4096] 294 -> 182; without a mask [1, 9, 2048] 41 -> 45,
+// [1, 10, 2048] 68 -> 57. The line is the share of the SMs' time that the blocks take if none works longer than the
+// longest item; a second item costs an SM a launch, which short items feel more.
+bool fwd128_few_items(int nb, long long heads, bool causal, int sms) {
+  if (nb * heads <= sms) return true;
+  const long long blocks = causal ? heads * nb * (nb + 1) / 2 : heads * nb * nb;
+  return blocks * 100 <= static_cast<long long>(sms) * nb * (nb >= 16 ? 70 : 59);
+}
+
+__global__ void __launch_bounds__(FWD128S_THREADS, 1)
+flash_fwd128_small_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
+                          const __grid_constant__ CUtensorMap tv, const FwdParams p) {
+  constexpr int D = 128;
+  constexpr int DB = D / 64;
+  constexpr int TILE_BYTES = DB * 16384;  // [128 x D] bf16 as DB swizzled blocks
+  constexpr int P_BYTES = 32768;          // [128 x 128] bf16 as 2 swizzled blocks
+  constexpr uint32_t TMEM_COLS = 512;
+  constexpr uint32_t OP_COL = 256;        // PV tiles start after the S tiles
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;  // the launcher requests exactly the bytes used; the base must be 1024-aligned
+  uint8_t* Qs = smem;
+  uint8_t* Ks = Qs + TILE_BYTES;
+  uint8_t* Vs = Ks + 2 * TILE_BYTES;
+  uint8_t* Ps = Vs + 2 * TILE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(Ps + 2 * P_BYTES);
+  uint64_t* q_full = bars;
+  uint64_t* k_full = bars + 1;
+  uint64_t* k_empty = bars + 3;
+  uint64_t* v_full = bars + 5;
+  uint64_t* v_empty = bars + 7;
+  uint64_t* s_full = bars + 9;
+  uint64_t* s_empty = bars + 11;
+  uint64_t* p_full = bars + 13;
+  uint64_t* p_empty = bars + 15;
+  uint64_t* o_full = bars + 17;
+  uint64_t* o_empty = bars + 19;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
+  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  if (smem_u32(smem_raw) & 1023u) {  // swizzled tiles need a 1024-byte aligned base
+    if (threadIdx.x == 0) record_status(p.status, STATUS_BAD_ARGUMENT, 0x5a11u);
+    return;
+  }
+  const int qt = gridDim.x - 1 - blockIdx.x;  // heaviest (most key blocks) first
+  const int bh = blockIdx.y;
+  const int b = bh / p.nh;
+  const int h = bh % p.nh;
+  const int n_blocks_all = (p.S + 127) >> 7;
+  const int n_kv = p.causal ? min(qt + 1, n_blocks_all) : n_blocks_all;
+
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&k_full[i], 1);
+      mbar_init(&k_empty[i], 1);
+      mbar_init(&v_full[i], 1);
+      mbar_init(&v_empty[i], 1);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&s_empty[i], 4);
+      mbar_init(&p_full[i], 4);
+      mbar_init(&p_empty[i], 1);
+      mbar_init(&o_full[i], 1);
+      mbar_init(&o_empty[i], 4);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tq);
+    tma_prefetch_desc(&tk);
+    tma_prefetch_desc(&tv);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();       // set-up above may overlap the tail of the preceding kernel (programmatic launch)
+  pdl_trigger();
+  const uint32_t tmem_base = *tmem_slot;
+  WaitCtx wctx{abort_flag, p.status, GFS_WAIT_LIMIT_NS};
+
+  if (warp == 0) {
+    if (lane == 0) {
+      mbar_arrive_expect_tx(q_full, TILE_BYTES);
+#pragma unroll
+      for (int db = 0; db < DB; ++db) tma_load_4d(Qs + db * 16384, &tq, q_full, db * 64, qt * 128, h, b);
+      for (int j = 0; j < n_kv; ++j) {
+        const int st = j & 1;
+        const uint32_t par = ((j >> 1) & 1) ^ 1u;
+        mbar_wait(&k_empty[st], par, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
+        mbar_arrive_expect_tx(&k_full[st], TILE_BYTES);
+#pragma unroll
+        for (int db = 0; db < DB; ++db)
+          tma_load_4d(Ks + st * TILE_BYTES + db * 16384, &tk, &k_full[st], db * 64, j * 128, h, b);
+        mbar_wait(&v_empty[st], par, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
+        mbar_arrive_expect_tx(&v_full[st], TILE_BYTES);
+#pragma unroll
+        for (int db = 0; db < DB; ++db)
+          tma_load_4d(Vs + st * TILE_BYTES + db * 16384, &tv, &v_full[st], db * 64, j * 128, h, b);
+      }
+      if (*abort_flag) {
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+      }
+    }
+  } else if (warp == 1) {
+    {  // whole warp, converged: the MMA / commit helpers elect the issuing lane
+      constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
+      constexpr uint32_t idesc_o = umma_idesc_bf16(128, D, 0, 1);
+      const uint32_t q_addr = smem_u32(Qs);
+      mbar_wait(q_full, 0, wctx, STATUS_TIMEOUT_PIPE_FULL);
+      auto issue_s = [&](int j) {
+        const int st = j & 1;                       // K/V stage
+        const uint32_t par = (j >> 1) & 1;
+        const int sb = j & 1;   // S / P / PV buffer
+        const uint32_t spar = (j >> 1) & 1;
+        mbar_wait(&k_full[st], par, wctx, STATUS_TIMEOUT_PIPE_FULL);
+        mbar_wait(&s_empty[sb], spar ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
+        tc_fence_after();
+        mma_kk<D / 16>(tmem_base + sb * 128, q_addr, 16384, smem_u32(Ks + st * TILE_BYTES), 16384, idesc_s, false);
+        umma_commit_e(&s_full[sb]);
+        umma_commit_e(&k_empty[st]);
+      };
+      issue_s(0);
+      for (int j = 0; j < n_kv; ++j) {
+        if (j + 1 < n_kv) issue_s(j + 1);
+        const int st = j & 1;
+        const uint32_t par = (j >> 1) & 1;
+        const int sb = j & 1;
+        const uint32_t spar = (j >> 1) & 1;
+        mbar_wait(&p_full[sb], spar, wctx, STATUS_TIMEOUT_SOFTMAX);
+        mbar_wait(&v_full[st], par, wctx, STATUS_TIMEOUT_PIPE_FULL);
+        mbar_wait(&o_empty[sb], spar ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
+        tc_fence_after();
+        mma_kmn<8>(tmem_base + OP_COL + sb * D, smem_u32(Ps + sb * P_BYTES), 16384, smem_u32(Vs + st * TILE_BYTES),
+                   16384, idesc_o, false);
+        umma_commit_e(&o_full[sb]);
+        umma_commit_e(&v_empty[st]);
+        umma_commit_e(&p_empty[sb]);
+      }
+    }
+  } else {
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;       // row inside the query tile
+    const int row_g = qt * 128 + r;          // query position
+    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+    const float sl2 = p.scale * LOG2E_F;
+    float m = -INFINITY, l = 0.f, alpha_prev = 0.f;
+    float o[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) o[i] = 0.f;
+
+    auto fold_pv = [&](int j, float alpha) {
+      const int st = j & 1;
+      mbar_wait(&o_full[st], (j >> 1) & 1, wctx, STATUS_TIMEOUT_SOFTMAX);
+      tc_fence_after();
+      const uint32_t o_addr = tmem_base + lane_base + OP_COL + st * D;
+      uint32_t wa[32], wb[32];
+      tmem_ld_32x32(o_addr, wa);
+#pragma unroll
+      for (int c = 0; c < D; c += 64) {
+        tmem_ld_wait_for(wa);
+        tmem_ld_32x32(o_addr + c + 32, wb);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[c + e] = fmaf(o[c + e], alpha, __uint_as_float(wa[e]));
+        tmem_ld_wait_for(wb);
+        if (c + 64 < D) tmem_ld_32x32(o_addr + c + 64, wa);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[c + 32 + e] = fmaf(o[c + 32 + e], alpha, __uint_as_float(wb[e]));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&o_empty[st]);
+    };
+
+    for (int j = 0; j < n_kv; ++j) {
+      const int st = j & 1;
+      const uint32_t par = (j >> 1) & 1;
+      const bool need_mask = (p.causal && j == qt) || ((j + 1) * 128 > p.S);
+      mbar_wait(&s_full[st], par, wctx, STATUS_TIMEOUT_SOFTMAX);
+      tc_fence_after();
+      const uint32_t s_addr = tmem_base + lane_base + st * 128;
+      // pass 1: row maximum (TMEM loads double buffered against the arithmetic)
+      float mx = -INFINITY;
+      uint32_t va[32], vb[32];
+      // Diagonal / tail block: dead scores become -inf in the registers and the block runs the same
+      // max / exponential code as every other block (a separate masked copy of that code executes
+      // once per CTA from a cold instruction cache and cost more than two unmasked blocks).
+      auto mask_chunk = [&](uint32_t (&v)[32], int c) {
+        if (need_mask) {
+          const int lim_c = p.causal ? row_g - j * 128 - c : 0x7fffffff;   // last live column of the chunk
+          const int lim = min(lim_c, p.S - 1 - j * 128 - c);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = (e > lim) ? 0xff800000u : v[e];
+        }
+      };
+      auto max_chunk = [&](uint32_t (&v)[32], int c) {
+        mask_chunk(v, c);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(v[e]));
+      };
+      tmem_ld_32x32(s_addr + 0, va);
+      tmem_ld_wait_for(va);
+      tmem_ld_32x32(s_addr + 32, vb);
+      max_chunk(va, 0);
+      tmem_ld_wait_for(vb);
+      tmem_ld_32x32(s_addr + 64, va);
+      max_chunk(vb, 32);
+      tmem_ld_wait_for(va);
+      tmem_ld_32x32(s_addr + 96, vb);
+      max_chunk(va, 64);
+      tmem_ld_wait_for(vb);
+      tmem_ld_32x32(s_addr + 0, va);  // first chunk of pass 2
+      max_chunk(vb, 96);
+      const float m_new = fmaxf(m, mx);
+      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;  // row with no live key so far
+      const float alpha = fast_exp2((m - m_use) * sl2);
+      const float moff = m_use * sl2;
+      mbar_wait(&p_empty[st], par ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
+      // pass 2: probabilities -> shared memory (bf16, swizzled K-major), row sum
+      float rs = 0.f;
+      uint8_t* prow = Ps + st * P_BYTES + r * 128;
+      auto prob_chunk = [&](uint32_t (&v)[32], int c) {
+        mask_chunk(v, c);
+        uint32_t packed[16];
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          const float x0 = fast_exp2(fmaf(__uint_as_float(v[e]), sl2, -moff));
+          const float x1 = fast_exp2(fmaf(__uint_as_float(v[e + 1]), sl2, -moff));
+          rs += x0 + x1;
+          packed[e >> 1] = pack_bf16x2(x0, x1);
+        }
+        uint8_t* blk = prow + (c >> 6) * 16384;
+        const int chunk0 = (c & 63) >> 3;
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4) {
+          const uint4 w = make_uint4(packed[4 * q4], packed[4 * q4 + 1], packed[4 * q4 + 2], packed[4 * q4 + 3]);
+          *reinterpret_cast<uint4*>(blk + ((((chunk0 + q4) ^ (r & 7)) & 7) << 4)) = w;
+        }
+      };
+      tmem_ld_wait_for(va);
+      tmem_ld_32x32(s_addr + 32, vb);
+      prob_chunk(va, 0);
+      tmem_ld_wait_for(vb);
+      tmem_ld_32x32(s_addr + 64, va);
+      prob_chunk(vb, 32);
+      tmem_ld_wait_for(va);
+      tmem_ld_32x32(s_addr + 96, vb);
+      prob_chunk(va, 64);
+      tmem_ld_wait_for(vb);
+      prob_chunk(vb, 96);
+      l = l * alpha + rs;
+      m = m_new;
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&s_empty[st]);
+        mbar_arrive(&p_full[st]);
+      }
+      if (j > 0) fold_pv(j - 1, alpha_prev);
+      alpha_prev = alpha;
+    }
+    fold_pv(n_kv - 1, alpha_prev);
+
+    const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
+    {
+      // every P V MMA has completed (the last fold waited for it): the P buffer serves as staging
+      uint8_t* stage = Ps + (r >> 5) * 4096;
+      const int row0 = row_g - lane;
+      __nv_bfloat16* g0 = p.O + row0 * p.o_ss + b * p.o_bs + h * p.o_hs;
+      // twice when a copy is wanted (rolled, to keep the registers of the loop above)
+#pragma unroll 1
+      for (int n_out = p.o_copy != 0 ? 2 : 1; n_out > 0; --n_out, g0 += p.o_copy) {
+#pragma unroll
+        for (int hf = 0; hf < D / 64; ++hf) {
+          uint32_t ow[32];
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            ow[e] = pack_out(o[hf * 64 + 2 * e] * inv_l, o[hf * 64 + 2 * e + 1] * inv_l, p.o_f16);
+          store_rows_32x64(stage, ow, lane, g0 + hf * 64, p.o_ss, p.S - row0);
+        }
+      }
+    }
+    if (row_g < p.S_pad) {
+      const float mm = (m == -INFINITY) ? 0.f : m;
+      p.lse[static_cast<size_t>(bh) * p.S_pad + row_g] = mm * sl2 + log2f(fmaxf(l, 1e-37f));
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
 constexpr int FWD128_CW = 8;                           // softmax warps of a pipeline
 constexpr int FWD128_FIRST_CW = 4;                     // warps 0, 1: TMA; 2, 3: MMAs (one each per pipeline)
 constexpr int FWD128_THREADS = 32 * (FWD128_FIRST_CW + 2 * FWD128_CW);
@@ -160,15 +503,16 @@ constexpr int FWD128_SMEM = 2 * FWD128_PIPE + FWD128_XCH + 512;
 // There are no columns left for P: it overwrites the scores it was made from, and the next block's scores
 // wait for its P V.
 //
-// The output accumulates in tensor memory, and the running maximum is only raised when it grows by more
-// than 2^8 (any consistent offset gives the same softmax; the stale one keeps exp2 arguments <= 8).
-// Raising it rescales the accumulator in tensor memory, which after the first blocks is rare.
+// The output accumulates in tensor memory and is rescaled there when the running maximum grows. (Raising the
+// maximum only when it grows by more than 2^8 saves 7 to 12 % of the time, but the largest probability of a row, exactly 1
+// with the true maximum, is then rounded to bf16 like the others: the output's error against 64 bits
+// was 2 % larger for scores of unit variance and 8 to 25 % for a standard deviation of 4.)
 //
 // Persistent: items are dealt heaviest first in a snake (left to right, then right to left), which evens
 // out the totals; all barrier parities run on counters that continue across items.
 //
-// us, one CTA per 128 rows with P through shared memory and the output folded into registers -> this:
-// [1, 8, 4096, 128] causal 103 -> 84, [4, 2, 2048, 128] 42 -> 41. At head_dim 64, where a block's products are
+// us, the kernel above -> this: [1, 8, 4096, 128] causal 100 -> 88, [1, 32, 4096, 128] 290 -> 182, [2, 16, 2048, 128]
+// without a mask 138 -> 105. At head_dim 64, where a block's products are
 // half as long, the kernel below is the faster one (75 against 78 us at [16, 12, 1024, 64]): its two tiles share
 // the K and V loads.
 __global__ void __launch_bounds__(FWD128_THREADS, 1)
@@ -379,31 +723,11 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         }
         const float mx = fmaxf(mx0, mx1);
         const float m_new = fmax3(m, mx, exchange(mx));
-        // raise the running maximum only when it grew by more than 2^8 (or was still -inf); both threads of
-        // a row decide alike
-        bool grow = false;
+        // the maximum of all keys so far: both threads of a row raise it alike
+        const bool grow = m_new > m;
         float alpha = 1.f;
-        if (m_new > m && (m == -INFINITY || (m_new - m) * sl2 > 8.f)) {
-          grow = true;
-          alpha = (m == -INFINITY) ? 0.f : fast_exp2((m - m_new) * sl2);
-        }
-        if (j > 0 && __any_sync(0xffffffffu, grow)) {
-          // rescale this warp's 32 accumulator rows in tensor memory (warp-collective accesses; rows whose
-          // maximum stays get factor 1), its half of the columns. P V of the previous block must be done.
-          mbar_wait(o_full, (g - 1) & 1, wctx, STATUS_TIMEOUT_SOFTMAX);
-          tc_fence_after();
-#pragma unroll 1
-          for (int cc = 0; cc < D / 2; cc += 16) {
-            uint32_t wv[16];
-            tmem_ld_32x16(o_addr + cc, wv);
-            tmem_ld_wait_for16(wv);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) wv[e] = __float_as_uint(__uint_as_float(wv[e]) * alpha);
-            tmem_st_32x16(o_addr + cc, wv);
-          }
-          tmem_st_wait();
-        }
         if (grow) {
+          alpha = (m == -INFINITY) ? 0.f : fast_exp2((m - m_new) * sl2);
           l2 = mul_f32x2(l2, pack_f32x2(alpha, alpha));
           m = m_new;
         }
@@ -420,6 +744,24 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
             pk[e >> 1] = pack_bf16x2(p0, p1);
           }
           tmem_st_32x16(p_addr + 16 * c, pk);
+        }
+        if (j > 0 && __any_sync(0xffffffffu, grow)) {
+          // rescale this warp's 32 accumulator rows in tensor memory (warp-collective accesses; rows whose
+          // maximum stays get factor 1), its half of the columns, while the registers of the scores are free. P V of
+          // the previous block is done: this block's scores were issued after it.
+          mbar_wait(o_full, (g - 1) & 1, wctx, STATUS_TIMEOUT_SOFTMAX);
+          tc_fence_after();
+          uint32_t wv[4][16];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld_32x16(o_addr + 16 * c, wv[c]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld_wait_for16(wv[c]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) wv[c][e] = __float_as_uint(__uint_as_float(wv[c][e]) * alpha);
+            tmem_st_32x16(o_addr + 16 * c, wv[c]);
+          }
         }
         tmem_st_wait();
         tc_fence_before();
@@ -1526,7 +1868,7 @@ int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* o_
   p.scale = scale; p.causal = causal; p.o_f16 = o_f16;
   p.status = gfs_host::status_words();
   const int nb = (S + 127) / 128;
-  static bool set64 = false, set128 = false;
+  static bool set64 = false, set128 = false, set128s = false;
   if (D == 64) {
     if (!set64) { if (set_smem(flash_fwd64_kernel, FWD64_SMEM)) return -10; set64 = true; }
     const int n_pairs = (nb + 1) / 2;
@@ -1535,8 +1877,14 @@ int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* o_
     gfs_host::launch_pdl(flash_fwd64_kernel, dim3(ctas), dim3(FWD64_THREADS), FWD64_SMEM, stream, *tq, *tk, *tv, p,
                          n_pairs, n_items);
   } else {
-    if (!set128) { if (set_smem(flash_fwd128_kernel, FWD128_SMEM)) return -10; set128 = true; }
     const int n_items = nb * B * nh;
+    if (fwd128_few_items(nb, static_cast<long long>(B) * nh, causal != 0, gfs_host::sm_count())) {
+      if (!set128s) { if (set_smem(flash_fwd128_small_kernel, FWD128S_SMEM)) return -10; set128s = true; }
+      gfs_host::launch_pdl(flash_fwd128_small_kernel, dim3(nb, B * nh), dim3(FWD128S_THREADS), FWD128S_SMEM, stream, *tq,
+                           *tk, *tv, p);
+      return cudaGetLastError() == cudaSuccess ? 0 : -11;
+    }
+    if (!set128) { if (set_smem(flash_fwd128_kernel, FWD128_SMEM)) return -10; set128 = true; }
     const int ctas = std::min(n_items, gfs_host::sm_count());
     gfs_host::launch_pdl(flash_fwd128_kernel, dim3(ctas), dim3(FWD128_THREADS), FWD128_SMEM, stream, *tq, *tk, *tv, p, nb,
                          n_items);

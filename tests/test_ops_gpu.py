@@ -377,3 +377,35 @@ def test_flash_attention_fp16_output_may_be_written_to(cuda_device, B, nh, S, D)
     o += 1.0
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         o.sum().backward()
+
+
+@pytest.mark.parametrize("B,nh,S,causal", [
+    (1, 148, 100, True), (1, 149, 100, True),        # one item per SM, one more
+    (1, 10, 2048, True), (1, 13, 2048, True),        # more items that find room behind short ones, and that do not
+    (1, 19, 1024, True), (1, 20, 1024, True), (1, 9, 2048, False), (1, 10, 2048, False)])
+def test_flash_forward_128_both_kernels(cuda_device, B, nh, S, causal):
+    """head_dim 128, both sides of the line between its two forward kernels, in bf16 and fp16 (with and without the copy
+    for the backward). Tolerance: one bf16 rounding of the output and of P (2^-9 each); fp16 inputs are rounded to bf16."""
+    from gpt_from_scratch_b200.ops.attention import apply_flash_attn, attention_reference
+    g = torch.Generator(device="cuda").manual_seed(S + nh)
+    q, k, v = (torch.randn(B, nh, S, 128, device=cuda_device, generator=g).bfloat16() for _ in range(3))
+    ref = attention_reference(q.double(), k.double(), v.double(), causal)
+    assert (apply_flash_attn(q, k, v, causal).double() - ref).norm() < 4e-3 * ref.norm()
+    q, k, v = (t.half() for t in (q, k, v))
+    plain = apply_flash_attn(q, k, v, causal)
+    assert (plain.double() - ref).norm() < 4e-3 * ref.norm()
+    assert torch.equal(apply_flash_attn(q.requires_grad_(), k, v, causal).detach(), plain)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("nh", [4, 40])
+def test_flash_forward_128_largest_probability_is_exact(cuda_device, nh, causal):
+    """Scores of standard deviation 4: a row is mostly its largest probability, which is 1 before the division, exact in
+    bf16, if the running maximum is the true one. What is left is the output's own rounding (1.66e-3 rms for bf16) and
+    a part of P's: 1.74e-3 measured; 2.04e-3 and 2.16e-3 with a maximum that lags by up to 2^8."""
+    from gpt_from_scratch_b200.ops.attention import apply_flash_attn, attention_reference
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k = (2 * torch.randn(1, nh, 1024, 128, device=cuda_device, generator=g) for _ in range(2))
+    q, k, v = (t.bfloat16() for t in (q, k, torch.randn(1, nh, 1024, 128, device=cuda_device, generator=g)))
+    ref = attention_reference(q.double(), k.double(), v.double(), causal)
+    assert (apply_flash_attn(q, k, v, causal).double() - ref).norm() < 1.9e-3 * ref.norm()
