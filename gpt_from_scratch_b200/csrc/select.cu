@@ -84,10 +84,14 @@ Choice choose(int M, int N, int K, int swi_mode, bool add, bool rope, int pair_m
   Choice c{Choice::PERSISTENT_CTA, 256, 1};
   const float t_tile = best_tile(tiles, kb, pairs, &c);
   // persistent CTAs: 128 x 256 tiles in waves; the addend, the rotation and the SwiGLU gradient are serial
-  // loads in its epilogue
+  // loads in its epilogue. Plain products of up to 128 columns have 128-column tiles and half the epilogue there. Judged
+  // by the same line, 27 of 129 measured ones went to kernels more than 5 % slower than the persistent one; with
+  // one of their own up to 12 K blocks, one (us, one-tile kernel -> here: 2010 x 48 x 104 5.2 -> 4.0, 3568 x 32 x 104
+  // 5.2 -> 4.0, 463 x 32 x 72 4.8 -> 3.7). With more K blocks the split over a cluster is the better one.
   const int waves = ceil_div(ceil_div(M, 128) * ceil_div(N, swi_mode == 1 ? 128 : 256), 148);
-  const float t_cta = 5.2f + 0.3f * kb * waves + 3.8f * (waves - 1) + (add ? 3.3f : 0.f) + (rope ? 9.5f : 0.f) +
-                      (swi_mode == 1 ? 2.0f : 0.f) + (swi_mode == 2 ? 6.0f : 0.f);
+  float t_cta = 5.2f + 0.3f * kb * waves + 3.8f * (waves - 1) + (add ? 3.3f : 0.f) + (rope ? 9.5f : 0.f) +
+                (swi_mode == 1 ? 2.0f : 0.f) + (swi_mode == 2 ? 6.0f : 0.f);
+  if (N <= 128 && kb <= 12 && swi_mode == 0 && !add && !rope) t_cta = 4.0f + 0.18f * kb * waves + (waves - 1);
   if (t_cta < t_tile) c = Choice{Choice::PERSISTENT_CTA, 256, 1};
   return c;
 }

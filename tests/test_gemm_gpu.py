@@ -249,3 +249,20 @@ def test_swiglu_backward_on_pairs(cuda_device, M, I, K):
     assert (out[M] == 7.0).all() and (out[:, 2 * I:] == 7.0).all()
     rel = (out[:M, :2 * I].double() - ref).norm() / ref.norm()
     assert rel < 5e-3, rel
+
+
+@pytest.mark.parametrize("N", [8, 120, 128, 136])
+@pytest.mark.parametrize("M,K", [(40, 72), (2010, 104), (304, 768), (304, 776), (304, 2200), (19200, 72)])
+def test_gemm_few_columns(cuda_device, M, N, K):
+    """Around the 128 columns up to which a plain product may stay on the persistent kernel's narrow tiles: one tile, a
+    wave with a ragged end, a long K loop, more tiles than SMs; with and without the addend that rules it out."""
+    from gpt_from_scratch_b200.ops.gemm import gemm_bf16
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    for a_mn, b_mn in ((False, False), (False, True), (True, True)):
+        a = torch.randn((K, M) if a_mn else (M, K), device=cuda_device, generator=g).bfloat16()
+        if a_mn and M % 8:
+            a = torch.nn.functional.pad(a, (0, 8 - M % 8))[:, :M]     # the pitch stays a multiple of 8 elements
+        b = torch.randn((K, N) if b_mn else (N, K), device=cuda_device, generator=g).bfloat16()
+        c = torch.randn(M, N, device=cuda_device, generator=g).bfloat16()
+        _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn), _ref(a, b, a_mn, b_mn, None), K)
+        _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn, addend=c), _ref(a, b, a_mn, b_mn, c), K)
