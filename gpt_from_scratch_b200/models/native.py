@@ -94,7 +94,7 @@ class _Plan:
 
     def __init__(self, model):
         self.dicts, self.keys, self.values = [], [], []
-        self.modules, self.tensors = [], []
+        self.modules, self.tensors, self.tables = [], [], []
 
         def read(place: dict, key: str):
             value = place[key]
@@ -109,14 +109,11 @@ class _Plan:
             self.modules.append(m)
             return m
 
-        def tensor(place: dict, name: str, dtype: torch.dtype, shape=None):
-            t = read(place, name)
-            _require(_native_tensor(t, dtype) and (shape is None or tuple(t.shape) == shape))
-            self.tensors.append(t)
-            return t
-
         def weight(m, *shape):
-            return tensor(m._parameters, "weight", torch.bfloat16, shape or None)
+            w = read(m._parameters, "weight")
+            _require(_native_tensor(w, torch.bfloat16) and (not shape or tuple(w.shape) == shape))
+            self.tensors.append(w)
+            return w
 
         def linear(parent, name: str, cls, *shape):
             m = child(parent, name, cls)
@@ -155,8 +152,10 @@ class _Plan:
             I = ws[5].shape[1]
             _require(ws[4].shape == (2 * I, H) and ws[5].shape == (H, I) and I % 8 == 0)
             rot = child(a, "rotary_emb", RotaryEmbedding)
-            cos, sin = (tensor(rot._buffers, k, torch.float32) for k in ("cos_cached", "sin_cached"))
+            cos, sin = read(rot._buffers, "cos_cached"), read(rot._buffers, "sin_cached")
+            _require(_native_tensor(cos, torch.float32) and _native_tensor(sin, torch.float32))
             _require(cos.shape == sin.shape and cos.dim() == 2 and cos.shape[1] == D // 2)
+            self.tables += (cos, sin)
             self.table_rows = min(self.table_rows or cos.shape[0], cos.shape[0])
             self.settings.add((nh, D, I, read(layer.__dict__, "dropout_prob")))
             self.rotaries.append(rot)
@@ -194,7 +193,7 @@ class _Plan:
     def _looks(self) -> tuple:
         ts = self.tensors
         return ([t.data_ptr() for t in ts], [t.shape for t in ts], [t.dtype for t in ts],
-                [t.is_contiguous() for t in ts])
+                [t.is_contiguous() for t in ts], [t.data_ptr() for t in self.tables])
 
     def current(self) -> bool:
         """True if nothing that the plan was built from has changed. (Loops in C: 60 us for 12 blocks.)"""
@@ -232,10 +231,11 @@ class _Plan:
 class _Pass:
     """The arguments of one pass: copies of its own, because the library reads them without the interpreter lock
     while other threads start passes of the same model, and because a backward may come long after its forward."""
-    __slots__ = ("plan", "S", "B", "dropout", "dims", "params")
+    __slots__ = ("plan", "S", "B", "dropout", "dims", "params", "gradients")
 
     def __init__(self, plan: _Plan, S: int, B: int, dropout: float):
         self.plan, self.S, self.B, self.dropout = plan, S, B, dropout     # the plan also keeps the tables alive
+        self.gradients = None           # addresses of the gradients of plan.all_params when the pass began
         d = self.dims = _Dims.from_buffer_copy(plan.dims)
         d.S, d.B, d.dropout_p = S, B, dropout
         d.pair_min_tiles = gemm_ops.pair_threshold()
@@ -254,13 +254,12 @@ class _Pass:
         for bp, s0, s1 in zip(self.params, seeds[0::2], seeds[1::2]):
             bp.seed[0], bp.seed[1] = s0, s1
 
-    def put_gradients(self, params) -> None:
-        """Where the blocks' weight gradients go, and whether they are added to what is there."""
-        for bp, ws in zip(params, self.plan.weights):
-            g, acc = bp.g, bp.accumulate
-            for k, w in enumerate(ws):
-                g[k] = w.grad.data_ptr()
-                acc[k] = _consume(w)
+    def put_gradients(self, params, addresses, add) -> None:
+        """Where the blocks' weight gradients go, and whether they are added to what is there (as :func:`_consume`
+        says; both in the order of ``plan.all_params``)."""
+        for i, bp in enumerate(params):
+            bp.g[:] = addresses[6 * i:6 * i + 6]
+            bp.accumulate[:] = add[6 * i:6 * i + 6]
 
     def for_backward(self, weights):
         """The blocks' arguments with ``weights`` (as autograd returns them) and their gradients."""
@@ -271,7 +270,8 @@ class _Pass:
                 t = next(it)
                 assert t.shape == w.shape and _native_tensor(t, torch.bfloat16), "a weight changed since the forward"
                 bp.w[k] = t.data_ptr()
-        self.put_gradients(params)
+        blocks = self.plan.all_params[:-3]
+        self.put_gradients(params, [w.grad.data_ptr() for w in blocks], [_consume(w) for w in blocks])
         return params
 
 
@@ -289,12 +289,22 @@ def _renew(model) -> _Plan | None:
     return plan
 
 
-def _observed(hooks) -> bool:
-    """A hook on a parameter other than the optimizer's own: it is called when the gradient is complete."""
-    for hook in hooks.values() if hooks else ():
-        if not getattr(hook, "clears_slice", False):
-            return True
-    return False
+def _sinks(params) -> list | None:
+    """Addresses of the gradients if every one goes to a slice of its own in the optimizer's buffer (what
+    GradSink.of asks for) and nobody waits for single ones or looks at them, else ``None``."""
+    addresses = []
+    for p in params:
+        attrs, g = p.__dict__, p.grad
+        if (g is None or not p.requires_grad or not attrs.get("_grad_sink_ok") or
+                attrs.get("_grad_ready_cb") is not None or p._post_accumulate_grad_hooks or not g.is_contiguous()):
+            return None
+        for hook in p._backward_hooks.values() if p._backward_hooks else ():
+            if not getattr(hook, "clears_slice", False):    # not the optimizer's own
+                return None
+        addresses.append(g.data_ptr())
+    if len(set(addresses)) != len(addresses) or any(a % 16 for a in addresses):
+        return None
+    return addresses
 
 
 def _autograd_is_watched() -> bool:
@@ -321,22 +331,14 @@ def plan_for(model, inputs: torch.Tensor) -> _Pass | None:
     dropout = plan.dropout_now()
     if inputs.device != plan.top[0].device or S > plan.table_rows or dropout is None:
         return None
+    run = _Pass(plan, S, inputs.shape[0], dropout)
     if torch.is_grad_enabled():
         if _autograd_is_watched():
             return None
-        slices = set()
-        for p in plan.all_params:
-            # every gradient goes to a slice of its own in the optimizer's buffer and nobody waits for single ones
-            if (not p.requires_grad or GradSink.of(p) is None or getattr(p, "_grad_ready_cb", None) is not None or
-                    p._post_accumulate_grad_hooks or _observed(p._backward_hooks)):
-                return None
-            g = p.grad
-            if not _native_tensor(g, torch.bfloat16):
-                return None
-            slices.add(g.data_ptr())
-        if len(slices) != len(plan.all_params):
+        run.gradients = _sinks(plan.all_params)
+        if run.gradients is None:
             return None
-    return _Pass(plan, S, inputs.shape[0], dropout)
+    return run
 
 
 def _stack_forward(run: _Pass, x: torch.Tensor, keep: bool):
@@ -476,11 +478,10 @@ def train_pass(model, inputs: torch.Tensor, labels: torch.Tensor):
     loss = torch.empty((), dtype=torch.float32, device=dev)
     if run.dropout > 0.0:
         run.draw_seeds()
-    fresh = [getattr(p, "_grad_fresh", False) for p in plan.all_params]
-    run.put_gradients(run.params)
-    for k, w in enumerate(plan.top):
-        top.g[k] = w.grad.data_ptr()
-        top.accumulate[k] = _consume(w)
+    fresh = [p.__dict__.get("_grad_fresh", False) for p in plan.all_params]
+    add = [_consume(p) for p in plan.all_params]
+    run.put_gradients(run.params, run.gradients, add)
+    top.g[:], top.accumulate[:] = run.gradients[-3:], add[-3:]
     launches = c_int(0)
     with _lib.nvtx("fused:model_step"):
         rc = lib.gfs_model_step(dims, run.params, byref(top), ids.data_ptr(), labels.data_ptr(), arena.data_ptr(),
