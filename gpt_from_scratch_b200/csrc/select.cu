@@ -4,7 +4,7 @@
 //   persistent CTAs    gemm.cu    128 x 256 per CTA
 //   one tile per CTA   gemm3.cu   128 x 64, 128 x 128 or 256 x 256 (pair), K split over a cluster
 //
-// From `pair_min_tiles` (60) tiles of 256 x 256 on, the persistent pairs always win. Below, a product is one
+// From `pair_min_tiles` (60) tiles of 256 x 256 on, the persistent pairs always win. Below, a product is mostly one
 // wave of whatever kernel runs it, and its time is a constant (launch, first TMA, epilogue) plus the K blocks
 // one CTA works through. The constants below were fitted to 110 measured (shape, kernel) pairs on B200: M 103 to
 // 4096, N 256 to 50304, K 103 to 50304, every layout, back to back in a CUDA graph; the fits are within 15 %.
@@ -79,7 +79,7 @@ Choice choose(int M, int N, int K, int swi_mode, bool add, bool rope, int pair_m
     return ceil_div(M, bn == 256 ? 256 : 128) * ceil_div(N, cols);
   };
   const int kb = ceil_div(K, 64);
-  const bool pairs = pair_min_tiles >= 0;
+  const bool pairs = pair_min_tiles >= 0, plain = swi_mode == 0 && !add && !rope;
   if (pairs && (K >= 256 || swi_mode != 0) && tiles(256) >= pair_min_tiles) return Choice{Choice::PERSISTENT_PAIR, 256, 1};
   Choice c{Choice::PERSISTENT_CTA, 256, 1};
   const float t_tile = best_tile(tiles, kb, pairs, &c);
@@ -91,8 +91,15 @@ Choice choose(int M, int N, int K, int swi_mode, bool add, bool rope, int pair_m
   const int waves = ceil_div(ceil_div(M, 128) * ceil_div(N, swi_mode == 1 ? 128 : 256), 148);
   float t_cta = 5.2f + 0.3f * kb * waves + 3.8f * (waves - 1) + (add ? 3.3f : 0.f) + (rope ? 9.5f : 0.f) +
                 (swi_mode == 1 ? 2.0f : 0.f) + (swi_mode == 2 ? 6.0f : 0.f);
-  if (N <= 128 && kb <= 12 && swi_mode == 0 && !add && !rope) t_cta = 4.0f + 0.18f * kb * waves + (waves - 1);
+  if (N <= 128 && kb <= 12 && plain) t_cta = 4.0f + 0.18f * kb * waves + (waves - 1);
   if (t_cta < t_tile) c = Choice{Choice::PERSISTENT_CTA, 256, 1};
+  // Persistent pairs from a third of the threshold on, where the K loop is long enough for their rate: 256 x 256 tiles
+  // ask least of shared memory and L2 (128 x 128 tiles on all SMs take 0.4 us per K block, not 0.27). Of 439 measured
+  // plain products 17 go there, none slower, up to 27 % faster: us, one-tile kernel or persistent CTAs -> here,
+  // 4576 x 656 x 8184 53 -> 45, 4393 x 760 x 2544 27 -> 20. (A lone weight gradient of 768 x 3072 x 16384 takes 77 us here and
+  // 69 with K split through a workspace, which callers on several streams would share; in a step it is part of a group.)
+  if (pairs && plain && K >= 256 && N > 128 && tiles(256) >= pair_min_tiles / 3 && 6.0f + 0.22f * kb < std::min(t_cta, t_tile))
+    c = Choice{Choice::PERSISTENT_PAIR, 256, 1};
   return c;
 }
 
@@ -101,7 +108,7 @@ Choice choose(int M, int N, int K, int swi_mode, bool add, bool rope, int pair_m
 extern "C" {
 
 // C[M,N] = op(A) op(B) (+ R); arguments as gfs_gemm_bf16_rope (R null: no addend). pair_min_tiles: number of
-// 256 x 256 tiles from which the persistent pair kernel is used; < 0: no kernel on CTA pairs.
+// 256 x 256 tiles from which the persistent pair kernel is always used; < 0: no kernel on CTA pairs.
 int gfs_linear(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,
                int ldr, int a_mn_major, int b_mn_major, const void* rope_cos, const void* rope_sin, int rope_cols,
                int rope_d, int rope_b, int pair_min_tiles, void* stream) {

@@ -46,7 +46,7 @@ class pair_min_tiles:
 
 
 def pair_threshold() -> int:
-    """Number of 256 x 256 tiles from which the persistent CTA-pair kernel serves a product; -1: no kernel
+    """Number of 256 x 256 tiles from which the persistent CTA-pair kernel always serves a product; -1: no kernel
     on CTA pairs. csrc/select.cu chooses by it."""
     return _PAIR_MIN_TILES if _PAIR_ENABLED else -1
 

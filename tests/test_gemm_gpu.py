@@ -266,3 +266,18 @@ def test_gemm_few_columns(cuda_device, M, N, K):
         c = torch.randn(M, N, device=cuda_device, generator=g).bfloat16()
         _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn), _ref(a, b, a_mn, b_mn, None), K)
         _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn, addend=c), _ref(a, b, a_mn, b_mn, c), K)
+
+
+@pytest.mark.parametrize("M,N,K", [(4393, 760, 2544), (623, 2208, 984), (1400, 768, 256), (768, 1288, 4104)])
+def test_gemm_below_the_pair_threshold(cuda_device, M, N, K):
+    """20 to 59 tiles of 256 x 256: a plain product may go to the persistent pairs, one with an addend may not."""
+    from gpt_from_scratch_b200.ops.gemm import gemm_bf16
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    for a_mn, b_mn in ((False, False), (False, True), (True, True)):
+        if a_mn and M % 8:
+            continue
+        a = torch.randn((K, M) if a_mn else (M, K), device=cuda_device, generator=g).bfloat16()
+        b = torch.randn((K, N) if b_mn else (N, K), device=cuda_device, generator=g).bfloat16()
+        c = torch.randn(M, N, device=cuda_device, generator=g).bfloat16()
+        _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn), _ref(a, b, a_mn, b_mn, None), K)
+        _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn, addend=c), _ref(a, b, a_mn, b_mn, c), K)
