@@ -616,3 +616,37 @@ def test_two_threads_train_and_evaluate(cuda_device):
     assert len(trained) == 40 and len(logits) == 80
     assert all(torch.equal(a, alone[0][0]) and torch.equal(b, alone[0][1]) for a, b in trained)
     assert all(torch.equal(a, logits_alone[0]) for a in logits)
+
+
+@pytest.mark.parametrize("H,heads,I,V,B,S", [(256, 4, 512, 512, 3, 50), (768, 12, 2048, 16384, 4, 256)])
+def test_native_step_adds_to_existing_gradients(cuda_device, H, heads, I, V, B, S):
+    """Two micro-batches without zero_grad in between: the second one's gradients are added, by kernels that are
+    launched alone and in groups, and to an embedding table that is not cleared. Tolerance: the module path, twice
+    that of one micro-batch."""
+    from gpt_from_scratch_b200.config import GPTConfig
+    from gpt_from_scratch_b200.engine import TrainEngine
+    from gpt_from_scratch_b200.models import native
+    from gpt_from_scratch_b200.parallel import parallel_state as ps
+    ps.set_device(cuda_device)
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_parallel_state(1)
+    cfg = GPTConfig(vocab_size=V, hidden_size=H, num_layers=2, num_attention_heads=heads, max_position_embeddings=S,
+                    intermediate_size=I)
+    g = torch.Generator().manual_seed(2)
+    batches = [torch.randint(0, V, (B, S + 1), generator=g).cuda() for _ in range(2)]
+    grads = []
+    for modules in (False, True):
+        eng = TrainEngine(cfg, seed=5)
+        eng.optimizer.overlap_grad_reduce = False
+        if modules:
+            eng.model.layers[-1].mlp.register_forward_hook(lambda *a: None)
+        eng.optimizer.zero_grad()
+        for t in batches:
+            x, y = t[:, :-1].contiguous(), t[:, 1:].contiguous()
+            if modules:
+                eng.forward_loss(x, y).backward()
+            else:
+                assert native.train_pass(eng.model, x, y) is not None
+        torch.cuda.synchronize()
+        grads.append(eng.optimizer.grad_buffer.double())
+    assert (grads[0] - grads[1]).norm() < 4e-3 * grads[1].norm()
