@@ -159,6 +159,11 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void*
                "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* src, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
+               "r"(smem_u32(src)), "r"(c0), "r"(c1)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all of this thread's stores have read their shared memory / are complete
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -730,7 +735,7 @@ __device__ __forceinline__ void named_barrier_arrive(int id, int nthreads) {
 // ----------------------------------------------------------------------------
 namespace gfs_host {
 
-// Encode a tiled bf16 tensor map with 128-byte swizzle. dims/strides are innermost
+// Encode a tiled bf16 tensor map with 128-byte swizzle (boxes of up to 32 columns: 64-byte). dims/strides are innermost
 // first; strides[0] is implied (2 bytes). Returns 0 on success.
 int encode_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                      const uint32_t* box);

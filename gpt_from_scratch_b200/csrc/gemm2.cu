@@ -55,28 +55,26 @@ constexpr int A_BYTES = BM * BK * 2;     // 16 KB
 constexpr int B_BYTES = BNH * BK * 2;    // 16 KB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int EPI_BYTES = 8 * 4096;     // one [32 rows x 128 B] transpose buffer per epilogue warp
-// Epilogue warps per CTA: 8 in the plain kernel (two per TMEM lane quarter, each taking half of the
-// tile's columns, so epilogues with real work per element still hide behind the next tile's
-// MMAs), also in the all-gather variant (its two push warps are cheap: 384 threads at up to 170
-// registers), also in the reduce-scatter variant (with four, its epilogue - 9000 cycles per tile -
-// was the longest phase of the small reduce-scatter GEMMs).
-__host__ __device__ constexpr int epi_warps(int comm) { return 8 + 0 * comm; }
+// Epilogue warps per CTA. Plain products: sixteen, one [32 rows x 64 columns] unit of the CTA's 128 x 256 half tile
+// each, results (and the addend) moving by TMA through 4 KB of shared memory per warp. At a K loop of 12 blocks (K = 768,
+// 7,100 cycles) eight warps with two units each, loads and stores of their own, took longer than the loop as soon as the
+// epilogue had anything to compute, and a kernel's last epilogue is never hidden. The price is one of six ring stages.
+// us, eight warps -> this, K = 768: [16384, 2304] with rotary epilogue 62 -> 49, [16384, 768] with addend 24 -> 20, SwiGLU
+// forward [16384, 2 x 3072] 142 -> 130 and backward 121 -> 117, LM head [8192, 50304] 626 -> 575.
+// The variants with collectives: eight (two per TMEM lane quarter, half of the tile's columns each), and two warps
+// for the transfers.
+__host__ __device__ constexpr int epi_warps(int comm) { return comm == COMM_NONE ? 16 : 8; }
 __host__ __device__ constexpr int threads2(int comm) { return 64 + 32 * epi_warps(comm) + (comm != 0 ? 64 : 0); }
+__host__ __device__ constexpr int stages2(int comm) { return comm == COMM_NONE ? 5 : STAGES; }
+__host__ __device__ constexpr int epi_bytes2(int comm) { return epi_warps(comm) * 4096; }
+constexpr int BAR_BYTES = 512;
+constexpr int XCH_BYTES = 8 * 32 * 8;   // SWI == 3: a (max, sum) pair per row and 128-column slice
 constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + 256 + 1024;
-// SWI == 4: the SwiGLU backward epilogue reads gate | up and writes their gradients with TMA, through two
-// [gate | up] slots of [32 rows x 64 columns] each per warp, paid for with half of the ring's stages. With a short K
-// loop what bounds that product is the 512 KB that a tile reads and writes there: loads by the epilogue's own threads
-// leave their latency (once per 64 columns) and the transposes exposed. With a long one the ring counts more.
-// us, loads by the threads -> TMA, [16384, K] x [K, 3072]: K 256 127 -> 109, 768 133 -> 121, 1024 139 -> 137,
-// 1280 141 -> 154, 2048 159 -> 209; [8192, K] x [K, 5632]: 512 121 -> 104, 1024 127 -> 127, 1536 133 -> 162.
-// (The forward's epilogue only writes; the same scheme there, with four ring stages, took 161 us instead of 151.)
-constexpr int SWI_TMA_MAX_K = 1024;
-__host__ __device__ constexpr bool epi_tma(int comm, int swi) { return comm == COMM_NONE && swi == 4; }
-__host__ __device__ constexpr int stages2(int comm, int swi) { return epi_tma(comm, swi) ? 3 : STAGES; }
-__host__ __device__ constexpr int epi_bytes2(int comm, int swi) { return epi_tma(comm, swi) ? 8 * 16384 : EPI_BYTES; }
-__host__ __device__ constexpr int smem2(int comm, int swi) {
-  return stages2(comm, swi) * STAGE_BYTES + epi_bytes2(comm, swi) + 512 + 1024;
+// (without a collective the base is used as it is, 1024-byte aligned)
+__host__ __device__ constexpr int smem2(int comm) {
+  return stages2(comm) * STAGE_BYTES + epi_bytes2(comm) + BAR_BYTES + (comm == COMM_NONE ? XCH_BYTES : 1024);
 }
+static_assert(smem2(COMM_NONE) <= 232448, "shared memory of an SM");
 
 struct Params2 {
   int M, N, K;
@@ -97,7 +95,7 @@ struct Params2 {
   int swi_I, swi_ld;
   __nv_bfloat16* swi_act;
   const __nv_bfloat16* swi_gu;
-  // SWI == 4: as 2, gate | up and their gradients through shared memory with TMA.
+  // SWI == 5: rotary embedding of the first rope_cols columns (without collectives; with them, a run-time switch).
   // SWI == 3 (LM head): besides storing the logits, every epilogue warp writes the online-softmax
   // statistics (max, sum exp(x - max)) of its 128 columns of each row, computed from the
   // bf16-rounded logits: ce_partials[(tile_n * 2 + column half) * M + row]. A small kernel
@@ -147,27 +145,340 @@ __device__ __forceinline__ void decode_tile2(const Params2& p, int t, int& m0, i
   }
 }
 
+// The epilogue of a warp of a plain product (COMM_NONE): rows [32 q, + 32) and one sixteenth of the columns of each of the
+// CTA's half tiles, a row per thread. Results leave through `slot` (4 KB, this warp's) by TMA, which clips what lies
+// outside the matrices and writes whole segments; the accumulator is handed back as soon as it has been read.
+//   SWI 0  64 columns; + R, which TMA has brought into the slot while the previous tiles were worked on
+//   SWI 5  64 columns, rotary embedding
+//   SWI 3  64 columns and their share of the row statistics
+//   SWI 1  32 gate and 32 up columns -> both and act
+//   SWI 2  64 columns of d_act in two chunks: gate | up of a chunk come into the slot, their gradients take their place
+// 64-column boxes are swizzled over 128-byte rows, 32-column ones (SWI 1, 2) over 64-byte rows, so that threads that
+// own rows meet no bank conflicts.
+template <int SWI>
+__device__ __forceinline__ void epilogue_plain(const Params2& p, const CUtensorMap& tmap_x, const CUtensorMap& tmap_y,
+                                               uint8_t* slot, uint64_t* bar, float2* xch_all, uint64_t* tmem_full,
+                                               uint64_t* tmem_empty, uint32_t tmem_base, int rank, int pair,
+                                               int num_pairs, int total_tiles, int ew, int q, const WaitCtx& wctx) {
+  const int lane = threadIdx.x & 31;
+  const int cg = ew >> 2;                                      // column group of the tile
+  constexpr int COLS = SWI == 1 ? 32 : 64;                     // output columns of this warp (SWI 1: of gate)
+  const int col_limit = (SWI == 1 || SWI == 2) ? p.swi_I : p.N;
+  const uint32_t sw128 = lane & 7, sw64 = (lane >> 1) & 3;
+  uint8_t* const row128 = slot + lane * 128;
+  uint8_t* const row64 = slot + lane * 64;
+  const bool has_add = SWI == 0 && p.R != nullptr;
+  auto tile_origin = [&](int t, int& row0, int& col0) {
+    row0 = (t / p.tiles_n) * 256 + rank * BM + q * 32;
+    col0 = (t % p.tiles_n) * (SWI == 1 ? BN / 2 : BN) + cg * COLS;
+  };
+  // loads into the slot, one box ahead: the addend of the next live tile, or the next chunk of gate | up
+  uint32_t n_box = 0;
+  int pf_t = pair, pf_h = 0;
+  auto prefetch = [&]() {
+    for (; pf_t < total_tiles; pf_t += num_pairs, pf_h = 0) {
+      int row0, col0;
+      tile_origin(pf_t, row0, col0);
+      col0 += 32 * pf_h;
+      if (row0 >= p.M || col0 >= col_limit) continue;
+      if (lane == 0) {
+        bulk_wait_read_all();             // the slot's previous results have left it
+        mbar_arrive_expect_tx(bar, 4096);
+        if (SWI == 2) {
+          tma_load_3d(slot, &tmap_x, bar, col0, 0, row0);
+          tma_load_3d(slot + 2048, &tmap_x, bar, col0, 1, row0);
+        } else {
+          tma_load_2d(slot, &tmap_x, bar, col0, row0);
+        }
+      }
+      if (SWI == 2 && pf_h == 0) pf_h = 1;
+      else { pf_h = 0; pf_t += num_pairs; }
+      return;
+    }
+  };
+  if (SWI == 2 || has_add) prefetch();
+
+  int acc = 0;
+  uint32_t acc_phase = 0;
+  uint32_t n_tile = 0;
+  for (int t = pair; t < total_tiles; t += num_pairs, ++n_tile) {
+    int row0, col0;
+    tile_origin(t, row0, col0);
+    const bool live = row0 < p.M && col0 < col_limit;
+    // rotary table entries of the vectors that this lane turns, the first half ahead of the accumulator
+    float4 cs[4], sn[4];
+    const int rrow = lane >> 3, gcol = col0 + (lane & 7) * 8;
+    const bool rope = SWI == 5 && live && col0 < p.rope_cols;
+    auto load_rope = [&](int i0) {
+      const int d2 = (gcol % p.rope_d) >> 1;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int s = min(row0 + (i0 + i) * 4 + rrow, p.M - 1) / p.rope_b;
+        const size_t at = static_cast<size_t>(s) * (p.rope_d >> 1) + d2;
+        cs[i] = *reinterpret_cast<const float4*>(p.rope_cos + at);
+        sn[i] = *reinterpret_cast<const float4*>(p.rope_sin + at);
+      }
+    };
+    if (rope) load_rope(0);
+    mbar_wait(&tmem_full[acc], acc_phase, wctx, STATUS_TIMEOUT_TMEM_FULL);
+    if (t == pair && ew == 0 && lane == 0) trace_stamp(p, TRACE_EPI_BEGIN);
+    tc_fence_after();
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + cg * COLS;
+    auto release = [&]() {      // the accumulator may be overwritten once all epilogue warps of the pair have read it
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty[acc]), 0));
+    };
+    auto slot_free = [&]() {    // the previous tile's results have left the slot
+      if (lane == 0) bulk_wait_read_all();
+      __syncwarp();
+    };
+    float ce_m = -INFINITY, ce_s = 0.f;
+    if (!live) {
+      release();
+    } else if (SWI == 1) {
+      uint32_t vg[32], vu[32];
+      tmem_ld_32x32(t_row, vg);
+      tmem_ld_32x32(t_row + BN / 2, vu);
+      slot_free();
+      tmem_ld_wait_for(vg);
+      tmem_ld_wait_for(vu);
+      release();
+      uint32_t pg[16], pu[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        pg[e] = pack_bf16x2(__uint_as_float(vg[2 * e]), __uint_as_float(vg[2 * e + 1]));
+        pu[e] = pack_bf16x2(__uint_as_float(vu[2 * e]), __uint_as_float(vu[2 * e + 1]));
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint8_t* at = row64 + ((j ^ sw64) << 4);
+        *reinterpret_cast<uint4*>(at) = make_uint4(pg[4 * j], pg[4 * j + 1], pg[4 * j + 2], pg[4 * j + 3]);
+        *reinterpret_cast<uint4*>(at + 2048) = make_uint4(pu[4 * j], pu[4 * j + 1], pu[4 * j + 2], pu[4 * j + 3]);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_3d(&tmap_y, slot, col0, 0, row0);
+        tma_store_3d(&tmap_y, slot + 2048, col0, 1, row0);
+        bulk_commit();
+      }
+      // act from the bf16-rounded projections, silu rounded to bf16 before the product
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const float2 g2 = unpack_bf16x2(pg[e]), u2 = unpack_bf16x2(pu[e]);
+        const float s0 = __bfloat162float(__float2bfloat16_rn(g2.x * sigmoid_f(g2.x)));
+        const float s1 = __bfloat162float(__float2bfloat16_rn(g2.y * sigmoid_f(g2.y)));
+        pg[e] = pack_bf16x2(s0 * u2.x, s1 * u2.y);
+      }
+      slot_free();
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<uint4*>(row64 + ((j ^ sw64) << 4)) =
+            make_uint4(pg[4 * j], pg[4 * j + 1], pg[4 * j + 2], pg[4 * j + 3]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&tmap_x, slot, col0, row0);
+        bulk_commit();
+      }
+    } else if (SWI == 2) {
+      uint32_t pd[32];    // d_act rounded to bf16, as when it is a tensor of its own
+      {
+        uint32_t va[32], vb[32];
+        tmem_ld_32x32(t_row, va);
+        tmem_ld_32x32(t_row + 32, vb);
+        tmem_ld_wait_for(va);
+        tmem_ld_wait_for(vb);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          pd[e] = pack_bf16x2(__uint_as_float(va[2 * e]), __uint_as_float(va[2 * e + 1]));
+          pd[16 + e] = pack_bf16x2(__uint_as_float(vb[2 * e]), __uint_as_float(vb[2 * e + 1]));
+        }
+      }
+      release();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (col0 + 32 * h >= col_limit) break;
+        mbar_wait(bar, n_box & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+        ++n_box;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint8_t* at = row64 + ((j ^ sw64) << 4);
+          uint4 g4 = *reinterpret_cast<const uint4*>(at), u4 = *reinterpret_cast<const uint4*>(at + 2048);
+          uint32_t *gp = &g4.x, *up = &u4.x;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 d2 = unpack_bf16x2(pd[16 * h + 4 * j + e]);
+            const float2 g2 = unpack_bf16x2(gp[e]), u2 = unpack_bf16x2(up[e]);
+            const float sg0 = sigmoid_f(g2.x), sg1 = sigmoid_f(g2.y);
+            gp[e] = pack_bf16x2(d2.x * u2.x * sg0 * (1.f + g2.x * (1.f - sg0)),
+                                d2.y * u2.y * sg1 * (1.f + g2.y * (1.f - sg1)));
+            up[e] = pack_bf16x2(d2.x * g2.x * sg0, d2.y * g2.y * sg1);
+          }
+          *reinterpret_cast<uint4*>(at) = g4;
+          *reinterpret_cast<uint4*>(at + 2048) = u4;
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_3d(&tmap_y, slot, col0 + 32 * h, 0, row0);
+          tma_store_3d(&tmap_y, slot + 2048, col0 + 32 * h, 1, row0);
+          bulk_commit();
+        }
+        prefetch();
+      }
+    } else {
+      uint32_t pk[32];    // this row's 64 columns, rounded to bf16
+      {
+        uint32_t va[32], vb[32];
+        tmem_ld_32x32(t_row, va);
+        tmem_ld_32x32(t_row + 32, vb);
+        if (!has_add) slot_free();
+        tmem_ld_wait_for(va);
+        tmem_ld_wait_for(vb);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          pk[e] = pack_bf16x2(__uint_as_float(va[2 * e]), __uint_as_float(va[2 * e + 1]));
+          pk[16 + e] = pack_bf16x2(__uint_as_float(vb[2 * e]), __uint_as_float(vb[2 * e + 1]));
+        }
+      }
+      release();
+      if (has_add) {
+        mbar_wait(bar, n_box & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+        ++n_box;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        uint8_t* at = row128 + ((j ^ sw128) << 4);
+        uint4 w = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+        if (has_add) {
+          const uint4 r4 = *reinterpret_cast<const uint4*>(at);
+          const uint32_t* rp = &r4.x;
+          uint32_t* wp = &w.x;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 a = unpack_bf16x2(wp[e]), r = unpack_bf16x2(rp[e]);
+            wp[e] = pack_bf16x2(a.x + r.x, a.y + r.y);
+          }
+        }
+        *reinterpret_cast<uint4*>(at) = w;
+      }
+      if (rope) {
+        // Turned in the transposed order, eight lanes to a row: the table's entries are then read as whole
+        // segments (by their rows' threads they would be 32 passes through the load / store unit each).
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (i == 4) load_rope(4);
+          const int r = i * 4 + rrow;
+          uint4* at = reinterpret_cast<uint4*>(slot + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+          if (gcol < p.rope_cols) {
+            uint4 w = *at;
+            const float2 a0 = unpack_bf16x2(w.x), a1 = unpack_bf16x2(w.y), a2 = unpack_bf16x2(w.z),
+                         a3 = unpack_bf16x2(w.w);
+            const float4 c = cs[i & 3], s = sn[i & 3];
+            float f[8] = {a0.x * c.x - a0.y * s.x, a0.x * s.x + a0.y * c.x, a1.x * c.y - a1.y * s.y,
+                          a1.x * s.y + a1.y * c.y, a2.x * c.z - a2.y * s.z, a2.x * s.z + a2.y * c.z,
+                          a3.x * c.w - a3.y * s.w, a3.x * s.w + a3.y * c.w};
+            w = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
+                           pack_bf16x2(f[6], f[7]));
+            *at = w;
+          }
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&tmap_y, slot, col0, row0);
+        bulk_commit();
+      }
+      if (has_add) prefetch();
+      if (SWI == 3) {
+        // fold the row's bf16-rounded values into (max, sum exp(x - max)); columns past N only exist in the last tile
+        constexpr float L2E = 1.4426950408889634f;
+        const int n_valid = p.N - col0;
+        if (n_valid < 64) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const uint32_t lo = (2 * e < n_valid) ? (pk[e] & 0xffffu) : 0xff80u;          // bf16 -inf
+            const uint32_t hi = (2 * e + 1 < n_valid) ? (pk[e] & 0xffff0000u) : 0xff800000u;
+            pk[e] = lo | hi;
+          }
+        }
+        float cm0 = -INFINITY, cm1 = -INFINITY;
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          cm0 = fmaxf(cm0, __uint_as_float(pk[e] << 16));
+          cm1 = fmaxf(cm1, __uint_as_float(pk[e] & 0xffff0000u));
+        }
+        ce_m = fmaxf(cm0, cm1);
+        const float off = (ce_m == -INFINITY) ? 0.f : ce_m * L2E;
+        float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          a0 += fast_exp2(fmaf(__uint_as_float(pk[e] << 16), L2E, -off));
+          a1 += fast_exp2(fmaf(__uint_as_float(pk[e] & 0xffff0000u), L2E, -off));
+        }
+        ce_s = a0 + a1;
+      }
+    }
+    if (SWI == 3) {
+      // Two warps share a 128-column slice: one hands its pair over, the other one folds and stores. They change
+      // parts with every tile, so the buffer is written by the warp that read it last and one barrier is enough.
+      float2* xch = xch_all + (q + 4 * (cg >> 1)) * 32 + lane;
+      const bool gives = (cg & 1) != static_cast<int>(n_tile & 1);
+      if (gives) *xch = make_float2(ce_m, ce_s);
+      named_barrier_sync(1 + q + 4 * (cg >> 1), 64);
+      const int part = col0 / 128;
+      if (!gives && row0 + lane < p.M) {
+        constexpr float L2E = 1.4426950408889634f;
+        const float2 o = *xch;
+        const float m = fmaxf(ce_m, o.x);
+        const float off = (m == -INFINITY) ? 0.f : m;
+        const float s = ce_s * fast_exp2((ce_m - off) * L2E) + o.y * fast_exp2((o.x - off) * L2E);
+        p.ce_partials[static_cast<size_t>(part) * p.M + row0 + lane] = make_float2(m, s);
+      }
+    }
+    if (ew == 0 && lane == 0) {
+      if (t == pair) trace_stamp(p, TRACE_EPI_FIRST);
+      trace_stamp(p, TRACE_EPI_LAST);
+    }
+    if (++acc == 2) {
+      acc = 0;
+      acc_phase ^= 1u;
+    }
+  }
+  if (lane == 0) bulk_wait_all();
+}
+
 template <bool A_MN, bool B_MN, int COMM, int SWI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads2(COMM), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
              const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y, const Params2 p) {
-  // tmap_x, tmap_y: all-gather: the local shard of A, unused; EPI_TMA: gate | up, d_gate | d_up
-  constexpr bool EPI_TMA = epi_tma(COMM, SWI);
-  constexpr int STAGES = stages2(COMM, SWI);
-  constexpr int EPI_BYTES = epi_bytes2(COMM, SWI);
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // tmap_x, tmap_y: all-gather: the local shard of A, unused; without a collective (see epilogue_plain): SWI 0 R, C;
+  // 1 act, gate | up; 2 gate | up, d_gate | d_up; 3, 5 unused, C
+  constexpr int STAGES = stages2(COMM);
+  constexpr int EPI_BYTES = epi_bytes2(COMM);
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if (COMM != COMM_NONE) {
+    smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  } else if (smem_u32(smem_raw) & 1023u) {   // both CTAs of a pair see the same offset
+    if (threadIdx.x == 0) record_status(p.status, STATUS_BAD_ARGUMENT, 0x5a14u);
+    return;
+  }
   uint8_t* tiles = smem;
   uint8_t* epi_smem = smem + STAGES * STAGE_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(epi_smem + EPI_BYTES);
   uint64_t* full_bar = bars;                      // [STAGES]  (used in the leader)
   uint64_t* empty_bar = bars + STAGES;            // [STAGES]  (one per CTA)
   uint64_t* tmem_full = bars + 2 * STAGES;        // [2]       (one per CTA)
-  uint64_t* tmem_empty = bars + 2 * STAGES + 2;   // [2]       (used in the leader, 8 arrivals)
+  uint64_t* tmem_empty = bars + 2 * STAGES + 2;   // [2]       (used in the leader)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
   uint32_t* rs_sent = tmem_slot + 2;   // [MAX_PEERS] reduce-scatter: (warp, tile) units stored for each peer
-  uint64_t* epi_full = reinterpret_cast<uint64_t*>(rs_sent + MAX_PEERS);   // [8 warps][2 slots], EPI_TMA
+  uint64_t* epi_full = reinterpret_cast<uint64_t*>(rs_sent + MAX_PEERS);   // [16 warps], without a collective
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -186,8 +497,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       mbar_init(&tmem_full[b], 1);
       mbar_init(&tmem_empty[b], 2 * epi_warps(COMM));
     }
-    if (EPI_TMA) {
-      for (int i = 0; i < 16; ++i) mbar_init(&epi_full[i], 1);
+    if (COMM == COMM_NONE) {
+      for (int i = 0; i < epi_warps(COMM); ++i) mbar_init(&epi_full[i], 1);
       tma_prefetch_desc(&tmap_x);
       tma_prefetch_desc(&tmap_y);
     }
@@ -325,6 +636,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   } else if (warp < 2 + epi_warps(COMM)) {
     // ------------------------------ epilogue (both CTAs, own accumulator half) ------------------------------
     constexpr int EW = epi_warps(COMM);
+    if constexpr (COMM == COMM_NONE) {
+      epilogue_plain<SWI>(p, tmap_x, tmap_y, epi_smem + (warp - 2) * 4096, &epi_full[warp - 2],
+                          reinterpret_cast<float2*>(epi_smem + EPI_BYTES + BAR_BYTES), tmem_full, tmem_empty, tmem_base,
+                          static_cast<int>(rank), pair, num_pairs, total_tiles, warp - 2, warp & 3, wctx);
+    } else {
     // all-gather variant: until the first accumulator is ready these warps help the two push warps
     if (COMM == COMM_ALLGATHER) {
       ag_push_rows(p.comm, static_cast<int>(threadIdx.x) - 64, COMM_THREADS + 32 * EW, 1);
@@ -332,41 +648,14 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     }
     bool rs_handed_over = false;                          // reduce-scatter: remote tiles handed to the signalling warp
     const int q = warp & 3;                               // TMEM lane quarter this warp may access
-    const int c_begin = (EW == 8) ? ((warp - 2) >> 2) * (BN / 2) : 0;   // this warp's column range of the tile
-    const int c_end = (EW == 8) ? c_begin + BN / 2 : BN;
+    const int c_begin = ((warp - 2) >> 2) * (BN / 2);     // this warp's column range of the tile
+    const int c_end = c_begin + BN / 2;
     int acc = 0;
     uint32_t acc_phase = 0;
     uint8_t* ebuf = epi_smem + (warp - 2) * 4096;
     const int rrow = lane >> 3;
     const int rch = lane & 7;
-    const bool has_add = !EPI_TMA && (p.R != nullptr);
-    // EPI_TMA: this warp's slots, and the loads of gate | up, one 64-column chunk ahead of the math
-    uint8_t* const slots = epi_smem + (warp - 2) * (EPI_BYTES / 8);
-    uint32_t n_chunk = 0;                   // chunks this warp has worked through (slot = parity)
-    int pf_t = pair, pf_c = c_begin - 64;   // the last chunk asked for
-    auto prefetch_chunk = [&](uint32_t n) { // the next chunk with anything in range, as the warp's n-th
-      while (true) {
-        pf_c += 64;
-        if (pf_c >= c_begin + BN / 2) {
-          pf_c = c_begin;
-          pf_t += num_pairs;
-        }
-        if (pf_t >= total_tiles) return;
-        const int row0 = (pf_t / p.tiles_n) * 256 + static_cast<int>(rank) * BM + q * 32;
-        const int col0 = (pf_t % p.tiles_n) * BN + pf_c;
-        if (row0 >= p.M || col0 >= p.N) continue;
-        if (lane == 0) {
-          uint64_t* bar = &epi_full[(warp - 2) * 2 + (n & 1)];
-          uint8_t* slot = slots + (n & 1) * 8192;
-          bulk_wait_read_all();             // the slot's previous results have left it
-          mbar_arrive_expect_tx(bar, 8192);
-          tma_load_3d(slot, &tmap_x, bar, col0, 0, row0);
-          tma_load_3d(slot + 4096, &tmap_x, bar, col0, 1, row0);
-        }
-        return;
-      }
-    };
-    if (EPI_TMA) prefetch_chunk(0);
+    const bool has_add = p.R != nullptr;
     // The addend of a 64-column chunk is fetched one chunk ahead (across tile boundaries too), so
     // its global-memory latency is covered by the previous chunk's work instead of stalling this one.
     uint4 pre[8];
@@ -393,61 +682,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       if (t == pair && warp == 2 && lane == 0) trace_stamp(p, TRACE_EPI_BEGIN);
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-      if (EPI_TMA) {
-        // A thread owns a row: the tiles' 16-byte chunks are swizzled (128-byte rows), so its accesses are free of
-        // bank conflicts, and rows and columns past the end are clipped by the tensor maps. gate | up are
-        // [row][half][column] to the maps, so the last gate columns cannot run into up.
-        const int row0 = m0 + q * 32;
-        const uint32_t sw = lane & 7;
-#pragma unroll 1
-        for (int c = c_begin; c < c_begin + BN / 2; c += 64) {
-          const int col0 = n0 + c;
-          if (row0 >= p.M || col0 >= p.N) break;
-          uint8_t* slot = slots + (n_chunk & 1) * 8192;
-          uint8_t* row = slot + lane * 128;
-          mbar_wait(&epi_full[(warp - 2) * 2 + (n_chunk & 1)], (n_chunk >> 1) & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
-          ++n_chunk;
-#pragma unroll 1
-          for (int h = 0; h < 2; ++h) {
-            uint32_t vd[32];
-            tmem_ld_32x32(t_row + c + 32 * h, vd);
-            // half way, when the previous chunk's results will have left the slot that the next one takes
-            if (h == 1) prefetch_chunk(n_chunk);
-            __syncwarp();
-            tmem_ld_wait_for(vd);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint8_t* at = row + (((4 * h + j) ^ sw) << 4);
-              uint4 g4 = *reinterpret_cast<const uint4*>(at), u4 = *reinterpret_cast<const uint4*>(at + 4096);
-              uint32_t *gp = &g4.x, *up = &u4.x;
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                // d_act rounded to bf16, as when it is a tensor of its own
-                const float2 d2 = unpack_bf16x2(
-                    pack_bf16x2(__uint_as_float(vd[8 * j + 2 * e]), __uint_as_float(vd[8 * j + 2 * e + 1])));
-                const float2 g2 = unpack_bf16x2(gp[e]), u2 = unpack_bf16x2(up[e]);
-                const float sg0 = sigmoid_f(g2.x), sg1 = sigmoid_f(g2.y);
-                gp[e] = pack_bf16x2(d2.x * u2.x * sg0 * (1.f + g2.x * (1.f - sg0)),
-                                    d2.y * u2.y * sg1 * (1.f + g2.y * (1.f - sg1)));
-                up[e] = pack_bf16x2(d2.x * g2.x * sg0, d2.y * g2.y * sg1);
-              }
-              *reinterpret_cast<uint4*>(at) = g4;
-              *reinterpret_cast<uint4*>(at + 4096) = u4;
-            }
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_3d(&tmap_y, slot, col0, 0, row0);
-            tma_store_3d(&tmap_y, slot + 4096, col0, 1, row0);
-            bulk_commit();
-          }
-        }
-      } else if (SWI == 1) {
+      if (SWI == 1) {
         // accumulator columns [0,128) are gate, [128,256) the matching up columns
         const int g0 = n0 >> 1;  // first gate column of the tile
-        const int sc_begin = (EW == 8) ? ((warp - 2) >> 2) * 64 : 0;
-        const int sc_end = (EW == 8) ? sc_begin + 64 : 128;
+        const int sc_begin = ((warp - 2) >> 2) * 64;
+        const int sc_end = sc_begin + 64;
 #pragma unroll 1
         for (int c = sc_begin; c < sc_end; c += 32) {
           if (g0 + c >= p.swi_I) break;
@@ -664,12 +903,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       }
       if (SWI == 3) {
         const int row = m0 + q * 32 + lane;
-        const int part = (n0 / BN) * 2 + ((EW == 8) ? ((warp - 2) >> 2) : 0);
-        if (row < p.M) {
-          p.ce_partials[static_cast<size_t>(part) * p.M + row] = make_float2(ce_m, ce_s);
-          // with four epilogue warps a warp covers all 256 columns: the tile's second slot is empty
-          if (EW != 8) p.ce_partials[static_cast<size_t>(part + 1) * p.M + row] = make_float2(-INFINITY, 0.f);
-        }
+        const int part = (n0 / BN) * 2 + ((warp - 2) >> 2);
+        if (row < p.M) p.ce_partials[static_cast<size_t>(part) * p.M + row] = make_float2(ce_m, ce_s);
       }
       }
       tc_fence_before();
@@ -704,7 +939,6 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         acc_phase ^= 1u;
       }
     }
-    if (EPI_TMA && lane == 0) bulk_wait_all();
     if (COMM == COMM_REDUCE_SCATTER) {
       if (!rs_handed_over) named_barrier_arrive(2, 32 * EW + COMM_THREADS);   // CTAs without local tiles
       // tiles done: join the reduction of this rank's row chunk (second share of the vectors)
@@ -718,6 +952,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       rs_reduce_rows(c.peer_buf[c.rank], c.world, c.rows_per_rank, p.N, c.rs_res, c.rs_ld_res, c.rs_out, c.rs_ld_out,
                      static_cast<size_t>(blockIdx.x) * RED_THREADS + COMM_THREADS + (threadIdx.x - 64),
                      static_cast<size_t>(gridDim.x) * RED_THREADS);
+    }
     }
   } else if (COMM == COMM_ALLGATHER) {
     // ------------------------------ all-gather push (warps 6-7) ------------------------------
@@ -1012,7 +1247,7 @@ template <bool A_MN, bool B_MN, int COMM = COMM_NONE, int SWI = 0>
 int launch2(const CUtensorMap* ta, const CUtensorMap* tb, const Params2& p, int grid, cudaStream_t stream,
             const CUtensorMap* tx = nullptr, const CUtensorMap* ty = nullptr) {
   auto kern = gemm2_kernel<A_MN, B_MN, COMM, SWI>;
-  constexpr int smem = smem2(COMM, SWI);
+  constexpr int smem = smem2(COMM);
   static bool attr_set = false;
   static int attr_dev = -1;
   int dev = 0;
@@ -1071,10 +1306,20 @@ int gfs_gemm2_bf16(const void* A, const void* B, void* C, const void* R, int M, 
   p.rope_cols = rope_cols; p.rope_d = rope_d; p.rope_b = rope_b > 0 ? rope_b : 1;
   const int pairs = std::min(p.tiles_m * p.tiles_n, gfs_host::sm_count() / 2);
   const int grid = 2 * pairs;
-  if (!a_mn_major && !b_mn_major) return launch2<false, false>(ta, tb, p, grid, stream);
-  if (!a_mn_major && b_mn_major) return launch2<false, true>(ta, tb, p, grid, stream);
-  if (a_mn_major && b_mn_major) return launch2<true, true>(ta, tb, p, grid, stream);
-  return launch2<true, false>(ta, tb, p, grid, stream);
+  const CUtensorMap* tx = R != nullptr ? gfs_host::tmap_2d_cached(R, M, N, ldr, 32, 64) : nullptr;
+  const CUtensorMap* ty = gfs_host::tmap_2d_cached(C, M, N, ldc, 32, 64);
+  if (ty == nullptr || (R != nullptr && tx == nullptr)) return -3;
+  if (rope_cos != nullptr) {
+    // the rotary epilogue here is that of a projection x W^T; other forms are the single-CTA kernel's
+    if (a_mn_major || b_mn_major || R != nullptr)
+      return gfs_gemm_bf16_rope(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn_major, b_mn_major, R != nullptr, nullptr, 0,
+                                1, rope_cos, rope_sin, rope_cols, rope_d, rope_b, stream_);
+    return launch2<false, false, COMM_NONE, 5>(ta, tb, p, grid, stream, tx, ty);
+  }
+  if (!a_mn_major && !b_mn_major) return launch2<false, false>(ta, tb, p, grid, stream, tx, ty);
+  if (!a_mn_major && b_mn_major) return launch2<false, true>(ta, tb, p, grid, stream, tx, ty);
+  if (a_mn_major && b_mn_major) return launch2<true, true>(ta, tb, p, grid, stream, tx, ty);
+  return launch2<true, false>(ta, tb, p, grid, stream, tx, ty);
 }
 
 // LM head with cross-entropy statistics: C[M, N] = A[M, K] @ B[N, K]^T (both K-major) and, per row,
@@ -1094,7 +1339,8 @@ int gfs_gemm2_bf16_ce(const void* A, const void* B, void* C, void* partials, int
   if (K < 256) return -20;
   const CUtensorMap* ta = gfs_host::tmap_2d_cached(A, M, K, lda, BM, 64);
   const CUtensorMap* tb = gfs_host::tmap_2d_cached(B, N, K, ldb, BNH, 64);
-  if (ta == nullptr || tb == nullptr) return -3;
+  const CUtensorMap* ty = gfs_host::tmap_2d_cached(C, M, N, ldc, 32, 64);
+  if (ta == nullptr || tb == nullptr || ty == nullptr) return -3;
   Params2 p{};
   p.M = M; p.N = N; p.K = K;
   p.ldc = ldc;
@@ -1106,7 +1352,7 @@ int gfs_gemm2_bf16_ce(const void* A, const void* B, void* C, void* partials, int
   p.rope_b = 1;
   p.ce_partials = static_cast<float2*>(partials);
   const int pairs = std::min(p.tiles_m * p.tiles_n, gfs_host::sm_count() / 2);
-  return launch2<false, false, COMM_NONE, 3>(ta, tb, p, 2 * pairs, stream);
+  return launch2<false, false, COMM_NONE, 3>(ta, tb, p, 2 * pairs, stream, nullptr, ty);
 }
 
 // SwiGLU-fused products of the MLP on CTA pairs; same contract as gfs_gemm_bf16_swiglu (gemm.cu):
@@ -1142,19 +1388,18 @@ int gfs_gemm2_bf16_swiglu(int mode, const void* a, const void* b, void* c, void*
                                       : gfs_host::tmap_2d_cached(b, K, I, ldb, 64, 64);
   if (ta == nullptr || tb == nullptr) return -3;
   const int pairs = std::min(p.tiles_m * p.tiles_n, gfs_host::sm_count() / 2);
-  if (mode == 1) return launch2<false, false, COMM_NONE, 1>(ta, tb, p, 2 * pairs, stream);
-  if (K > SWI_TMA_MAX_K) return launch2<false, true, COMM_NONE, 2>(ta, tb, p, 2 * pairs, stream);
-  // gate | up as [row][half][column], in boxes of one warp's 32 rows x 64 columns
-  auto epi_map = [&](const void* base, int ld) {
+  // gate | up as [row][half][column] (the last gate columns must not run into up), in boxes of 32 rows x 32 columns
+  auto halves = [&](const void* base, int ld) {
     const uint64_t dims[3] = {static_cast<uint64_t>(I), 2, static_cast<uint64_t>(M)};
     const uint64_t strides[3] = {2, static_cast<uint64_t>(I) * 2, static_cast<uint64_t>(ld) * 2};
-    const uint32_t box[3] = {64, 1, 32};
+    const uint32_t box[3] = {32, 1, 32};
     return gfs_host::tmap_nd_cached(base, 3, dims, strides, box);
   };
-  const CUtensorMap* tx = epi_map(extra, ld_extra);
-  const CUtensorMap* ty = epi_map(c, ldc);
+  const CUtensorMap* ty = halves(c, ldc);
+  const CUtensorMap* tx = mode == 1 ? gfs_host::tmap_2d_cached(extra, M, I, ld_extra, 32, 32) : halves(extra, ld_extra);
   if (tx == nullptr || ty == nullptr) return -3;
-  return launch2<false, true, COMM_NONE, 4>(ta, tb, p, 2 * pairs, stream, tx, ty);
+  if (mode == 1) return launch2<false, false, COMM_NONE, 1>(ta, tb, p, 2 * pairs, stream, tx, ty);
+  return launch2<false, true, COMM_NONE, 2>(ta, tb, p, 2 * pairs, stream, tx, ty);
 }
 
 // Fused collective + GEMM on CTA pairs; same contract as gfs_gemm_bf16_comm (gemm.cu) with the

@@ -281,3 +281,76 @@ def test_gemm_below_the_pair_threshold(cuda_device, M, N, K):
         c = torch.randn(M, N, device=cuda_device, generator=g).bfloat16()
         _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn), _ref(a, b, a_mn, b_mn, None), K)
         _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn, addend=c), _ref(a, b, a_mn, b_mn, c), K)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (33, 72, 64), (95, 264, 392), (700, 1096, 72), (5000, 2056, 256)])
+def test_pair_kernel_epilogues_at_edges(cuda_device, M, N, K):
+    """Rows, columns and K that end inside a warp's 32 x 64 box of the pair kernel, from one tile to several per CTA: plain,
+    with an addend (aliasing the output too), rotary, SwiGLU forward and the row statistics of the LM head. Nothing outside
+    the results is written. Tolerance as in _check."""
+    from gpt_from_scratch_b200.ops import _lib
+    from gpt_from_scratch_b200.ops.rope import rope_reference
+    lib, st = _lib.lib(), _lib.stream_ptr()
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g).bfloat16()  # noqa: E731
+
+    def guarded(n):
+        return torch.full((M + 1, n + 8), 7.0, device=cuda_device, dtype=torch.bfloat16)
+
+    def outside_untouched(t, n):
+        assert (t[M] == 7.0).all() and (t[:, n:] == 7.0).all()
+
+    x, w, r = rnd(M, K), rnd(N, K), rnd(M, N)
+    ref = x.float() @ w.float().t()
+    for addend in (None, r):
+        out = guarded(N)
+        assert lib.gfs_gemm2_bf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), _lib.ptr(addend), M, N, K, K, K, out.stride(0),
+                                  N if addend is not None else 0, 0, 0, 0, 0, 0, 0, 1, st) == 0
+        _check(out[:M, :N], ref if addend is None else ref + addend.float(), K)
+        outside_untouched(out, N)
+    acc = r.clone()
+    assert lib.gfs_gemm2_bf16(x.data_ptr(), w.data_ptr(), acc.data_ptr(), acc.data_ptr(), M, N, K, K, K, N, N, 0, 0, 0, 0, 0,
+                              0, 1, st) == 0
+    _check(acc, ref + r.float(), K)
+
+    # rotary: heads of 8 columns, the first half of them turned (the line lies inside a box); with an addend too
+    B, D = (3, 8) if M % 3 == 0 else (1, 8)
+    S, turned = M // B, N // 16 * 8
+    ang = torch.rand(S, D // 2, device=cuda_device, generator=g) * 6.28
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    rr = ref.view(S, B, N // 8, 8).clone()
+    rr[:, :, :turned // 8] = rope_reference(rr[:, :, :turned // 8], cos, sin)
+    for addend in (None, r):
+        out = guarded(N)
+        assert lib.gfs_gemm2_bf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), _lib.ptr(addend), M, N, K, K, K, out.stride(0),
+                                  N if addend is not None else 0, 0, 0, cos.data_ptr(), sin.data_ptr(), turned, D, B,
+                                  st) == 0
+        _check(out[:M, :N], rr.view(M, N) if addend is None else rr.view(M, N) + addend.float(), K)
+        outside_untouched(out, N)
+
+    # SwiGLU forward with I = N
+    wg = rnd(2 * N, K) * 0.3
+    gu, act = guarded(2 * N), guarded(N)
+    assert lib.gfs_gemm2_bf16_swiglu(1, x.data_ptr(), wg.data_ptr(), gu.data_ptr(), act.data_ptr(), M, N, K, K, K,
+                                     gu.stride(0), act.stride(0), st) == 0
+    _check(gu[:M, :2 * N], x.float() @ wg.float().t(), K)
+    gate, up = gu[:M, :N].float(), gu[:M, N:2 * N].float()
+    _check(act[:M, :N], torch.nn.functional.silu(gate) * up, K)
+    outside_untouched(gu, 2 * N)
+    outside_untouched(act, N)
+
+    # row statistics of 128-column slices of the rounded logits (K >= 256 by contract)
+    if K >= 256:
+        logits = guarded(N)
+        parts = torch.full((lib.gfs_gemm2_ce_parts(N), M, 2), 7.0, device=cuda_device)
+        assert lib.gfs_gemm2_bf16_ce(x.data_ptr(), w.data_ptr(), logits.data_ptr(), parts.data_ptr(), M, N, K, K, K,
+                                     logits.stride(0), st) == 0
+        outside_untouched(logits, N)
+        m = parts[..., 0].max(dim=0).values
+        s = (parts[..., 1] * torch.exp(parts[..., 0] - m)).sum(dim=0)     # empty slices: (-inf, 0)
+        assert torch.equal(m, logits[:M, :N].float().max(dim=1).values)
+        lse = torch.logsumexp(logits[:M, :N].double(), dim=1)
+        # fp32 sums of exponentials of 2^-22 relative error: a few 1e-6 of an lse of the order of its maximum
+        assert ((m.double() + s.double().log()) - lse).abs().max() < 1e-5 * lse.abs().max().clamp(min=1)
+    torch.cuda.synchronize()
+    _lib.raise_on_status()
