@@ -4,10 +4,10 @@
 // shared-memory traffic per FLOP, which is what bounds the single-CTA kernel in gemm.cu
 // (operand reads plus TMA writes exceed 128 B/clk/SM at full tensor rate).
 //
-// Roles per CTA (6 warps): warp 0 TMA producer (loads its own A rows and its half of B into
+// Roles per CTA: warp 0 TMA producer (loads its own A rows and its half of B into
 // its own shared memory; both CTAs' loads complete on the LEADER's "full" barrier), warp 1
 // MMA issuer (leader CTA only; both CTAs' warp 1 take part in the paired TMEM allocation),
-// warps 2-5 epilogue (each CTA drains its own accumulator half). Barriers that must be seen
+// then eight or sixteen epilogue warps (each CTA drains its own accumulator half). Barriers that must be seen
 // by both CTAs are signalled twice (own address and the peer's address obtained with
 // mapa), so no multicast form of any instruction is used. TMA loads are plain per-CTA loads.
 //
@@ -55,26 +55,31 @@ constexpr int A_BYTES = BM * BK * 2;     // 16 KB
 constexpr int B_BYTES = BNH * BK * 2;    // 16 KB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int EPI_BYTES = 8 * 4096;     // one [32 rows x 128 B] transpose buffer per epilogue warp
-// Epilogue warps per CTA. Plain products: sixteen, one [32 rows x 64 columns] unit of the CTA's 128 x 256 half tile
-// each, results (and the addend) moving by TMA through 4 KB of shared memory per warp. At a K loop of 12 blocks (K = 768,
-// 7,100 cycles) eight warps with two units each, loads and stores of their own, took longer than the loop as soon as the
-// epilogue had anything to compute, and a kernel's last epilogue is never hidden. The price is one of six ring stages.
-// us, eight warps -> this, K = 768: [16384, 2304] with rotary epilogue 62 -> 49, [16384, 768] with addend 24 -> 20, SwiGLU
-// forward [16384, 2 x 3072] 142 -> 130 and backward 121 -> 117, LM head [8192, 50304] 626 -> 575.
-// The variants with collectives: eight (two per TMEM lane quarter, half of the tile's columns each), and two warps
-// for the transfers.
-__host__ __device__ constexpr int epi_warps(int comm) { return comm == COMM_NONE ? 16 : 8; }
-__host__ __device__ constexpr int threads2(int comm) { return 64 + 32 * epi_warps(comm) + (comm != 0 ? 64 : 0); }
-__host__ __device__ constexpr int stages2(int comm) { return comm == COMM_NONE ? 5 : STAGES; }
-__host__ __device__ constexpr int epi_bytes2(int comm) { return epi_warps(comm) * 4096; }
+// Epilogue warps per CTA (template parameter EW).
+// Sixteen, for products without a collective and a K loop of up to 16 blocks: one [32 rows x 64 columns] unit of the CTA's
+// 128 x 256 half tile each, results (and the addend) moving by TMA through 4 KB of shared memory per warp. At K = 768 (7,100
+// cycles) eight warps with two units each, loads and stores of their own, took longer than the loop as soon as the
+// epilogue had anything to compute, and a kernel's last epilogue is never hidden. The price is one of six ring stages
+// (SWI == 2: two, for 6 KB per warp: gate | up on the way in and the results on the way out), which a long loop feels.
+// us, eight warps -> sixteen, K = 768: [16384, 2304] with rotary epilogue 62 -> 48, [16384, 768] with addend 24 -> 20,
+// SwiGLU forward [16384, 2 x 3072] 138 -> 124 and backward 119 -> 102, LM head [8192, 50304] 626 -> 575; K = 2048, inside
+// a training step of 8192 tokens: SwiGLU forward [., 2 x 5632] 259 -> 280, backward 165 -> 197, without an epilogue's work
+// equal, with the rotary one 176 -> 159 (which is why that one always has sixteen).
+// Eight, for the others (two per TMEM lane quarter, half of the tile's columns each); variants with collectives have two
+// more warps for the transfers.
+constexpr int EW16_MAX_K = 1024;
+__host__ __device__ constexpr int threads2(int comm, int ew) { return 64 + 32 * ew + (comm != 0 ? 64 : 0); }
+__host__ __device__ constexpr int slot_bytes2(int ew, int swi) { return ew == 16 && swi == 2 ? 6144 : 4096; }
+__host__ __device__ constexpr int stages2(int ew, int swi) { return ew != 16 ? STAGES : swi == 2 ? 4 : 5; }
+__host__ __device__ constexpr int epi_bytes2(int ew, int swi) { return ew * slot_bytes2(ew, swi); }
 constexpr int BAR_BYTES = 512;
 constexpr int XCH_BYTES = 8 * 32 * 8;   // SWI == 3: a (max, sum) pair per row and 128-column slice
 constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + 256 + 1024;
-// (without a collective the base is used as it is, 1024-byte aligned)
-__host__ __device__ constexpr int smem2(int comm) {
-  return stages2(comm) * STAGE_BYTES + epi_bytes2(comm) + BAR_BYTES + (comm == COMM_NONE ? XCH_BYTES : 1024);
+// (with sixteen warps the base is used as it is, 1024-byte aligned)
+__host__ __device__ constexpr int smem2(int ew, int swi) {
+  return stages2(ew, swi) * STAGE_BYTES + epi_bytes2(ew, swi) + BAR_BYTES + (ew == 16 ? XCH_BYTES : 1024);
 }
-static_assert(smem2(COMM_NONE) <= 232448, "shared memory of an SM");
+static_assert(smem2(16, 0) <= 232448 && smem2(16, 2) <= 232448, "shared memory of an SM");
 
 struct Params2 {
   int M, N, K;
@@ -163,18 +168,19 @@ __device__ __forceinline__ void decode_tile2(const Params2& p, int t, int& m0, i
   }
 }
 
-// The epilogue of a warp of a plain product (COMM_NONE): rows [32 q, + 32) and one sixteenth of the columns of each of the
+// The epilogue of a warp where there are sixteen: rows [32 q, + 32) and one sixteenth of the columns of each of the
 // CTA's half tiles, a row per thread. Results leave through `slot` (4 KB, this warp's) by TMA, which clips what lies
 // outside the matrices and writes whole segments; the accumulator is handed back as soon as it has been read.
 //   SWI 0  64 columns; + R, which TMA has brought into the slot while the previous tiles were worked on
 //   SWI 5  64 columns, rotary embedding
 //   SWI 3  64 columns and their share of the row statistics
 //   SWI 1  32 gate and 32 up columns -> both and act
-//   SWI 2  64 columns of d_act in two chunks: gate | up of a chunk come into the slot, their gradients take their place
+//   SWI 2  64 columns of d_act in two chunks: gate | up of a chunk come into the slot one chunk ahead (the next box is asked
+//          for as soon as this one is in registers), their gradients leave one after the other through 2 KB behind it
 // 64-column boxes are swizzled over 128-byte rows, 32-column ones (SWI 1, 2) over 64-byte rows, so that threads that
 // own rows meet no bank conflicts.
 template <int SWI>
-__device__ __forceinline__ void epilogue_plain(const Params2& p, const CUtensorMap& tmap_x, const CUtensorMap& tmap_y,
+__device__ __forceinline__ void epilogue16(const Params2& p, const CUtensorMap& tmap_x, const CUtensorMap& tmap_y,
                                                uint8_t* slot, uint64_t* bar, float2* xch_all, uint64_t* tmem_full,
                                                uint64_t* tmem_empty, uint32_t tmem_base, int rank, int pair,
                                                int num_pairs, int total_tiles, int ew, int q, const WaitCtx& wctx) {
@@ -202,7 +208,7 @@ __device__ __forceinline__ void epilogue_plain(const Params2& p, const CUtensorM
       col0 += 32 * pf_h;
       if (row0 >= p.M || col0 >= col_limit) continue;
       if (lane == 0) {
-        bulk_wait_read_all();             // the slot's previous results have left it
+        if (SWI != 2) bulk_wait_read_all();   // the slot's previous results have left it
         mbar_arrive_expect_tx(bar, 4096);
         if (SWI == 2) {
           tma_load_3d(slot, &tmap_x, bar, col0, 0, row0);
@@ -303,50 +309,66 @@ __device__ __forceinline__ void epilogue_plain(const Params2& p, const CUtensorM
         bulk_commit();
       }
     } else if (SWI == 2) {
-      uint32_t pd[32];    // d_act rounded to bf16, as when it is a tensor of its own
-      {
-        uint32_t va[32], vb[32];
-        tmem_ld_32x32(t_row, va);
-        tmem_ld_32x32(t_row + 32, vb);
-        tmem_ld_wait_for(va);
-        tmem_ld_wait_for(vb);
+      const uint64_t one2 = pack_f32x2(1.f, 1.f), neg_one2 = pack_f32x2(-1.f, -1.f);
+      auto pair_of = [](uint32_t u) {
+        const float2 f = unpack_bf16x2(u);
+        return pack_f32x2(f.x, f.y);
+      };
+      auto packed = [](uint64_t v) {
+        const float2 f = unpack_f32x2(v);
+        return pack_bf16x2(f.x, f.y);
+      };
+      const int chunks = col0 + 32 < col_limit ? 2 : 1;
+#pragma unroll 1
+      for (int h = 0; h < chunks; ++h) {
+        uint32_t pd[16];    // d_act rounded to bf16, as when it is a tensor of its own
+        {
+          uint32_t va[32];
+          tmem_ld_32x32(t_row + 32 * h, va);
+          tmem_ld_wait_for(va);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          pd[e] = pack_bf16x2(__uint_as_float(va[2 * e]), __uint_as_float(va[2 * e + 1]));
-          pd[16 + e] = pack_bf16x2(__uint_as_float(vb[2 * e]), __uint_as_float(vb[2 * e + 1]));
+          for (int e = 0; e < 16; ++e)
+            pd[e] = pack_bf16x2(__uint_as_float(va[2 * e]), __uint_as_float(va[2 * e + 1]));
         }
-      }
-      release();
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (col0 + 32 * h >= col_limit) break;
+        if (h == chunks - 1) release();
         mbar_wait(bar, n_box & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
         ++n_box;
+        uint4 g4[4], u4[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          uint8_t* at = row64 + ((j ^ sw64) << 4);
-          uint4 g4 = *reinterpret_cast<const uint4*>(at), u4 = *reinterpret_cast<const uint4*>(at + 2048);
-          uint32_t *gp = &g4.x, *up = &u4.x;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 d2 = unpack_bf16x2(pd[16 * h + 4 * j + e]);
-            const float2 g2 = unpack_bf16x2(gp[e]), u2 = unpack_bf16x2(up[e]);
-            const float sg0 = sigmoid_f(g2.x), sg1 = sigmoid_f(g2.y);
-            gp[e] = pack_bf16x2(d2.x * u2.x * sg0 * (1.f + g2.x * (1.f - sg0)),
-                                d2.y * u2.y * sg1 * (1.f + g2.y * (1.f - sg1)));
-            up[e] = pack_bf16x2(d2.x * g2.x * sg0, d2.y * g2.y * sg1);
-          }
-          *reinterpret_cast<uint4*>(at) = g4;
-          *reinterpret_cast<uint4*>(at + 2048) = u4;
+          const uint8_t* at = row64 + ((j ^ sw64) << 4);
+          g4[j] = *reinterpret_cast<const uint4*>(at);
+          u4[j] = *reinterpret_cast<const uint4*>(at + 2048);
         }
-        fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
-          tma_store_3d(&tmap_y, slot, col0 + 32 * h, 0, row0);
-          tma_store_3d(&tmap_y, slot + 2048, col0 + 32 * h, 1, row0);
-          bulk_commit();
-        }
         prefetch();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint32_t *gp = &g4[j].x, *up = &u4[j].x;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {   // two columns per instruction of the FMA pipe
+            const float2 g = unpack_bf16x2(gp[e]);
+            const uint64_t g2 = pack_f32x2(g.x, g.y), d2 = pair_of(pd[4 * j + e]);
+            const uint64_t s2 = pack_f32x2(sigmoid_f(g.x), sigmoid_f(g.y));
+            // d_gate = d up sigma (1 + gate (1 - sigma)), d_up = d gate sigma
+            const uint64_t t2 = fma_f32x2(g2, fma_f32x2(s2, neg_one2, one2), one2);
+            up[e] = packed(mul_f32x2(mul_f32x2(mul_f32x2(d2, pair_of(up[e])), s2), t2));
+            gp[e] = packed(mul_f32x2(mul_f32x2(d2, g2), s2));
+          }
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {      // d_gate (in u4), d_up (in g4)
+          slot_free();
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<uint4*>(row64 + 4096 + ((j ^ sw64) << 4)) = half == 0 ? u4[j] : g4[j];
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&tmap_y, slot + 4096, col0 + 32 * h, half, row0);
+            bulk_commit();
+          }
+        }
       }
     } else {
       uint32_t pk[32];    // this row's 64 columns, rounded to bf16
@@ -472,17 +494,17 @@ __device__ __forceinline__ void epilogue_plain(const Params2& p, const CUtensorM
   if (lane == 0) bulk_wait_all();
 }
 
-template <bool A_MN, bool B_MN, int COMM, int SWI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads2(COMM), 1)
+template <bool A_MN, bool B_MN, int COMM, int SWI, int EW>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads2(COMM, EW), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
              const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y, const Params2 p) {
-  // tmap_x, tmap_y: all-gather: the local shard of A, unused; without a collective (see epilogue_plain): SWI 0 R, C;
+  // tmap_x, tmap_y: all-gather: the local shard of A, unused; with sixteen epilogue warps: SWI 0 R, C;
   // 1 act, gate | up; 2 gate | up, d_gate | d_up; 3, 5 unused, C
-  constexpr int STAGES = stages2(COMM);
-  constexpr int EPI_BYTES = epi_bytes2(COMM);
+  constexpr int STAGES = stages2(EW, SWI);
+  constexpr int EPI_BYTES = epi_bytes2(EW, SWI);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
-  if (COMM != COMM_NONE) {
+  if (EW != 16) {
     smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   } else if (smem_u32(smem_raw) & 1023u) {   // both CTAs of a pair see the same offset
     if (threadIdx.x == 0) record_status(p.status, STATUS_BAD_ARGUMENT, 0x5a14u);
@@ -498,7 +520,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
   uint32_t* rs_sent = tmem_slot + 2;   // [MAX_PEERS] reduce-scatter: (warp, tile) units stored for each peer
-  uint64_t* epi_full = reinterpret_cast<uint64_t*>(rs_sent + MAX_PEERS);   // [16 warps], without a collective
+  uint64_t* epi_full = reinterpret_cast<uint64_t*>(rs_sent + MAX_PEERS);   // [warp], sixteen of them
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -515,10 +537,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tmem_full[b], 1);
-      mbar_init(&tmem_empty[b], 2 * epi_warps(COMM));
+      mbar_init(&tmem_empty[b], 2 * EW);
     }
-    if (COMM == COMM_NONE) {
-      for (int i = 0; i < epi_warps(COMM); ++i) mbar_init(&epi_full[i], 1);
+    if (EW == 16) {
+      for (int i = 0; i < EW; ++i) mbar_init(&epi_full[i], 1);
       tma_prefetch_desc(&tmap_x);
       tma_prefetch_desc(&tmap_y);
     }
@@ -653,11 +675,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         }
       }
     }
-  } else if (warp < 2 + epi_warps(COMM)) {
+  } else if (warp < 2 + EW) {
     // ------------------------------ epilogue (both CTAs, own accumulator half) ------------------------------
-    constexpr int EW = epi_warps(COMM);
-    if constexpr (COMM == COMM_NONE) {
-      epilogue_plain<SWI>(p, tmap_x, tmap_y, epi_smem + (warp - 2) * 4096, &epi_full[warp - 2],
+    if constexpr (EW == 16) {
+      epilogue16<SWI>(p, tmap_x, tmap_y, epi_smem + (warp - 2) * slot_bytes2(EW, SWI), &epi_full[warp - 2],
                           reinterpret_cast<float2*>(epi_smem + EPI_BYTES + BAR_BYTES), tmem_full, tmem_empty, tmem_base,
                           static_cast<int>(rank), pair, num_pairs, total_tiles, warp - 2, warp & 3, wctx);
     } else {
@@ -979,16 +1000,16 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     // Every CTA pushes its slice of the local shard into every rank's gathered buffer
     // (own rank first), then bumps that rank's counter for this source.
     // (the epilogue warps push too, before their first tile: see the top of the epilogue branch)
-    ag_push_rows(p.comm, static_cast<int>(threadIdx.x) - (threads2(COMM) - COMM_THREADS) + 32 * epi_warps(COMM),
-                 COMM_THREADS + 32 * epi_warps(COMM), 1);
+    ag_push_rows(p.comm, static_cast<int>(threadIdx.x) - (threads2(COMM, EW) - COMM_THREADS) + 32 * EW,
+                 COMM_THREADS + 32 * EW, 1);
   } else if (COMM == COMM_REDUCE_SCATTER) {
     // ------------------------------ reduce (warps 6-7) ------------------------------
     // Wait until every rank (this one included) has delivered all partial tiles of our row
     // chunk, then sum the staged partials in rank order, add the residual, round once.
     const CommParams& c = p.comm;
-    const int ct = threadIdx.x - (threads2(COMM) - COMM_THREADS);
+    const int ct = threadIdx.x - (threads2(COMM, EW) - COMM_THREADS);
     // every epilogue warp of this CTA has stored its tiles for the peers: the owners learn how many (warp, tile) units this CTA delivered to each of them
-    named_barrier_sync(2, 32 * epi_warps(COMM) + COMM_THREADS);
+    named_barrier_sync(2, 32 * EW + COMM_THREADS);
     if (ct < c.world && ct != c.rank) {
       const uint32_t n = rs_sent[ct];
       if (n != 0u) red_release_sys_add_u32(c.peer_flags[ct] + c.rank, n);   // release: cumulative over the barrier
@@ -1001,7 +1022,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     if (ct == 0) trace_stamp(p, TRACE_RED_BEGIN);
     // these 64 threads take the first share of the vectors; the epilogue warps take the rest once
     // their tiles are done (see the end of the epilogue loop)
-    constexpr int RED_THREADS = COMM_THREADS + 32 * epi_warps(COMM);
+    constexpr int RED_THREADS = COMM_THREADS + 32 * EW;
     rs_reduce_rows(c.peer_buf[c.rank], c.world, c.rows_per_rank, p.N, c.rs_res, c.rs_ld_res, c.rs_out, c.rs_ld_out,
                    static_cast<size_t>(blockIdx.x) * RED_THREADS + ct, static_cast<size_t>(gridDim.x) * RED_THREADS);
     if (ct == 0) trace_stamp(p, TRACE_RED_END);
@@ -1271,11 +1292,11 @@ int panel_rows(const Params2& p) {
 // their phase stamps (TraceSlot); null (the default) switches tracing off.
 static unsigned long long* g_trace = nullptr;
 
-template <bool A_MN, bool B_MN, int COMM = COMM_NONE, int SWI = 0>
+template <bool A_MN, bool B_MN, int COMM, int SWI, int EW>
 int launch2(const CUtensorMap* ta, const CUtensorMap* tb, const Params2& p, int grid, cudaStream_t stream,
             const CUtensorMap* tx = nullptr, const CUtensorMap* ty = nullptr) {
-  auto kern = gemm2_kernel<A_MN, B_MN, COMM, SWI>;
-  constexpr int smem = smem2(COMM);
+  auto kern = gemm2_kernel<A_MN, B_MN, COMM, SWI, EW>;
+  constexpr int smem = smem2(EW, SWI);
   static bool attr_set = false;
   static int attr_dev = -1;
   int dev = 0;
@@ -1289,7 +1310,7 @@ int launch2(const CUtensorMap* ta, const CUtensorMap* tb, const Params2& p, int 
   Params2 pt = p;
   pt.trace = g_trace;
   if (COMM == COMM_NONE) pt.group_m = panel_rows(p);
-  if (gfs_host::launch_pdl(kern, dim3(grid), dim3(threads2(COMM)), smem, stream, *ta, *tb, tx ? *tx : *ta,
+  if (gfs_host::launch_pdl(kern, dim3(grid), dim3(threads2(COMM, EW)), smem, stream, *ta, *tb, tx ? *tx : *ta,
                            ty ? *ty : *ta, pt) != cudaSuccess)
     return -11;
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
@@ -1335,20 +1356,27 @@ int gfs_gemm2_bf16(const void* A, const void* B, void* C, const void* R, int M, 
   p.rope_cols = rope_cols; p.rope_d = rope_d; p.rope_b = rope_b > 0 ? rope_b : 1;
   const int pairs = std::min(p.tiles_m * p.tiles_n, gfs_host::sm_count() / 2);
   const int grid = 2 * pairs;
-  const CUtensorMap* tx = R != nullptr ? gfs_host::tmap_2d_cached(R, M, N, ldr, 32, 64) : nullptr;
-  const CUtensorMap* ty = gfs_host::tmap_2d_cached(C, M, N, ldc, 32, 64);
-  if (ty == nullptr || (R != nullptr && tx == nullptr)) return -3;
+  const bool ew16 = K <= EW16_MAX_K || rope_cos != nullptr;
+  const CUtensorMap* tx = ew16 && R != nullptr ? gfs_host::tmap_2d_cached(R, M, N, ldr, 32, 64) : nullptr;
+  const CUtensorMap* ty = ew16 ? gfs_host::tmap_2d_cached(C, M, N, ldc, 32, 64) : nullptr;
+  if (ew16 && (ty == nullptr || (R != nullptr && tx == nullptr))) return -3;
   if (rope_cos != nullptr) {
     // the rotary epilogue here is that of a projection x W^T; other forms are the single-CTA kernel's
     if (a_mn_major || b_mn_major || R != nullptr)
       return gfs_gemm_bf16_rope(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn_major, b_mn_major, R != nullptr, nullptr, 0,
                                 1, rope_cos, rope_sin, rope_cols, rope_d, rope_b, stream_);
-    return launch2<false, false, COMM_NONE, 5>(ta, tb, p, grid, stream, tx, ty);
+    return launch2<false, false, COMM_NONE, 5, 16>(ta, tb, p, grid, stream, tx, ty);
   }
-  if (!a_mn_major && !b_mn_major) return launch2<false, false>(ta, tb, p, grid, stream, tx, ty);
-  if (!a_mn_major && b_mn_major) return launch2<false, true>(ta, tb, p, grid, stream, tx, ty);
-  if (a_mn_major && b_mn_major) return launch2<true, true>(ta, tb, p, grid, stream, tx, ty);
-  return launch2<true, false>(ta, tb, p, grid, stream, tx, ty);
+  if (ew16) {
+    if (!a_mn_major && !b_mn_major) return launch2<false, false, COMM_NONE, 0, 16>(ta, tb, p, grid, stream, tx, ty);
+    if (!a_mn_major && b_mn_major) return launch2<false, true, COMM_NONE, 0, 16>(ta, tb, p, grid, stream, tx, ty);
+    if (a_mn_major && b_mn_major) return launch2<true, true, COMM_NONE, 0, 16>(ta, tb, p, grid, stream, tx, ty);
+    return launch2<true, false, COMM_NONE, 0, 16>(ta, tb, p, grid, stream, tx, ty);
+  }
+  if (!a_mn_major && !b_mn_major) return launch2<false, false, COMM_NONE, 0, 8>(ta, tb, p, grid, stream);
+  if (!a_mn_major && b_mn_major) return launch2<false, true, COMM_NONE, 0, 8>(ta, tb, p, grid, stream);
+  if (a_mn_major && b_mn_major) return launch2<true, true, COMM_NONE, 0, 8>(ta, tb, p, grid, stream);
+  return launch2<true, false, COMM_NONE, 0, 8>(ta, tb, p, grid, stream);
 }
 
 // LM head with cross-entropy statistics: C[M, N] = A[M, K] @ B[N, K]^T (both K-major) and, per row,
@@ -1381,7 +1409,8 @@ int gfs_gemm2_bf16_ce(const void* A, const void* B, void* C, void* partials, int
   p.rope_b = 1;
   p.ce_partials = static_cast<float2*>(partials);
   const int pairs = std::min(p.tiles_m * p.tiles_n, gfs_host::sm_count() / 2);
-  return launch2<false, false, COMM_NONE, 3>(ta, tb, p, 2 * pairs, stream, nullptr, ty);
+  if (K > EW16_MAX_K) return launch2<false, false, COMM_NONE, 3, 8>(ta, tb, p, 2 * pairs, stream);
+  return launch2<false, false, COMM_NONE, 3, 16>(ta, tb, p, 2 * pairs, stream, nullptr, ty);
 }
 
 // SwiGLU-fused products of the MLP on CTA pairs; same contract as gfs_gemm_bf16_swiglu (gemm.cu):
@@ -1417,6 +1446,9 @@ int gfs_gemm2_bf16_swiglu(int mode, const void* a, const void* b, void* c, void*
                                       : gfs_host::tmap_2d_cached(b, K, I, ldb, 64, 64);
   if (ta == nullptr || tb == nullptr) return -3;
   const int pairs = std::min(p.tiles_m * p.tiles_n, gfs_host::sm_count() / 2);
+  if (K > EW16_MAX_K)
+    return mode == 1 ? launch2<false, false, COMM_NONE, 1, 8>(ta, tb, p, 2 * pairs, stream)
+                     : launch2<false, true, COMM_NONE, 2, 8>(ta, tb, p, 2 * pairs, stream);
   // gate | up as [row][half][column] (the last gate columns must not run into up), in boxes of 32 rows x 32 columns
   auto halves = [&](const void* base, int ld) {
     const uint64_t dims[3] = {static_cast<uint64_t>(I), 2, static_cast<uint64_t>(M)};
@@ -1427,8 +1459,8 @@ int gfs_gemm2_bf16_swiglu(int mode, const void* a, const void* b, void* c, void*
   const CUtensorMap* ty = halves(c, ldc);
   const CUtensorMap* tx = mode == 1 ? gfs_host::tmap_2d_cached(extra, M, I, ld_extra, 32, 32) : halves(extra, ld_extra);
   if (tx == nullptr || ty == nullptr) return -3;
-  if (mode == 1) return launch2<false, false, COMM_NONE, 1>(ta, tb, p, 2 * pairs, stream, tx, ty);
-  return launch2<false, true, COMM_NONE, 2>(ta, tb, p, 2 * pairs, stream, tx, ty);
+  if (mode == 1) return launch2<false, false, COMM_NONE, 1, 16>(ta, tb, p, 2 * pairs, stream, tx, ty);
+  return launch2<false, true, COMM_NONE, 2, 16>(ta, tb, p, 2 * pairs, stream, tx, ty);
 }
 
 // Fused collective + GEMM on CTA pairs; same contract as gfs_gemm_bf16_comm (gemm.cu) with the
@@ -1497,7 +1529,7 @@ static int gemm2_comm_impl(int mode, const void* a, int lda, const void* B, int 
     c.rs_ld_out = ldo;
     c.rs_res = static_cast<const __nv_bfloat16*>(residual);
     c.rs_ld_res = ldr;
-    increment = static_cast<unsigned int>((rows_per_rank / 256) * p.tiles_n * 2 * epi_warps(COMM_REDUCE_SCATTER));  // (warp, tile) units per pair tile
+    increment = static_cast<unsigned int>((rows_per_rank / 256) * p.tiles_n * 2 * 8);  // (warp, tile) units per pair tile
   }
   if ((reinterpret_cast<uintptr_t>(a_base) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(out)) & 15)
     return -2;
@@ -1523,17 +1555,17 @@ static int gemm2_comm_impl(int mode, const void* a, int lda, const void* B, int 
   }
   *target_inout += increment;
   c.target = *target_inout;
-  if (swi_mode == 1) return launch2<false, false, COMM_ALLGATHER, 1>(ta, tb, p, grid, stream, ta_local);
-  if (swi_mode == 2) return launch2<false, true, COMM_ALLGATHER, 2>(ta, tb, p, grid, stream, ta_local);
+  if (swi_mode == 1) return launch2<false, false, COMM_ALLGATHER, 1, 8>(ta, tb, p, grid, stream, ta_local);
+  if (swi_mode == 2) return launch2<false, true, COMM_ALLGATHER, 2, 8>(ta, tb, p, grid, stream, ta_local);
   if (ce_partials != nullptr) {
     p.ce_partials = static_cast<float2*>(ce_partials);
-    return launch2<false, false, COMM_ALLGATHER, 3>(ta, tb, p, grid, stream, ta_local);
+    return launch2<false, false, COMM_ALLGATHER, 3, 8>(ta, tb, p, grid, stream, ta_local);
   }
   if (mode == COMM_ALLGATHER)
-    return b_mn_major ? launch2<false, true, COMM_ALLGATHER>(ta, tb, p, grid, stream, ta_local)
-                      : launch2<false, false, COMM_ALLGATHER>(ta, tb, p, grid, stream, ta_local);
-  return b_mn_major ? launch2<false, true, COMM_REDUCE_SCATTER>(ta, tb, p, grid, stream)
-                    : launch2<false, false, COMM_REDUCE_SCATTER>(ta, tb, p, grid, stream);
+    return b_mn_major ? launch2<false, true, COMM_ALLGATHER, 0, 8>(ta, tb, p, grid, stream, ta_local)
+                      : launch2<false, false, COMM_ALLGATHER, 0, 8>(ta, tb, p, grid, stream, ta_local);
+  return b_mn_major ? launch2<false, true, COMM_REDUCE_SCATTER, 0, 8>(ta, tb, p, grid, stream)
+                    : launch2<false, false, COMM_REDUCE_SCATTER, 0, 8>(ta, tb, p, grid, stream);
 }
 
 int gfs_gemm2_bf16_comm(int mode, const void* a, int lda, const void* B, int ldb, void* out, int ldo,
