@@ -650,3 +650,24 @@ def test_native_step_adds_to_existing_gradients(cuda_device, H, heads, I, V, B, 
         torch.cuda.synchronize()
         grads.append(eng.optimizer.grad_buffer.double())
     assert (grads[0] - grads[1]).norm() < 4e-3 * grads[1].norm()
+
+
+@pytest.mark.parametrize("H", [8, 256, 264, 2048])
+def test_embedding_backward_run_lengths(cuda_device, H):
+    """Runs of equal ids around the numbers that a warp reads at once (8 rows, 32 keys), and columns around the 256 of a
+    warp: bit for bit the fp32 sum in the order of the positions, rounded once, on top of what is in the gradient."""
+    from gpt_from_scratch_b200.ops.embedding import embedding_bwd_native
+    counts = [1, 2, 7, 8, 9, 31, 32, 33, 64, 65, 257]
+    g = torch.Generator(device="cuda").manual_seed(H)
+    ids = torch.repeat_interleave(torch.arange(len(counts), device=cuda_device) * 3, torch.tensor(counts, device=cuda_device))
+    ids = ids[torch.randperm(ids.numel(), generator=g, device=cuda_device)].view(1, -1)
+    S = ids.shape[1]
+    dout = torch.randn(S, 1, H, device=cuda_device, generator=g).bfloat16()
+    dW = torch.randn(40, H, device=cuda_device, generator=g).bfloat16()
+    for accumulate in (False, True):
+        got = dW.clone()
+        embedding_bwd_native(ids, dout, got, 0, 40, accumulate=accumulate)
+        acc = dW.float() if accumulate else torch.zeros(40, H, device=cuda_device)
+        for s in range(S):
+            acc[ids[0, s]] += dout[s, 0].float()
+        assert torch.equal(got, acc.bfloat16())
