@@ -409,3 +409,29 @@ def test_flash_forward_128_largest_probability_is_exact(cuda_device, nh, causal)
     q, k, v = (t.bfloat16() for t in (q, k, torch.randn(1, nh, 1024, 128, device=cuda_device, generator=g)))
     ref = attention_reference(q.double(), k.double(), v.double(), causal)
     assert (apply_flash_attn(q, k, v, causal).double() - ref).norm() < 1.9e-3 * ref.norm()
+
+
+@pytest.mark.parametrize("rows,H", [(1, 8), (9, 256), (1184, 264), (1185, 264), (2500, 8), (2500, 1024), (2500, 1032),
+                                    (2500, 2048), (2500, 2056), (80000, 64)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_rmsnorm_backward_ring(cuda_device, rows, H, residual):
+    """Both sides of the lines at 1024 and 2048 columns and at a CTA per SM, a last vector that not every lane has, more
+    than 32 rows per warp; against float64, weight gradients included. The normalised value is rounded to bf16
+    (2^-9), as are the results."""
+    from gpt_from_scratch_b200.ops import _lib
+    lib = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g).bfloat16()  # noqa: E731
+    x, dy, res, w = rnd(rows, H), rnd(rows, H), rnd(rows, H), (rnd(H).float() * 0.2 + 1).bfloat16()
+    rstd = (x.float().pow(2).mean(1) + 1e-5).rsqrt().contiguous()
+    dx = torch.full((rows + 1, H), 7.0, device=cuda_device, dtype=torch.bfloat16)
+    dw = torch.empty(H, device=cuda_device, dtype=torch.bfloat16)
+    partial = torch.empty(lib.gfs_rmsnorm_bwd_parts(rows) * H, device=cuda_device)
+    assert lib.gfs_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), res.data_ptr() if residual else 0,
+                               dx.data_ptr(), dw.data_ptr(), partial.data_ptr(), rows, H, 0, _lib.stream_ptr()) == 0
+    xd, dyd, wd, r = x.double(), dy.double(), w.double(), rstd.double()[:, None]
+    ref = r * dyd * wd - xd * r ** 3 * (dyd * wd * xd).mean(1, keepdim=True) + (res.double() if residual else 0)
+    assert (dx[rows] == 7.0).all()
+    assert (dx[:rows].double() - ref).norm() < 3e-3 * ref.norm()
+    ref_w = (dyd * (xd * r)).sum(0)
+    assert (dw.double() - ref_w).norm() < 6e-3 * (dyd * xd * r).pow(2).sum(0).sqrt().norm()
