@@ -1492,7 +1492,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();       // set-up above may overlap the tail of the preceding kernel (programmatic launch)
+  // Set-up above may overlap the tail of the preceding kernel (programmatic launch). The dQ kernel reads nothing that the
+  // preceding dK / dV kernel writes, and that one had waited for everything before it when it let this one start: it
+  // waits at its end, so that its completion means that of both. us per backward: [1, 12, 130, 64] 14.0 -> 12.2,
+  // [2, 4, 256, 64] 14.9 -> 13.1, [3, 12, 777, 64] 32.2 -> 31.3, [16, 12, 1024, 64] 163.6 -> 162.4.
+  if (MODE == 0) pdl_wait();
   pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
   WaitCtx wctx{abort_flag, p.status, GFS_WAIT_LIMIT_NS};
@@ -1789,6 +1793,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
     }
   }
 
+  if (MODE == 1) pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
