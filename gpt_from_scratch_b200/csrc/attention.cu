@@ -815,7 +815,7 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 // ---------------------------------------------------------------------------
 // Forward, head_dim 64: two 128-row query tiles per CTA.
 //
-// One CTA per SM; warps 2-5 run the softmax of tile A and warps 6-9 that of tile B (one thread
+// One CTA per SM; warps 4-7 run the softmax of tile A and warps 8-11 that of tile B (one thread
 // per query row, so no cross-thread reductions), which gives every scheduler two independent
 // softmax warps while K/V tiles are fetched once for 256 query rows. S, P V and P each live
 // in tensor memory (S_A S_B | PV_A PV_B | P_A P_B = 512 columns): the probabilities are
@@ -823,7 +823,13 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 // memory. K/V use a 4-stage ring (three: 111.1 us, four: 109.4 us at the GPT-124M shape with an
 // earlier version; six stages measured 1.5 % slower than four with this one).
 // ---------------------------------------------------------------------------
-constexpr int FWD64_THREADS = 64 + 256;
+constexpr int FWD64_FIRST_SW = 4;                   // warps 0: TMA, 1: MMAs, 2 and 3: idle; then the softmax warps
+constexpr int FWD64_THREADS = 32 * (FWD64_FIRST_SW + 8);
+// Registers: 384 threads x 168 at the launch = 128 x 72 + 256 x 216. A softmax thread holds the 128 scores of its row and
+// their packed probabilities; with 168 the exponentials' sums and products could not be paired (spills). us, 168 registers
+// and scalar arithmetic -> this: [16, 12, 1024, 64] 64.4 -> 59.3, [8, 12, 2048, 64] 94.3 -> 89.0,
+// [4, 12, 4096, 64] 163 -> 155, [3, 12, 777, 64] 15.7 -> 15.0, [2, 4, 256, 64] 7.6 -> 7.4.
+constexpr int FWD64_REGS_IO = 72, FWD64_REGS_SOFTMAX = 216;
 constexpr int FWD64_KS = 4;
 constexpr int FWD64_SMEM = 2 * 16384 + FWD64_KS * 32768 + 512;
 
@@ -922,6 +928,8 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     nbk = (qb < nb) ? (p.causal ? min(qb + 1, nb) : nb) : 0;
   };
 
+  if (warp < FWD64_FIRST_SW) {
+  setmaxnreg_dec<FWD64_REGS_IO>();
   if (warp == 0) {
     if (lane == 0) {
       int g = 0;      // key blocks loaded so far (ring position)
@@ -1059,8 +1067,10 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
         it[1] += n_x[1] > 0;
       }
     }
+  }
   } else {
-    const int x = (warp - 2) >> 2;           // query tile of this warp
+    setmaxnreg_inc<FWD64_REGS_SOFTMAX>();
+    const int x = (warp - FWD64_FIRST_SW) >> 2;   // query tile of this warp
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
@@ -1068,6 +1078,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     const uint32_t o_addr = tmem_base + lane_base + OP_COL + x * 64;
     const uint32_t p_addr = tmem_base + lane_base + P_COL + x * 64;
     const float sl2 = p.scale * LOG2E_F;
+    const uint64_t sl2_2 = pack_f32x2(sl2, sl2);
     int cdone = 0;  // blocks of this tile processed in earlier items
     {
       for (int rnd = 0; rnd * G < n_items; ++rnd) {
@@ -1153,14 +1164,14 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
             m = m_new;
           }
           const float moff = ((m == -INFINITY) ? 0.f : m) * sl2;
-          float rs0 = 0.f, rs1 = 0.f;
+          const uint64_t moff2 = pack_f32x2(-moff, -moff);
+          uint64_t rs2 = 0;                        // two columns per instruction of the FMA pipe
           auto prob_chunk = [&](const uint32_t (&v)[32], uint32_t (&packed)[16]) {
 #pragma unroll
             for (int e = 0; e < 32; e += 2) {
-              const float x0 = fast_exp2(fmaf(__uint_as_float(v[e]), sl2, -moff));
-              const float x1 = fast_exp2(fmaf(__uint_as_float(v[e + 1]), sl2, -moff));
-              rs0 += x0;
-              rs1 += x1;
+              const float2 y = unpack_f32x2(fma_f32x2(pack_u32x2(v[e], v[e + 1]), sl2_2, moff2));
+              const float x0 = fast_exp2(y.x), x1 = fast_exp2(y.y);
+              rs2 = add_f32x2(rs2, pack_f32x2(x0, x1));
               packed[e >> 1] = pack_bf16x2(x0, x1);
             }
           };
@@ -1169,7 +1180,8 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           prob_chunk(v1, p1);
           prob_chunk(v2, p2);
           prob_chunk(v3, p3);
-          l += rs0 + rs1;
+          const float2 rs = unpack_f32x2(rs2);
+          l += rs.x + rs.y;
           // P of the previous block is read by its P V MMA: overwrite it only when that is done
           if (j > 0) {
             mbar_wait(&o_full[x], (c - 1) & 1, wctx, STATUS_TIMEOUT_SOFTMAX);

@@ -475,6 +475,11 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_addr) {
 // this CTA no longer objects to the next kernel's CTAs being scheduled on SMs that become free.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Registers per thread of the calling warpgroup from here on (all four warps call it).
+template <int N>
+__device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(

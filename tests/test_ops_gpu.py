@@ -435,3 +435,22 @@ def test_rmsnorm_backward_ring(cuda_device, rows, H, residual):
     assert (dx[:rows].double() - ref).norm() < 3e-3 * ref.norm()
     ref_w = (dyd * (xd * r)).sum(0)
     assert (dw.double() - ref_w).norm() < 6e-3 * (dyd * xd * r).pow(2).sum(0).sqrt().norm()
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("B,nh,S", [(7, 23, 333), (5, 30, 70), (2, 75, 257), (1, 160, 640)])
+def test_flash_attention_many_items(cuda_device, B, nh, S, causal):
+    """More work items than SMs at head_dim 64: pairs of query tiles with and without a second one, one to five key blocks;
+    the output once more in fp16, which is stored twice."""
+    from gpt_from_scratch_b200.ops.attention import apply_flash_attn, attention_reference
+    g = torch.Generator(device="cuda").manual_seed(S)
+    for dtype in (torch.bfloat16, torch.float16):
+        q, k, v = (torch.randn(B, nh, S, 64, device=cuda_device, generator=g).to(dtype).requires_grad_() for _ in range(3))
+        do = torch.randn(B, nh, S, 64, device=cuda_device, generator=g).to(dtype)
+        o = apply_flash_attn(q, k, v, causal)
+        got = (o, *torch.autograd.grad(o, (q, k, v), do))
+        qf, kf, vf = (t.detach().bfloat16().float().requires_grad_() for t in (q, k, v))
+        of = attention_reference(qf, kf, vf, causal)
+        for name, a, b in zip(("O", "dQ", "dK", "dV"), got, (of, *torch.autograd.grad(of, (qf, kf, vf), do.float()))):
+            rel = (a.float() - b).norm() / b.norm()
+            assert rel < 1e-2, f"{name}: relative error {rel:.4g}"       # as in test_flash_attention_tile_edges
