@@ -88,6 +88,7 @@ struct Params2 {
   const __nv_bfloat16* R;  // addend (may alias C) or null
   int tiles_m, tiles_n, kblocks;
   int group_m;             // see tile_coords
+  int early_b, late_wait;  // gfs_host::LaunchHints (without collectives)
   uint32_t* status;
   const float* rope_cos;
   const float* rope_sin;
@@ -558,9 +559,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   tc_fence_before();
   cluster_sync_all();  // barriers of both CTAs initialised, TMEM allocated
   tc_fence_after();
-  // everything above ran while the preceding kernel of the stream may still have been draining
-  pdl_wait();
-  pdl_trigger();
+  // Everything above ran while the preceding kernel of the stream may still have been draining. With early_b the TMA warp
+  // waits after its first loads of B, with late_wait everybody at the end.
+  const bool late_wait = COMM == COMM_NONE && p.late_wait != 0;
+  const bool early_b = COMM == COMM_NONE && p.early_b != 0 && !late_wait;
+  if (!late_wait && !(early_b && warp == 0)) pdl_wait();
+  if (!(early_b && warp == 0)) pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
   WaitCtx wctx{abort_flag, p.status, GFS_WAIT_LIMIT_NS};
 
@@ -579,6 +583,34 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       int stage = 0;
       uint32_t phase = 0;
       uint32_t chunk_ready = 0;  // all-gather: chunks whose arrival has been observed
+      auto load_b = [&](int st, int k0, int n0) {
+        uint8_t* sb = tiles + st * STAGE_BYTES + A_BYTES;
+        const uint32_t bar = mapa_u32(smem_u32(&full_bar[st]), 0);
+        if (SWI == 1) {
+          // n0 counts interleaved tile columns: gate rows [g0, g0 + 128) for the leader, the
+          // matching up rows [I + g0, ...) for the other CTA
+          const int g0 = (n0 - static_cast<int>(rank) * BNH) >> 1;
+          tma_load_2d_pair(sb, &tmap_b, bar, k0, (rank == 0 ? 0 : p.swi_I) + g0);
+        } else if (!B_MN) {
+          tma_load_2d_pair(sb, &tmap_b, bar, k0, n0);
+        } else {
+#pragma unroll
+          for (int i = 0; i < BNH / 64; ++i) tma_load_2d_pair(sb + i * 8192, &tmap_b, bar, n0 + 64 * i, k0);
+        }
+      };
+      int early = 0;             // stages whose B is on its way
+      if (early_b) {
+        int m0, n0, chunk;
+        decode_tile2<COMM>(p, pair, m0, n0, chunk);
+        n0 += static_cast<int>(rank) * BNH;
+        early = min(STAGES, p.kblocks);
+        for (int kb = 0; kb < early; ++kb) {
+          if (leader) mbar_arrive_expect_tx(&full_bar[kb], 2 * STAGE_BYTES);
+          load_b(kb, kb * BK, n0);
+        }
+        pdl_wait();
+        pdl_trigger();
+      }
       for (int t = pair; t < total_tiles; t += num_pairs) {
         int m0, n0, chunk;
         decode_tile2<COMM>(p, t, m0, n0, chunk);
@@ -600,9 +632,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         for (int kb = 0; kb < p.kblocks; ++kb) {
           mbar_wait(&empty_bar[stage], phase ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
           uint8_t* sa = tiles + stage * STAGE_BYTES;
-          uint8_t* sb = sa + A_BYTES;
           // the leader's barrier counts the bytes of both CTAs
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
+          if (leader && early == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
           const uint32_t bar = mapa_u32(smem_u32(&full_bar[stage]), 0);
           const int k0 = kb * BK;
           if (!A_MN) {
@@ -612,17 +643,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < BM / 64; ++i) tma_load_2d_pair(sa + i * 8192, &tmap_a, bar, m0 + 64 * i, k0);
           }
-          if (SWI == 1) {
-            // n0 counts interleaved tile columns: gate rows [g0, g0 + 128) for the leader, the
-            // matching up rows [I + g0, ...) for the other CTA
-            const int g0 = (n0 - static_cast<int>(rank) * BNH) >> 1;
-            tma_load_2d_pair(sb, &tmap_b, bar, k0, (rank == 0 ? 0 : p.swi_I) + g0);
-          } else if (!B_MN) {
-            tma_load_2d_pair(sb, &tmap_b, bar, k0, n0);
-          } else {
-#pragma unroll
-            for (int i = 0; i < BNH / 64; ++i) tma_load_2d_pair(sb + i * 8192, &tmap_b, bar, n0 + 64 * i, k0);
-          }
+          if (early == 0) load_b(stage, k0, n0);
+          else --early;
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
@@ -1028,6 +1050,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     if (ct == 0) trace_stamp(p, TRACE_RED_END);
   }
 
+  if (late_wait) pdl_wait();
   // nobody leaves while the partner may still touch this CTA's shared memory / barriers
   tc_fence_before();
   __syncthreads();
@@ -1059,6 +1082,7 @@ struct GroupProblem {
 
 struct GroupParams {
   int ngroups, total_tiles;
+  int late_wait;         // gfs_host::LaunchHints
   GroupProblem g[MAX_GROUP];
   uint32_t* status;
 };
@@ -1114,7 +1138,7 @@ gemm2_grouped_kernel(const __grid_constant__ GroupMaps maps, const __grid_consta
   tc_fence_before();
   cluster_sync_all();
   tc_fence_after();
-  pdl_wait();
+  if (p.late_wait == 0) pdl_wait();
   pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
   WaitCtx wctx{abort_flag, p.status, GFS_WAIT_LIMIT_NS};
@@ -1273,6 +1297,7 @@ gemm2_grouped_kernel(const __grid_constant__ GroupMaps maps, const __grid_consta
     }
   }
 
+  if (p.late_wait) pdl_wait();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();
@@ -1309,7 +1334,11 @@ int launch2(const CUtensorMap* ta, const CUtensorMap* tb, const Params2& p, int 
   }
   Params2 pt = p;
   pt.trace = g_trace;
-  if (COMM == COMM_NONE) pt.group_m = panel_rows(p);
+  if (COMM == COMM_NONE) {
+    pt.group_m = panel_rows(p);
+    pt.early_b = gfs_host::launch_hints().early_b;
+    pt.late_wait = gfs_host::launch_hints().late_wait;
+  }
   if (gfs_host::launch_pdl(kern, dim3(grid), dim3(threads2(COMM, EW)), smem, stream, *ta, *tb, tx ? *tx : *ta,
                            ty ? *ty : *ta, pt) != cudaSuccess)
     return -11;
@@ -1622,6 +1651,7 @@ int gfs_gemm2_wgrad_grouped(int n, const unsigned long long* A, const unsigned l
   GroupMaps maps;
   GroupParams p{};
   p.ngroups = n;
+  p.late_wait = gfs_host::launch_hints().late_wait;
   p.status = gfs_host::status_words();
   int total = 0;
   for (int i = 0; i < n; ++i) {

@@ -52,6 +52,7 @@ template <int NG>
 struct TileParams {
   TileProblem g[NG];
   int ngroups, split;
+  int early_b, late_wait;   // gfs_host::LaunchHints
   uint32_t* status;
   const float* rope_cos;    // rotary embedding of the first rope_cols columns (see gemm.cu)
   const float* rope_sin;
@@ -279,8 +280,11 @@ gemm_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constan
   if (split > 1) cluster_sync();   // also: every CTA of the cluster runs before its shared memory is written
   else __syncthreads();
   tc_fence_after();
-  pdl_wait();       // set-up above may overlap the tail of the preceding kernel (programmatic launch)
-  pdl_trigger();
+  // Set-up above may overlap the tail of the preceding kernel (programmatic launch). With early_b the TMA warp waits after
+  // its first loads of B, with late_wait everybody at the end.
+  const bool early_b = p.early_b != 0 && p.late_wait == 0;
+  if (p.late_wait == 0 && !(early_b && warp == 0)) pdl_wait();
+  if (!(early_b && warp == 0)) pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
   WaitCtx wctx{abort_flag, p.status, GFS_WAIT_LIMIT_NS};
   const int kb0 = rank * g.per_split;
@@ -288,19 +292,8 @@ gemm_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constan
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const int i = kb - kb0, stage = i % STAGES;
-        mbar_wait(&empty_bar[stage], ((i / STAGES) & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
-        uint8_t* sa = tiles + stage * C_::STAGE_BYTES;
-        uint8_t* sb = sa + C_::A_BYTES;
-        mbar_arrive_expect_tx(&full_bar[stage], C_::STAGE_BYTES);
-        const int k0 = kb * BK;
-        if (!A_MN) {
-          tma_load_2d(sa, &maps.a[gi], &full_bar[stage], k0, m0);
-        } else {
-#pragma unroll
-          for (int j = 0; j < BM / 64; ++j) tma_load_2d(sa + j * 8192, &maps.a[gi], &full_bar[stage], m0 + 64 * j, k0);
-        }
+      auto load_b = [&](int stage, int k0) {
+        uint8_t* sb = tiles + stage * C_::STAGE_BYTES + C_::A_BYTES;
         if (!B_MN) {
           if (p.swi_mode == 1) {   // BN/2 gate rows + the matching up rows (tensor map box = BN/2 rows)
             tma_load_2d(sb, &maps.b[gi], &full_bar[stage], k0, n0 >> 1);
@@ -312,6 +305,33 @@ gemm_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constan
 #pragma unroll
           for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, &maps.b[gi], &full_bar[stage], n0 + 64 * j, k0);
         }
+      };
+      auto load_a = [&](int stage, int k0) {
+        uint8_t* sa = tiles + stage * C_::STAGE_BYTES;
+        if (!A_MN) {
+          tma_load_2d(sa, &maps.a[gi], &full_bar[stage], k0, m0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < BM / 64; ++j) tma_load_2d(sa + j * 8192, &maps.a[gi], &full_bar[stage], m0 + 64 * j, k0);
+        }
+      };
+      int i = 0;
+      if (early_b) {
+        const int n = min(STAGES, kb1 - kb0);
+        for (int e = 0; e < n; ++e) {
+          mbar_arrive_expect_tx(&full_bar[e], C_::STAGE_BYTES);
+          load_b(e, (kb0 + e) * BK);
+        }
+        pdl_wait();
+        pdl_trigger();
+        for (; i < n; ++i) load_a(i, (kb0 + i) * BK);
+      }
+      for (; i < kb1 - kb0; ++i) {
+        const int stage = i % STAGES, k0 = (kb0 + i) * BK;
+        mbar_wait(&empty_bar[stage], ((i / STAGES) & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
+        mbar_arrive_expect_tx(&full_bar[stage], C_::STAGE_BYTES);
+        load_a(stage, k0);
+        load_b(stage, k0);
       }
       if (*abort_flag) {
         for (int i = 0; i < 64; ++i) __nanosleep(1000);   // copies in flight land before the memory is released
@@ -351,6 +371,7 @@ gemm_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constan
     else __syncthreads();
   });
 
+  if (p.late_wait) pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -425,8 +446,9 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
   tc_fence_before();
   cluster_sync();   // barriers of all CTAs initialised, TMEM allocated
   tc_fence_after();
-  pdl_wait();
-  pdl_trigger();
+  const bool early_b = p.early_b != 0 && p.late_wait == 0;   // as above
+  if (p.late_wait == 0 && !(early_b && warp == 0)) pdl_wait();
+  if (!(early_b && warp == 0)) pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
   WaitCtx wctx{abort_flag, p.status, GFS_WAIT_LIMIT_NS};
   const int kb0 = z * g.per_split;
@@ -435,20 +457,12 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
   if (warp == 0) {
     if (lane == 0) {
       const int nb = n0 + half * BNH;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const int i = kb - kb0, stage = i % PAIR_STAGES;
-        mbar_wait(&empty_bar[stage], ((i / PAIR_STAGES) & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
-        uint8_t* sa = tiles + stage * PAIR_STAGE_BYTES;
-        uint8_t* sb = sa + 16384;
-        if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * PAIR_STAGE_BYTES);   // the bytes of both CTAs
+      auto begin = [&](int stage) {      // the leader's barrier counts the bytes of both CTAs
+        if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * PAIR_STAGE_BYTES);
+      };
+      auto load_b = [&](int stage, int k0) {
+        uint8_t* sb = tiles + stage * PAIR_STAGE_BYTES + 16384;
         const uint32_t bar = mapa_u32(smem_u32(&full_bar[stage]), lead);
-        const int k0 = kb * BK;
-        if (!A_MN) {
-          tma_load_2d_pair(sa, &maps.a[gi], bar, k0, m0);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 2; ++j) tma_load_2d_pair(sa + j * 8192, &maps.a[gi], bar, m0 + 64 * j, k0);
-        }
         if (!B_MN) {
           // SwiGLU forward: 128 gate rows for the leader, the matching up rows for the other CTA
           tma_load_2d_pair(sb, &maps.b[gi], bar, k0, p.swi_mode == 1 ? half * p.swi_I + (n0 >> 1) : nb);
@@ -456,6 +470,34 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
 #pragma unroll
           for (int j = 0; j < 2; ++j) tma_load_2d_pair(sb + j * 8192, &maps.b[gi], bar, nb + 64 * j, k0);
         }
+      };
+      auto load_a = [&](int stage, int k0) {
+        uint8_t* sa = tiles + stage * PAIR_STAGE_BYTES;
+        const uint32_t bar = mapa_u32(smem_u32(&full_bar[stage]), lead);
+        if (!A_MN) {
+          tma_load_2d_pair(sa, &maps.a[gi], bar, k0, m0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) tma_load_2d_pair(sa + j * 8192, &maps.a[gi], bar, m0 + 64 * j, k0);
+        }
+      };
+      int i = 0;
+      if (early_b) {
+        const int n = min(PAIR_STAGES, kb1 - kb0);
+        for (int e = 0; e < n; ++e) {
+          begin(e);
+          load_b(e, (kb0 + e) * BK);
+        }
+        pdl_wait();
+        pdl_trigger();
+        for (; i < n; ++i) load_a(i, (kb0 + i) * BK);
+      }
+      for (; i < kb1 - kb0; ++i) {
+        const int stage = i % PAIR_STAGES, k0 = (kb0 + i) * BK;
+        mbar_wait(&empty_bar[stage], ((i / PAIR_STAGES) & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
+        begin(stage);
+        load_a(stage, k0);
+        load_b(stage, k0);
       }
       if (*abort_flag) {
         for (int i = 0; i < 64; ++i) __nanosleep(1000);
@@ -504,6 +546,7 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
     else __syncthreads();
   });
 
+  if (p.late_wait) pdl_wait();
   // nobody leaves while the partner may still touch this CTA's shared memory / barriers
   tc_fence_before();
   __syncthreads();
@@ -594,6 +637,8 @@ int gfs_gemm_tile(const void* A, const void* B, void* C, const void* R, int M, i
   TileParams<1> p{};
   p.ngroups = 1;
   p.split = split;
+  p.early_b = gfs_host::launch_hints().early_b;
+  p.late_wait = gfs_host::launch_hints().late_wait;
   p.status = gfs_host::status_words();
   p.rope_cos = static_cast<const float*>(rope_cos);
   p.rope_sin = static_cast<const float*>(rope_sin);
@@ -632,6 +677,8 @@ int gfs_gemm_tile_wgrad_grouped(int n, const unsigned long long* A, const unsign
   TileParams<MAX_GROUP> p{};
   p.ngroups = n;
   p.split = split;
+  p.early_b = gfs_host::launch_hints().early_b;
+  p.late_wait = gfs_host::launch_hints().late_wait;
   p.status = gfs_host::status_words();
   p.rope_b = 1;
   int total = 0;

@@ -117,9 +117,10 @@ int tiles256(int m, int n) { return ((m + 255) / 256) * ((n + 255) / 256); }
 
 bool use_pair(const GfsBlockDims& d, int tiles) { return d.pair_min_tiles >= 0 && tiles >= d.pair_min_tiles; }
 
-// C[M,N] = op(A) op(B) (+ R), R with the pitch of C
+// C[M,N] = op(A) op(B) (+ R), R with the pitch of C. B is a weight, which no kernel of a pass writes.
 int product(const GfsBlockDims& d, const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda,
             int ldb, int ldc, int a_mn, int b_mn, void* stream) {
+  const gfs_host::WithHints hints(true, false);
   return gfs_linear(A, B, C, R, M, N, K, lda, ldb, ldc, R != nullptr ? ldc : 0, a_mn, b_mn, nullptr, nullptr, 0, d.D,
                     d.B, d.pair_min_tiles, stream);
 }
@@ -130,8 +131,10 @@ struct WgradGroup {
   u64 A[MAX], B[MAX], C[MAX];
   int M[MAX], N[MAX], K[MAX], lda[MAX], ldb[MAX], ldc[MAX], acc[MAX];
   int n = 0, tiles = 0;
-  int flush(int* launches, void* stream) {
+  // late: the kernel launched last is a product that writes nothing these read (see gfs_host::LaunchHints)
+  int flush(int* launches, void* stream, bool late) {
     if (n == 0) return 0;
+    const gfs_host::WithHints hints(false, late);
     const int rc = gfs_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, acc, stream);
     n = tiles = 0;
     ++*launches;
@@ -139,7 +142,8 @@ struct WgradGroup {
   }
 };
 
-// dW[N_out, N_in] (+)= dY[T, N_out]^T X[T, N_in]
+// dW[N_out, N_in] (+)= dY[T, N_out]^T X[T, N_in]. Called right after a product of the gradient chain that also reads dY:
+// nothing launched here depends on that product, and it may fill the SMs that its last wave leaves idle.
 int weight_grad(const GfsBlockDims& d, WgradGroup& grp, const void* dY, const void* X, void* dW, int accumulate, int T,
                 int n_out, int n_in, int* launches, void* stream) {
   const int tiles = tiles256(n_out, n_in);
@@ -152,11 +156,13 @@ int weight_grad(const GfsBlockDims& d, WgradGroup& grp, const void* dY, const vo
     grp.lda[i] = n_out; grp.ldb[i] = n_in; grp.ldc[i] = n_in;
     grp.acc[i] = accumulate;
     grp.tiles += tiles;
-    if (grp.n == WgradGroup::MAX || grp.tiles >= d.pair_min_tiles) return grp.flush(launches, stream);
+    if (grp.n == WgradGroup::MAX || grp.tiles >= d.pair_min_tiles) return grp.flush(launches, stream, true);
     return 0;
   }
   ++*launches;
-  return product(d, dY, X, dW, accumulate ? dW : nullptr, n_out, n_in, T, n_out, n_in, n_in, 1, 1, stream);
+  const gfs_host::WithHints hints(false, true);
+  return gfs_linear(dY, X, dW, accumulate ? dW : nullptr, n_out, n_in, T, n_out, n_in, n_in, accumulate ? n_in : 0, 1, 1,
+                    nullptr, nullptr, 0, d.D, d.B, d.pair_min_tiles, stream);
 }
 
 bool dims_ok(const GfsBlockDims& d) {
@@ -202,6 +208,7 @@ int gfs_blocks_forward(const GfsBlockDims* dp, const GfsBlockParams* layers, con
          *y2 = base + a.y2, *rstd2 = base + a.rstd2, *gu = base + a.gu, *ac = base + a.act, *x2 = base + a.x2;
     char* qkv = base + a.qkv;
     GFS_TRY(gfs_rmsnorm_fwd(x, p.w[W_NORM1], y1, rstd1, T, H, p.eps[0], stream));
+    const gfs_host::WithHints hints(true, false);   // (of the products; B is a weight)
     GFS_TRY(gfs_linear(y1, p.w[W_QKV], qkv, nullptr, T, 3 * H, H, H, H, 3 * H, 0, 0, 0, p.cos_table, p.sin_table, 2 * H,
                        d.D, d.B, d.pair_min_tiles, stream));   // q and k leave rotated
     GFS_TRY(gfs_flash_fwd(qkv, qkv + 2 * static_cast<size_t>(H), qkv + 4 * static_cast<size_t>(H), attn, nullptr, lse,
@@ -295,8 +302,11 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
       GFS_TRY(gfs_dropout_residual(dout, nullptr, s + b.dmask, n_el, d.dropout_p, p.seed[1], 1, stream));
       dm = s + b.dmask;
     }
-    GFS_TRY(gfs_linear_swiglu(2, dm, p.w[W_DOWN], dgu, const_cast<void*>(gu), T, I, H, H, I, 2 * I, 2 * I,
-                              d.pair_min_tiles, stream));
+    {
+      const gfs_host::WithHints hints(true, false);
+      GFS_TRY(gfs_linear_swiglu(2, dm, p.w[W_DOWN], dgu, const_cast<void*>(gu), T, I, H, H, I, 2 * I, 2 * I,
+                                d.pair_min_tiles, stream));
+    }
     int rc = weight_grad(d, grp, dm, ac, p.g[W_DOWN], p.accumulate[W_DOWN], T, H, I, launches, stream);
     if (rc != 0) return rc;
     GFS_TRY(product(d, dgu, p.w[W_GATE_UP], dy, nullptr, T, H, 2 * I, 2 * I, H, H, 0, 1, stream));
@@ -318,9 +328,10 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
                           d.nh, d.D, st, scale, 1, p.cos_table, p.sin_table, nullptr, stream));
     *launches += 2;   // a pre-pass and two main kernels
     GFS_TRY(product(d, dqkv, p.w[W_QKV], dy, nullptr, T, H, 3 * H, 3 * H, H, H, 0, 1, stream));
+    const int launched = *launches;
     rc = weight_grad(d, grp, dqkv, y1, p.g[W_QKV], p.accumulate[W_QKV], T, 3 * H, H, launches, stream);
     if (rc != 0) return rc;
-    rc = grp.flush(launches, stream);   // its operands are overwritten by the next block
+    rc = grp.flush(launches, stream, *launches == launched);   // its operands are overwritten by the next block
     if (rc != 0) return rc;
     void* dnext = l == 0 ? dx : s + b.dx[l & 1];
     GFS_TRY(norm_bwd(dy, input_of(l), p.w[W_NORM1], rstd1, dx1, dnext, p.g[W_NORM1], p.accumulate[W_NORM1]));
@@ -434,8 +445,9 @@ int step_until_embedding(const GfsBlockDims& d, const GfsBlockParams* layers, co
   GFS_TRY(gfs_ce_bwd(logits, lse, targets, nullptr, g_row, T, V, V, 0, stream));
   GFS_TRY(product(d, logits, t.w_out, dy, nullptr, T, H, V, V, H, H, 0, 1, stream));
   WgradGroup grp;
+  const int launched = *launches;
   rc = weight_grad(d, grp, logits, y, t.g_out, t.acc_out, T, V, H, launches, stream);
-  if (rc == 0) rc = grp.flush(launches, stream);
+  if (rc == 0) rc = grp.flush(launches, stream, *launches == launched);
   if (rc != 0) return rc;
   rc = gfs_blocks_backward(&d, layers, t.w_final, t.g_final, t.acc_final, x0, act, rstd, dy, scratch, dx0, launches,
                            stream);
