@@ -568,17 +568,22 @@ struct AdamArgs {
   const float* step_dev;
   double beta1_d, beta2_d;
 };
+// beta^n by squaring (a few roundings of double precision); pow() twice on one thread was 2 of the 11 us of a small update.
+__device__ __forceinline__ double power(double beta, unsigned int n) {
+  double r = 1.0;
+  for (; n != 0u; n >>= 1, beta *= beta)
+    if (n & 1u) r *= beta;
+  return r;
+}
 // Called by all threads of the CTA (contains a __syncthreads when step_dev is set).
 __device__ __forceinline__ void adam_bias_corrections(const AdamArgs& a, float& bc1, float& bc2_sqrt) {
   bc1 = a.bias_corr1;
   bc2_sqrt = a.bias_corr2_sqrt;
   if (a.step_dev != nullptr) {
     __shared__ float s_bc[2];
-    if (threadIdx.x == 0) {
-      const double t = static_cast<double>(*a.step_dev);
-      s_bc[0] = static_cast<float>(1.0 - pow(a.beta1_d, t));
-      s_bc[1] = static_cast<float>(sqrt(1.0 - pow(a.beta2_d, t)));
-    }
+    const unsigned int t = static_cast<unsigned int>(*a.step_dev);   // a whole number
+    if (threadIdx.x == 0) s_bc[0] = static_cast<float>(1.0 - power(a.beta1_d, t));
+    if (threadIdx.x == 32) s_bc[1] = static_cast<float>(sqrt(1.0 - power(a.beta2_d, t)));
     __syncthreads();
     bc1 = s_bc[0];
     bc2_sqrt = s_bc[1];

@@ -439,6 +439,8 @@ struct DwReduceBatch {
 
 __global__ void rmsnorm_dw_reduce_multi_kernel(const __grid_constant__ DwReduceBatch b, int H) {
   __shared__ float sm[32][33];
+  pdl_wait();
+  pdl_trigger();
   const int l = blockIdx.y;
   const float* __restrict__ partial = b.partial[l];
   __nv_bfloat16* __restrict__ dw = b.dw[l];
@@ -508,6 +510,8 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
 __global__ void dropout_residual_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                                         __nv_bfloat16* __restrict__ out, long long nvec, float p,
                                         unsigned long long seed, int backward) {
+  pdl_wait();
+  pdl_trigger();
   const unsigned int drop_below = static_cast<unsigned int>(p * 256.f + 0.5f);  // byte < drop_below -> dropped
   const float scale = 256.f / static_cast<float>(256u - drop_below);           // 1 / (realised keep probability)
   for (long long v = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; v < nvec;
@@ -581,6 +585,8 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const 
 __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ W,
                                      __nv_bfloat16* __restrict__ out, int B, int S, int H, int v0, int v1, int s0,
                                      int s_count) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= s_count * B) return;
@@ -829,7 +835,8 @@ int gfs_rmsnorm_dw_reduce_multi(int n, const unsigned long long* partial, const 
     b.parts[i] = parts[i];
     b.accumulate[i] = accumulate[i];
   }
-  rmsnorm_dw_reduce_multi_kernel<<<dim3((H + 31) / 32, n), dim3(32, 32), 0, static_cast<cudaStream_t>(stream)>>>(b, H);
+  gfs_host::launch_pdl(rmsnorm_dw_reduce_multi_kernel, dim3((H + 31) / 32, n), dim3(32, 32), 0,
+                       static_cast<cudaStream_t>(stream), b, H);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -854,9 +861,10 @@ int gfs_dropout_residual(const void* x, const void* residual, void* out, long lo
   if (!(p >= 0.f) || p >= 1.f) return -1;
   const long long nvec = n >> 3;
   const int blocks = static_cast<int>(std::min<long long>((nvec + 255) / 256, static_cast<long long>(gfs_host::sm_count()) * 16));
-  dropout_residual_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual),
-      static_cast<__nv_bfloat16*>(out), nvec, p, seed, backward);
+  gfs_host::launch_pdl(dropout_residual_kernel, dim3(blocks), dim3(256), 0,
+                       static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x),
+                       static_cast<const __nv_bfloat16*>(residual), static_cast<__nv_bfloat16*>(out), nvec, p, seed,
+                       backward);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -885,9 +893,10 @@ int gfs_embedding_fwd(const void* ids, const void* W, void* out, int B, int S, i
   const int rows = s_count * B;
   if (rows == 0) return 0;
   const int warps = 8;
-  embedding_fwd_kernel<<<(rows + warps - 1) / warps, warps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const long long*>(ids), static_cast<const __nv_bfloat16*>(W), static_cast<__nv_bfloat16*>(out), B, S,
-      H, v0, v1, s0, s_count);
+  gfs_host::launch_pdl(embedding_fwd_kernel, dim3((rows + warps - 1) / warps), dim3(warps *
+                       32), 0, static_cast<cudaStream_t>(stream), static_cast<const long long*>(ids),
+                       static_cast<const __nv_bfloat16*>(W), static_cast<__nv_bfloat16*>(out), B, S, H, v0, v1, s0,
+                       s_count);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -43,6 +43,8 @@ __global__ void __launch_bounds__(CE_THREADS)
 ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
               float* __restrict__ stats, float* __restrict__ lse, float* __restrict__ loss, int Vp, long ld, int v0,
               int single_rank, int tb, long long* __restrict__ rows_target) {
+  pdl_wait();
+  pdl_trigger();
   const int row = blockIdx.x;
   const __nv_bfloat16* z = logits + static_cast<size_t>(row) * ld;
   const int nvec = Vp >> 3;
@@ -108,6 +110,8 @@ ce_from_partials_kernel(const float2* __restrict__ partials, const __nv_bfloat16
                         float* __restrict__ loss, int parts, int M, int Vp, long ld, int v0, int single_rank, int tb,
                         long long* __restrict__ rows_target) {
   __shared__ float2 part_res[CE_PW][32];
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * 32 + lane;
   float gm = -INFINITY, gs = 0.f;
@@ -170,6 +174,8 @@ __global__ void ce_combine_kernel(const float* __restrict__ stats_all, float* __
 __global__ void ce_bwd_kernel(__nv_bfloat16* __restrict__ logits, const float* __restrict__ lse,
                               const long long* __restrict__ target, const float* __restrict__ grad_rows, float grad_all,
                               int M, int Vp, long ld, int v0) {
+  pdl_wait();
+  pdl_trigger();
   const int nvec = Vp >> 3;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nvec) return;
@@ -222,6 +228,8 @@ constexpr int SUMSQ_MAX_BLOCKS = 1024;
 __global__ void __launch_bounds__(SUMSQ_THREADS)
 sumsq_bf16_kernel(const __nv_bfloat16* __restrict__ x, long long n, float* __restrict__ out,
                   float* __restrict__ scratch) {
+  pdl_wait();
+  pdl_trigger();
   float acc = 0.f;
   const long long nvec = n >> 3;
   for (long long v = blockIdx.x * static_cast<long long>(SUMSQ_THREADS) + threadIdx.x; v < nvec;
@@ -280,9 +288,12 @@ __global__ void adamw_kernel(const __nv_bfloat16* __restrict__ grad, float* __re
                              float* __restrict__ exp_avg, float* __restrict__ exp_avg_sq,
                              __nv_bfloat16* __restrict__ param_out, long long n, const float* __restrict__ sumsq,
                              float* __restrict__ norm_out, AdamArgs a) {
+  pdl_wait();
+  pdl_trigger();
   float coef = a.grad_scale;
   if (sumsq != nullptr) {
-    const float norm = sqrtf(*sumsq) * a.grad_scale;
+    // (not through the read-only path: the kernel before this one writes it)
+    const float norm = sqrtf(*reinterpret_cast<const volatile float*>(sumsq)) * a.grad_scale;
     if (norm_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *norm_out = norm;
     if (a.clip > 0.f && norm > a.clip) coef *= a.clip / (norm + 1e-6f);
   }
@@ -334,6 +345,8 @@ __global__ void adamw_kernel(const __nv_bfloat16* __restrict__ grad, float* __re
 // Mean of n floats by one CTA, in a fixed order.
 __global__ void __launch_bounds__(1024) mean_f32_kernel(const float* __restrict__ x, float* __restrict__ out, int n) {
   __shared__ float sm[32];
+  pdl_wait();
+  pdl_trigger();
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += 1024) s += x[i];
   s = warp_sum(s);
@@ -367,10 +380,11 @@ int gfs_ce_fwd(const void* logits, const void* target, void* stats, void* lse, v
                int v0, int single_rank, int target_batch, void* rows_target, void* stream) {
   if ((Vp & 7) || (ld & 7) || target_batch < 0 || (target_batch > 0 && M % target_batch != 0)) return -1;
   if (M == 0) return 0;
-  ce_fwd_kernel<<<M, CE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(logits), static_cast<const long long*>(target), static_cast<float*>(stats),
-      static_cast<float*>(lse), static_cast<float*>(loss), Vp, ld, v0, single_rank, target_batch,
-      static_cast<long long*>(rows_target));
+  gfs_host::launch_pdl(ce_fwd_kernel, dim3(M), dim3(CE_THREADS), 0,
+                       static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(logits),
+                       static_cast<const long long*>(target), static_cast<float*>(stats), static_cast<float*>(lse),
+                       static_cast<float*>(loss), Vp, ld, v0, single_rank, target_batch,
+                       static_cast<long long*>(rows_target));
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -379,11 +393,11 @@ int gfs_ce_from_partials(const void* partials, const void* logits, const void* t
                          void* rows_target, void* stream) {
   if (M == 0) return 0;
   if (target_batch < 0 || (target_batch > 0 && M % target_batch != 0)) return -1;
-  ce_from_partials_kernel<<<(M + 31) / 32, 32 * CE_PW, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const float2*>(partials), static_cast<const __nv_bfloat16*>(logits),
-      static_cast<const long long*>(target), static_cast<float*>(stats), static_cast<float*>(lse),
-      static_cast<float*>(loss), parts, M, Vp, ld, v0, single_rank, target_batch,
-      static_cast<long long*>(rows_target));
+  gfs_host::launch_pdl(ce_from_partials_kernel, dim3((M + 31) / 32), dim3(32 * CE_PW), 0,
+                       static_cast<cudaStream_t>(stream), static_cast<const float2*>(partials),
+                       static_cast<const __nv_bfloat16*>(logits), static_cast<const long long*>(target),
+                       static_cast<float*>(stats), static_cast<float*>(lse), static_cast<float*>(loss), parts, M,
+                       Vp, ld, v0, single_rank, target_batch, static_cast<long long*>(rows_target));
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -399,16 +413,18 @@ int gfs_ce_bwd(void* logits, const void* lse, const void* target, const void* gr
   if ((Vp & 7) || (ld & 7)) return -1;
   if (M == 0 || Vp == 0) return 0;
   const dim3 grid(((Vp >> 3) + 255) / 256, std::min((M + 3) / 4, 1024));
-  ce_bwd_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(logits), static_cast<const float*>(lse), static_cast<const long long*>(target),
-      static_cast<const float*>(grad_rows), grad_all, M, Vp, ld, v0);
+  gfs_host::launch_pdl(ce_bwd_kernel, grid, dim3(256), 0, static_cast<cudaStream_t>(stream),
+                       static_cast<__nv_bfloat16*>(logits), static_cast<const float*>(lse),
+                       static_cast<const long long*>(target), static_cast<const float*>(grad_rows), grad_all, M, Vp,
+                       ld, v0);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 int gfs_mean_f32(const void* x, void* out, int n, void* stream) {
   if (n <= 0) return -1;
-  mean_f32_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const float*>(x),
-                                                                     static_cast<float*>(out), n);
+  gfs_host::launch_pdl(mean_f32_kernel, dim3(1), dim3(1024), 0,
+                       static_cast<cudaStream_t>(stream), static_cast<const float*>(x), static_cast<float*>(out),
+                       n);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -419,8 +435,9 @@ int gfs_sumsq_bf16(const void* x, long long n, void* out, void* scratch, void* s
   const long long nvec = n >> 3;
   long long blocks = (nvec + SUMSQ_THREADS - 1) / SUMSQ_THREADS;
   blocks = std::max<long long>(1, std::min<long long>(blocks, std::min(SUMSQ_MAX_BLOCKS, gfs_host::sm_count() * 4)));
-  sumsq_bf16_kernel<<<static_cast<int>(blocks), SUMSQ_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), n, static_cast<float*>(out), static_cast<float*>(scratch));
+  gfs_host::launch_pdl(sumsq_bf16_kernel, dim3(static_cast<int>(blocks)), dim3(SUMSQ_THREADS),
+                       0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x), n,
+                       static_cast<float*>(out), static_cast<float*>(scratch));
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -437,10 +454,11 @@ int gfs_adamw_step(const void* grad, void* master, void* exp_avg, void* exp_avg_
              bias_corr2_sqrt, clip, grad_scale, static_cast<const float*>(step_dev), beta1, beta2};
   const long long blocks =
       std::max<long long>(1, std::min<long long>((n / 4 + 255) / 256, static_cast<long long>(gfs_host::sm_count()) * 16));
-  adamw_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(grad), static_cast<float*>(master), static_cast<float*>(exp_avg),
-      static_cast<float*>(exp_avg_sq), static_cast<__nv_bfloat16*>(param_out), n, static_cast<const float*>(sumsq),
-      static_cast<float*>(norm_out), a);
+  gfs_host::launch_pdl(adamw_kernel, dim3(static_cast<int>(blocks)), dim3(256), 0,
+                       static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(grad),
+                       static_cast<float*>(master), static_cast<float*>(exp_avg), static_cast<float*>(exp_avg_sq),
+                       static_cast<__nv_bfloat16*>(param_out), n, static_cast<const float*>(sumsq),
+                       static_cast<float*>(norm_out), a);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -384,8 +384,8 @@ struct StepLayout {
   }
 };
 
-// The id sort of the embedding backward needs only the ids: it runs beside the forward on a stream of
-// its own (one per thread and device, so that neither threads nor captures meet in its events; given back when
+// The id sort of the embedding backward needs only the ids, the clearing of its gradient nothing: they run beside the
+// forward on a stream of their own (one per thread and device, so that neither threads nor captures meet in its events; given back when
 // the thread ends).
 struct SideStream {
   cudaStream_t stream = nullptr;
@@ -410,7 +410,7 @@ SideStream* side_stream() {
   return &s;
 }
 
-// The step without the embedding's backward (but with its gradient cleared): logits, loss, and back.
+// The step without the embedding's backward: logits, loss, and back.
 int step_until_embedding(const GfsBlockDims& d, const GfsBlockParams* layers, const GfsModelTop& t, const void* ids,
                          const void* labels, char* m, const StepLayout& lay, const u64* act, void* loss, int* launches,
                          cudaStream_t stream) {
@@ -449,10 +449,8 @@ int step_until_embedding(const GfsBlockDims& d, const GfsBlockParams* layers, co
   rc = weight_grad(d, grp, logits, y, t.g_out, t.acc_out, T, V, H, launches, stream);
   if (rc == 0) rc = grp.flush(launches, stream, *launches == launched);
   if (rc != 0) return rc;
-  rc = gfs_blocks_backward(&d, layers, t.w_final, t.g_final, t.acc_final, x0, act, rstd, dy, scratch, dx0, launches,
-                           stream);
-  if (rc != 0) return rc;
-  return !t.acc_emb && cudaMemsetAsync(t.g_emb, 0, 2 * static_cast<size_t>(V) * H, stream) != cudaSuccess ? -11 : 0;
+  return gfs_blocks_backward(&d, layers, t.w_final, t.g_final, t.acc_final, x0, act, rstd, dy, scratch, dx0, launches,
+                             stream);
 }
 
 }  // namespace
@@ -484,7 +482,10 @@ int gfs_model_step(const GfsBlockDims* dp, const GfsBlockParams* layers, const G
   if (side == nullptr) return -10;
   if (cudaEventRecord(side->fork, st) != cudaSuccess || cudaStreamWaitEvent(side->stream, side->fork, 0) != cudaSuccess)
     return -11;
-  const int shift = gfs_embedding_sort_keys(ids, m + lay.keys, d.B, d.S, 0, t.V, side->stream);
+  int shift = gfs_embedding_sort_keys(ids, m + lay.keys, d.B, d.S, 0, t.V, side->stream);
+  if (shift >= 0 && !t.acc_emb &&
+      cudaMemsetAsync(t.g_emb, 0, 2 * static_cast<size_t>(t.V) * d.H, side->stream) != cudaSuccess)
+    shift = -11;
   if (cudaEventRecord(side->join, side->stream) != cudaSuccess) {
     cudaStreamSynchronize(side->stream);
     return -11;

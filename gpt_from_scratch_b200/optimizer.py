@@ -385,7 +385,7 @@ class DistributedOptimizer:
             adam_ops.sumsq_bf16(shard, self._sumsq[0:1])
             if self._rep_index_shard is not None and not self.reference_quirks:
                 self._sumsq[1] = shard.index_select(0, self._rep_index_shard).float().pow(2).sum()
-            else:
+            elif self.tp_world_size > 1:     # (with one rank nobody reads it)
                 self._sumsq[1:2].zero_()     # (a scalar assignment would be a host-to-device copy)
             sumsq = self._global_sumsq(self._sumsq)
         lr, beta1, beta2, eps, wd = self._hyper()
