@@ -16,7 +16,13 @@
 // Split K over a cluster of s CTAs: CTA r of the cluster owns rows [r * 128/s, +128/s) of the tile. Every
 // CTA writes the rows of its partial tile into their owners' staging areas (st.shared::cluster), one
 // cluster barrier, and the owner sums the s partials in rank order (deterministic) in its epilogue. The staging
-// area is s x (128/s) rows whatever s is.
+// area is s x (128/s) rows whatever s is. (Bulk copies out of the dead operand ring, counted on a barrier of the owner's,
+// instead of the threads' scattered stores: 6.0 against 5.3 us at 130 x 768 x 768, split 4.)
+//
+// A kernel of a few microseconds executes its code once, so what counts in the epilogue is how much of it there is: every
+// kind (EPI_*) is a variant of its own, and vectors past the end skip theirs. One epilogue for all kinds, six
+// vectors unrolled, took 3,700 of the 12,500 cycles of an unsplit 512 x 256 x 256 product for the 5 vectors of a thread.
+// us in a chain of products, that -> this: 512 x 256 x 256 5.5 -> 4.1, 130 x 768 x 768 unsplit 7.2 -> 5.8.
 //
 // Operand layouts, addend, rotary and SwiGLU epilogues as in gemm.cu; values are rounded once, from fp32.
 #include <algorithm>
@@ -33,6 +39,8 @@ constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int THREADS = 192;
 constexpr int MAX_GROUP = 4;
+// Epilogues: (+ addend) / SwiGLU forward / SwiGLU backward / rotary embedding (+ addend)
+enum Epi : int { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_SWIGLU_BWD = 2, EPI_ROPE = 3 };
 
 struct TileProblem {
   int M, N;
@@ -57,7 +65,7 @@ struct TileParams {
   const float* rope_cos;    // rotary embedding of the first rope_cols columns (see gemm.cu)
   const float* rope_sin;
   int rope_cols, rope_d, rope_b;
-  int swi_mode, swi_I, swi_ld;   // SwiGLU forward (1) / backward (2), as in gemm.cu
+  int swi_I, swi_ld;             // SwiGLU, as in gemm.cu
   __nv_bfloat16* swi_act;
   const __nv_bfloat16* swi_gu;
 };
@@ -92,21 +100,23 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 // The epilogue of one CTA, called by all its threads: rows [rank * rows_per_cta, ...) of the tile at (m0, n0)
 // are the sums of `split` fp32 slabs in `staging`. `sync` makes the slabs visible; the addends of the first
 // vectors are fetched before it, while the K loop still runs.
-template <int BN, int NT, int NG, typename Sync>
+template <int BN, int NT, int EPI, int NG, typename Sync>
 __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const TileProblem& g, const float* staging,
                                               int split, int rank, int m0, int n0, Sync sync) {
   constexpr int PITCH = BN + 4;   // floats per staging row: 16-byte chunks of consecutive rows hit different banks
   const int rows_per_cta = (BM + split - 1) / split;
   const int rows_here = min(BM, (rank + 1) * rows_per_cta) - rank * rows_per_cta;
   const int row_base = m0 + rank * rows_per_cta;
-  if (p.swi_mode == 1) {
+  if constexpr (EPI == EPI_SWIGLU) {
     constexpr int VPR = BN / 16;   // vectors of gate columns per row
     sync();
+#pragma unroll 1
     for (int v = threadIdx.x; v < rows_here * VPR; v += NT) {
       const int lr = v / VPR, c = (v % VPR) * 8;
       const int row = row_base + lr, col = (n0 >> 1) + c;
       if (row >= g.M || col + 8 > p.swi_I) continue;
       float gt[8] = {0, 0, 0, 0, 0, 0, 0, 0}, up[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 1
       for (int r = 0; r < split; ++r) {
         const float* src = staging + (r * rows_per_cta + lr) * PITCH + c;
 #pragma unroll
@@ -127,12 +137,11 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
       *reinterpret_cast<uint4*>(dst + p.swi_I) = wu;
       *reinterpret_cast<uint4*>(p.swi_act + static_cast<size_t>(row) * p.swi_ld + col) = pack8(a);
     }
-    return;
-  }
+  } else {
   constexpr int VPR = BN / 8;
   constexpr int NPRE = 6;        // vectors of a thread whose addend is fetched early
   uint4 pre[NPRE];
-  const bool has_add = g.R != nullptr;
+  const bool has_add = EPI != EPI_SWIGLU_BWD && g.R != nullptr;
   if (has_add) {
 #pragma unroll
     for (int i = 0; i < NPRE; ++i) {
@@ -150,13 +159,14 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
     const int row = row_base + lr, col = n0 + c;
     if (lr >= rows_here || row >= g.M || col + 8 > g.N) return;
     float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 1
     for (int r = 0; r < split; ++r) {
       const float4* src = reinterpret_cast<const float4*>(staging + (r * rows_per_cta + lr) * PITCH + c);
       const float4 a = src[0], b = src[1];
       f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
       f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
     }
-    if (p.swi_mode == 2) {
+    if constexpr (EPI == EPI_SWIGLU_BWD) {
       // f holds d_act; turn it into d_gate and d_up
       const __nv_bfloat16* gp = p.swi_gu + static_cast<size_t>(row) * p.swi_ld + col;
       float gt[8], up[8], dg[8], du[8];
@@ -173,7 +183,7 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
       *reinterpret_cast<uint4*>(dst + p.swi_I) = pack8(du);
       return;
     }
-    if (p.rope_cos != nullptr && col < p.rope_cols) {
+    if (EPI == EPI_ROPE && col < p.rope_cols) {
       const size_t ti = static_cast<size_t>(row / p.rope_b) * (p.rope_d >> 1) + ((col % p.rope_d) >> 1);
       const float4 cs = *reinterpret_cast<const float4*>(p.rope_cos + ti);
       const float4 sn = *reinterpret_cast<const float4*>(p.rope_sin + ti);
@@ -191,11 +201,19 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
     }
     *reinterpret_cast<uint4*>(g.C + static_cast<size_t>(row) * g.ldc + col) = pack8(f);
   };
+  const int n_vec = rows_here * VPR;
+  int v = threadIdx.x;
+  if (has_add) {
 #pragma unroll
-  for (int i = 0; i < NPRE; ++i) finish(threadIdx.x + i * NT, true, pre[i]);
+    for (int i = 0; i < NPRE; ++i, v += NT) {
+      if (v >= n_vec) return;
+      finish(v, true, pre[i]);
+    }
+  }
   const uint4 none = make_uint4(0, 0, 0, 0);
-#pragma unroll 2
-  for (int v = threadIdx.x + NPRE * NT; v < rows_here * VPR; v += NT) finish(v, false, none);
+#pragma unroll 1
+  for (; v < n_vec; v += NT) finish(v, false, none);
+  }
 }
 
 // One accumulator row (this lane's) from tensor memory to the staging area of the CTA that owns it. `owner`:
@@ -229,7 +247,7 @@ __device__ __forceinline__ void stage_row(uint32_t t_row, float* staging, int sl
   }
 }
 
-template <bool A_MN, bool B_MN, int BN, int NG>
+template <bool A_MN, bool B_MN, int BN, int NG, int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constant__ TileParams<NG> p) {
   using C_ = Cfg<BN>;
@@ -295,7 +313,7 @@ gemm_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constan
       auto load_b = [&](int stage, int k0) {
         uint8_t* sb = tiles + stage * C_::STAGE_BYTES + C_::A_BYTES;
         if (!B_MN) {
-          if (p.swi_mode == 1) {   // BN/2 gate rows + the matching up rows (tensor map box = BN/2 rows)
+          if (EPI == EPI_SWIGLU) {   // BN/2 gate rows + the matching up rows (tensor map box = BN/2 rows)
             tma_load_2d(sb, &maps.b[gi], &full_bar[stage], k0, n0 >> 1);
             tma_load_2d(sb + (BN / 2) * 128, &maps.b[gi], &full_bar[stage], k0, p.swi_I + (n0 >> 1));
           } else {
@@ -366,7 +384,7 @@ gemm_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constan
     tc_fence_before();
   }
 
-  tile_epilogue<BN, THREADS>(p, g, staging, split, rank, m0, n0, [&]() {
+  tile_epilogue<BN, THREADS, EPI>(p, g, staging, split, rank, m0, n0, [&]() {
     if (split > 1) cluster_sync();
     else __syncthreads();
   });
@@ -392,7 +410,7 @@ constexpr int PAIR_THREADS = 320;   // TMA, MMA, eight warps that drain the accu
 constexpr int PAIR_TOTAL = PAIR_STAGES * PAIR_STAGE_BYTES + 256 + 1024;
 static_assert((BM + 1) * 260 * 4 <= PAIR_STAGES * PAIR_STAGE_BYTES, "staging fits the ring");
 
-template <bool A_MN, bool B_MN, int NG>
+template <bool A_MN, bool B_MN, int NG, int EPI>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constant__ TileParams<NG> p) {
   constexpr int BN = 256, BNH = 128, PITCH = BN + 4;
@@ -465,7 +483,7 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
         const uint32_t bar = mapa_u32(smem_u32(&full_bar[stage]), lead);
         if (!B_MN) {
           // SwiGLU forward: 128 gate rows for the leader, the matching up rows for the other CTA
-          tma_load_2d_pair(sb, &maps.b[gi], bar, k0, p.swi_mode == 1 ? half * p.swi_I + (n0 >> 1) : nb);
+          tma_load_2d_pair(sb, &maps.b[gi], bar, k0, EPI == EPI_SWIGLU ? half * p.swi_I + (n0 >> 1) : nb);
         } else {
 #pragma unroll
           for (int j = 0; j < 2; ++j) tma_load_2d_pair(sb + j * 8192, &maps.b[gi], bar, nb + 64 * j, k0);
@@ -541,7 +559,7 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
                      row - owner * rows_per_cta, split > 1, static_cast<uint32_t>(2 * owner + half), c0, c0 + BNH);
     tc_fence_before();
   }
-  tile_epilogue<BN, PAIR_THREADS>(p, g, staging, split, z, m0, n0, [&]() {
+  tile_epilogue<BN, PAIR_THREADS, EPI>(p, g, staging, split, z, m0, n0, [&]() {
     if (split > 1) cluster_sync();
     else __syncthreads();
   });
@@ -583,17 +601,26 @@ int launch_clustered(Kern kern, int threads, int smem, int cluster, const Maps& 
   return cudaLaunchKernelEx(&cfg, kern, maps, p) == cudaSuccess ? 0 : -11;
 }
 
-template <bool A_MN, bool B_MN, int NG>
+template <bool A_MN, bool B_MN, int NG, int EPI>
 int launch_tile(int bn, const TileMaps<NG>& maps, const TileParams<NG>& p, int ctas, cudaStream_t stream) {
   static bool set64[64] = {}, set128[64] = {}, set256[64] = {};
   if (bn == 64)
-    return launch_clustered(gemm_tile_kernel<A_MN, B_MN, 64, NG>, THREADS, Cfg<64>::TOTAL, p.split, maps, p, ctas, stream,
-                            set64);
+    return launch_clustered(gemm_tile_kernel<A_MN, B_MN, 64, NG, EPI>, THREADS, Cfg<64>::TOTAL, p.split, maps, p, ctas,
+                            stream, set64);
   if (bn == 128)
-    return launch_clustered(gemm_tile_kernel<A_MN, B_MN, 128, NG>, THREADS, Cfg<128>::TOTAL, p.split, maps, p, ctas,
+    return launch_clustered(gemm_tile_kernel<A_MN, B_MN, 128, NG, EPI>, THREADS, Cfg<128>::TOTAL, p.split, maps, p, ctas,
                             stream, set128);
-  return launch_clustered(gemm_pair_tile_kernel<A_MN, B_MN, NG>, PAIR_THREADS, PAIR_TOTAL, 2 * p.split, maps, p, 2 * ctas,
-                          stream, set256);
+  return launch_clustered(gemm_pair_tile_kernel<A_MN, B_MN, NG, EPI>, PAIR_THREADS, PAIR_TOTAL, 2 * p.split, maps, p,
+                          2 * ctas, stream, set256);
+}
+
+template <int EPI>
+int launch_layout(int a_mn, int b_mn, int bn, const TileMaps<1>& maps, const TileParams<1>& p, int ctas,
+                  cudaStream_t stream) {
+  if (!a_mn) return b_mn ? launch_tile<false, true, 1, EPI>(bn, maps, p, ctas, stream)
+                         : launch_tile<false, false, 1, EPI>(bn, maps, p, ctas, stream);
+  return b_mn ? launch_tile<true, true, 1, EPI>(bn, maps, p, ctas, stream)
+              : launch_tile<true, false, 1, EPI>(bn, maps, p, ctas, stream);
 }
 
 // Splits 5 to 7 round the rows of a CTA up so far that `split` slabs of them exceed the staging area's 129 rows.
@@ -643,7 +670,7 @@ int gfs_gemm_tile(const void* A, const void* B, void* C, const void* R, int M, i
   p.rope_cos = static_cast<const float*>(rope_cos);
   p.rope_sin = static_cast<const float*>(rope_sin);
   p.rope_cols = rope_cols; p.rope_d = rope_d; p.rope_b = rope_b > 0 ? rope_b : 1;
-  p.swi_mode = swi_mode; p.swi_I = N; p.swi_ld = swi_ld;
+  p.swi_I = N; p.swi_ld = swi_ld;
   if (swi_mode == 1) p.swi_act = static_cast<__nv_bfloat16*>(swi_extra);
   if (swi_mode == 2) p.swi_gu = static_cast<const __nv_bfloat16*>(swi_extra);
   TileProblem& g = p.g[0];
@@ -659,10 +686,10 @@ int gfs_gemm_tile(const void* A, const void* B, void* C, const void* R, int M, i
   g.R = static_cast<const __nv_bfloat16*>(R);
   const int bm = bn == 256 ? 256 : BM;
   const int ctas = (M + bm - 1) / bm * g.tiles_n * split;
-  if (!a_mn_major) return b_mn_major ? launch_tile<false, true, 1>(bn, maps, p, ctas, stream)
-                                     : launch_tile<false, false, 1>(bn, maps, p, ctas, stream);
-  return b_mn_major ? launch_tile<true, true, 1>(bn, maps, p, ctas, stream)
-                    : launch_tile<true, false, 1>(bn, maps, p, ctas, stream);
+  if (swi_mode == 1) return launch_tile<false, false, 1, EPI_SWIGLU>(bn, maps, p, ctas, stream);
+  if (swi_mode == 2) return launch_tile<false, true, 1, EPI_SWIGLU_BWD>(bn, maps, p, ctas, stream);
+  return rope_cos != nullptr ? launch_layout<EPI_ROPE>(a_mn_major, b_mn_major, bn, maps, p, ctas, stream)
+                             : launch_layout<EPI_PLAIN>(a_mn_major, b_mn_major, bn, maps, p, ctas, stream);
 }
 
 // Grouped weight gradients with this kernel: same contract as gfs_gemm2_wgrad_grouped.
@@ -711,7 +738,7 @@ int gfs_gemm_tile_wgrad_grouped(int n, const unsigned long long* A, const unsign
     p.g[i].tile_begin = INT_MAX;
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  return launch_tile<true, true, MAX_GROUP>(bn, maps, p, total * split, stream);
+  return launch_tile<true, true, MAX_GROUP, EPI_PLAIN>(bn, maps, p, total * split, stream);
 }
 
 }  // extern "C"
