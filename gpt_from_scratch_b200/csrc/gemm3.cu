@@ -22,7 +22,10 @@
 // A kernel of a few microseconds executes its code once, so what counts in the epilogue is how much of it there is: every
 // kind (EPI_*) is a variant of its own, and vectors past the end skip theirs. One epilogue for all kinds, six
 // vectors unrolled, took 3,700 of the 12,500 cycles of an unsplit 512 x 256 x 256 product for the 5 vectors of a thread.
-// us in a chain of products, that -> this: 512 x 256 x 256 5.5 -> 4.1, 130 x 768 x 768 unsplit 7.2 -> 5.8.
+// us in a chain of products, that -> this: 512 x 256 x 256 5.5 -> 4.1, 130 x 768 x 768 unsplit 7.2 -> 5.8. What
+// an epilogue reads (addend, rotation table, gate and up) is fetched six vectors at a time, the first six before the
+// accumulator is ready; read where it is used, each vector waited for memory: 1040 x 768 x 768 with the SwiGLU gradient
+// 9.0 -> 7.1, with the rotation 8.2 -> 7.0.
 //
 // Operand layouts, addend, rotary and SwiGLU epilogues as in gemm.cu; values are rounded once, from fp32.
 #include <algorithm>
@@ -139,24 +142,36 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
     }
   } else {
   constexpr int VPR = BN / 8;
-  constexpr int NPRE = 6;        // vectors of a thread whose addend is fetched early
-  uint4 pre[NPRE];
+  constexpr int NPRE = 6;        // vectors of a thread whose operands are fetched together, the first before the wait
+  constexpr bool TABLE = EPI == EPI_SWIGLU_BWD || EPI == EPI_ROPE;
+  uint4 pre[NPRE], aux[TABLE ? NPRE : 1], aux2[TABLE ? NPRE : 1];   // addend; gate and up, or cos and sin
   const bool has_add = EPI != EPI_SWIGLU_BWD && g.R != nullptr;
-  if (has_add) {
+  static_assert(NT % VPR == 0, "a thread's vectors lie in the same columns");
+  const int c = (threadIdx.x % VPR) * 8, col = n0 + c;
+  const int rope_col = EPI == EPI_ROPE ? (col % p.rope_d) >> 1 : 0;
+  auto fetch = [&](int v0) {
 #pragma unroll
     for (int i = 0; i < NPRE; ++i) {
-      const int v = threadIdx.x + i * NT;
-      const int lr = v / VPR, c = (v % VPR) * 8;
-      const int row = row_base + lr, col = n0 + c;
-      pre[i] = make_uint4(0, 0, 0, 0);
-      if (lr < rows_here && row < g.M && col + 8 <= g.N)
-        pre[i] = *reinterpret_cast<const uint4*>(g.R + static_cast<size_t>(row) * g.ldr + col);
+      const int lr = v0 / VPR + i * (NT / VPR), row = row_base + lr;
+      if (lr >= rows_here || row >= g.M || col + 8 > g.N) continue;
+      if (has_add) pre[i] = *reinterpret_cast<const uint4*>(g.R + static_cast<size_t>(row) * g.ldr + col);
+      if constexpr (EPI == EPI_SWIGLU_BWD) {
+        const __nv_bfloat16* gp = p.swi_gu + static_cast<size_t>(row) * p.swi_ld + col;
+        aux[i] = *reinterpret_cast<const uint4*>(gp);
+        aux2[i] = *reinterpret_cast<const uint4*>(gp + p.swi_I);
+      }
+      if (EPI == EPI_ROPE && col < p.rope_cols) {
+        const size_t ti = static_cast<size_t>(row / p.rope_b) * (p.rope_d >> 1) + rope_col;
+        aux[i] = *reinterpret_cast<const uint4*>(p.rope_cos + ti);
+        aux2[i] = *reinterpret_cast<const uint4*>(p.rope_sin + ti);
+      }
     }
-  }
+  };
+  const bool fetches = TABLE || has_add;
+  if (fetches) fetch(threadIdx.x);
   sync();
-  auto finish = [&](int v, bool have_pre, const uint4& addend) {
-    const int lr = v / VPR, c = (v % VPR) * 8;
-    const int row = row_base + lr, col = n0 + c;
+  auto finish = [&](int v, const uint4& addend, const uint4& t0, const uint4& t1) {
+    const int lr = v / VPR, row = row_base + lr;
     if (lr >= rows_here || row >= g.M || col + 8 > g.N) return;
     float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll 1
@@ -168,10 +183,9 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
     }
     if constexpr (EPI == EPI_SWIGLU_BWD) {
       // f holds d_act; turn it into d_gate and d_up
-      const __nv_bfloat16* gp = p.swi_gu + static_cast<size_t>(row) * p.swi_ld + col;
       float gt[8], up[8], dg[8], du[8];
-      unpack8(*reinterpret_cast<const uint4*>(gp), gt);
-      unpack8(*reinterpret_cast<const uint4*>(gp + p.swi_I), up);
+      unpack8(t0, gt);
+      unpack8(t1, up);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float sg = sigmoid_f(gt[e]);
@@ -184,9 +198,8 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
       return;
     }
     if (EPI == EPI_ROPE && col < p.rope_cols) {
-      const size_t ti = static_cast<size_t>(row / p.rope_b) * (p.rope_d >> 1) + ((col % p.rope_d) >> 1);
-      const float4 cs = *reinterpret_cast<const float4*>(p.rope_cos + ti);
-      const float4 sn = *reinterpret_cast<const float4*>(p.rope_sin + ti);
+      const float4 cs = make_float4(__uint_as_float(t0.x), __uint_as_float(t0.y), __uint_as_float(t0.z), __uint_as_float(t0.w));
+      const float4 sn = make_float4(__uint_as_float(t1.x), __uint_as_float(t1.y), __uint_as_float(t1.z), __uint_as_float(t1.w));
       const float a0 = f[0], a1 = f[1], a2 = f[2], a3 = f[3], a4 = f[4], a5 = f[5], a6 = f[6], a7 = f[7];
       f[0] = a0 * cs.x - a1 * sn.x; f[1] = a0 * sn.x + a1 * cs.x;
       f[2] = a2 * cs.y - a3 * sn.y; f[3] = a2 * sn.y + a3 * cs.y;
@@ -195,7 +208,7 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
     }
     if (has_add) {
       float r8[8];
-      unpack8(have_pre ? addend : *reinterpret_cast<const uint4*>(g.R + static_cast<size_t>(row) * g.ldr + col), r8);
+      unpack8(addend, r8);
 #pragma unroll
       for (int e = 0; e < 8; ++e) f[e] += r8[e];
     }
@@ -203,16 +216,22 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
   };
   const int n_vec = rows_here * VPR;
   int v = threadIdx.x;
-  if (has_add) {
+  if (!fetches) {
+    const uint4 none = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+    for (; v < n_vec; v += NT) finish(v, none, none, none);
+    return;
+  }
+#pragma unroll 1
+  while (true) {
 #pragma unroll
     for (int i = 0; i < NPRE; ++i, v += NT) {
       if (v >= n_vec) return;
-      finish(v, true, pre[i]);
+      finish(v, pre[i], aux[TABLE ? i : 0], aux2[TABLE ? i : 0]);
     }
+    if (v >= n_vec) return;
+    fetch(v);
   }
-  const uint4 none = make_uint4(0, 0, 0, 0);
-#pragma unroll 1
-  for (; v < n_vec; v += NT) finish(v, false, none);
   }
 }
 
