@@ -6,8 +6,13 @@
 //
 // From `pair_min_tiles` (60) tiles of 256 x 256 on, the persistent pairs always win. Below, a product is mostly one
 // wave of whatever kernel runs it, and its time is a constant (launch, first TMA, epilogue) plus the K blocks
-// one CTA works through. The constants below were fitted to 110 measured (shape, kernel) pairs on B200: M 103 to
-// 4096, N 256 to 50304, K 103 to 50304, every layout, back to back in a CUDA graph; the fits are within 15 %.
+// one CTA works through. The constants of the persistent kernels were fitted to 110 measured (shape, kernel) pairs on
+// B200: M 103 to 4096, N 256 to 50304, K 103 to 50304, every layout, back to back in a CUDA graph; the fits are within 15 %.
+// Those of the tiles were fitted again when their epilogues had become shorter: M 64 to 2331, N 128 to 3072, K 256 to 4096,
+// every epilogue, and weight gradients over 130 to 8192 rows, each with every tile and split that fits one wave. Of 142 products
+// 7 are more than 4 % slower than the best of their tiles, the worst 6 %, by 0.3 us; with the constants before, unsplit 128 x 128 tiles
+// lost to the persistent kernel (512 x 3072 x 768 8.7 us there, 7.0 as tiles; 2331 x 768 x 3072 18.5 and 15.1) and small
+// K was split (512 x 1024 x 256 4.3 us split in two, 3.9 whole). A step of two blocks of hidden 256 as a graph: 210 -> 201 us.
 // us per launch, before (persistent kernels, K split through a workspace and a second launch) -> with this rule:
 // 512 x 768 x 256 with rotary epilogue 16.5 -> 5.5, 130 x 768 x 3072 with addend 18.6 -> 7.7,
 // 2048 x 768 x 2304 21.4 -> 16.3, weight gradient 768 x 768 x 2331 20.8 -> 9.8.
@@ -36,20 +41,24 @@ int wave_of_clusters(int c) {
   }
 }
 
+// What a tile's epilogue does beside storing the sums (gemm3.cu)
+enum Extra { NONE = 0, ADDEND = 1, ROTATION = 2, SWIGLU = 3, SWIGLU_GRAD = 4 };
+
 struct TileShape {
   int bn;               // columns of the tile
   int cluster;          // CTAs per tile without a split
-  float base, per_kblock, split_cost;
+  float base, per_kblock, split_base, split_cost;   // a split over s CTAs costs split_base + s * split_cost
+  float extra[5];       // by Extra, for a whole tile; a CTA of a split tile does its share of the rows
 };
 constexpr TileShape kShapes[3] = {
-    {64, 1, 4.2f, 0.21f, 0.4f},     // 96 cycles per MMA (A and B read for 64 columns), 64-column epilogue
-    {128, 1, 6.3f, 0.265f, 0.7f},   // 128 cycles per MMA: shared-memory reads
-    {256, 2, 8.2f, 0.29f, 2.6f},    // tensor-bound, but 256 columns per row in the epilogue
+    {64, 1, 3.0f, 0.21f, 0.0f, 0.25f, {0.f, 0.2f, 1.3f, 0.6f, 1.2f}},   // 96 cycles per MMA (A and B read for 64 columns)
+    {128, 1, 4.0f, 0.225f, 0.5f, 0.3f, {0.f, 0.55f, 3.2f, 1.1f, 2.45f}},   // 128 cycles per MMA: shared-memory reads
+    {256, 2, 5.5f, 0.28f, 1.0f, 0.8f, {0.f, 0.85f, 4.4f, 1.2f, 3.5f}},     // tensor-bound, 256 columns per row to store
 };
 
 // Best one-wave tile for `tiles(bn)` tiles of 128 (bn = 256: 256) rows. us, or a huge number if none fits.
 template <typename Tiles>
-float best_tile(Tiles tiles, int kblocks, bool pairs, Choice* c) {
+float best_tile(Tiles tiles, int kblocks, bool pairs, Extra extra, Choice* c) {
   float best = 1e30f;
   for (const TileShape& s : kShapes) {
     if (s.bn == 256 && !pairs) continue;
@@ -60,7 +69,8 @@ float best_tile(Tiles tiles, int kblocks, bool pairs, Choice* c) {
       if (per * (split - 1) >= kblocks) break;              // a CTA without K blocks
       const int cluster = s.cluster * split;
       if (n * cluster > wave_of_clusters(cluster)) break;
-      const float t = s.base + s.per_kblock * per + (split > 1 ? s.split_cost : 0.f);
+      float t = s.base + s.per_kblock * per + s.extra[extra] / split;
+      if (split > 1) t += s.split_base + s.split_cost * split + (extra != NONE ? 0.3f : 0.f);
       if (t < best) {
         best = t;
         *c = Choice{Choice::TILE, s.bn, split};
@@ -82,7 +92,8 @@ Choice choose(int M, int N, int K, int swi_mode, bool add, bool rope, int pair_m
   const bool pairs = pair_min_tiles >= 0, plain = swi_mode == 0 && !add && !rope;
   if (pairs && (K >= 256 || swi_mode != 0) && tiles(256) >= pair_min_tiles) return Choice{Choice::PERSISTENT_PAIR, 256, 1};
   Choice c{Choice::PERSISTENT_CTA, 256, 1};
-  const float t_tile = best_tile(tiles, kb, pairs, &c);
+  const Extra extra = swi_mode == 1 ? SWIGLU : swi_mode == 2 ? SWIGLU_GRAD : rope ? ROTATION : add ? ADDEND : NONE;
+  const float t_tile = best_tile(tiles, kb, pairs, extra, &c);
   // persistent CTAs: 128 x 256 tiles in waves; the addend, the rotation and the SwiGLU gradient are serial
   // loads in its epilogue. Plain products of up to 128 columns have 128-column tiles and half the epilogue there. Judged
   // by the same line, 27 of 129 measured ones went to kernels more than 5 % slower than the persistent one; with
@@ -164,7 +175,7 @@ int gfs_wgrad_grouped(int n, const unsigned long long* A, const unsigned long lo
   const float t_pair = 6.5f + 0.3f * kb * ceil_div(tiles(256), 74);
   // Unsplit 256 x 256 tiles on pairs are that kernel's tiles without its persistence: 95 us instead of 86 for the
   // three small gradients of a block at 16384 tokens (hidden 768, FFN 3072).
-  if (kb == kb_min && best_tile(tiles, kb, true, &c) < t_pair && c.kernel == Choice::TILE && (c.bn != 256 || c.split > 1))
+  if (kb == kb_min && best_tile(tiles, kb, true, NONE, &c) < t_pair && c.kernel == Choice::TILE && (c.bn != 256 || c.split > 1))
     return gfs_gemm_tile_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, accumulate, c.bn, c.split, stream);
   return gfs_gemm2_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, accumulate, stream);
 }
