@@ -9,8 +9,8 @@
 // one CTA works through. The constants of the persistent kernels were fitted to 110 measured (shape, kernel) pairs on
 // B200: M 103 to 4096, N 256 to 50304, K 103 to 50304, every layout, back to back in a CUDA graph; the fits are within 15 %.
 // Those of the tiles were fitted again when their epilogues had become shorter: M 64 to 2331, N 128 to 3072, K 256 to 4096,
-// every epilogue, and weight gradients over 130 to 8192 rows, each with every tile and split that fits one wave. Of 142 products
-// 7 are more than 4 % slower than the best of their tiles, the worst 6 %, by 0.3 us; with the constants before, unsplit 128 x 128 tiles
+// every epilogue, and weight gradients over 130 to 8192 rows, each with every tile and split that fits one wave. Of 188
+// choices four are more than 4.5 % slower than the best tile, none of those by more than 1.1 us; with the constants before, unsplit 128 x 128 tiles
 // lost to the persistent kernel (512 x 3072 x 768 8.7 us there, 7.0 as tiles; 2331 x 768 x 3072 18.5 and 15.1) and small
 // K was split (512 x 1024 x 256 4.3 us split in two, 3.9 whole). A step of two blocks of hidden 256 as a graph: 210 -> 201 us.
 // us per launch, before (persistent kernels, K split through a workspace and a second launch) -> with this rule:
