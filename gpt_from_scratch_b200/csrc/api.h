@@ -33,6 +33,10 @@ int gfs_wgrad_grouped(int n, const unsigned long long* A, const unsigned long lo
                       const int* M, const int* N, const int* K, const int* lda, const int* ldb, const int* ldc,
                       const int* accumulate, void* stream);
 int gfs_rmsnorm_fwd(const void* x, const void* w, void* y, void* rstd, int rows, int H, float eps, void* stream);
+int gfs_dropout_residual_norm(const void* z, const void* residual, void* x, const void* w, void* y, void* rstd, int rows,
+                              int H, float eps, float p, unsigned long long seed, void* stream);
+int gfs_rmsnorm_bwd_dropout(const void* dy, const void* x, const void* w, const void* rstd, const void* dres, void* dx,
+                            void* dmask, void* partial, int rows, int H, float p, unsigned long long seed, void* stream);
 int gfs_rmsnorm_bwd_parts(int rows);
 int gfs_rmsnorm_bwd(const void* dy, const void* x, const void* w, const void* rstd, const void* dres, void* dx,
                     void* dw, void* partial, int rows, int H, int accumulate_dw, void* stream);

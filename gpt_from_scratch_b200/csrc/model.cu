@@ -195,7 +195,6 @@ int gfs_blocks_forward(const GfsBlockDims* dp, const GfsBlockParams* layers, con
   if (!dims_ok(d)) return -1;
   const ActLayout a(d);
   const int T = d.S * d.B, H = d.H, I = d.I;
-  const long long n_el = static_cast<long long>(T) * H;
   const float scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(d.D)));
   const bool drop = d.dropout_p > 0.f;
   const long long tok = 3ll * H;   // a token of the packed [S, B, 3, nh, D] projection
@@ -207,7 +206,7 @@ int gfs_blocks_forward(const GfsBlockDims* dp, const GfsBlockParams* layers, con
     void *y1 = base + a.y1, *rstd1 = base + a.rstd1, *attn = base + a.attn, *lse = base + a.lse, *x1 = base + a.x1,
          *y2 = base + a.y2, *rstd2 = base + a.rstd2, *gu = base + a.gu, *ac = base + a.act, *x2 = base + a.x2;
     char* qkv = base + a.qkv;
-    GFS_TRY(gfs_rmsnorm_fwd(x, p.w[W_NORM1], y1, rstd1, T, H, p.eps[0], stream));
+    if (!drop || l == 0) GFS_TRY(gfs_rmsnorm_fwd(x, p.w[W_NORM1], y1, rstd1, T, H, p.eps[0], stream));
     const gfs_host::WithHints hints(true, false);   // (of the products; B is a weight)
     GFS_TRY(gfs_linear(y1, p.w[W_QKV], qkv, nullptr, T, 3 * H, H, H, H, 3 * H, 0, 0, 0, p.cos_table, p.sin_table, 2 * H,
                        d.D, d.B, d.pair_min_tiles, stream));   // q and k leave rotated
@@ -217,19 +216,25 @@ int gfs_blocks_forward(const GfsBlockDims* dp, const GfsBlockParams* layers, con
       GFS_TRY(product(d, attn, p.w[W_OUT], x1, x, T, H, H, H, H, H, 0, 0, stream));
     } else {
       GFS_TRY(product(d, attn, p.w[W_OUT], tmp, nullptr, T, H, H, H, H, H, 0, 0, stream));
-      GFS_TRY(gfs_dropout_residual(tmp, x, x1, n_el, d.dropout_p, p.seed[0], 0, stream));
+      GFS_TRY(gfs_dropout_residual_norm(tmp, x, x1, p.w[W_NORM2], y2, rstd2, T, H, p.eps[1], d.dropout_p, p.seed[0],
+                                        stream));
     }
-    GFS_TRY(gfs_rmsnorm_fwd(x1, p.w[W_NORM2], y2, rstd2, T, H, p.eps[1], stream));
+    if (!drop) GFS_TRY(gfs_rmsnorm_fwd(x1, p.w[W_NORM2], y2, rstd2, T, H, p.eps[1], stream));
     GFS_TRY(gfs_linear_swiglu(1, y2, p.w[W_GATE_UP], gu, ac, T, I, H, H, H, 2 * I, I, d.pair_min_tiles, stream));
     if (!drop) {
       GFS_TRY(product(d, ac, p.w[W_DOWN], x2, x1, T, H, I, I, I, H, 0, 0, stream));
     } else {
       GFS_TRY(product(d, ac, p.w[W_DOWN], tmp, nullptr, T, H, I, I, I, H, 0, 0, stream));
-      GFS_TRY(gfs_dropout_residual(tmp, x1, x2, n_el, d.dropout_p, p.seed[1], 0, stream));
+      // with the next block's first norm, or the final one
+      const bool last = l + 1 == d.n_layers;
+      char* next = last ? nullptr : reinterpret_cast<char*>(act[l + 1]);
+      GFS_TRY(gfs_dropout_residual_norm(tmp, x1, x2, last ? w_final : layers[l + 1].w[W_NORM1],
+                                        last ? y_final : next + a.y1, last ? rstd_final : next + a.rstd1, T, H,
+                                        last ? d.eps_final : layers[l + 1].eps[0], d.dropout_p, p.seed[1], stream));
     }
     x = x2;
   }
-  GFS_TRY(gfs_rmsnorm_fwd(x, w_final, y_final, rstd_final, T, H, d.eps_final, stream));
+  if (!drop || d.n_layers == 0) GFS_TRY(gfs_rmsnorm_fwd(x, w_final, y_final, rstd_final, T, H, d.eps_final, stream));
   return 0;
 }
 
@@ -272,9 +277,16 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
     return rc;
   };
   auto norm_bwd = [&](const void* dyp, const void* xp, const void* w, const void* rstd, const void* dres, void* dxp,
-                      void* g, int acc) -> int {
+                      void* g, int acc, void* masked, u64 seed) -> int {
     void* part = s + b.partial + b.partial_stride * n_partial++;
-    int rc = gfs_rmsnorm_bwd(dyp, xp, w, rstd, dres, dxp, nullptr, part, T, H, 0, stream);
+    int rc = masked != nullptr ? gfs_rmsnorm_bwd_dropout(dyp, xp, w, rstd, dres, dxp, masked, part, T, H, d.dropout_p,
+                                                         seed, stream)
+                               : gfs_rmsnorm_bwd(dyp, xp, w, rstd, dres, dxp, nullptr, part, T, H, 0, stream);
+    if (rc == 1) {
+      rc = gfs_rmsnorm_bwd(dyp, xp, w, rstd, dres, dxp, nullptr, part, T, H, 0, stream);
+      if (rc == 0) rc = gfs_dropout_residual(dxp, nullptr, masked, n_el, d.dropout_p, seed, 1, stream);
+      ++*launches;
+    }
     if (rc != 0) return rc;
     red_p[n_red] = reinterpret_cast<u64>(part);
     red_g[n_red] = reinterpret_cast<u64>(g);
@@ -288,7 +300,11 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
   };
   // gradient of the current block's output; the two buffers alternate
   void* dout = d.n_layers == 0 ? dx : s + b.dx[d.n_layers & 1];
-  GFS_TRY(norm_bwd(dy_final, input_of(d.n_layers), w_final, rstd_final, nullptr, dout, g_final, accumulate_final));
+  // with dropout: the gradients of the MLP's and of the attention's output, masked where dout and dx1 are written
+  void* m_mlp = drop && d.n_layers > 0 ? s + b.dmask : nullptr;
+  void* m_attn = drop ? s + b.dmask + align256(2 * static_cast<size_t>(n_el)) : nullptr;
+  GFS_TRY(norm_bwd(dy_final, input_of(d.n_layers), w_final, rstd_final, nullptr, dout, g_final, accumulate_final, m_mlp,
+                   m_mlp ? layers[d.n_layers - 1].seed[1] : 0));
   for (int l = d.n_layers - 1; l >= 0; --l) {
     const GfsBlockParams& p = layers[l];
     const char* base = reinterpret_cast<const char*>(act[l]);
@@ -297,11 +313,7 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
     const char* qkv = base + a.qkv;
     WgradGroup grp;
     // gradient of the MLP's output
-    const void* dm = dout;
-    if (drop) {
-      GFS_TRY(gfs_dropout_residual(dout, nullptr, s + b.dmask, n_el, d.dropout_p, p.seed[1], 1, stream));
-      dm = s + b.dmask;
-    }
+    const void* dm = drop ? m_mlp : dout;
     {
       const gfs_host::WithHints hints(true, false);
       GFS_TRY(gfs_linear_swiglu(2, dm, p.w[W_DOWN], dgu, const_cast<void*>(gu), T, I, H, H, I, 2 * I, 2 * I,
@@ -312,14 +324,10 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
     GFS_TRY(product(d, dgu, p.w[W_GATE_UP], dy, nullptr, T, H, 2 * I, 2 * I, H, H, 0, 1, stream));
     rc = weight_grad(d, grp, dgu, y2, p.g[W_GATE_UP], p.accumulate[W_GATE_UP], T, 2 * I, H, launches, stream);
     if (rc != 0) return rc;
-    GFS_TRY(norm_bwd(dy, x1, p.w[W_NORM2], rstd2, dout, dx1, p.g[W_NORM2], p.accumulate[W_NORM2]));
+    GFS_TRY(norm_bwd(dy, x1, p.w[W_NORM2], rstd2, dout, dx1, p.g[W_NORM2], p.accumulate[W_NORM2], m_attn,
+                     p.seed[0]));
     // attention
-    const void* da = dx1;
-    if (drop) {
-      void* m = s + b.dmask + align256(2 * static_cast<size_t>(n_el));
-      GFS_TRY(gfs_dropout_residual(dx1, nullptr, m, n_el, d.dropout_p, p.seed[0], 1, stream));
-      da = m;
-    }
+    const void* da = drop ? m_attn : dx1;
     GFS_TRY(product(d, da, p.w[W_OUT], dattn, nullptr, T, H, H, H, H, H, 0, 1, stream));
     rc = weight_grad(d, grp, da, attn, p.g[W_OUT], p.accumulate[W_OUT], T, H, H, launches, stream);
     if (rc != 0) return rc;
@@ -334,7 +342,8 @@ int gfs_blocks_backward(const GfsBlockDims* dp, const GfsBlockParams* layers, co
     rc = grp.flush(launches, stream, *launches == launched);   // its operands are overwritten by the next block
     if (rc != 0) return rc;
     void* dnext = l == 0 ? dx : s + b.dx[l & 1];
-    GFS_TRY(norm_bwd(dy, input_of(l), p.w[W_NORM1], rstd1, dx1, dnext, p.g[W_NORM1], p.accumulate[W_NORM1]));
+    GFS_TRY(norm_bwd(dy, input_of(l), p.w[W_NORM1], rstd1, dx1, dnext, p.g[W_NORM1], p.accumulate[W_NORM1],
+                     l > 0 ? m_mlp : nullptr, l > 0 ? layers[l - 1].seed[1] : 0));
     dout = dnext;
   }
   return flush_norms();

@@ -86,6 +86,8 @@ def _declare(lib: ctypes.CDLL) -> None:
         "gfs_gemm_bf16_comm": ([i, vp, i, vp, i, vp, i, vp, i, i, i, i, i, i, i, ulp, ulp, uip, vp, vp, i, i, i,
                                 ctypes.c_longlong, vp], i),
         "gfs_rmsnorm_dw_reduce_multi": ([i, ulp, ulp, ip, ip, i, vp], i),
+        "gfs_dropout_residual_norm": ([vp, vp, vp, vp, vp, vp, i, i, f, f, ctypes.c_ulonglong, vp], i),
+        "gfs_rmsnorm_bwd_dropout": ([vp, vp, vp, vp, vp, vp, vp, vp, i, i, f, ctypes.c_ulonglong, vp], i),
         "gfs_dropout_residual": ([vp, vp, vp, ctypes.c_longlong, f, ctypes.c_ulonglong, i, vp], i),
         "gfs_gemm2_ce_parts": ([i], i),
         "gfs_gemm2_bf16_ce": ([vp, vp, vp, vp, i, i, i, i, i, i, vp], i),

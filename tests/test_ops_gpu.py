@@ -437,6 +437,36 @@ def test_rmsnorm_backward_ring(cuda_device, rows, H, residual):
     assert (dw.double() - ref_w).norm() < 6e-3 * (dyd * xd * r).pow(2).sum(0).sqrt().norm()
 
 
+@pytest.mark.parametrize("rows,H", [(1, 8), (9, 1024), (77, 1032), (33, 2048), (5, 4104), (1184, 264), (1185, 264),
+                                    (2500, 1024), (2500, 1032), (2500, 2048), (1300, 2056)])
+@pytest.mark.parametrize("p", [0.0, 0.1, 0.999])
+def test_rmsnorm_with_dropout(cuda_device, rows, H, p):
+    """The norm that makes its input from a branch's dropped output, and the norm's backward that also writes that branch's
+    gradient: the bits of the two kernels each, at the lines of both (columns kept in registers, rows per CTA)."""
+    from gpt_from_scratch_b200.ops import _lib
+    lib, st, seed = _lib.lib(), _lib.stream_ptr, 0x9876543210fedcba
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g).bfloat16()  # noqa: E731
+    z, res, dy, w = rnd(rows, H), rnd(rows, H), rnd(rows, H), (rnd(H).float() * 0.2 + 1).bfloat16()
+    out = [[torch.full((rows + 1, H), 7.0, device=cuda_device, dtype=torch.bfloat16) for _ in range(4)] for _ in range(2)]
+    rstd = [torch.zeros(rows, device=cuda_device) for _ in range(2)]
+    partial = [torch.zeros(lib.gfs_rmsnorm_bwd_parts(rows) * H, device=cuda_device) for _ in range(2)]
+    P = lambda t: t.data_ptr()  # noqa: E731
+    x, y, dx, dm = out[0]
+    assert lib.gfs_dropout_residual(P(z), P(res), P(x), rows * H, p, seed, 0, st()) == 0
+    assert lib.gfs_rmsnorm_fwd(P(x), P(w), P(y), P(rstd[0]), rows, H, 1e-5, st()) == 0
+    assert lib.gfs_rmsnorm_bwd(P(dy), P(x), P(w), P(rstd[0]), P(res), P(dx), 0, P(partial[0]), rows, H, 0, st()) == 0
+    assert lib.gfs_dropout_residual(P(dx), 0, P(dm), rows * H, p, seed, 1, st()) == 0
+    x2, y2, dx2, dm2 = out[1]
+    assert lib.gfs_dropout_residual_norm(P(z), P(res), P(x2), P(w), P(y2), P(rstd[1]), rows, H, 1e-5, p, seed, st()) == 0
+    rc = lib.gfs_rmsnorm_bwd_dropout(P(dy), P(x2), P(w), P(rstd[1]), P(res), P(dx2), P(dm2), P(partial[1]), rows, H, p, seed,
+                                     st())
+    assert rc == (1 if rows <= 1184 or H > 2048 else 0)
+    assert torch.equal(x, x2) and torch.equal(y, y2) and torch.equal(rstd[0], rstd[1])
+    if rc == 0:
+        assert torch.equal(dx, dx2) and torch.equal(dm, dm2) and torch.equal(partial[0], partial[1])
+
+
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("B,nh,S", [(7, 23, 333), (5, 30, 70), (2, 75, 257), (1, 160, 640)])
 def test_flash_attention_many_items(cuda_device, B, nh, S, causal):
