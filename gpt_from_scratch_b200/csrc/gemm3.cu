@@ -25,7 +25,7 @@
 // us in a chain of products, that -> this: 512 x 256 x 256 5.5 -> 4.1, 130 x 768 x 768 unsplit 7.2 -> 5.8. What
 // an epilogue reads (addend, rotation table, gate and up) is fetched six vectors at a time, the first six before the
 // accumulator is ready; read where it is used, each vector waited for memory: 1040 x 768 x 768 with the SwiGLU gradient
-// 9.0 -> 7.1, with the rotation 8.2 -> 7.0.
+// 9.0 -> 7.1, with the rotation 8.2 -> 7.2.
 //
 // Operand layouts, addend, rotary and SwiGLU epilogues as in gemm.cu; values are rounded once, from fp32.
 #include <algorithm>
@@ -141,97 +141,97 @@ __device__ __forceinline__ void tile_epilogue(const TileParams<NG>& p, const Til
       *reinterpret_cast<uint4*>(p.swi_act + static_cast<size_t>(row) * p.swi_ld + col) = pack8(a);
     }
   } else {
-  constexpr int VPR = BN / 8;
-  constexpr int NPRE = 6;        // vectors of a thread whose operands are fetched together, the first before the wait
-  constexpr bool TABLE = EPI == EPI_SWIGLU_BWD || EPI == EPI_ROPE;
-  uint4 pre[NPRE], aux[TABLE ? NPRE : 1], aux2[TABLE ? NPRE : 1];   // addend; gate and up, or cos and sin
-  const bool has_add = EPI != EPI_SWIGLU_BWD && g.R != nullptr;
-  static_assert(NT % VPR == 0, "a thread's vectors lie in the same columns");
-  const int c = (threadIdx.x % VPR) * 8, col = n0 + c;
-  const int rope_col = EPI == EPI_ROPE ? (col % p.rope_d) >> 1 : 0;
-  auto fetch = [&](int v0) {
+    constexpr int VPR = BN / 8;
+    constexpr int NPRE = 6;        // vectors of a thread whose operands are fetched together, the first before the wait
+    constexpr bool TABLE = EPI == EPI_SWIGLU_BWD || EPI == EPI_ROPE;
+    uint4 pre[NPRE], aux[TABLE ? NPRE : 1], aux2[TABLE ? NPRE : 1];   // addend; gate and up, or cos and sin
+    const bool has_add = EPI != EPI_SWIGLU_BWD && g.R != nullptr;
+    static_assert(NT % VPR == 0, "a thread's vectors lie in the same columns");
+    const int c = (threadIdx.x % VPR) * 8, col = n0 + c;
+    const int rope_col = EPI == EPI_ROPE ? (col % p.rope_d) >> 1 : 0;
+    auto fetch = [&](int v0) {
 #pragma unroll
-    for (int i = 0; i < NPRE; ++i) {
-      const int lr = v0 / VPR + i * (NT / VPR), row = row_base + lr;
-      if (lr >= rows_here || row >= g.M || col + 8 > g.N) continue;
-      if (has_add) pre[i] = *reinterpret_cast<const uint4*>(g.R + static_cast<size_t>(row) * g.ldr + col);
+      for (int i = 0; i < NPRE; ++i) {
+        const int lr = v0 / VPR + i * (NT / VPR), row = row_base + lr;
+        if (lr >= rows_here || row >= g.M || col + 8 > g.N) continue;
+        if (has_add) pre[i] = *reinterpret_cast<const uint4*>(g.R + static_cast<size_t>(row) * g.ldr + col);
+        if constexpr (EPI == EPI_SWIGLU_BWD) {
+          const __nv_bfloat16* gp = p.swi_gu + static_cast<size_t>(row) * p.swi_ld + col;
+          aux[i] = *reinterpret_cast<const uint4*>(gp);
+          aux2[i] = *reinterpret_cast<const uint4*>(gp + p.swi_I);
+        }
+        if (EPI == EPI_ROPE && col < p.rope_cols) {
+          const size_t ti = static_cast<size_t>(row / p.rope_b) * (p.rope_d >> 1) + rope_col;
+          aux[i] = *reinterpret_cast<const uint4*>(p.rope_cos + ti);
+          aux2[i] = *reinterpret_cast<const uint4*>(p.rope_sin + ti);
+        }
+      }
+    };
+    const bool fetches = TABLE || has_add;
+    if (fetches) fetch(threadIdx.x);
+    sync();
+    auto finish = [&](int v, const uint4& addend, const uint4& t0, const uint4& t1) {
+      const int lr = v / VPR, row = row_base + lr;
+      if (lr >= rows_here || row >= g.M || col + 8 > g.N) return;
+      float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+      for (int r = 0; r < split; ++r) {
+        const float4* src = reinterpret_cast<const float4*>(staging + (r * rows_per_cta + lr) * PITCH + c);
+        const float4 a = src[0], b = src[1];
+        f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+        f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+      }
       if constexpr (EPI == EPI_SWIGLU_BWD) {
-        const __nv_bfloat16* gp = p.swi_gu + static_cast<size_t>(row) * p.swi_ld + col;
-        aux[i] = *reinterpret_cast<const uint4*>(gp);
-        aux2[i] = *reinterpret_cast<const uint4*>(gp + p.swi_I);
+        // f holds d_act; turn it into d_gate and d_up
+        float gt[8], up[8], dg[8], du[8];
+        unpack8(t0, gt);
+        unpack8(t1, up);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float sg = sigmoid_f(gt[e]);
+          dg[e] = f[e] * up[e] * sg * (1.f + gt[e] * (1.f - sg));
+          du[e] = f[e] * gt[e] * sg;
+        }
+        __nv_bfloat16* dst = g.C + static_cast<size_t>(row) * g.ldc + col;
+        *reinterpret_cast<uint4*>(dst) = pack8(dg);
+        *reinterpret_cast<uint4*>(dst + p.swi_I) = pack8(du);
+        return;
       }
       if (EPI == EPI_ROPE && col < p.rope_cols) {
-        const size_t ti = static_cast<size_t>(row / p.rope_b) * (p.rope_d >> 1) + rope_col;
-        aux[i] = *reinterpret_cast<const uint4*>(p.rope_cos + ti);
-        aux2[i] = *reinterpret_cast<const uint4*>(p.rope_sin + ti);
+        const float4 cs = make_float4(__uint_as_float(t0.x), __uint_as_float(t0.y), __uint_as_float(t0.z), __uint_as_float(t0.w));
+        const float4 sn = make_float4(__uint_as_float(t1.x), __uint_as_float(t1.y), __uint_as_float(t1.z), __uint_as_float(t1.w));
+        const float a0 = f[0], a1 = f[1], a2 = f[2], a3 = f[3], a4 = f[4], a5 = f[5], a6 = f[6], a7 = f[7];
+        f[0] = a0 * cs.x - a1 * sn.x; f[1] = a0 * sn.x + a1 * cs.x;
+        f[2] = a2 * cs.y - a3 * sn.y; f[3] = a2 * sn.y + a3 * cs.y;
+        f[4] = a4 * cs.z - a5 * sn.z; f[5] = a4 * sn.z + a5 * cs.z;
+        f[6] = a6 * cs.w - a7 * sn.w; f[7] = a6 * sn.w + a7 * cs.w;
       }
-    }
-  };
-  const bool fetches = TABLE || has_add;
-  if (fetches) fetch(threadIdx.x);
-  sync();
-  auto finish = [&](int v, const uint4& addend, const uint4& t0, const uint4& t1) {
-    const int lr = v / VPR, row = row_base + lr;
-    if (lr >= rows_here || row >= g.M || col + 8 > g.N) return;
-    float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 1
-    for (int r = 0; r < split; ++r) {
-      const float4* src = reinterpret_cast<const float4*>(staging + (r * rows_per_cta + lr) * PITCH + c);
-      const float4 a = src[0], b = src[1];
-      f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
-      f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
-    }
-    if constexpr (EPI == EPI_SWIGLU_BWD) {
-      // f holds d_act; turn it into d_gate and d_up
-      float gt[8], up[8], dg[8], du[8];
-      unpack8(t0, gt);
-      unpack8(t1, up);
+      if (has_add) {
+        float r8[8];
+        unpack8(addend, r8);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float sg = sigmoid_f(gt[e]);
-        dg[e] = f[e] * up[e] * sg * (1.f + gt[e] * (1.f - sg));
-        du[e] = f[e] * gt[e] * sg;
+        for (int e = 0; e < 8; ++e) f[e] += r8[e];
       }
-      __nv_bfloat16* dst = g.C + static_cast<size_t>(row) * g.ldc + col;
-      *reinterpret_cast<uint4*>(dst) = pack8(dg);
-      *reinterpret_cast<uint4*>(dst + p.swi_I) = pack8(du);
+      *reinterpret_cast<uint4*>(g.C + static_cast<size_t>(row) * g.ldc + col) = pack8(f);
+    };
+    const int n_vec = rows_here * VPR;
+    int v = threadIdx.x;
+    if (!fetches) {
+      const uint4 none = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+      for (; v < n_vec; v += NT) finish(v, none, none, none);
       return;
     }
-    if (EPI == EPI_ROPE && col < p.rope_cols) {
-      const float4 cs = make_float4(__uint_as_float(t0.x), __uint_as_float(t0.y), __uint_as_float(t0.z), __uint_as_float(t0.w));
-      const float4 sn = make_float4(__uint_as_float(t1.x), __uint_as_float(t1.y), __uint_as_float(t1.z), __uint_as_float(t1.w));
-      const float a0 = f[0], a1 = f[1], a2 = f[2], a3 = f[3], a4 = f[4], a5 = f[5], a6 = f[6], a7 = f[7];
-      f[0] = a0 * cs.x - a1 * sn.x; f[1] = a0 * sn.x + a1 * cs.x;
-      f[2] = a2 * cs.y - a3 * sn.y; f[3] = a2 * sn.y + a3 * cs.y;
-      f[4] = a4 * cs.z - a5 * sn.z; f[5] = a4 * sn.z + a5 * cs.z;
-      f[6] = a6 * cs.w - a7 * sn.w; f[7] = a6 * sn.w + a7 * cs.w;
-    }
-    if (has_add) {
-      float r8[8];
-      unpack8(addend, r8);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] += r8[e];
-    }
-    *reinterpret_cast<uint4*>(g.C + static_cast<size_t>(row) * g.ldc + col) = pack8(f);
-  };
-  const int n_vec = rows_here * VPR;
-  int v = threadIdx.x;
-  if (!fetches) {
-    const uint4 none = make_uint4(0, 0, 0, 0);
 #pragma unroll 1
-    for (; v < n_vec; v += NT) finish(v, none, none, none);
-    return;
-  }
-#pragma unroll 1
-  while (true) {
+    while (true) {
 #pragma unroll
-    for (int i = 0; i < NPRE; ++i, v += NT) {
+      for (int i = 0; i < NPRE; ++i, v += NT) {
+        if (v >= n_vec) return;
+        finish(v, pre[i], aux[TABLE ? i : 0], aux2[TABLE ? i : 0]);
+      }
       if (v >= n_vec) return;
-      finish(v, pre[i], aux[TABLE ? i : 0], aux2[TABLE ? i : 0]);
+      fetch(v);
     }
-    if (v >= n_vec) return;
-    fetch(v);
-  }
   }
 }
 
