@@ -160,18 +160,28 @@ const CUtensorMap* tmap_nd_cached(const void* base, int rank, const uint64_t* di
   return m;
 }
 
+// Zeroed device words, also when this thread is capturing a stream (an operator that is captured without having run before):
+// an allocation or a blocking clear would invalidate the capture unless its mode is relaxed for the while.
+static uint32_t* zeroed_words(size_t bytes) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  uint32_t* p = nullptr;
+  cudaStream_t s = nullptr;
+  bool ok = cudaMalloc(&p, bytes) == cudaSuccess && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+  ok = ok && cudaMemsetAsync(p, 0, bytes, s) == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess;
+  if (s != nullptr) cudaStreamDestroy(s);
+  if (!ok && p != nullptr) cudaFree(p);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return ok ? p : nullptr;
+}
+
 uint32_t* status_words() {
   static std::mutex mu;
   static uint32_t* per_dev[64] = {nullptr};
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
-  if (per_dev[dev] == nullptr) {
-    uint32_t* p = nullptr;
-    if (cudaMalloc(&p, 64 * sizeof(uint32_t)) != cudaSuccess) return nullptr;
-    cudaMemset(p, 0, 64 * sizeof(uint32_t));
-    per_dev[dev] = p;
-  }
+  if (per_dev[dev] == nullptr) per_dev[dev] = zeroed_words(64 * sizeof(uint32_t));
   return per_dev[dev];
 }
 

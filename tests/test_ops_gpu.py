@@ -1,5 +1,8 @@
 """Numerics of the single-GPU kernels against fp32 PyTorch references."""
 import math
+import pathlib
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -484,3 +487,40 @@ def test_flash_attention_many_items(cuda_device, B, nh, S, causal):
         for name, a, b in zip(("O", "dQ", "dK", "dV"), got, (of, *torch.autograd.grad(of, (qf, kf, vf), do.float()))):
             rel = (a.float() - b).norm() / b.norm()
             assert rel < 1e-2, f"{name}: relative error {rel:.4g}"       # as in test_flash_attention_tile_edges
+
+
+@pytest.mark.parametrize("op", ["rmsnorm", "linear"])
+def test_first_call_may_be_captured(cuda_device, op):
+    """A process whose first use of the library is inside a graph capture: what is set up on first use must not invalidate
+    the capture. rmsnorm: more rows than two CTAs of eight warps per SM have warps, so that its backward is the kernel
+    with bounded waits, which has status words."""
+    code = f"""
+import torch
+from gpt_from_scratch_b200.ops import _lib
+from gpt_from_scratch_b200.ops.gemm import gemm_bf16
+from gpt_from_scratch_b200.ops.rmsnorm import rmsnorm, rmsnorm_reference
+g = torch.Generator(device='cuda').manual_seed(1)
+x, dy = (torch.randn(2500, 256, device='cuda', generator=g).bfloat16() for _ in range(2))
+w = torch.ones(256, device='cuda', dtype=torch.bfloat16).requires_grad_()
+x.requires_grad_()
+graph = torch.cuda.CUDAGraph()
+torch.cuda.synchronize()
+with torch.cuda.graph(graph):
+    if {op!r} == 'rmsnorm':
+        got, = torch.autograd.grad(rmsnorm(x, w, 1e-5), (x,), dy)
+    else:
+        got = gemm_bf16(x.detach(), dy[:256])
+graph.replay()
+if {op!r} == 'rmsnorm':
+    xd = x.detach().double().requires_grad_()
+    ref, = torch.autograd.grad(rmsnorm_reference(xd, w.detach().double(), 1e-5), (xd,), dy.double())
+else:
+    ref = x.detach().double() @ dy[:256].double().t()
+torch.cuda.synchronize()
+_lib.raise_on_status()
+assert (got.double() - ref).norm() < 3e-3 * ref.norm()      # results rounded to bf16, 2^-9
+print('captured')
+"""
+    run = subprocess.run([sys.executable, "-c", code], cwd=pathlib.Path(__file__).resolve().parent.parent, text=True,
+                         capture_output=True, timeout=300)
+    assert run.returncode == 0 and "captured" in run.stdout, run.stderr[-2000:]
