@@ -1822,10 +1822,6 @@ const CUtensorMap* make_map(const void* base, int D, int S, int nh, int B, const
   return gfs_host::tmap_nd_cached(base, 4, dims, strides, box);
 }
 
-template <typename K>
-int set_smem(K kern, int bytes) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess ? 0 : -10;
-}
 
 bool strides_ok(const long long* st, int n) {
   for (int i = 0; i < n; ++i)
@@ -1885,9 +1881,9 @@ int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* o_
   p.scale = scale; p.causal = causal; p.o_f16 = o_f16;
   p.status = gfs_host::status_words();
   const int nb = (S + 127) / 128;
-  static bool set64 = false, set128 = false, set128s = false;
+  static gfs_host::SmemLimit limit64, limit128, limit128s;
   if (D == 64) {
-    if (!set64) { if (set_smem(flash_fwd64_kernel, FWD64_SMEM)) return -10; set64 = true; }
+    if (!limit64.raise(flash_fwd64_kernel, FWD64_SMEM)) return -10;
     const int n_pairs = (nb + 1) / 2;
     const int n_items = n_pairs * B * nh;
     const int ctas = std::min(n_items, gfs_host::sm_count());
@@ -1896,12 +1892,12 @@ int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* o_
   } else {
     const int n_items = nb * B * nh;
     if (fwd128_few_items(nb, static_cast<long long>(B) * nh, causal != 0, gfs_host::sm_count())) {
-      if (!set128s) { if (set_smem(flash_fwd128_small_kernel, FWD128S_SMEM)) return -10; set128s = true; }
+      if (!limit128s.raise(flash_fwd128_small_kernel, FWD128S_SMEM)) return -10;
       gfs_host::launch_pdl(flash_fwd128_small_kernel, dim3(nb, B * nh), dim3(FWD128S_THREADS), FWD128S_SMEM, stream, *tq,
                            *tk, *tv, p);
       return cudaGetLastError() == cudaSuccess ? 0 : -11;
     }
-    if (!set128) { if (set_smem(flash_fwd128_kernel, FWD128_SMEM)) return -10; set128 = true; }
+    if (!limit128.raise(flash_fwd128_kernel, FWD128_SMEM)) return -10;
     const int ctas = std::min(n_items, gfs_host::sm_count());
     gfs_host::launch_pdl(flash_fwd128_kernel, dim3(ctas), dim3(FWD128_THREADS), FWD128_SMEM, stream, *tq, *tk, *tv, p, nb,
                          n_items);
@@ -1971,7 +1967,7 @@ int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, co
   const int n_rt = (S + 127) / 128;
   const int n_items = n_rt * B * nh;
   const int ctas = std::min(n_items, gfs_host::sm_count());
-  static bool set_done[4] = {false, false, false, false};
+  static gfs_host::SmemLimit limits[4];
   // mode 0: dK, dV
   BwdParams p0 = p;
   p0.out1 = static_cast<__nv_bfloat16*>(dk); p0.o1_ss = sdk[0]; p0.o1_bs = sdk[1]; p0.o1_hs = sdk[2];
@@ -1981,22 +1977,22 @@ int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, co
   p1.out2 = nullptr; p1.o2_ss = p1.o2_bs = p1.o2_hs = 0;
   if (D == 64) {
     constexpr int smem0 = BwdShape<64, 0>::SMEM;
-    if (!set_done[0]) { if (set_smem(flash_bwd_kernel<64, 0>, smem0)) return -10; set_done[0] = true; }
+    if (!limits[0].raise(flash_bwd_kernel<64, 0>, smem0)) return -10;
     gfs_host::launch_pdl(flash_bwd_kernel<64, 0>, dim3(ctas), dim3(BWD_THREADS), smem0, stream, *k128, *v128,
                          *q64, *do64, p0, n_rt, n_items);
     if (cudaGetLastError() != cudaSuccess) return -12;
     constexpr int smem1 = BwdShape<64, 1>::SMEM;
-    if (!set_done[1]) { if (set_smem(flash_bwd_kernel<64, 1>, smem1)) return -10; set_done[1] = true; }
+    if (!limits[1].raise(flash_bwd_kernel<64, 1>, smem1)) return -10;
     gfs_host::launch_pdl(flash_bwd_kernel<64, 1>, dim3(ctas), dim3(BWD_THREADS), smem1, stream, *q128, *do128,
                          *k64, *v64, p1, n_rt, n_items);
   } else {
     constexpr int smem0 = BwdShape<128, 0>::SMEM;
-    if (!set_done[2]) { if (set_smem(flash_bwd_kernel<128, 0>, smem0)) return -10; set_done[2] = true; }
+    if (!limits[2].raise(flash_bwd_kernel<128, 0>, smem0)) return -10;
     gfs_host::launch_pdl(flash_bwd_kernel<128, 0>, dim3(ctas), dim3(BWD_THREADS), smem0, stream, *k128, *v128,
                          *q64, *do64, p0, n_rt, n_items);
     if (cudaGetLastError() != cudaSuccess) return -12;
     constexpr int smem1 = BwdShape<128, 1>::SMEM;
-    if (!set_done[3]) { if (set_smem(flash_bwd_kernel<128, 1>, smem1)) return -10; set_done[3] = true; }
+    if (!limits[3].raise(flash_bwd_kernel<128, 1>, smem1)) return -10;
     gfs_host::launch_pdl(flash_bwd_kernel<128, 1>, dim3(ctas), dim3(BWD_THREADS), smem1, stream, *q128, *do128,
                          *k64, *v64, p1, n_rt, n_items);
   }

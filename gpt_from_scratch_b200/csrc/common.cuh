@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace gfs {
 
 // ----------------------------------------------------------------------------
@@ -764,6 +766,25 @@ uint32_t* status_words();
 int sm_count();
 // Programmatic dependent launch allowed (GFS_PDL, default on).
 bool pdl_enabled();
+
+// The limit on a kernel's dynamic shared memory belongs to the device: one of these per kernel (a static of its launcher),
+// which raises it once for each device that the kernel is launched on. Devices past the 64th: every time.
+class SmemLimit {
+ public:
+  template <typename Kern>
+  bool raise(Kern kern, int bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+    if (raised_.load(std::memory_order_relaxed) & bit) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+    raised_.fetch_or(bit, std::memory_order_relaxed);
+    return true;
+  }
+
+ private:
+  std::atomic<unsigned long long> raised_{0};
+};
 
 // Launch with programmatic stream serialization: the kernel's CTAs may become resident and run
 // their set-up while the preceding kernel of the stream drains; the kernel must call

@@ -839,26 +839,16 @@ static int rmsnorm_bwd_any(const void* dy, const void* x, const void* w, const v
   const __nv_bfloat16* a_res = static_cast<const __nv_bfloat16*>(dres);
   __nv_bfloat16* a_dx = static_cast<__nv_bfloat16*>(dx);
   float* a_part = static_cast<float*>(partial);
-  auto ensure_smem = [&](auto kern, int& done) -> int {
-    if (smem > 48 * 1024 && done < static_cast<int>(smem)) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
-        return -10;
-      done = 200 * 1024;
-    }
-    return 0;
+  auto too_much = [&](auto kern, gfs_host::SmemLimit& limit) {
+    return smem > 48 * 1024 && !limit.raise(kern, 200 * 1024);
   };
-  static int set_gen = 0, set_r4 = 0, set_r8 = 0;
+  static gfs_host::SmemLimit limit_gen, limit_r4, limit_r8;
   auto ring = [&](auto nv, auto with_drop) -> int {
     constexpr int NV = decltype(nv)::value;
     constexpr bool DROP = decltype(with_drop)::value;
-    static bool set = false;
+    static gfs_host::SmemLimit limit;
     auto kern = rmsnorm_bwd_ring_kernel<NV, DROP>;
-    if (!set) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NormBwdShape<NV>::smem(256 * NV)) !=
-          cudaSuccess)
-        return -10;
-      set = true;
-    }
+    if (!limit.raise(kern, NormBwdShape<NV>::smem(256 * NV))) return -10;
     gfs_host::launch_pdl(kern, dim3(parts), dim3(NormBwdShape<NV>::WARPS * 32), NormBwdShape<NV>::smem(H), stream, a_dy,
                          a_x, a_w, a_rstd, a_res, a_dx, a_part, rows, H, rows_per_cta, gfs_host::status_words(),
                          static_cast<__nv_bfloat16*>(dmask), drop);
@@ -875,15 +865,15 @@ static int rmsnorm_bwd_any(const void* dy, const void* x, const void* w, const v
     const std::integral_constant<int, 8> nv;
     if (const int rc = dmask ? ring(nv, std::true_type{}) : ring(nv, std::false_type{})) return rc;
   } else if (H <= 1024) {
-    if (ensure_smem(rmsnorm_bwd_reg_kernel<4>, set_r4)) return -10;
+    if (too_much(rmsnorm_bwd_reg_kernel<4>, limit_r4)) return -10;
     gfs_host::launch_pdl(rmsnorm_bwd_reg_kernel<4>, dim3(parts), dim3(warps * 32), smem, stream, a_dy, a_x, a_w, a_rstd,
                          a_res, a_dx, a_part, rows, H, rows_per_cta);
   } else if (H <= 2048) {
-    if (ensure_smem(rmsnorm_bwd_reg_kernel<8>, set_r8)) return -10;
+    if (too_much(rmsnorm_bwd_reg_kernel<8>, limit_r8)) return -10;
     gfs_host::launch_pdl(rmsnorm_bwd_reg_kernel<8>, dim3(parts), dim3(warps * 32), smem, stream, a_dy, a_x, a_w, a_rstd,
                          a_res, a_dx, a_part, rows, H, rows_per_cta);
   } else {
-    if (ensure_smem(rmsnorm_bwd_kernel, set_gen)) return -10;
+    if (too_much(rmsnorm_bwd_kernel, limit_gen)) return -10;
     gfs_host::launch_pdl(rmsnorm_bwd_kernel, dim3(parts), dim3(warps * 32), smem, stream, a_dy, a_x, a_w, a_rstd, a_res,
                          a_dx, a_part, rows, H, rows_per_cta);
   }
@@ -1020,13 +1010,8 @@ int gfs_embedding_sort_keys(const void* ids_bs, void* keys, int B, int S, int v0
   if (shift < 0) return shift;
   const int n = static_cast<int>(n64), npow2 = 1 << shift;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(embedding_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 4) !=
-        cudaSuccess)
-      return -10;
-    attr_set = true;
-  }
+  static gfs_host::SmemLimit limit;
+  if (!limit.raise(embedding_sort_kernel, 32768 * 4)) return -10;
   embedding_sort_kernel<<<1, SORT_THREADS, npow2 * sizeof(uint32_t), stream>>>(
       static_cast<const long long*>(ids_bs), static_cast<uint32_t*>(keys), n, npow2, shift, B, S, v0, v1);
   return cudaGetLastError() == cudaSuccess ? shift : -11;

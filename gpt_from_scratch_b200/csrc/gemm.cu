@@ -581,15 +581,8 @@ template <bool A_MN, bool B_MN, int BN, int STAGES, int COMM = COMM_NONE>
 int launch_variant(const CUtensorMap* ta, const CUtensorMap* tb, const GemmParams& p, int grid, cudaStream_t stream) {
   using Cfg = SmemCfg<BN, STAGES>;
   auto kern = gemm_bf16_kernel<A_MN, B_MN, BN, STAGES, COMM>;
-  static bool attr_set = false;
-  static int attr_dev = -1;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_set || attr_dev != dev) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::TOTAL) != cudaSuccess) return -10;
-    attr_set = true;
-    attr_dev = dev;
-  }
+  static gfs_host::SmemLimit limit;
+  if (!limit.raise(kern, Cfg::TOTAL)) return -10;
   if (gfs_host::launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS + (COMM != COMM_NONE ? COMM_THREADS : 0)), Cfg::TOTAL,
                            stream, *ta, *tb, p) != cudaSuccess)
     return -11;

@@ -1322,16 +1322,8 @@ int launch2(const CUtensorMap* ta, const CUtensorMap* tb, const Params2& p, int 
             const CUtensorMap* tx = nullptr, const CUtensorMap* ty = nullptr) {
   auto kern = gemm2_kernel<A_MN, B_MN, COMM, SWI, EW>;
   constexpr int smem = smem2(EW, SWI);
-  static bool attr_set = false;
-  static int attr_dev = -1;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_set || attr_dev != dev) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return -10;
-    attr_set = true;
-    attr_dev = dev;
-  }
+  static gfs_host::SmemLimit limit;
+  if (!limit.raise(kern, smem)) return -10;
   Params2 pt = p;
   pt.trace = g_trace;
   if (COMM == COMM_NONE) {
@@ -1679,17 +1671,8 @@ int gfs_gemm2_wgrad_grouped(int n, const unsigned long long* A, const unsigned l
     p.g[i].tile_begin = 0x7fffffff;
   }
   p.total_tiles = total;
-  static bool attr_set = false;
-  static int attr_dev = -1;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_set || attr_dev != dev) {
-    if (cudaFuncSetAttribute(gemm2_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL) !=
-        cudaSuccess)
-      return -10;
-    attr_set = true;
-    attr_dev = dev;
-  }
+  static gfs_host::SmemLimit limit;
+  if (!limit.raise(gemm2_grouped_kernel, SMEM_TOTAL)) return -10;
   const int pairs = std::min(total, gfs_host::sm_count() / 2);
   if (gfs_host::launch_pdl(gemm2_grouped_kernel, dim3(2 * pairs), dim3(THREADS), SMEM_TOTAL, stream, maps, p) !=
       cudaSuccess)

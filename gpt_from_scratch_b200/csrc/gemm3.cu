@@ -595,14 +595,8 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
 // Launch with `cluster` CTAs per cluster (and programmatic stream serialization).
 template <typename Kern, typename Maps, typename Params>
 int launch_clustered(Kern kern, int threads, int smem, int cluster, const Maps& maps, const Params& p, int ctas,
-                     cudaStream_t stream, bool* attr_set) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return -10;
-  if (!attr_set[dev]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -10;
-    attr_set[dev] = true;
-  }
+                     cudaStream_t stream, gfs_host::SmemLimit& limit) {
+  if (!limit.raise(kern, smem)) return -10;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(threads);
@@ -622,15 +616,15 @@ int launch_clustered(Kern kern, int threads, int smem, int cluster, const Maps& 
 
 template <bool A_MN, bool B_MN, int NG, int EPI>
 int launch_tile(int bn, const TileMaps<NG>& maps, const TileParams<NG>& p, int ctas, cudaStream_t stream) {
-  static bool set64[64] = {}, set128[64] = {}, set256[64] = {};
+  static gfs_host::SmemLimit limit64, limit128, limit256;
   if (bn == 64)
     return launch_clustered(gemm_tile_kernel<A_MN, B_MN, 64, NG, EPI>, THREADS, Cfg<64>::TOTAL, p.split, maps, p, ctas,
-                            stream, set64);
+                            stream, limit64);
   if (bn == 128)
     return launch_clustered(gemm_tile_kernel<A_MN, B_MN, 128, NG, EPI>, THREADS, Cfg<128>::TOTAL, p.split, maps, p, ctas,
-                            stream, set128);
+                            stream, limit128);
   return launch_clustered(gemm_pair_tile_kernel<A_MN, B_MN, NG, EPI>, PAIR_THREADS, PAIR_TOTAL, 2 * p.split, maps, p,
-                          2 * ctas, stream, set256);
+                          2 * ctas, stream, limit256);
 }
 
 template <int EPI>
