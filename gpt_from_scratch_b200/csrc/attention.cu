@@ -1507,7 +1507,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
   // Set-up above may overlap the tail of the preceding kernel (programmatic launch). The dQ kernel reads nothing that the
   // preceding dK / dV kernel writes, and that one had waited for everything before it when it let this one start: it
   // waits at its end, so that its completion means that of both. us per backward: [1, 12, 130, 64] 14.0 -> 12.2,
-  // [2, 4, 256, 64] 14.9 -> 13.1, [3, 12, 777, 64] 32.2 -> 31.3, [16, 12, 1024, 64] 163.6 -> 162.4.
+  // [2, 4, 256, 64] 14.9 -> 13.1, [3, 12, 777, 64] 32.2 -> 31.3, [16, 12, 1024, 64] 163.6 -> 162.4. (launch_hints.h has
+  // what this means for the kernel that follows.)
   if (MODE == 0) pdl_wait();
   pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
@@ -1912,6 +1913,7 @@ int gfs_flash_fwd(const void* q, const void* k, const void* v, void* o, void* o_
 // un-rotated projections.
 // do_bf16: null for bf16 tensors; otherwise o, dO, dq, dk and dv are fp16 (q, k, v stay bf16) and this is
 // scratch for a contiguous bf16 [B, nh, S, D] copy of dO.
+// dq shares no memory with anything that is read for dk and dv, nor with them: its kernel runs beside theirs.
 int gfs_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dO, const void* lse,
                   void* dvec, void* dq, void* dk, void* dv, int S, int B, int nh, int D, const long long* strides,
                   float scale, int causal, const void* rope_cos, const void* rope_sin, void* do_bf16, void* stream_) {

@@ -15,6 +15,8 @@
 
 #include <atomic>
 
+#include "launch_hints.h"
+
 namespace gfs {
 
 // ----------------------------------------------------------------------------
@@ -788,7 +790,7 @@ class SmemLimit {
 
 // Launch with programmatic stream serialization: the kernel's CTAs may become resident and run
 // their set-up while the preceding kernel of the stream drains; the kernel must call
-// gfs::pdl_wait() before its first access to global memory. Inside a stream capture the
+// gfs::pdl_wait() before its first access to global memory, or keep to launch_hints.h. Inside a stream capture the
 // dependency becomes a programmatic edge of the graph.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
@@ -803,31 +805,9 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+  launch_hints().late_wait = false;
+  return e;
 }
-
-// What the caller of the GEMM launchers knows about the kernel that precedes the launch in the stream (this thread's
-// launches inside a WithHints scope). Both rest on every kernel with pdl_wait() calling it before pdl_trigger(): when such
-// a kernel's successor starts, everything before that kernel has completed.
-//   early_b    the preceding kernel does not write operand B (a weight): its first tiles are fetched ahead of pdl_wait()
-//   late_wait  the preceding kernel (which has waited before its trigger) writes nothing this one reads and reads nothing
-//              it writes: it starts on SMs as they become free and waits only at its end, so that its
-//              completion still means that of everything before it. Never for two launches in a row.
-// us a pass, without -> with: two blocks of hidden 256, a step as a graph 245 -> 235; twelve of hidden 768, logits of 130
-// tokens 580 -> 558, a step of 8 x 1024 tokens 10920 -> 10840, of 4 x 512 with dropout 4562 -> 4536.
-struct LaunchHints {
-  bool early_b, late_wait;
-};
-inline LaunchHints& launch_hints() {
-  static thread_local LaunchHints h = {false, false};
-  return h;
-}
-struct WithHints {
-  LaunchHints before;
-  WithHints(bool early_b, bool late_wait) : before(launch_hints()) { launch_hints() = LaunchHints{early_b, late_wait}; }
-  ~WithHints() { launch_hints() = before; }
-  WithHints(const WithHints&) = delete;
-  WithHints& operator=(const WithHints&) = delete;
-};
 
 }  // namespace gfs_host

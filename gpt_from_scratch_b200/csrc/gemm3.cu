@@ -611,7 +611,9 @@ int launch_clustered(Kern kern, int threads, int smem, int cluster, const Maps& 
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, maps, p) == cudaSuccess ? 0 : -11;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, maps, p);
+  gfs_host::launch_hints().late_wait = false;
+  return e == cudaSuccess ? 0 : -11;
 }
 
 template <bool A_MN, bool B_MN, int NG, int EPI>

@@ -131,7 +131,7 @@ struct WgradGroup {
   u64 A[MAX], B[MAX], C[MAX];
   int M[MAX], N[MAX], K[MAX], lda[MAX], ldb[MAX], ldc[MAX], acc[MAX];
   int n = 0, tiles = 0;
-  // late: the kernel launched last is a product that writes nothing these read (see gfs_host::LaunchHints)
+  // late: the kernel launched last is a product that writes nothing these read (see launch_hints.h)
   int flush(int* launches, void* stream, bool late) {
     if (n == 0) return 0;
     const gfs_host::WithHints hints(false, late);

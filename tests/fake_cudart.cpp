@@ -9,8 +9,12 @@
 #include <map>
 #include <utility>
 
+#include "api.h"
+#include "launch_hints.h"
+
 namespace {
 int device = 0, launches = 0;
+int late_waits = 0;         // one bit for each launch, the last one lowest
 cudaError_t last_error = cudaSuccess;
 std::map<std::pair<const void*, int>, int> limits;
 
@@ -19,6 +23,7 @@ cudaError_t launch(const void* func, size_t smem) {
   const size_t limit = it == limits.end() ? 48 * 1024 : it->second;
   if (smem > limit) return last_error = cudaErrorInvalidValue;
   ++launches;
+  late_waits = late_waits << 1 | (gfs_host::launch_hints().late_wait ? 1 : 0);
   return cudaSuccess;
 }
 CUresult encode(CUtensorMap* out) {
@@ -30,6 +35,16 @@ CUresult encode(CUtensorMap* out) {
 extern "C" {
 void fake_set_device(int dev) { device = dev; }
 int fake_launches() { return launches; }
+
+// three products of M x N x K in a scope in which the first one waits late
+int fake_late_waits(int M, int N, int K) {
+  late_waits = 0;
+  const gfs_host::WithHints hints(true, true);
+  void* p = reinterpret_cast<void*>(1 << 20);
+  for (int i = 0; i < 3; ++i)
+    if (gfs_linear(p, p, p, nullptr, M, N, K, K, K, N, 0, 0, 0, nullptr, nullptr, 0, 0, 1, 60, nullptr) != 0) return -1;
+  return late_waits << 1 | (gfs_host::launch_hints().early_b ? 1 : 0);
+}
 
 cudaError_t cudaGetDevice(int* dev) { *dev = device; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return std::exchange(last_error, cudaSuccess); }

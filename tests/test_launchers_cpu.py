@@ -23,6 +23,7 @@ def fake(tmp_path_factory):
     include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
     out = tmp_path_factory.mktemp("fake") / "libgfs_fake.so"
     subprocess.run(["g++", "-shared", "-fPIC", "-std=c++17", "-Wl,-Bsymbolic", "-I", include,
+                    "-I", str(native_build.CSRC),
                     os.path.join(HERE, "fake_cudart.cpp"), *map(str, sorted(native_build.BUILD_DIR.glob("*.o"))),
                     "-o", str(out)], check=True)
     lib = ctypes.CDLL(str(out), mode=os.RTLD_LAZY | os.RTLD_LOCAL)
@@ -59,3 +60,9 @@ def test_every_device_of_a_process_is_served(fake, call):
         assert CALLS[call](fake) == 0, f"device {dev}"
         assert fake.fake_launches() > before
     fake.fake_set_device(0)
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 64, 256), (512, 3072, 768), (16384, 2048, 2048), (8000, 48, 104)])
+def test_late_wait_is_for_one_launch(fake, M, N, K):
+    """Tiles, persistent pairs, persistent CTAs: two late-waiting kernels in a row would be three running at once."""
+    assert fake.fake_late_waits(M, N, K) == 0b1001       # first of three launches; early_b stays
