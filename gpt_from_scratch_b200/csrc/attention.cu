@@ -292,9 +292,7 @@ flash_fwd128_small_kernel(const __grid_constant__ CUtensorMap tq, const __grid_c
         for (int db = 0; db < DB; ++db)
           tma_load_4d(Vs + st * TILE_BYTES + db * 16384, &tv, &v_full[st], db * 64, j * 128, h, b);
       }
-      if (*abort_flag) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      }
+      settle_copies(wctx);
     }
   } else if (warp == 1) {
     {  // whole warp, converged: the MMA / commit helpers elect the issuing lane
@@ -611,9 +609,7 @@ flash_fwd128_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         }
       }
       if (v_prev >= 0) load(Vs, tv, v_full, v_empty, gv++, v_prev * 128, bh_prev);
-      if (*abort_flag) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      }
+      settle_copies(wctx);
     }
   } else if (warp < FWD128_FIRST_CW) {
     // whole warp, converged: the MMA / commit helpers elect the issuing lane. The blocks of all items are one
@@ -956,9 +952,7 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
           tma_load_4d(Vs + st * 16384, &tv, &v_full[st], 0, j * 128, h, b);
         }
       }
-      if (*abort_flag) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      }
+      settle_copies(wctx);
     }
   } else if (warp == 1) {
     {  // whole warp, converged: the MMA / commit helpers elect the issuing lane
@@ -1547,9 +1541,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tr1, const __grid_constant_
           }
         }
       }
-      if (*abort_flag) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      }
+      settle_copies(wctx);
     }
   } else if (warp == 1) {
     // Score MMAs (whole warp, converged: the MMA / commit helpers elect the issuing lane); runs ahead as

@@ -129,6 +129,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   }
 }
 
+// A thread whose copies may still be in flight when a wait has given up stays until they have landed: the shared memory that
+// they write must not be another CTA's by then.
+__device__ __forceinline__ void settle_copies(const WaitCtx& ctx) {
+  if (*ctx.abort_flag) {
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  }
+}
+
 // ----------------------------------------------------------------------------
 // TMA (bulk tensor copies global -> shared of this CTA, completion on an mbarrier)
 // ----------------------------------------------------------------------------

@@ -332,7 +332,7 @@ rmsnorm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
     const float rs = __shfl_sync(0xffffffffu, rs_lane, k & 31);
     const int slot = k % SLOTS;
     const uint8_t* src = ring + slot * (3 * row_bytes);
-    mbar_wait(&full[slot], (k / SLOTS) & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+    if (!__all_sync(0xffffffffu, mbar_wait(&full[slot], (k / SLOTS) & 1, wctx, STATUS_TIMEOUT_PIPE_FULL))) break;
     uint64_t dot2 = 0;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -386,6 +386,7 @@ rmsnorm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
     __syncwarp();                           // the slot has been read
     if (lane == 0 && row + SLOTS * WARPS < r1) fetch(row + SLOTS * WARPS, slot);
   }
+  settle_copies(wctx);
   __syncthreads();                          // all rows of all warps: the ring is free
   float* red = reinterpret_cast<float*>(ring_smem);   // [WARPS][H]
 #pragma unroll

@@ -221,10 +221,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
         }
       }
-      if (*abort_flag) {
-        // let copies that are still in flight land before the CTA's shared memory is released
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      }
+      settle_copies(wctx);
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------

@@ -492,6 +492,7 @@ __device__ __forceinline__ void epilogue16(const Params2& p, const CUtensorMap& 
       acc_phase ^= 1u;
     }
   }
+  settle_copies(wctx);
   if (lane == 0) bulk_wait_all();
 }
 
@@ -651,9 +652,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           }
         }
       }
-      if (*abort_flag) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      }
+      settle_copies(wctx);
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader only) ------------------------------
@@ -1173,9 +1172,7 @@ gemm2_grouped_kernel(const __grid_constant__ GroupMaps maps, const __grid_consta
           }
         }
       }
-      if (*abort_flag) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      }
+      settle_copies(wctx);
     }
   } else if (warp == 1) {
     if (leader) {  // whole warp, converged: the MMA / commit helpers elect the issuing lane

@@ -370,9 +370,7 @@ gemm_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_constan
         load_a(stage, k0);
         load_b(stage, k0);
       }
-      if (*abort_flag) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);   // copies in flight land before the memory is released
-      }
+      settle_copies(wctx);
     }
     __syncwarp();
   } else if (warp == 1) {   // whole warp, converged: the MMA / commit helpers elect the issuing lane
@@ -536,9 +534,7 @@ gemm_pair_tile_kernel(const __grid_constant__ TileMaps<NG> maps, const __grid_co
         load_a(stage, k0);
         load_b(stage, k0);
       }
-      if (*abort_flag) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-      }
+      settle_copies(wctx);
     }
     __syncwarp();
   } else if (warp == 1) {
