@@ -731,11 +731,13 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           dst[i] = *reinterpret_cast<const uint4*>(p.R + static_cast<size_t>(grow) * p.ldr + gc);
       }
     };
-    if (has_add && pair < total_tiles) {
+    auto load_addend_of_tile = [&](int t) {   // this warp's first chunk there
+      if (t >= total_tiles) return;
       int fm0, fn0, fchunk;
-      decode_tile2<COMM>(p, pair, fm0, fn0, fchunk);
+      decode_tile2<COMM>(p, t, fm0, fn0, fchunk);
       load_addend(pre, fm0 + static_cast<int>(rank) * BM, fn0 + c_begin);
-    }
+    };
+    if (has_add) load_addend_of_tile(pair);
     for (int t = pair; t < total_tiles; t += num_pairs) {
       int m0, n0, chunk;
       decode_tile2<COMM>(p, t, m0, n0, chunk);
@@ -806,6 +808,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         }
       } else {
       float ce_m = -INFINITY, ce_s = 0.f;   // SWI == 3: running statistics of this lane's row
+      if (has_add && n0 + c_begin >= p.N) load_addend_of_tile(t + num_pairs);   // no chunk of this tile does it
 #pragma unroll 1
       for (int c = c_begin; c < c_end; c += 64) {
         const int col0 = n0 + c;
@@ -829,13 +832,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         if (has_add) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) cur[i] = pre[i];
-          if (c + 64 < c_end && col0 + 64 < p.N) {
-            load_addend(pre, m0, col0 + 64);
-          } else if (t + num_pairs < total_tiles) {
-            int nm0, nn0, nchunk;
-            decode_tile2<COMM>(p, t + num_pairs, nm0, nn0, nchunk);
-            load_addend(pre, nm0 + static_cast<int>(rank) * BM, nn0 + c_begin);
-          }
+          if (c + 64 < c_end && col0 + 64 < p.N) load_addend(pre, m0, col0 + 64);
+          else load_addend_of_tile(t + num_pairs);
         }
         uint32_t va[32], vb[32];
         tmem_ld_32x32(t_row + c, va);

@@ -354,3 +354,18 @@ def test_pair_kernel_epilogues_at_edges(cuda_device, M, N, K):
         assert ((m.double() + s.double().log()) - lse).abs().max() < 1e-5 * lse.abs().max().clamp(min=1)
     torch.cuda.synchronize()
     _lib.raise_on_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 1032), (95, 264, 1096), (5000, 2056, 1032)])
+def test_pair_kernel_epilogues_long_k(cuda_device, M, N, K):
+    """The same epilogues behind K loops that keep eight epilogue warps: one tile with rows, columns and K ending inside it, and
+    several tiles per CTA."""
+    test_pair_kernel_epilogues_at_edges(cuda_device, M, N, K)
+
+
+@pytest.mark.parametrize("M,N,K", [(2100, 27656, 776), (4200, 17480, 1208)])
+def test_pair_kernel_panels(cuda_device, M, N, K):
+    """B of more than 40 MB is walked in panels of eight tile rows: a last panel of one row that is cut off, behind one and
+    behind two whole panels, with sixteen and with eight epilogue warps."""
+    assert 2 * N * K >= 40 << 20
+    test_pair_kernel_epilogues_at_edges(cuda_device, M, N, K)
