@@ -102,7 +102,7 @@ struct Params2 {
   int swi_I, swi_ld;
   __nv_bfloat16* swi_act;
   const __nv_bfloat16* swi_gu;
-  // SWI == 5: rotary embedding of the first rope_cols columns (without collectives; with them, a run-time switch).
+  // SWI == 5: rotary embedding of the first rope_cols columns (sixteen warps; with eight, a run-time switch).
   // SWI == 3 (LM head): besides storing the logits, every epilogue warp writes the online-softmax
   // statistics (max, sum exp(x - max)) of its 128 columns of each row, computed from the
   // bf16-rounded logits: ce_partials[(tile_n * 2 + column half) * M + row]. A small kernel
@@ -1372,17 +1372,13 @@ int gfs_gemm2_bf16(const void* A, const void* B, void* C, const void* R, int M, 
   p.rope_cols = rope_cols; p.rope_d = rope_d; p.rope_b = rope_b > 0 ? rope_b : 1;
   const int pairs = std::min(p.tiles_m * p.tiles_n, gfs_host::sm_count() / 2);
   const int grid = 2 * pairs;
-  const bool ew16 = K <= EW16_MAX_K || rope_cos != nullptr;
+  // the sixteen-warp rotary epilogue is that of a projection x W^T; the eight-warp kernel rotates by a run-time switch
+  const bool projection = !a_mn_major && !b_mn_major && R == nullptr;
+  const bool ew16 = rope_cos != nullptr ? projection : K <= EW16_MAX_K;
   const CUtensorMap* tx = ew16 && R != nullptr ? gfs_host::tmap_2d_cached(R, M, N, ldr, 32, 64) : nullptr;
   const CUtensorMap* ty = ew16 ? gfs_host::tmap_2d_cached(C, M, N, ldc, 32, 64) : nullptr;
   if (ew16 && (ty == nullptr || (R != nullptr && tx == nullptr))) return -3;
-  if (rope_cos != nullptr) {
-    // the rotary epilogue here is that of a projection x W^T; other forms are the single-CTA kernel's
-    if (a_mn_major || b_mn_major || R != nullptr)
-      return gfs_gemm_bf16_rope(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn_major, b_mn_major, R != nullptr, nullptr, 0,
-                                1, rope_cos, rope_sin, rope_cols, rope_d, rope_b, stream_);
-    return launch2<false, false, COMM_NONE, 5, 16>(ta, tb, p, grid, stream, tx, ty);
-  }
+  if (ew16 && rope_cos != nullptr) return launch2<false, false, COMM_NONE, 5, 16>(ta, tb, p, grid, stream, tx, ty);
   if (ew16) {
     if (!a_mn_major && !b_mn_major) return launch2<false, false, COMM_NONE, 0, 16>(ta, tb, p, grid, stream, tx, ty);
     if (!a_mn_major && b_mn_major) return launch2<false, true, COMM_NONE, 0, 16>(ta, tb, p, grid, stream, tx, ty);

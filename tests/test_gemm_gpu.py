@@ -369,3 +369,42 @@ def test_pair_kernel_panels(cuda_device, M, N, K):
     behind two whole panels, with sixteen and with eight epilogue warps."""
     assert 2 * N * K >= 40 << 20
     test_pair_kernel_epilogues_at_edges(cuda_device, M, N, K)
+
+
+@pytest.mark.parametrize("bn,split", [(64, 1), (128, 2), (256, 1)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+def test_rope_with_addend_and_other_layouts(cuda_device, bn, split, a_mn, b_mn):
+    """The rotary epilogue for every operand layout, with and without an addend: tile kernels, the pair kernel and the rule
+    that chooses. Against fp32, tolerance as in _check."""
+    from gpt_from_scratch_b200.ops import _lib
+    from gpt_from_scratch_b200.ops.gemm import gemm_bf16
+    from gpt_from_scratch_b200.ops.rope import rope_reference
+    S, B, nh, D, K = 46, 4, 3, 64, 328
+    M, N = S * B, 3 * nh * D
+    g = torch.Generator(device="cuda").manual_seed(bn)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g).bfloat16()  # noqa: E731
+    a, b, r = rnd(K, M) if a_mn else rnd(M, K), rnd(K, N) if b_mn else rnd(N, K), rnd(M, N)
+    ang = torch.rand(S, D // 2, device=cuda_device, generator=g) * 6.28
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    ref = _ref(a, b, a_mn, b_mn, None).view(S, B, 3 * nh, D)
+    ref = torch.cat((rope_reference(ref[:, :, :2 * nh], cos, sin), ref[:, :, 2 * nh:]), dim=2).view(M, N)
+    for addend in (None, r):
+        want = ref if addend is None else ref + addend.float()
+        out = torch.empty(M, N, device=cuda_device, dtype=torch.bfloat16)
+        assert _lib.lib().gfs_gemm_tile(a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(addend), M, N, K, a.stride(0),
+                                        b.stride(0), N, N if addend is not None else 0, int(a_mn), int(b_mn), cos.data_ptr(),
+                                        sin.data_ptr(), 2 * nh * D, D, B, 0, 0, 0, bn, split, _lib.stream_ptr()) == 0
+        _check(out, want, K)
+        for pair in (None, True):
+            _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn, addend=addend, rope=(cos, sin, 2 * nh * D, D, B),
+                             pair=pair), want, K)
+
+
+@pytest.mark.parametrize("K", [512, 1032])
+def test_pair_kernel_addend_of_one_row(cuda_device, K):
+    """An addend whose rows are the same memory (a bias as an expanded view), on both sides of the line in K."""
+    from gpt_from_scratch_b200.ops.gemm import gemm_bf16
+    g = torch.Generator(device="cuda").manual_seed(K)
+    M, N = 600, 520
+    a, b, bias = (torch.randn(*s, device=cuda_device, generator=g).bfloat16() for s in ((M, K), (N, K), (N,)))
+    _check(gemm_bf16(a, b, addend=bias.expand(M, N), pair=True), _ref(a, b, False, False, bias.expand(M, N)), K)
