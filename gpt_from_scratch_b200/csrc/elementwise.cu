@@ -722,52 +722,113 @@ embedding_sort_kernel(const long long* __restrict__ ids_bs, uint32_t* __restrict
   for (int i = threadIdx.x; i < n; i += SORT_THREADS) keys_out[i] = sk[i];
 }
 
-// Segmented sum over the sorted keys: a warp owns 256 columns of one run of equal vocabulary rows and adds the run's
-// dout rows in key order (deterministic); dW rows are accumulated (bf16, fp32 sum). The longest run bounds the time: the
-// commonest token of a text is some 3 % of it, 245 rows of 8192 tokens. One warp per run, a row per iteration, was 245
-// memory latencies for each 256 columns of the row in turn; now the column blocks run side by side, 32 keys come in one
-// load, and the loads of EMB_AHEAD rows are in flight together (the order of the additions is the same). us, that -> this:
-// 8192 tokens of text at H 768 239 -> 40, at H 2048 706 -> 79; 16384 uniform tokens at 768, runs of one or two, 25 -> 32.
+// Segmented sum over the sorted keys, dout rows added in key order (deterministic); dW rows are accumulated (bf16, fp32
+// sum). A warp per position; the first warps of a run of equal vocabulary rows share its columns, 256 at a time. The longest
+// run bounds the time of a text (its commonest token is some 3 % of it, 245 rows of 8192 tokens), so its column blocks are
+// worked on side by side, with EMB_AHEAD rows in flight and 32 keys per load. Uniform tokens are runs of one or two rows,
+// and what counts there is the number of warps and what each does before its first row: the keys around its
+// position come in one load, from which it knows its run, and two column blocks are in flight together. Few positions leave the chip
+// idle: then several warps (blockIdx.y) stand for one.
+// us, a warp per run -> a warp per run and column block -> this: 16384 uniform tokens at H 768 11.5 -> 18.3 -> 9.9, at 2048
+// 53 -> 62 -> 38; 8192 tokens of text at 768 108 -> 28 -> 20. (EMB_AHEAD 16 takes 14 for the text, but 14.6 for the uniform
+// tokens: fewer warps fit.)
 constexpr int EMB_AHEAD = 8;
+// A load that stays where it is written: the compiler would move each one down to its addition, one latency after the other.
+__device__ __forceinline__ uint4 load_now(const __nv_bfloat16* p) {
+  uint4 x;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "l"(p));
+  return x;
+}
+constexpr int EMB_BACK = 15;                           // keys ahead of the position in a warp's first load
 __global__ void embedding_bwd_keys_kernel(const uint32_t* __restrict__ keys, const __nv_bfloat16* __restrict__ dout,
                                           __nv_bfloat16* __restrict__ dW, int n, int H, int shift) {
   const int lane = threadIdx.x & 31;
   const int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (p >= n) return;
-  const uint32_t key = keys[p];
+  const int near = p - EMB_BACK + lane;
+  const uint32_t k0 = near >= 0 && near < n ? keys[near] : 0xFFFFFFFFu;
+  const uint32_t key = __shfl_sync(0xffffffffu, k0, EMB_BACK);
   if (key == 0xFFFFFFFFu) return;
-  const uint32_t row = key >> shift;
-  if (p > 0 && (keys[p - 1] >> shift) == row) return;  // not the start of a run
-  const uint32_t mask = (1u << shift) - 1u;
-  const int v = blockIdx.y * 32 + lane;
-  const bool active = v < (H >> 3);                    // idle lanes still take part in the shuffles
-  __nv_bfloat16* dst = dW + static_cast<size_t>(row) * H + 8 * v;
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (active) load8(dst, acc);
-  for (int q = p;; q += 32) {
-    const uint32_t k = q + lane < n ? keys[q + lane] : 0xFFFFFFFFu;
-    const uint32_t in_run = __ballot_sync(0xffffffffu, k != 0xFFFFFFFFu && (k >> shift) == row);
-    const int cnt = in_run == 0xffffffffu ? 32 : __ffs(~in_run) - 1;
-    for (int i = 0; i < cnt; i += EMB_AHEAD) {
-      uint4 x[EMB_AHEAD];
+  const uint32_t row = key >> shift, mask = (1u << shift) - 1u;
+  auto run_lanes = [&](uint32_t k) { return __ballot_sync(0xffffffffu, k != 0xFFFFFFFFu && (k >> shift) == row); };
+  const uint32_t same = run_lanes(k0);
+  const uint32_t other = ~same & ((1u << EMB_BACK) - 1u);
+  const int back = other != 0u ? __clz(other) - (32 - EMB_BACK) : EMB_BACK;   // rows of the run ahead of this one (or more)
+  const int here = __ffs(~(same >> EMB_BACK)) - 1;     // and from this one on, as far as the load reaches
+  const int nvec = H >> 3, blocks = (nvec + 31) >> 5;
+  const int sharers = min(min(blocks, EMB_BACK), back + here);
+  if (back >= sharers) return;
+  const int cb0 = back * gridDim.y + blockIdx.y, cb_step = sharers * gridDim.y;   // this warp's column blocks
+  __nv_bfloat16* const dst = dW + static_cast<size_t>(row) * H;
+  auto add = [](float (&acc)[8], const uint4& x) {
+    const float2 a = unpack_bf16x2(x.x), b = unpack_bf16x2(x.y), c = unpack_bf16x2(x.z), d = unpack_bf16x2(x.w);
+    acc[0] += a.x; acc[1] += a.y; acc[2] += b.x; acc[3] += b.y;
+    acc[4] += c.x; acc[5] += c.y; acc[6] += d.x; acc[7] += d.y;
+  };
+  const int first = EMB_BACK - back;                   // lane of the run's first key
+  if (back + here <= 2) {
+    const uint32_t r0 = __shfl_sync(0xffffffffu, k0, first) & mask;
+    const uint32_t r1 = __shfl_sync(0xffffffffu, k0, first + back + here - 1) & mask;
+    const bool two = back + here == 2;
+    const __nv_bfloat16 *s0 = dout + static_cast<size_t>(r0) * H, *s1 = dout + static_cast<size_t>(r1) * H;
+    for (int cb = cb0; cb < blocks; cb += 2 * cb_step) {
+      uint4 old[2], x0[2], x1[2];
 #pragma unroll
-      for (int u = 0; u < EMB_AHEAD; ++u) {
-        const uint32_t src = __shfl_sync(0xffffffffu, k, min(i + u, cnt - 1)) & mask;
-        x[u] = make_uint4(0, 0, 0, 0);
-        if (active && i + u < cnt) x[u] = *reinterpret_cast<const uint4*>(dout + static_cast<size_t>(src) * H + 8 * v);
+      for (int u = 0; u < 2; ++u) {
+        const int v = (cb + u * cb_step) * 32 + lane;
+        old[u] = x0[u] = x1[u] = make_uint4(0, 0, 0, 0);
+        if (v >= nvec) continue;
+        old[u] = *reinterpret_cast<const uint4*>(dst + 8 * v);
+        x0[u] = *reinterpret_cast<const uint4*>(s0 + 8 * v);
+        if (two) x1[u] = *reinterpret_cast<const uint4*>(s1 + 8 * v);
       }
 #pragma unroll
-      for (int u = 0; u < EMB_AHEAD; ++u) {
-        if (i + u >= cnt) break;
-        const float2 a = unpack_bf16x2(x[u].x), b = unpack_bf16x2(x[u].y), c = unpack_bf16x2(x[u].z),
-                     d = unpack_bf16x2(x[u].w);
-        acc[0] += a.x; acc[1] += a.y; acc[2] += b.x; acc[3] += b.y;
-        acc[4] += c.x; acc[5] += c.y; acc[6] += d.x; acc[7] += d.y;
+      for (int u = 0; u < 2; ++u) {
+        const int v = (cb + u * cb_step) * 32 + lane;
+        if (v >= nvec) continue;
+        const float2 a = unpack_bf16x2(old[u].x), b = unpack_bf16x2(old[u].y), c = unpack_bf16x2(old[u].z),
+                     d = unpack_bf16x2(old[u].w);
+        float acc[8] = {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y};
+        add(acc, x0[u]);
+        if (two) add(acc, x1[u]);
+        store8(dst + 8 * v, acc);
       }
     }
-    if (cnt < 32) break;
+    return;
   }
-  if (active) store8(dst, acc);
+  for (int cb = cb0; cb < blocks; cb += cb_step) {
+    const int v = cb * 32 + lane;
+    const __nv_bfloat16* src = dout + 8 * min(v, nvec - 1);   // (idle lanes read what others read: no branch per load)
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (v < nvec) load8(dst + 8 * v, acc);
+    uint32_t k = k0;
+    for (int from = first, cnt = back + here, q = p + here;; q += 32) {   // rows of lanes [from, from + cnt)
+      const bool more = from + cnt == 32;              // the run may go on behind these keys
+      const uint32_t next = more && q + lane < n ? keys[q + lane] : 0xFFFFFFFFu;
+      for (int i = 0; i < cnt; i += EMB_AHEAD) {
+        uint4 x[EMB_AHEAD];
+#pragma unroll
+        for (int u = 0; u < EMB_AHEAD; ++u) {
+          const uint32_t r = __shfl_sync(0xffffffffu, k, from + min(i + u, cnt - 1)) & mask;
+          x[u] = load_now(src + static_cast<size_t>(r) * H);
+        }
+        if (i + EMB_AHEAD <= cnt) {
+#pragma unroll
+          for (int u = 0; u < EMB_AHEAD; ++u) add(acc, x[u]);
+        } else {
+#pragma unroll
+          for (int u = 0; u < EMB_AHEAD - 1; ++u)
+            if (i + u < cnt) add(acc, x[u]);
+        }
+      }
+      if (!more) break;
+      const uint32_t in_run = run_lanes(next);
+      from = 0;
+      cnt = in_run == 0xffffffffu ? 32 : __ffs(~in_run) - 1;
+      k = next;
+    }
+    if (v < nvec) store8(dst + 8 * v, acc);
+  }
 }
 
 inline int grid_for(size_t work_items, int threads, int max_blocks_per_sm = 16) {
@@ -1022,8 +1083,9 @@ int gfs_embedding_bwd_keys(const void* keys, const void* dout, void* dW, int n, 
   if ((H & 7) || shift <= 0 || shift > 31) return -1;
   if (n == 0) return 0;
   const int warps = 8;
-  const dim3 grid((n + warps - 1) / warps, ((H >> 3) + 31) / 32);
-  embedding_bwd_keys_kernel<<<grid, warps * 32, 0, static_cast<cudaStream_t>(stream_)>>>(
+  // as many warps per position as one wave of the chip (32 per SM) has room for, and columns for
+  const int share = std::max(1, std::min((H / 8 + 31) / 32, gfs_host::sm_count() * 32 / n));
+  embedding_bwd_keys_kernel<<<dim3((n + warps - 1) / warps, share), warps * 32, 0, static_cast<cudaStream_t>(stream_)>>>(
       static_cast<const uint32_t*>(keys), static_cast<const __nv_bfloat16*>(dout), static_cast<__nv_bfloat16*>(dW), n, H,
       shift);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;

@@ -524,3 +524,23 @@ print('captured')
     run = subprocess.run([sys.executable, "-c", code], cwd=pathlib.Path(__file__).resolve().parent.parent, text=True,
                          capture_output=True, timeout=300)
     assert run.returncode == 0 and "captured" in run.stdout, run.stderr[-2000:]
+
+
+@pytest.mark.parametrize("repeat", [1, 12])
+@pytest.mark.parametrize("H", [8, 264, 768, 4200])
+def test_embedding_backward_runs_behind_one_load_of_keys(cuda_device, H, repeat):
+    """Runs around the 31 keys that a warp's first load brings, and the 32 of each further one, between runs of one row, from
+    the first position to the last; positions that several warps share and, with more of them, one each: bit for bit the fp32
+    sum in the order of the positions, rounded once."""
+    from gpt_from_scratch_b200.ops.embedding import embedding_bwd_native
+    counts = [3, 1, 30, 1, 2, 62, 63, 1, 94, 95, 96, 1] * repeat
+    g = torch.Generator(device="cuda").manual_seed(H)
+    ids = torch.repeat_interleave(torch.arange(len(counts), device=cuda_device), torch.tensor(counts, device=cuda_device))
+    ids = ids[torch.randperm(ids.numel(), generator=g, device=cuda_device)].view(1, -1)
+    dout = torch.randn(ids.shape[1], 1, H, device=cuda_device, generator=g).bfloat16()
+    dW = torch.randn(len(counts), H, device=cuda_device, generator=g).bfloat16()
+    acc = dW.float()
+    embedding_bwd_native(ids, dout, dW, 0, len(counts), accumulate=True)
+    for s in range(ids.shape[1]):
+        acc[ids[0, s]] += dout[s, 0].float()
+    assert torch.equal(dW, acc.bfloat16())
