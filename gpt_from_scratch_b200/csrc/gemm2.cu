@@ -61,13 +61,23 @@ constexpr int EPI_BYTES = 8 * 4096;     // one [32 rows x 128 B] transpose buffe
 // cycles) eight warps with two units each, loads and stores of their own, took longer than the loop as soon as the
 // epilogue had anything to compute, and a kernel's last epilogue is never hidden. The price is one of six ring stages
 // (SWI == 2: two, for 6 KB per warp: gate | up on the way in and the results on the way out), which a long loop feels.
-// us, eight warps -> sixteen, K = 768: [16384, 2304] with rotary epilogue 62 -> 48, [16384, 768] with addend 24 -> 20,
-// SwiGLU forward [16384, 2 x 3072] 138 -> 124 and backward 119 -> 102, LM head [8192, 50304] 626 -> 575; K = 2048, inside
-// a training step of 8192 tokens: SwiGLU forward [., 2 x 5632] 259 -> 280, backward 165 -> 197, without an epilogue's work
-// equal, with the rotary one 176 -> 159 (which is why that one always has sixteen).
+// Both sides, us, eight -> sixteen warps (SwiGLU backward up to K 1024: eight with TMA boxes of 64 columns, a variant that is
+// gone):
+//   K                              256         512         768         1024        1152        1280        1536        2048
+//   SwiGLU fwd [8192, 2 x 3072]  57 -> 46    72 -> 58    82 -> 69   100 -> 95   108 -> 104  115 -> 116  128 -> 136  164 -> 173
+//   SwiGLU bwd [8192, 3072]      56 -> 54    69 -> 66    68 -> 62    84 -> 75    86 -> 78    85 -> 80    92 -> 95   105 -> 118
+//   LM head [4096, 32000]       128 -> 97   174 -> 139  213 -> 181  260 -> 244  299 -> 300  279 -> 299  351 -> 374  452 -> 463
+//   addend [8192, 2304]          26 -> 19    31 -> 23    35 -> 30    41 -> 38.5  42 -> 41    46 -> 47    51 -> 54    65 -> 69
+//   rotary [8192, 2304]          34 -> 19    38 -> 23    43 -> 29    51 -> 38    53 -> 40    55 -> 43    62 -> 51    76 -> 68
+// The rotary one always has sixteen. A plain epilogue has nothing to compute, and the line for it lies lower (and above one
+// tile per pair: a last epilogue alone is as short with eight, and the CTAs are set up sooner):
+//   plain, K                       256         384         512         576         640         768         1024
+//   [4096, 1024], 64 tiles        7.3 -> 7.6  8.7 -> 9.0 11.1 -> 11.5 12.0 -> 12.4 12.5 -> 12.8 13.6 -> 14.0 15.5 -> 15.9
+//   [8192, 768], 96 tiles         9.6 -> 9.1 10.6 -> 10.1 11.8 -> 11.7 13.8 -> 13.3 12.7 -> 12.7 14.2 -> 14.6 15.4 -> 15.7
+//   [8192, 2304], 288 tiles      16.8 -> 14.5 18.3 -> 15.9 19.3 -> 17.7 20.4 -> 19.1 21.0 -> 20.2 23.3 -> 23.0 28.9 -> 29.3
 // Eight, for the others (two per TMEM lane quarter, half of the tile's columns each); variants with collectives have two
 // more warps for the transfers.
-constexpr int EW16_MAX_K = 1024;
+constexpr int EW16_MAX_K = 1024, EW16_PLAIN_MAX_K = 640;
 __host__ __device__ constexpr int threads2(int comm, int ew) { return 64 + 32 * ew + (comm != 0 ? 64 : 0); }
 __host__ __device__ constexpr int slot_bytes2(int ew, int swi) { return ew == 16 && swi == 2 ? 6144 : 4096; }
 __host__ __device__ constexpr int stages2(int ew, int swi) { return ew != 16 ? STAGES : swi == 2 ? 4 : 5; }
@@ -1374,7 +1384,9 @@ int gfs_gemm2_bf16(const void* A, const void* B, void* C, const void* R, int M, 
   const int grid = 2 * pairs;
   // the sixteen-warp rotary epilogue is that of a projection x W^T; the eight-warp kernel rotates by a run-time switch
   const bool projection = !a_mn_major && !b_mn_major && R == nullptr;
-  const bool ew16 = rope_cos != nullptr ? projection : K <= EW16_MAX_K;
+  const bool ew16 = rope_cos != nullptr ? projection
+                    : R != nullptr      ? K <= EW16_MAX_K
+                                        : K <= EW16_PLAIN_MAX_K && p.tiles_m * p.tiles_n > pairs;
   const CUtensorMap* tx = ew16 && R != nullptr ? gfs_host::tmap_2d_cached(R, M, N, ldr, 32, 64) : nullptr;
   const CUtensorMap* ty = ew16 ? gfs_host::tmap_2d_cached(C, M, N, ldc, 32, 64) : nullptr;
   if (ew16 && (ty == nullptr || (R != nullptr && tx == nullptr))) return -3;

@@ -408,3 +408,17 @@ def test_pair_kernel_addend_of_one_row(cuda_device, K):
     M, N = 600, 520
     a, b, bias = (torch.randn(*s, device=cuda_device, generator=g).bfloat16() for s in ((M, K), (N, K), (N,)))
     _check(gemm_bf16(a, b, addend=bias.expand(M, N), pair=True), _ref(a, b, False, False, bias.expand(M, N)), K)
+
+
+@pytest.mark.parametrize("K", [640, 648])
+@pytest.mark.parametrize("M,N", [(512, 9472), (500, 9480)])
+def test_pair_kernel_plain_at_the_lines(cuda_device, M, N, K):
+    """Plain products on both sides of the lines between sixteen and eight epilogue warps: K, and a tile per CTA pair (74 on 148
+    SMs) or one column of tiles more."""
+    from gpt_from_scratch_b200.ops.gemm import gemm_bf16
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    for a_mn, b_mn in ((False, False), (False, True), (True, True)):
+        m = M - M % 8 if a_mn else M       # the pitch is a multiple of 8 elements
+        a = torch.randn((K, m) if a_mn else (m, K), device=cuda_device, generator=g).bfloat16()
+        b = torch.randn((K, N) if b_mn else (N, K), device=cuda_device, generator=g).bfloat16()
+        _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn, pair=True), _ref(a, b, a_mn, b_mn, None), K)
