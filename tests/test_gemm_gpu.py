@@ -422,3 +422,17 @@ def test_pair_kernel_plain_at_the_lines(cuda_device, M, N, K):
         a = torch.randn((K, m) if a_mn else (m, K), device=cuda_device, generator=g).bfloat16()
         b = torch.randn((K, N) if b_mn else (N, K), device=cuda_device, generator=g).bfloat16()
         _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn, pair=True), _ref(a, b, a_mn, b_mn, None), K)
+
+
+@pytest.mark.parametrize("M,N,K", [(854, 1400, 3032), (1988, 896, 2808), (494, 1536, 2056)])
+def test_gemm_long_k_with_odd_pitches(cuda_device, M, N, K):
+    """Operands whose rows begin within a 32-byte sector, behind 32 K blocks and more: other tiles are chosen for them."""
+    from gpt_from_scratch_b200.ops.gemm import gemm_bf16
+    g = torch.Generator(device="cuda").manual_seed(M)
+    for a_mn, b_mn in ((False, False), (False, True), (True, True), (True, False)):
+        m = M - M % 8 if a_mn else M
+        a = torch.randn((K, m) if a_mn else (m, K), device=cuda_device, generator=g).bfloat16()
+        b = torch.randn((K, N) if b_mn else (N, K), device=cuda_device, generator=g).bfloat16()
+        c = torch.randn(m, N, device=cuda_device, generator=g).bfloat16()
+        _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn), _ref(a, b, a_mn, b_mn, None), K)
+        _check(gemm_bf16(a, b, a_mn_major=a_mn, b_mn_major=b_mn, addend=c), _ref(a, b, a_mn, b_mn, c), K)
