@@ -183,11 +183,14 @@ int gfs_wgrad_grouped(int n, const unsigned long long* A, const unsigned long lo
     return t;
   };
   Choice c{Choice::PERSISTENT_PAIR, 256, 1};
-  // the persistent grouped kernel: one wave of pairs, an epilogue of four warps
-  const float t_pair = 6.5f + 0.3f * kb * ceil_div(tiles(256), 74);
+  const bool adds = std::any_of(accumulate, accumulate + n, [](int a) { return a != 0; });
+  // the persistent grouped kernel: one wave of pairs, an epilogue of four warps, which reads what it adds to late. (Of 122 groups
+  // that add to existing gradients, three go to other tiles for it, 4 to 10 % faster: three of hidden 128 and 192.)
+  const float t_pair = 6.5f + 0.3f * kb * ceil_div(tiles(256), 74) + (adds ? 2.5f : 0.f);
   // Unsplit 256 x 256 tiles on pairs are that kernel's tiles without its persistence: 95 us instead of 86 for the
   // three small gradients of a block at 16384 tokens (hidden 768, FFN 3072).
-  if (kb == kb_min && best_tile(tiles, kb, true, NONE, 0, &c) < t_pair && c.kernel == Choice::TILE && (c.bn != 256 || c.split > 1))
+  if (kb == kb_min && best_tile(tiles, kb, true, adds ? ADDEND : NONE, 0, &c) < t_pair && c.kernel == Choice::TILE &&
+      (c.bn != 256 || c.split > 1))
     return gfs_gemm_tile_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, accumulate, c.bn, c.split, stream);
   return gfs_gemm2_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, accumulate, stream);
 }
