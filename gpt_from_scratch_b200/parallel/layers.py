@@ -75,6 +75,7 @@ class _LinearFn(torch.autograd.Function):
         ctx.sink = sink
         ctx.has_res = residual is not None
         ctx.in_shape = x.shape
+        ctx.is_head = ce_stats
         y = y2.view(*x.shape[:-1], weight.shape[0])
         if not ce_stats:
             return y
@@ -99,6 +100,10 @@ class _LinearFn(torch.autograd.Function):
         sink = ctx.sink
         if sink is not None:
             gemm_ops.linear_wgrad_to_sink(dy2, x2, sink)
+            if ctx.is_head:
+                # a launch of its own, as in the native passes: in a group with the last block's gradients other
+                # tiles may be chosen, and their roundings would be the only ones that tell the paths apart
+                gemm_ops.flush_wgrad()
         elif ctx.needs_input_grad[1]:
             dw = gemm_ops.linear_wgrad(dy2, x2)
         dres = dy if ctx.has_res else None
