@@ -598,7 +598,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
     load8(base + I + c, u);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float sg = __fdividef(1.f, 1.f + __expf(-g[e]));
+      const float sg = sigmoid_f(g[e]);
       // silu rounded to bf16 before the product, as two separate bf16 ops would do
       o[e] = round_bf16(g[e] * sg) * u[e];
     }
@@ -620,7 +620,7 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const 
     load8(dact + static_cast<size_t>(row) * I + c, d);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float sg = __fdividef(1.f, 1.f + __expf(-g[e]));
+      const float sg = sigmoid_f(g[e]);
       const float silu = g[e] * sg;
       dg[e] = d[e] * u[e] * sg * (1.f + g[e] * (1.f - sg));
       du[e] = d[e] * silu;

@@ -544,3 +544,19 @@ def test_embedding_backward_runs_behind_one_load_of_keys(cuda_device, H, repeat)
     for s in range(ids.shape[1]):
         acc[ids[0, s]] += dout[s, 0].float()
     assert torch.equal(dW, acc.bfloat16())
+
+
+@pytest.mark.parametrize("M,H,I,pair", [(130, 256, 384, False), (3000, 264, 1528, False), (512, 256, 384, True),
+                                        (512, 1032, 384, True)])
+def test_swiglu_fused_and_alone_agree(cuda_device, M, H, I, pair):
+    """The activation of every product with a SwiGLU epilogue (tiles, persistent CTAs, pairs with sixteen and eight epilogue
+    warps) has the bits of the kernel that makes it from the stored projection."""
+    from gpt_from_scratch_b200.ops import gemm as gemm_ops
+    from gpt_from_scratch_b200.ops.mlp_fused import swiglu_gemm_fwd
+    from gpt_from_scratch_b200.ops.swiglu import swiglu
+    g = torch.Generator(device="cuda").manual_seed(M + H)
+    x = torch.randn(M, H, device=cuda_device, generator=g).bfloat16()
+    w = (torch.randn(2 * I, H, device=cuda_device, generator=g) * 0.2).bfloat16()
+    with gemm_ops.pair_min_tiles(1 if pair else 10 ** 9):
+        gu, act = swiglu_gemm_fwd(x, w)
+    assert torch.equal(act, swiglu(gu))
