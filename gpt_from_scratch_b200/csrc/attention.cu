@@ -925,143 +925,143 @@ flash_fwd64_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   };
 
   if (warp < FWD64_FIRST_SW) {
-  setmaxnreg_dec<FWD64_REGS_IO>();
-  if (warp == 0) {
-    if (lane == 0) {
-      int g = 0;      // key blocks loaded so far (ring position)
-      for (int rnd = 0; rnd * G < n_items; ++rnd) {
-        const int w = snake(rnd);
-        if (w >= n_items) break;
-        const int item = rnd;
-        int qp, bh, na, nbk;
-        decode(w, qp, bh, na, nbk);
-        const int b = bh / p.nh, h = bh % p.nh;
-        const int n_kv = max(na, nbk);
-        mbar_wait(q_empty, (item & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);  // previous item's S MMAs done
-        mbar_arrive_expect_tx(q_full, 2 * 16384);
-        tma_load_4d(Qs, &tq, q_full, 0, (2 * qp) * 128, h, b);
-        tma_load_4d(Qs + 16384, &tq, q_full, 0, (2 * qp + 1) * 128, h, b);   // rows past S are zero-filled
-        for (int j = 0; j < n_kv; ++j, ++g) {
-          const int st = g % KS;
-          const uint32_t par = ((g / KS) & 1) ^ 1u;
-          mbar_wait(&k_empty[st], par, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
-          mbar_arrive_expect_tx(&k_full[st], 16384);
-          tma_load_4d(Ks + st * 16384, &tk, &k_full[st], 0, j * 128, h, b);
-          mbar_wait(&v_empty[st], par, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
-          mbar_arrive_expect_tx(&v_full[st], 16384);
-          tma_load_4d(Vs + st * 16384, &tv, &v_full[st], 0, j * 128, h, b);
+    setmaxnreg_dec<FWD64_REGS_IO>();
+    if (warp == 0) {
+      if (lane == 0) {
+        int g = 0;      // key blocks loaded so far (ring position)
+        for (int rnd = 0; rnd * G < n_items; ++rnd) {
+          const int w = snake(rnd);
+          if (w >= n_items) break;
+          const int item = rnd;
+          int qp, bh, na, nbk;
+          decode(w, qp, bh, na, nbk);
+          const int b = bh / p.nh, h = bh % p.nh;
+          const int n_kv = max(na, nbk);
+          mbar_wait(q_empty, (item & 1) ^ 1u, wctx, STATUS_TIMEOUT_PIPE_EMPTY);  // previous item's S MMAs done
+          mbar_arrive_expect_tx(q_full, 2 * 16384);
+          tma_load_4d(Qs, &tq, q_full, 0, (2 * qp) * 128, h, b);
+          tma_load_4d(Qs + 16384, &tq, q_full, 0, (2 * qp + 1) * 128, h, b);   // rows past S are zero-filled
+          for (int j = 0; j < n_kv; ++j, ++g) {
+            const int st = g % KS;
+            const uint32_t par = ((g / KS) & 1) ^ 1u;
+            mbar_wait(&k_empty[st], par, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
+            mbar_arrive_expect_tx(&k_full[st], 16384);
+            tma_load_4d(Ks + st * 16384, &tk, &k_full[st], 0, j * 128, h, b);
+            mbar_wait(&v_empty[st], par, wctx, STATUS_TIMEOUT_PIPE_EMPTY);
+            mbar_arrive_expect_tx(&v_full[st], 16384);
+            tma_load_4d(Vs + st * 16384, &tv, &v_full[st], 0, j * 128, h, b);
+          }
         }
+        settle_copies(wctx);
       }
-      settle_copies(wctx);
-    }
-  } else if (warp == 1) {
-    {  // whole warp, converged: the MMA / commit helpers elect the issuing lane
-      constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
-      constexpr uint32_t idesc_o = umma_idesc_bf16(128, D, 0, 1);
-      int g0 = 0;            // ring position of this item's first key block
-      int cx[2] = {0, 0};    // blocks processed so far per query tile (barrier phase counters)
-      int it[2] = {0, 0};    // items in which the tile had blocks (phase of o_empty)
-      for (int rnd = 0; rnd * G < n_items; ++rnd) {
-        const int w = snake(rnd);
-        if (w >= n_items) break;
-        const int item = rnd;
-        int qp, bh, n_x[2];
-        decode(w, qp, bh, n_x[0], n_x[1]);
-        const int n_kv = max(n_x[0], n_x[1]);
-        mbar_wait(q_full, item & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
-        auto issue_s = [&](int x, int j) {
-          const int g = g0 + j;
-          mbar_wait(&k_full[g % KS], (g / KS) & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
-          tc_fence_after();
-          mma_kk<D / 16>(tmem_base + S_COL + x * 128, smem_u32(Qs + x * 16384), 0, smem_u32(Ks + (g % KS) * 16384),
-                         0, idesc_s, false);
-          umma_commit_e(&s_full[x]);
-        };
-        // S(0) of this item may only overwrite S once the softmax has consumed the previous
-        // item's last block of that tile; that is guaranteed because the previous item's last
-        // P V of the tile was issued after its p_full, and we issue in program order.
-        if (n_x[0] > 0) issue_s(0, 0);
-        if (n_x[1] > 0) issue_s(1, 0);
-        if (n_kv > 0) umma_commit_e(&k_empty[g0 % KS]);
-        if (n_kv == 1) umma_commit_e(q_empty);
-        // Event loop over both query tiles. Two kinds of events per tile: "scores read out"
-        // (s_free: the softmax warps hold block j's scores in registers) lets S(j+1) be issued
-        // into the same columns while the exponentials of block j are still being computed, so
-        // the next scores are ready when the softmax gets there; "probabilities stored" (p_full)
-        // lets P V(j) be issued. Every wait here is a poll, so a tile that is ahead (bounded by
-        // the K/V ring, whose stages are released when both tiles have used a
-        // block) never blocks the warp that the other tile needs.
-        int s_iss[2] = {n_x[0] > 0 ? 1 : 0, n_x[1] > 0 ? 1 : 0};   // S MMAs issued per tile
-        int pv_iss[2] = {0, 0};                                     // P V MMAs issued per tile
-        uint32_t spins = 0;
-        uint64_t spin_t0 = 0;
-        bool dead = false;
-        while ((pv_iss[0] < n_x[0] || pv_iss[1] < n_x[1]) && !dead) {
-          bool progressed = false;
+    } else if (warp == 1) {
+      {  // whole warp, converged: the MMA / commit helpers elect the issuing lane
+        constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
+        constexpr uint32_t idesc_o = umma_idesc_bf16(128, D, 0, 1);
+        int g0 = 0;            // ring position of this item's first key block
+        int cx[2] = {0, 0};    // blocks processed so far per query tile (barrier phase counters)
+        int it[2] = {0, 0};    // items in which the tile had blocks (phase of o_empty)
+        for (int rnd = 0; rnd * G < n_items; ++rnd) {
+          const int w = snake(rnd);
+          if (w >= n_items) break;
+          const int item = rnd;
+          int qp, bh, n_x[2];
+          decode(w, qp, bh, n_x[0], n_x[1]);
+          const int n_kv = max(n_x[0], n_x[1]);
+          mbar_wait(q_full, item & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+          auto issue_s = [&](int x, int j) {
+            const int g = g0 + j;
+            mbar_wait(&k_full[g % KS], (g / KS) & 1, wctx, STATUS_TIMEOUT_PIPE_FULL);
+            tc_fence_after();
+            mma_kk<D / 16>(tmem_base + S_COL + x * 128, smem_u32(Qs + x * 16384), 0, smem_u32(Ks + (g % KS) * 16384),
+                           0, idesc_s, false);
+            umma_commit_e(&s_full[x]);
+          };
+          // S(0) of this item may only overwrite S once the softmax has consumed the previous
+          // item's last block of that tile; that is guaranteed because the previous item's last
+          // P V of the tile was issued after its p_full, and we issue in program order.
+          if (n_x[0] > 0) issue_s(0, 0);
+          if (n_x[1] > 0) issue_s(1, 0);
+          if (n_kv > 0) umma_commit_e(&k_empty[g0 % KS]);
+          if (n_kv == 1) umma_commit_e(q_empty);
+          // Event loop over both query tiles. Two kinds of events per tile: "scores read out"
+          // (s_free: the softmax warps hold block j's scores in registers) lets S(j+1) be issued
+          // into the same columns while the exponentials of block j are still being computed, so
+          // the next scores are ready when the softmax gets there; "probabilities stored" (p_full)
+          // lets P V(j) be issued. Every wait here is a poll, so a tile that is ahead (bounded by
+          // the K/V ring, whose stages are released when both tiles have used a
+          // block) never blocks the warp that the other tile needs.
+          int s_iss[2] = {n_x[0] > 0 ? 1 : 0, n_x[1] > 0 ? 1 : 0};   // S MMAs issued per tile
+          int pv_iss[2] = {0, 0};                                     // P V MMAs issued per tile
+          uint32_t spins = 0;
+          uint64_t spin_t0 = 0;
+          bool dead = false;
+          while ((pv_iss[0] < n_x[0] || pv_iss[1] < n_x[1]) && !dead) {
+            bool progressed = false;
 #pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            const int ot = x ^ 1;
-            const int bn = s_iss[x];          // next block whose S is to be issued
-            if (bn > 0 && bn < n_x[x]) {
-              const int gb = g0 + bn;
-              if (mbar_try_wait(&s_free[x], (cx[x] + bn - 1) & 1) &&
-                  mbar_try_wait(&k_full[gb % KS], (gb / KS) & 1)) {
-                tc_fence_after();
-                mma_kk<D / 16>(tmem_base + S_COL + x * 128, smem_u32(Qs + x * 16384), 0,
-                               smem_u32(Ks + (gb % KS) * 16384), 0, idesc_s, false);
-                umma_commit_e(&s_full[x]);
-                s_iss[x] = bn + 1;
-                // the K block is free once both tiles' S MMAs on it have been issued
-                if (s_iss[ot] > bn || bn >= n_x[ot]) umma_commit_e(&k_empty[gb % KS]);
-                if (s_iss[0] >= n_x[0] && s_iss[1] >= n_x[1]) umma_commit_e(q_empty);   // the item's last S
-                progressed = true;
+            for (int x = 0; x < 2; ++x) {
+              const int ot = x ^ 1;
+              const int bn = s_iss[x];          // next block whose S is to be issued
+              if (bn > 0 && bn < n_x[x]) {
+                const int gb = g0 + bn;
+                if (mbar_try_wait(&s_free[x], (cx[x] + bn - 1) & 1) &&
+                    mbar_try_wait(&k_full[gb % KS], (gb / KS) & 1)) {
+                  tc_fence_after();
+                  mma_kk<D / 16>(tmem_base + S_COL + x * 128, smem_u32(Qs + x * 16384), 0,
+                                 smem_u32(Ks + (gb % KS) * 16384), 0, idesc_s, false);
+                  umma_commit_e(&s_full[x]);
+                  s_iss[x] = bn + 1;
+                  // the K block is free once both tiles' S MMAs on it have been issued
+                  if (s_iss[ot] > bn || bn >= n_x[ot]) umma_commit_e(&k_empty[gb % KS]);
+                  if (s_iss[0] >= n_x[0] && s_iss[1] >= n_x[1]) umma_commit_e(q_empty);   // the item's last S
+                  progressed = true;
+                }
+              }
+              const int j = pv_iss[x];
+              if (j < n_x[x]) {
+                const int c = cx[x] + j;
+                const int g = g0 + j;
+                if (mbar_try_wait(&p_full[x], c & 1) && mbar_try_wait(&v_full[g % KS], (g / KS) & 1)) {
+                  // the accumulator is overwritten once per item: wait until the softmax warps
+                  // have read the previous item's result out of it
+                  if (j == 0) mbar_wait(&o_empty[x], (it[x] & 1) ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
+                  tc_fence_after();
+                  mma_tmn<8>(tmem_base + OP_COL + x * 64, tmem_base + P_COL + x * 64, smem_u32(Vs + (g % KS) * 16384),
+                             0, idesc_o, j > 0);
+                  umma_commit_e(&o_full[x]);
+                  pv_iss[x] = j + 1;
+                  if (pv_iss[ot] > j || j >= n_x[ot]) umma_commit_e(&v_empty[g % KS]);
+                  progressed = true;
+                }
               }
             }
-            const int j = pv_iss[x];
-            if (j < n_x[x]) {
-              const int c = cx[x] + j;
-              const int g = g0 + j;
-              if (mbar_try_wait(&p_full[x], c & 1) && mbar_try_wait(&v_full[g % KS], (g / KS) & 1)) {
-                // the accumulator is overwritten once per item: wait until the softmax warps
-                // have read the previous item's result out of it
-                if (j == 0) mbar_wait(&o_empty[x], (it[x] & 1) ^ 1u, wctx, STATUS_TIMEOUT_SOFTMAX);
-                tc_fence_after();
-                mma_tmn<8>(tmem_base + OP_COL + x * 64, tmem_base + P_COL + x * 64, smem_u32(Vs + (g % KS) * 16384),
-                           0, idesc_o, j > 0);
-                umma_commit_e(&o_full[x]);
-                pv_iss[x] = j + 1;
-                if (pv_iss[ot] > j || j >= n_x[ot]) umma_commit_e(&v_empty[g % KS]);
-                progressed = true;
-              }
-            }
-          }
-          if (progressed) {
-            spins = 0;
-            spin_t0 = 0;
-          } else if (((++spins) & 0xfffu) == 0u) {
-            // bounded like mbar_wait: give up (status recorded) when nothing becomes ready in time
-            if (*abort_flag) {
-              dead = true;
-            } else {
-              const uint64_t now = globaltimer_ns();
-              if (spin_t0 == 0) {
-                spin_t0 = now;
-              } else if (now - spin_t0 > GFS_WAIT_LIMIT_NS) {
-                *abort_flag = 1u;
-                record_status(p.status, STATUS_TIMEOUT_SOFTMAX, (blockIdx.x << 8) | 0xE1u);
+            if (progressed) {
+              spins = 0;
+              spin_t0 = 0;
+            } else if (((++spins) & 0xfffu) == 0u) {
+              // bounded like mbar_wait: give up (status recorded) when nothing becomes ready in time
+              if (*abort_flag) {
                 dead = true;
+              } else {
+                const uint64_t now = globaltimer_ns();
+                if (spin_t0 == 0) {
+                  spin_t0 = now;
+                } else if (now - spin_t0 > GFS_WAIT_LIMIT_NS) {
+                  *abort_flag = 1u;
+                  record_status(p.status, STATUS_TIMEOUT_SOFTMAX, (blockIdx.x << 8) | 0xE1u);
+                  dead = true;
+                }
               }
             }
           }
+          g0 += n_kv;
+          cx[0] += n_x[0];
+          cx[1] += n_x[1];
+          it[0] += n_x[0] > 0;
+          it[1] += n_x[1] > 0;
         }
-        g0 += n_kv;
-        cx[0] += n_x[0];
-        cx[1] += n_x[1];
-        it[0] += n_x[0] > 0;
-        it[1] += n_x[1] > 0;
       }
     }
-  }
   } else {
     setmaxnreg_inc<FWD64_REGS_SOFTMAX>();
     const int x = (warp - FWD64_FIRST_SW) >> 2;   // query tile of this warp

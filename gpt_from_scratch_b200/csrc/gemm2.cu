@@ -713,326 +713,326 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
                           reinterpret_cast<float2*>(epi_smem + EPI_BYTES + BAR_BYTES), tmem_full, tmem_empty, tmem_base,
                           static_cast<int>(rank), pair, num_pairs, total_tiles, warp - 2, warp & 3, wctx);
     } else {
-    // all-gather variant: until the first accumulator is ready these warps help the two push warps
-    if (COMM == COMM_ALLGATHER) {
-      ag_push_rows(p.comm, static_cast<int>(threadIdx.x) - 64, COMM_THREADS + 32 * EW, 1);
-      if (warp == 2 && lane == 0) trace_stamp(p, TRACE_PUSH_DONE);
-    }
-    bool rs_handed_over = false;                          // reduce-scatter: remote tiles handed to the signalling warp
-    const int q = warp & 3;                               // TMEM lane quarter this warp may access
-    const int c_begin = ((warp - 2) >> 2) * (BN / 2);     // this warp's column range of the tile
-    const int c_end = c_begin + BN / 2;
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    uint8_t* ebuf = epi_smem + (warp - 2) * 4096;
-    const int rrow = lane >> 3;
-    const int rch = lane & 7;
-    const bool has_add = p.R != nullptr;
-    // The addend of a 64-column chunk is fetched one chunk ahead (across tile boundaries too), so
-    // its global-memory latency is covered by the previous chunk's work instead of stalling this one.
-    uint4 pre[8];
-    auto load_addend = [&](uint4 (&dst)[8], int mm0, int col0) {
-      const int gc = col0 + rch * 8;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int grow = mm0 + q * 32 + i * 4 + rrow;
-        dst[i] = make_uint4(0, 0, 0, 0);
-        if (grow < p.M && gc + 8 <= p.N)
-          dst[i] = *reinterpret_cast<const uint4*>(p.R + static_cast<size_t>(grow) * p.ldr + gc);
+      // all-gather variant: until the first accumulator is ready these warps help the two push warps
+      if (COMM == COMM_ALLGATHER) {
+        ag_push_rows(p.comm, static_cast<int>(threadIdx.x) - 64, COMM_THREADS + 32 * EW, 1);
+        if (warp == 2 && lane == 0) trace_stamp(p, TRACE_PUSH_DONE);
       }
-    };
-    auto load_addend_of_tile = [&](int t) {   // this warp's first chunk there
-      if (t >= total_tiles) return;
-      int fm0, fn0, fchunk;
-      decode_tile2<COMM>(p, t, fm0, fn0, fchunk);
-      load_addend(pre, fm0 + static_cast<int>(rank) * BM, fn0 + c_begin);
-    };
-    if (has_add) load_addend_of_tile(pair);
-    for (int t = pair; t < total_tiles; t += num_pairs) {
-      int m0, n0, chunk;
-      decode_tile2<COMM>(p, t, m0, n0, chunk);
-      m0 += static_cast<int>(rank) * BM;
-      mbar_wait(&tmem_full[acc], acc_phase, wctx, STATUS_TIMEOUT_TMEM_FULL);
-      if (t == pair && warp == 2 && lane == 0) trace_stamp(p, TRACE_EPI_BEGIN);
-      tc_fence_after();
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-      if (SWI == 1) {
-        // accumulator columns [0,128) are gate, [128,256) the matching up columns
-        const int g0 = n0 >> 1;  // first gate column of the tile
-        const int sc_begin = ((warp - 2) >> 2) * 64;
-        const int sc_end = sc_begin + 64;
-#pragma unroll 1
-        for (int c = sc_begin; c < sc_end; c += 32) {
-          if (g0 + c >= p.swi_I) break;
-          uint32_t vg[32], vu[32];
-          tmem_ld_32x32(t_row + c, vg);
-          tmem_ld_32x32(t_row + BN / 2 + c, vu);
-          tmem_ld_wait();
-          uint32_t pa[16];
-          uint8_t* myrow = ebuf + lane * 128;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint4 wg, wu;
-            uint32_t* wgp = &wg.x;
-            uint32_t* wup = &wu.x;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              wgp[e] = pack_bf16x2(__uint_as_float(vg[8 * j + 2 * e]), __uint_as_float(vg[8 * j + 2 * e + 1]));
-              wup[e] = pack_bf16x2(__uint_as_float(vu[8 * j + 2 * e]), __uint_as_float(vu[8 * j + 2 * e + 1]));
-              // act from the bf16-rounded projections, silu rounded to bf16 before the product
-              const float2 g2 = unpack_bf16x2(wgp[e]), u2 = unpack_bf16x2(wup[e]);
-              const float s0 = __bfloat162float(__float2bfloat16_rn(g2.x * sigmoid_f(g2.x)));
-              const float s1 = __bfloat162float(__float2bfloat16_rn(g2.y * sigmoid_f(g2.y)));
-              pa[4 * j + e] = pack_bf16x2(s0 * u2.x, s1 * u2.y);
-            }
-            *reinterpret_cast<uint4*>(myrow + ((j ^ (lane & 7)) << 4)) = wg;
-            *reinterpret_cast<uint4*>(myrow + (((4 + j) ^ (lane & 7)) << 4)) = wu;
-          }
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {  // gate | up halves of the projection
-            const int r = i * 4 + rrow;
-            const int grow = m0 + q * 32 + r;
-            const int lc = g0 + c + (rch & 3) * 8;  // column inside [0, I)
-            const uint4 w = *reinterpret_cast<const uint4*>(ebuf + r * 128 + ((rch ^ (r & 7)) << 4));
-            if (grow < p.M && lc + 8 <= p.swi_I)
-              *reinterpret_cast<uint4*>(p.C + static_cast<size_t>(grow) * p.ldc + (rch >= 4 ? p.swi_I : 0) + lc) = w;
-          }
-          __syncwarp();
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            *reinterpret_cast<uint4*>(myrow + ((j ^ (lane & 7)) << 4)) =
-                make_uint4(pa[4 * j], pa[4 * j + 1], pa[4 * j + 2], pa[4 * j + 3]);
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {  // act: 32 columns per row, 4 lanes per row
-            const int r = i * 8 + (lane >> 2);
-            const int ch = lane & 3;
-            const int grow = m0 + q * 32 + r;
-            const int lc = g0 + c + ch * 8;
-            const uint4 w = *reinterpret_cast<const uint4*>(ebuf + r * 128 + ((ch ^ (r & 7)) << 4));
-            if (grow < p.M && lc + 8 <= p.swi_I)
-              *reinterpret_cast<uint4*>(p.swi_act + static_cast<size_t>(grow) * p.swi_ld + lc) = w;
-          }
-          __syncwarp();
-        }
-      } else {
-      float ce_m = -INFINITY, ce_s = 0.f;   // SWI == 3: running statistics of this lane's row
-      if (has_add && n0 + c_begin >= p.N) load_addend_of_tile(t + num_pairs);   // no chunk of this tile does it
-#pragma unroll 1
-      for (int c = c_begin; c < c_end; c += 64) {
-        const int col0 = n0 + c;
-        if (col0 >= p.N) break;
-        const int gcol = col0 + rch * 8;
-        uint4 cur[8];
-        uint4 gq[8], uq[8];
-        if (SWI == 2) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int grow = m0 + q * 32 + i * 4 + rrow;
-            gq[i] = make_uint4(0, 0, 0, 0);
-            uq[i] = make_uint4(0, 0, 0, 0);
-            if (grow < p.M && gcol + 8 <= p.N) {
-              const __nv_bfloat16* gp = p.swi_gu + static_cast<size_t>(grow) * p.swi_ld + gcol;
-              gq[i] = *reinterpret_cast<const uint4*>(gp);
-              uq[i] = *reinterpret_cast<const uint4*>(gp + p.swi_I);
-            }
-          }
-        }
-        if (has_add) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) cur[i] = pre[i];
-          if (c + 64 < c_end && col0 + 64 < p.N) load_addend(pre, m0, col0 + 64);
-          else load_addend_of_tile(t + num_pairs);
-        }
-        uint32_t va[32], vb[32];
-        tmem_ld_32x32(t_row + c, va);
-        tmem_ld_32x32(t_row + c + 32, vb);
-        tmem_ld_wait();
-        uint8_t* myrow = ebuf + lane * 128;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint4 w;
-          w.x = pack_bf16x2(__uint_as_float(va[8 * j + 0]), __uint_as_float(va[8 * j + 1]));
-          w.y = pack_bf16x2(__uint_as_float(va[8 * j + 2]), __uint_as_float(va[8 * j + 3]));
-          w.z = pack_bf16x2(__uint_as_float(va[8 * j + 4]), __uint_as_float(va[8 * j + 5]));
-          w.w = pack_bf16x2(__uint_as_float(va[8 * j + 6]), __uint_as_float(va[8 * j + 7]));
-          *reinterpret_cast<uint4*>(myrow + ((j ^ (lane & 7)) << 4)) = w;
-          w.x = pack_bf16x2(__uint_as_float(vb[8 * j + 0]), __uint_as_float(vb[8 * j + 1]));
-          w.y = pack_bf16x2(__uint_as_float(vb[8 * j + 2]), __uint_as_float(vb[8 * j + 3]));
-          w.z = pack_bf16x2(__uint_as_float(vb[8 * j + 4]), __uint_as_float(vb[8 * j + 5]));
-          w.w = pack_bf16x2(__uint_as_float(vb[8 * j + 6]), __uint_as_float(vb[8 * j + 7]));
-          *reinterpret_cast<uint4*>(myrow + (((4 + j) ^ (lane & 7)) << 4)) = w;
-        }
-        if (SWI == 3) {
-          // this lane still holds its own row's 64 columns: fold their bf16-rounded values (read
-          // back from the words it just wrote for the transpose) into the row's running
-          // (max, sum-exp). Columns past N only exist in the last tile (warp-uniform test).
-          constexpr float L2E = 1.4426950408889634f;
-          const int n_valid = min(64, p.N - col0);
-          uint32_t pk[32];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint4 t = *reinterpret_cast<const uint4*>(myrow + ((j ^ (lane & 7)) << 4));
-            pk[4 * j + 0] = t.x; pk[4 * j + 1] = t.y; pk[4 * j + 2] = t.z; pk[4 * j + 3] = t.w;
-          }
-          if (n_valid < 64) {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              const uint32_t lo = (2 * e < n_valid) ? (pk[e] & 0xffffu) : 0xff80u;          // bf16 -inf
-              const uint32_t hi = (2 * e + 1 < n_valid) ? (pk[e] & 0xffff0000u) : 0xff800000u;
-              pk[e] = lo | hi;
-            }
-          }
-          float cm0 = -INFINITY, cm1 = -INFINITY;
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            cm0 = fmaxf(cm0, __uint_as_float(pk[e] << 16));
-            cm1 = fmaxf(cm1, __uint_as_float(pk[e] & 0xffff0000u));
-          }
-          const float nm = fmaxf(ce_m, fmaxf(cm0, cm1));
-          const float off = (nm == -INFINITY) ? 0.f : nm * L2E;
-          float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            a0 += fast_exp2(fmaf(__uint_as_float(pk[e] << 16), L2E, -off));
-            a1 += fast_exp2(fmaf(__uint_as_float(pk[e] & 0xffff0000u), L2E, -off));
-          }
-          ce_s = ce_s * fast_exp2((ce_m == -INFINITY) ? -INFINITY : (ce_m - nm) * L2E) + (a0 + a1);
-          ce_m = nm;
-        }
-        __syncwarp();
+      bool rs_handed_over = false;                          // reduce-scatter: remote tiles handed to the signalling warp
+      const int q = warp & 3;                               // TMEM lane quarter this warp may access
+      const int c_begin = ((warp - 2) >> 2) * (BN / 2);     // this warp's column range of the tile
+      const int c_end = c_begin + BN / 2;
+      int acc = 0;
+      uint32_t acc_phase = 0;
+      uint8_t* ebuf = epi_smem + (warp - 2) * 4096;
+      const int rrow = lane >> 3;
+      const int rch = lane & 7;
+      const bool has_add = p.R != nullptr;
+      // The addend of a 64-column chunk is fetched one chunk ahead (across tile boundaries too), so
+      // its global-memory latency is covered by the previous chunk's work instead of stalling this one.
+      uint4 pre[8];
+      auto load_addend = [&](uint4 (&dst)[8], int mm0, int col0) {
+        const int gc = col0 + rch * 8;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int r = i * 4 + rrow;
-          const int grow = m0 + q * 32 + r;
-          uint4 w = *reinterpret_cast<const uint4*>(ebuf + r * 128 + ((rch ^ (r & 7)) << 4));
-          if (SWI == 2) {
-            // w holds 8 values of d_act; turn them into d_gate and d_up
-            if (grow < p.M && gcol + 8 <= p.N) {
-              const uint32_t* dw = &w.x;
-              const uint32_t* gw = &gq[i].x;
-              const uint32_t* uw = &uq[i].x;
-              uint4 og, ou;
-              uint32_t* ogp = &og.x;
-              uint32_t* oup = &ou.x;
+          const int grow = mm0 + q * 32 + i * 4 + rrow;
+          dst[i] = make_uint4(0, 0, 0, 0);
+          if (grow < p.M && gc + 8 <= p.N)
+            dst[i] = *reinterpret_cast<const uint4*>(p.R + static_cast<size_t>(grow) * p.ldr + gc);
+        }
+      };
+      auto load_addend_of_tile = [&](int t) {   // this warp's first chunk there
+        if (t >= total_tiles) return;
+        int fm0, fn0, fchunk;
+        decode_tile2<COMM>(p, t, fm0, fn0, fchunk);
+        load_addend(pre, fm0 + static_cast<int>(rank) * BM, fn0 + c_begin);
+      };
+      if (has_add) load_addend_of_tile(pair);
+      for (int t = pair; t < total_tiles; t += num_pairs) {
+        int m0, n0, chunk;
+        decode_tile2<COMM>(p, t, m0, n0, chunk);
+        m0 += static_cast<int>(rank) * BM;
+        mbar_wait(&tmem_full[acc], acc_phase, wctx, STATUS_TIMEOUT_TMEM_FULL);
+        if (t == pair && warp == 2 && lane == 0) trace_stamp(p, TRACE_EPI_BEGIN);
+        tc_fence_after();
+        const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
+        if (SWI == 1) {
+          // accumulator columns [0,128) are gate, [128,256) the matching up columns
+          const int g0 = n0 >> 1;  // first gate column of the tile
+          const int sc_begin = ((warp - 2) >> 2) * 64;
+          const int sc_end = sc_begin + 64;
+#pragma unroll 1
+          for (int c = sc_begin; c < sc_end; c += 32) {
+            if (g0 + c >= p.swi_I) break;
+            uint32_t vg[32], vu[32];
+            tmem_ld_32x32(t_row + c, vg);
+            tmem_ld_32x32(t_row + BN / 2 + c, vu);
+            tmem_ld_wait();
+            uint32_t pa[16];
+            uint8_t* myrow = ebuf + lane * 128;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint4 wg, wu;
+              uint32_t* wgp = &wg.x;
+              uint32_t* wup = &wu.x;
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const float2 d2 = unpack_bf16x2(dw[e]), g2 = unpack_bf16x2(gw[e]), u2 = unpack_bf16x2(uw[e]);
-                const float sg0 = sigmoid_f(g2.x), sg1 = sigmoid_f(g2.y);
-                ogp[e] = pack_bf16x2(d2.x * u2.x * sg0 * (1.f + g2.x * (1.f - sg0)),
-                                     d2.y * u2.y * sg1 * (1.f + g2.y * (1.f - sg1)));
-                oup[e] = pack_bf16x2(d2.x * g2.x * sg0, d2.y * g2.y * sg1);
+                wgp[e] = pack_bf16x2(__uint_as_float(vg[8 * j + 2 * e]), __uint_as_float(vg[8 * j + 2 * e + 1]));
+                wup[e] = pack_bf16x2(__uint_as_float(vu[8 * j + 2 * e]), __uint_as_float(vu[8 * j + 2 * e + 1]));
+                // act from the bf16-rounded projections, silu rounded to bf16 before the product
+                const float2 g2 = unpack_bf16x2(wgp[e]), u2 = unpack_bf16x2(wup[e]);
+                const float s0 = __bfloat162float(__float2bfloat16_rn(g2.x * sigmoid_f(g2.x)));
+                const float s1 = __bfloat162float(__float2bfloat16_rn(g2.y * sigmoid_f(g2.y)));
+                pa[4 * j + e] = pack_bf16x2(s0 * u2.x, s1 * u2.y);
               }
-              __nv_bfloat16* dst = p.C + static_cast<size_t>(grow) * p.ldc + gcol;
-              *reinterpret_cast<uint4*>(dst) = og;
-              *reinterpret_cast<uint4*>(dst + p.swi_I) = ou;
+              *reinterpret_cast<uint4*>(myrow + ((j ^ (lane & 7)) << 4)) = wg;
+              *reinterpret_cast<uint4*>(myrow + (((4 + j) ^ (lane & 7)) << 4)) = wu;
             }
-          } else if (grow < p.M && gcol + 8 <= p.N) {
-            if (has_add || p.rope_cos != nullptr) {
-              float f[8];
-              const float2 x0 = unpack_bf16x2(w.x), x1 = unpack_bf16x2(w.y), x2 = unpack_bf16x2(w.z),
-                           x3 = unpack_bf16x2(w.w);
-              f[0] = x0.x; f[1] = x0.y; f[2] = x1.x; f[3] = x1.y; f[4] = x2.x; f[5] = x2.y; f[6] = x3.x; f[7] = x3.y;
-              if (p.rope_cos != nullptr && gcol < p.rope_cols) {
-                const int half = p.rope_d >> 1;
-                const size_t ti = static_cast<size_t>(grow / p.rope_b) * half + ((gcol % p.rope_d) >> 1);
-                const float4 cs = *reinterpret_cast<const float4*>(p.rope_cos + ti);
-                const float4 sn = *reinterpret_cast<const float4*>(p.rope_sin + ti);
-                const float a0 = f[0], a1 = f[1], a2 = f[2], a3 = f[3], a4 = f[4], a5 = f[5], a6 = f[6], a7 = f[7];
-                f[0] = a0 * cs.x - a1 * sn.x; f[1] = a0 * sn.x + a1 * cs.x;
-                f[2] = a2 * cs.y - a3 * sn.y; f[3] = a2 * sn.y + a3 * cs.y;
-                f[4] = a4 * cs.z - a5 * sn.z; f[5] = a4 * sn.z + a5 * cs.z;
-                f[6] = a6 * cs.w - a7 * sn.w; f[7] = a6 * sn.w + a7 * cs.w;
-              }
-              if (has_add) {
-                const uint4 rr = cur[i];
-                const float2 r0 = unpack_bf16x2(rr.x), r1 = unpack_bf16x2(rr.y), r2 = unpack_bf16x2(rr.z),
-                             r3 = unpack_bf16x2(rr.w);
-                f[0] += r0.x; f[1] += r0.y; f[2] += r1.x; f[3] += r1.y;
-                f[4] += r2.x; f[5] += r2.y; f[6] += r3.x; f[7] += r3.y;
-              }
-              w.x = pack_bf16x2(f[0], f[1]);
-              w.y = pack_bf16x2(f[2], f[3]);
-              w.z = pack_bf16x2(f[4], f[5]);
-              w.w = pack_bf16x2(f[6], f[7]);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {  // gate | up halves of the projection
+              const int r = i * 4 + rrow;
+              const int grow = m0 + q * 32 + r;
+              const int lc = g0 + c + (rch & 3) * 8;  // column inside [0, I)
+              const uint4 w = *reinterpret_cast<const uint4*>(ebuf + r * 128 + ((rch ^ (r & 7)) << 4));
+              if (grow < p.M && lc + 8 <= p.swi_I)
+                *reinterpret_cast<uint4*>(p.C + static_cast<size_t>(grow) * p.ldc + (rch >= 4 ? p.swi_I : 0) + lc) = w;
             }
-            __nv_bfloat16* dst;
-            if (COMM == COMM_REDUCE_SCATTER) {
-              // partial rows go to their owner's staging area, slot of this (source) rank
-              dst = p.comm.peer_buf[chunk] +
-                    (static_cast<size_t>(p.comm.rank) * p.comm.rows_per_rank +
-                     (grow - chunk * p.comm.rows_per_rank)) * p.N + gcol;
-            } else {
-              dst = p.C + static_cast<size_t>(grow) * p.ldc + gcol;
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              *reinterpret_cast<uint4*>(myrow + ((j ^ (lane & 7)) << 4)) =
+                  make_uint4(pa[4 * j], pa[4 * j + 1], pa[4 * j + 2], pa[4 * j + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {  // act: 32 columns per row, 4 lanes per row
+              const int r = i * 8 + (lane >> 2);
+              const int ch = lane & 3;
+              const int grow = m0 + q * 32 + r;
+              const int lc = g0 + c + ch * 8;
+              const uint4 w = *reinterpret_cast<const uint4*>(ebuf + r * 128 + ((ch ^ (r & 7)) << 4));
+              if (grow < p.M && lc + 8 <= p.swi_I)
+                *reinterpret_cast<uint4*>(p.swi_act + static_cast<size_t>(grow) * p.swi_ld + lc) = w;
             }
-            *reinterpret_cast<uint4*>(dst) = w;
+            __syncwarp();
           }
-        }
-        __syncwarp();
-      }
-      if (SWI == 3) {
-        const int row = m0 + q * 32 + lane;
-        const int part = (n0 / BN) * 2 + ((warp - 2) >> 2);
-        if (row < p.M) p.ce_partials[static_cast<size_t>(part) * p.M + row] = make_float2(ce_m, ce_s);
-      }
-      }
-      tc_fence_before();
-      __syncwarp();
-      // the accumulator buffer may be overwritten once all epilogue warps of the pair are done
-      if (COMM == COMM_REDUCE_SCATTER) {
-        // Signalling the owner needs a system-scope release, which costs several microseconds (it
-        // waits for every store in flight). It is therefore not done per tile: tiles for the peers
-        // come first in every CTA's order; when this warp moves on to the local chunk (or runs out
-        // of tiles) it hands the count to the reduction warps, which signal the owners (one release
-        // per destination for the whole CTA) while the epilogue warps work on the local chunk. Local tiles only
-        // need device scope.
-        if (chunk != p.comm.rank) {
-          if (lane == 0) atomicAdd(&rs_sent[chunk], 1u);
         } else {
-          if (!rs_handed_over) {
-            named_barrier_arrive(2, 32 * EW + COMM_THREADS);
-            rs_handed_over = true;
+          float ce_m = -INFINITY, ce_s = 0.f;   // SWI == 3: running statistics of this lane's row
+          if (has_add && n0 + c_begin >= p.N) load_addend_of_tile(t + num_pairs);   // no chunk of this tile does it
+#pragma unroll 1
+          for (int c = c_begin; c < c_end; c += 64) {
+            const int col0 = n0 + c;
+            if (col0 >= p.N) break;
+            const int gcol = col0 + rch * 8;
+            uint4 cur[8];
+            uint4 gq[8], uq[8];
+            if (SWI == 2) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int grow = m0 + q * 32 + i * 4 + rrow;
+                gq[i] = make_uint4(0, 0, 0, 0);
+                uq[i] = make_uint4(0, 0, 0, 0);
+                if (grow < p.M && gcol + 8 <= p.N) {
+                  const __nv_bfloat16* gp = p.swi_gu + static_cast<size_t>(grow) * p.swi_ld + gcol;
+                  gq[i] = *reinterpret_cast<const uint4*>(gp);
+                  uq[i] = *reinterpret_cast<const uint4*>(gp + p.swi_I);
+                }
+              }
+            }
+            if (has_add) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) cur[i] = pre[i];
+              if (c + 64 < c_end && col0 + 64 < p.N) load_addend(pre, m0, col0 + 64);
+              else load_addend_of_tile(t + num_pairs);
+            }
+            uint32_t va[32], vb[32];
+            tmem_ld_32x32(t_row + c, va);
+            tmem_ld_32x32(t_row + c + 32, vb);
+            tmem_ld_wait();
+            uint8_t* myrow = ebuf + lane * 128;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint4 w;
+              w.x = pack_bf16x2(__uint_as_float(va[8 * j + 0]), __uint_as_float(va[8 * j + 1]));
+              w.y = pack_bf16x2(__uint_as_float(va[8 * j + 2]), __uint_as_float(va[8 * j + 3]));
+              w.z = pack_bf16x2(__uint_as_float(va[8 * j + 4]), __uint_as_float(va[8 * j + 5]));
+              w.w = pack_bf16x2(__uint_as_float(va[8 * j + 6]), __uint_as_float(va[8 * j + 7]));
+              *reinterpret_cast<uint4*>(myrow + ((j ^ (lane & 7)) << 4)) = w;
+              w.x = pack_bf16x2(__uint_as_float(vb[8 * j + 0]), __uint_as_float(vb[8 * j + 1]));
+              w.y = pack_bf16x2(__uint_as_float(vb[8 * j + 2]), __uint_as_float(vb[8 * j + 3]));
+              w.z = pack_bf16x2(__uint_as_float(vb[8 * j + 4]), __uint_as_float(vb[8 * j + 5]));
+              w.w = pack_bf16x2(__uint_as_float(vb[8 * j + 6]), __uint_as_float(vb[8 * j + 7]));
+              *reinterpret_cast<uint4*>(myrow + (((4 + j) ^ (lane & 7)) << 4)) = w;
+            }
+            if (SWI == 3) {
+              // this lane still holds its own row's 64 columns: fold their bf16-rounded values (read
+              // back from the words it just wrote for the transpose) into the row's running
+              // (max, sum-exp). Columns past N only exist in the last tile (warp-uniform test).
+              constexpr float L2E = 1.4426950408889634f;
+              const int n_valid = min(64, p.N - col0);
+              uint32_t pk[32];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const uint4 t = *reinterpret_cast<const uint4*>(myrow + ((j ^ (lane & 7)) << 4));
+                pk[4 * j + 0] = t.x; pk[4 * j + 1] = t.y; pk[4 * j + 2] = t.z; pk[4 * j + 3] = t.w;
+              }
+              if (n_valid < 64) {
+#pragma unroll
+                for (int e = 0; e < 32; ++e) {
+                  const uint32_t lo = (2 * e < n_valid) ? (pk[e] & 0xffffu) : 0xff80u;          // bf16 -inf
+                  const uint32_t hi = (2 * e + 1 < n_valid) ? (pk[e] & 0xffff0000u) : 0xff800000u;
+                  pk[e] = lo | hi;
+                }
+              }
+              float cm0 = -INFINITY, cm1 = -INFINITY;
+#pragma unroll
+              for (int e = 0; e < 32; ++e) {
+                cm0 = fmaxf(cm0, __uint_as_float(pk[e] << 16));
+                cm1 = fmaxf(cm1, __uint_as_float(pk[e] & 0xffff0000u));
+              }
+              const float nm = fmaxf(ce_m, fmaxf(cm0, cm1));
+              const float off = (nm == -INFINITY) ? 0.f : nm * L2E;
+              float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+              for (int e = 0; e < 32; ++e) {
+                a0 += fast_exp2(fmaf(__uint_as_float(pk[e] << 16), L2E, -off));
+                a1 += fast_exp2(fmaf(__uint_as_float(pk[e] & 0xffff0000u), L2E, -off));
+              }
+              ce_s = ce_s * fast_exp2((ce_m == -INFINITY) ? -INFINITY : (ce_m - nm) * L2E) + (a0 + a1);
+              ce_m = nm;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int r = i * 4 + rrow;
+              const int grow = m0 + q * 32 + r;
+              uint4 w = *reinterpret_cast<const uint4*>(ebuf + r * 128 + ((rch ^ (r & 7)) << 4));
+              if (SWI == 2) {
+                // w holds 8 values of d_act; turn them into d_gate and d_up
+                if (grow < p.M && gcol + 8 <= p.N) {
+                  const uint32_t* dw = &w.x;
+                  const uint32_t* gw = &gq[i].x;
+                  const uint32_t* uw = &uq[i].x;
+                  uint4 og, ou;
+                  uint32_t* ogp = &og.x;
+                  uint32_t* oup = &ou.x;
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) {
+                    const float2 d2 = unpack_bf16x2(dw[e]), g2 = unpack_bf16x2(gw[e]), u2 = unpack_bf16x2(uw[e]);
+                    const float sg0 = sigmoid_f(g2.x), sg1 = sigmoid_f(g2.y);
+                    ogp[e] = pack_bf16x2(d2.x * u2.x * sg0 * (1.f + g2.x * (1.f - sg0)),
+                                         d2.y * u2.y * sg1 * (1.f + g2.y * (1.f - sg1)));
+                    oup[e] = pack_bf16x2(d2.x * g2.x * sg0, d2.y * g2.y * sg1);
+                  }
+                  __nv_bfloat16* dst = p.C + static_cast<size_t>(grow) * p.ldc + gcol;
+                  *reinterpret_cast<uint4*>(dst) = og;
+                  *reinterpret_cast<uint4*>(dst + p.swi_I) = ou;
+                }
+              } else if (grow < p.M && gcol + 8 <= p.N) {
+                if (has_add || p.rope_cos != nullptr) {
+                  float f[8];
+                  const float2 x0 = unpack_bf16x2(w.x), x1 = unpack_bf16x2(w.y), x2 = unpack_bf16x2(w.z),
+                               x3 = unpack_bf16x2(w.w);
+                  f[0] = x0.x; f[1] = x0.y; f[2] = x1.x; f[3] = x1.y; f[4] = x2.x; f[5] = x2.y; f[6] = x3.x; f[7] = x3.y;
+                  if (p.rope_cos != nullptr && gcol < p.rope_cols) {
+                    const int half = p.rope_d >> 1;
+                    const size_t ti = static_cast<size_t>(grow / p.rope_b) * half + ((gcol % p.rope_d) >> 1);
+                    const float4 cs = *reinterpret_cast<const float4*>(p.rope_cos + ti);
+                    const float4 sn = *reinterpret_cast<const float4*>(p.rope_sin + ti);
+                    const float a0 = f[0], a1 = f[1], a2 = f[2], a3 = f[3], a4 = f[4], a5 = f[5], a6 = f[6], a7 = f[7];
+                    f[0] = a0 * cs.x - a1 * sn.x; f[1] = a0 * sn.x + a1 * cs.x;
+                    f[2] = a2 * cs.y - a3 * sn.y; f[3] = a2 * sn.y + a3 * cs.y;
+                    f[4] = a4 * cs.z - a5 * sn.z; f[5] = a4 * sn.z + a5 * cs.z;
+                    f[6] = a6 * cs.w - a7 * sn.w; f[7] = a6 * sn.w + a7 * cs.w;
+                  }
+                  if (has_add) {
+                    const uint4 rr = cur[i];
+                    const float2 r0 = unpack_bf16x2(rr.x), r1 = unpack_bf16x2(rr.y), r2 = unpack_bf16x2(rr.z),
+                                 r3 = unpack_bf16x2(rr.w);
+                    f[0] += r0.x; f[1] += r0.y; f[2] += r1.x; f[3] += r1.y;
+                    f[4] += r2.x; f[5] += r2.y; f[6] += r3.x; f[7] += r3.y;
+                  }
+                  w.x = pack_bf16x2(f[0], f[1]);
+                  w.y = pack_bf16x2(f[2], f[3]);
+                  w.z = pack_bf16x2(f[4], f[5]);
+                  w.w = pack_bf16x2(f[6], f[7]);
+                }
+                __nv_bfloat16* dst;
+                if (COMM == COMM_REDUCE_SCATTER) {
+                  // partial rows go to their owner's staging area, slot of this (source) rank
+                  dst = p.comm.peer_buf[chunk] +
+                        (static_cast<size_t>(p.comm.rank) * p.comm.rows_per_rank +
+                         (grow - chunk * p.comm.rows_per_rank)) * p.N + gcol;
+                } else {
+                  dst = p.C + static_cast<size_t>(grow) * p.ldc + gcol;
+                }
+                *reinterpret_cast<uint4*>(dst) = w;
+              }
+            }
+            __syncwarp();
           }
-          if (lane == 0) red_release_gpu_add_u32(p.comm.peer_flags[chunk] + p.comm.rank, 1u);
+          if (SWI == 3) {
+            const int row = m0 + q * 32 + lane;
+            const int part = (n0 / BN) * 2 + ((warp - 2) >> 2);
+            if (row < p.M) p.ce_partials[static_cast<size_t>(part) * p.M + row] = make_float2(ce_m, ce_s);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        // the accumulator buffer may be overwritten once all epilogue warps of the pair are done
+        if (COMM == COMM_REDUCE_SCATTER) {
+          // Signalling the owner needs a system-scope release, which costs several microseconds (it
+          // waits for every store in flight). It is therefore not done per tile: tiles for the peers
+          // come first in every CTA's order; when this warp moves on to the local chunk (or runs out
+          // of tiles) it hands the count to the reduction warps, which signal the owners (one release
+          // per destination for the whole CTA) while the epilogue warps work on the local chunk. Local tiles only
+          // need device scope.
+          if (chunk != p.comm.rank) {
+            if (lane == 0) atomicAdd(&rs_sent[chunk], 1u);
+          } else {
+            if (!rs_handed_over) {
+              named_barrier_arrive(2, 32 * EW + COMM_THREADS);
+              rs_handed_over = true;
+            }
+            if (lane == 0) red_release_gpu_add_u32(p.comm.peer_flags[chunk] + p.comm.rank, 1u);
+          }
+        }
+        if (lane == 0) {
+          mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty[acc]), 0));
+          if (warp == 2) {
+            if (t == pair) trace_stamp(p, TRACE_EPI_FIRST);
+            trace_stamp(p, TRACE_EPI_LAST);
+          }
+        }
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1u;
         }
       }
-      if (lane == 0) {
-        mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty[acc]), 0));
-        if (warp == 2) {
-          if (t == pair) trace_stamp(p, TRACE_EPI_FIRST);
-          trace_stamp(p, TRACE_EPI_LAST);
-        }
+      if (COMM == COMM_REDUCE_SCATTER) {
+        if (!rs_handed_over) named_barrier_arrive(2, 32 * EW + COMM_THREADS);   // CTAs without local tiles
+        // tiles done: join the reduction of this rank's row chunk (second share of the vectors)
+        const CommParams& c = p.comm;
+        bool ok = true;
+        for (int src = 0; src < c.world; ++src)
+          ok = wait_flag_reached(c.peer_flags[c.rank] + src, c.target, c.wait_ns, p.status,
+                                 0xB8000000u | (src << 8) | c.rank) && ok;
+        if (!ok) *abort_flag = 1u;
+        constexpr int RED_THREADS = COMM_THREADS + 32 * EW;
+        rs_reduce_rows(c.peer_buf[c.rank], c.world, c.rows_per_rank, p.N, c.rs_res, c.rs_ld_res, c.rs_out, c.rs_ld_out,
+                       static_cast<size_t>(blockIdx.x) * RED_THREADS + COMM_THREADS + (threadIdx.x - 64),
+                       static_cast<size_t>(gridDim.x) * RED_THREADS);
       }
-      if (++acc == 2) {
-        acc = 0;
-        acc_phase ^= 1u;
-      }
-    }
-    if (COMM == COMM_REDUCE_SCATTER) {
-      if (!rs_handed_over) named_barrier_arrive(2, 32 * EW + COMM_THREADS);   // CTAs without local tiles
-      // tiles done: join the reduction of this rank's row chunk (second share of the vectors)
-      const CommParams& c = p.comm;
-      bool ok = true;
-      for (int src = 0; src < c.world; ++src)
-        ok = wait_flag_reached(c.peer_flags[c.rank] + src, c.target, c.wait_ns, p.status,
-                               0xB8000000u | (src << 8) | c.rank) && ok;
-      if (!ok) *abort_flag = 1u;
-      constexpr int RED_THREADS = COMM_THREADS + 32 * EW;
-      rs_reduce_rows(c.peer_buf[c.rank], c.world, c.rows_per_rank, p.N, c.rs_res, c.rs_ld_res, c.rs_out, c.rs_ld_out,
-                     static_cast<size_t>(blockIdx.x) * RED_THREADS + COMM_THREADS + (threadIdx.x - 64),
-                     static_cast<size_t>(gridDim.x) * RED_THREADS);
-    }
     }
   } else if (COMM == COMM_ALLGATHER) {
-    // ------------------------------ all-gather push (warps 6-7) ------------------------------
+    // ------------------------------ all-gather push (the last two warps) ------------------------------
     // Every CTA pushes its slice of the local shard into every rank's gathered buffer
     // (own rank first), then bumps that rank's counter for this source.
     // (the epilogue warps push too, before their first tile: see the top of the epilogue branch)
     ag_push_rows(p.comm, static_cast<int>(threadIdx.x) - (threads2(COMM, EW) - COMM_THREADS) + 32 * EW,
                  COMM_THREADS + 32 * EW, 1);
   } else if (COMM == COMM_REDUCE_SCATTER) {
-    // ------------------------------ reduce (warps 6-7) ------------------------------
+    // ------------------------------ reduce (the last two warps) ------------------------------
     // Wait until every rank (this one included) has delivered all partial tiles of our row
     // chunk, then sum the staged partials in rank order, add the residual, round once.
     const CommParams& c = p.comm;
@@ -1622,9 +1622,8 @@ int gfs_gemm2_bf16_comm_swiglu(int swi_mode, const void* a, int lda, const void*
 
 // Vocabulary-parallel LM head under sequence parallelism: the all-gather GEMM
 // (logits[M, N] = gather(a)[M, K] @ B[N, K]^T, B K-major) whose epilogue also writes the
-// cross-entropy statistics of gfs_gemm2_bf16_ce: partials is float2 [gfs_gemm2_ce_parts(N)][M]
-// (the second slot of every 256-column tile holds the empty pair (-inf, 0): four epilogue warps
-// per CTA here, each covering the tile's full width). Returns -20 like gfs_gemm2_bf16_comm.
+// cross-entropy statistics of gfs_gemm2_bf16_ce: partials is float2 [gfs_gemm2_ce_parts(N)][M]. Returns -20 like
+// gfs_gemm2_bf16_comm.
 int gfs_gemm2_bf16_allgather_ce(const void* a, int lda, const void* B, int ldb, void* out, int ldo, void* partials,
                                 int M, int N, int K, int world, int rank, const unsigned long long* peer_bufs,
                                 const unsigned long long* peer_flags, unsigned int* target_inout, long long wait_ns,

@@ -101,8 +101,10 @@ class _LinearFn(torch.autograd.Function):
         if sink is not None:
             gemm_ops.linear_wgrad_to_sink(dy2, x2, sink)
             if ctx.is_head:
-                # a launch of its own, as in the native passes: in a group with the last block's gradients other
-                # tiles may be chosen, and their roundings would be the only ones that tell the paths apart
+                # a launch of its own, as in the native passes: in a group with the last block's gradients other tiles may be
+                # chosen, and their roundings would be the only ones that tell the paths apart (a hidden-768 model's logits by
+                # 4e-3 after three steps). All weight gradients of a pass, us in groups -> with this: V 1024, H 256, two blocks,
+                # 512 tokens 15.3 -> 15.7; V 4096, H 256, four, 2048 tokens 55.7 -> 55.8; V 1024, H 768, two, 2331 tokens 84 -> 94.
                 gemm_ops.flush_wgrad()
         elif ctx.needs_input_grad[1]:
             dw = gemm_ops.linear_wgrad(dy2, x2)
