@@ -49,27 +49,19 @@ struct TileShape {
   int cluster;          // CTAs per tile without a split
   float base, per_kblock, split_base, split_cost;   // a split over s CTAs costs split_base + s * split_cost
   float extra[5];       // by Extra, for a whole tile; a CTA of a split tile does its share of the rows
-  float odd_pitch[3];   // more per K block, by the number of operands with an odd pitch (see odd_pitches)
 };
+// (Operands whose rows begin within a 32-byte sector, pitches of 8 mod 16, are not priced: a K block of a 128 x 128 tile takes
+// up to 0.4 us for them. 854 x 1400 x 3032 with addend takes 25 to 27 us there and would take 20 to 21 on 256 x 256 tiles split in two,
+// 1988 x 896 x 2808 22.5 and 20; another split sums in another order, so models of such widths would train to other bits.)
 constexpr TileShape kShapes[3] = {
-    // 96 cycles per MMA (A and B read for 64 columns)
-    {64, 1, 3.0f, 0.21f, 0.0f, 0.25f, {0.f, 0.2f, 1.3f, 0.6f, 1.2f}, {0.f, 0.04f, 0.08f}},
-    // 128 cycles per MMA: shared-memory reads
-    {128, 1, 4.0f, 0.225f, 0.5f, 0.3f, {0.f, 0.55f, 3.2f, 1.1f, 2.45f}, {0.f, 0.065f, 0.165f}},
-    // tensor-bound, 256 columns per row to store
-    {256, 2, 5.5f, 0.28f, 1.0f, 0.8f, {0.f, 0.85f, 4.4f, 1.2f, 3.5f}, {0.f, 0.095f, 0.15f}},
+    {64, 1, 3.0f, 0.21f, 0.0f, 0.25f, {0.f, 0.2f, 1.3f, 0.6f, 1.2f}},   // 96 cycles per MMA (A and B read for 64 columns)
+    {128, 1, 4.0f, 0.225f, 0.5f, 0.3f, {0.f, 0.55f, 3.2f, 1.1f, 2.45f}},   // 128 cycles per MMA: shared-memory reads
+    {256, 2, 5.5f, 0.28f, 1.0f, 0.8f, {0.f, 0.85f, 4.4f, 1.2f, 3.5f}},     // tensor-bound, 256 columns per row to store
 };
-constexpr float kOddPitchCta[3] = {0.f, 0.12f, 0.25f}, kOddPitchPair[3] = {0.f, 0.08f, 0.16f};   // persistent kernels
-
-// Operands whose rows do not begin on 32-byte sectors: a TMA box then reads a sector more per row, and a K block takes up to
-// 0.4 us where it took 0.23. All kernels suffer, 128 x 128 tiles most, which tells only in long loops (in short ones the
-// constants above fit well enough): counted from 32 K blocks on. us with addend, 128 x 128 tiles, the choice without this, and
-// 256 x 256 tiles split in two: 854 x 1400 x 3032 25 to 27 by layout and 20 to 21, 1988 x 896 x 2808 22.5 and 20.
-int odd_pitches(int lda, int ldb, int kblocks) { return kblocks < 32 ? 0 : (lda % 16 != 0) + (ldb % 16 != 0); }
 
 // Best one-wave tile for `tiles(bn)` tiles of 128 (bn = 256: 256) rows. us, or a huge number if none fits.
 template <typename Tiles>
-float best_tile(Tiles tiles, int kblocks, bool pairs, Extra extra, int odd, Choice* c) {
+float best_tile(Tiles tiles, int kblocks, bool pairs, Extra extra, Choice* c) {
   float best = 1e30f;
   for (const TileShape& s : kShapes) {
     if (s.bn == 256 && !pairs) continue;
@@ -80,7 +72,7 @@ float best_tile(Tiles tiles, int kblocks, bool pairs, Extra extra, int odd, Choi
       if (per * (split - 1) >= kblocks) break;              // a CTA without K blocks
       const int cluster = s.cluster * split;
       if (n * cluster > wave_of_clusters(cluster)) break;
-      float t = s.base + (s.per_kblock + s.odd_pitch[odd]) * per + s.extra[extra] / split;
+      float t = s.base + s.per_kblock * per + s.extra[extra] / split;
       if (split > 1) t += s.split_base + s.split_cost * split + (extra != NONE ? 0.3f : 0.f);
       if (t < best) {
         best = t;
@@ -94,25 +86,25 @@ float best_tile(Tiles tiles, int kblocks, bool pairs, Extra extra, int odd, Choi
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // cols(bn): output columns covered by a tile of bn accumulator columns.
-Choice choose(int M, int N, int K, int lda, int ldb, int swi_mode, bool add, bool rope, int pair_min_tiles) {
+Choice choose(int M, int N, int K, int swi_mode, bool add, bool rope, int pair_min_tiles) {
   auto tiles = [&](int bn) {
     const int cols = swi_mode == 1 ? bn / 2 : bn;
     return ceil_div(M, bn == 256 ? 256 : 128) * ceil_div(N, cols);
   };
-  const int kb = ceil_div(K, 64), odd = odd_pitches(lda, ldb, kb);
+  const int kb = ceil_div(K, 64);
   const bool pairs = pair_min_tiles >= 0, plain = swi_mode == 0 && !add && !rope;
   if (pairs && (K >= 256 || swi_mode != 0) && tiles(256) >= pair_min_tiles) return Choice{Choice::PERSISTENT_PAIR, 256, 1};
   Choice c{Choice::PERSISTENT_CTA, 256, 1};
   const Extra extra = swi_mode == 1 ? SWIGLU : swi_mode == 2 ? SWIGLU_GRAD : rope ? ROTATION : add ? ADDEND : NONE;
-  const float t_tile = best_tile(tiles, kb, pairs, extra, odd, &c);
+  const float t_tile = best_tile(tiles, kb, pairs, extra, &c);
   // persistent CTAs: 128 x 256 tiles in waves; the addend, the rotation and the SwiGLU gradient are serial
   // loads in its epilogue. Plain products of up to 128 columns have 128-column tiles and half the epilogue there. Judged
   // by the same line, 27 of 129 measured ones went to kernels more than 5 % slower than the persistent one; with
   // one of their own up to 12 K blocks, one (us, one-tile kernel -> here: 2010 x 48 x 104 5.2 -> 4.0, 3568 x 32 x 104
   // 5.2 -> 4.0, 463 x 32 x 72 4.8 -> 3.7). With more K blocks the split over a cluster is the better one.
   const int waves = ceil_div(ceil_div(M, 128) * ceil_div(N, swi_mode == 1 ? 128 : 256), 148);
-  float t_cta = 5.2f + (0.3f + kOddPitchCta[odd]) * kb * waves + 3.8f * (waves - 1) + (add ? 3.3f : 0.f) +
-                (rope ? 9.5f : 0.f) + (swi_mode == 1 ? 2.0f : 0.f) + (swi_mode == 2 ? 6.0f : 0.f);
+  float t_cta = 5.2f + 0.3f * kb * waves + 3.8f * (waves - 1) + (add ? 3.3f : 0.f) + (rope ? 9.5f : 0.f) +
+                (swi_mode == 1 ? 2.0f : 0.f) + (swi_mode == 2 ? 6.0f : 0.f);
   if (N <= 128 && kb <= 12 && plain) t_cta = 4.0f + 0.18f * kb * waves + (waves - 1);
   if (t_cta < t_tile) c = Choice{Choice::PERSISTENT_CTA, 256, 1};
   // Persistent pairs from a third of the threshold on, where the K loop is long enough for their rate: 256 x 256 tiles
@@ -120,8 +112,7 @@ Choice choose(int M, int N, int K, int lda, int ldb, int swi_mode, bool add, boo
   // plain products 17 go there, none slower, up to 27 % faster: us, one-tile kernel or persistent CTAs -> here,
   // 4576 x 656 x 8184 53 -> 45, 4393 x 760 x 2544 27 -> 20. (A lone weight gradient of 768 x 3072 x 16384 takes 77 us here and
   // 69 with K split through a workspace, which callers on several streams would share; in a step it is part of a group.)
-  if (pairs && plain && K >= 256 && N > 128 && tiles(256) >= pair_min_tiles / 3 &&
-      6.0f + (0.22f + kOddPitchPair[odd]) * kb < std::min(t_cta, t_tile))
+  if (pairs && plain && K >= 256 && N > 128 && tiles(256) >= pair_min_tiles / 3 && 6.0f + 0.22f * kb < std::min(t_cta, t_tile))
     c = Choice{Choice::PERSISTENT_PAIR, 256, 1};
   return c;
 }
@@ -136,7 +127,7 @@ int gfs_linear(const void* A, const void* B, void* C, const void* R, int M, int 
                int ldr, int a_mn_major, int b_mn_major, const void* rope_cos, const void* rope_sin, int rope_cols,
                int rope_d, int rope_b, int pair_min_tiles, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const Choice c = choose(M, N, K, lda, ldb, 0, R != nullptr, rope_cos != nullptr, pair_min_tiles);
+  const Choice c = choose(M, N, K, 0, R != nullptr, rope_cos != nullptr, pair_min_tiles);
   switch (c.kernel) {
     case Choice::PERSISTENT_PAIR:
       return gfs_gemm2_bf16(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn_major, b_mn_major, rope_cos, rope_sin,
@@ -155,7 +146,7 @@ int gfs_linear_swiglu(int mode, const void* a, const void* b, void* c, void* ext
                       int ldb, int ldc, int ld_extra, int pair_min_tiles, void* stream) {
   if (mode != 1 && mode != 2) return -1;
   if (M <= 0 || I <= 0 || K <= 0) return 0;
-  const Choice ch = choose(M, I, K, lda, ldb, mode, false, false, pair_min_tiles);
+  const Choice ch = choose(M, I, K, mode, false, false, pair_min_tiles);
   switch (ch.kernel) {
     case Choice::PERSISTENT_PAIR:
       return gfs_gemm2_bf16_swiglu(mode, a, b, c, extra, M, I, K, lda, ldb, ldc, ld_extra, stream);
@@ -189,7 +180,7 @@ int gfs_wgrad_grouped(int n, const unsigned long long* A, const unsigned long lo
   const float t_pair = 6.5f + 0.3f * kb * ceil_div(tiles(256), 74) + (adds ? 2.5f : 0.f);
   // Unsplit 256 x 256 tiles on pairs are that kernel's tiles without its persistence: 95 us instead of 86 for the
   // three small gradients of a block at 16384 tokens (hidden 768, FFN 3072).
-  if (kb == kb_min && best_tile(tiles, kb, true, adds ? ADDEND : NONE, 0, &c) < t_pair && c.kernel == Choice::TILE &&
+  if (kb == kb_min && best_tile(tiles, kb, true, adds ? ADDEND : NONE, &c) < t_pair && c.kernel == Choice::TILE &&
       (c.bn != 256 || c.split > 1))
     return gfs_gemm_tile_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, accumulate, c.bn, c.split, stream);
   return gfs_gemm2_wgrad_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, accumulate, stream);

@@ -426,7 +426,7 @@ def test_pair_kernel_plain_at_the_lines(cuda_device, M, N, K):
 
 @pytest.mark.parametrize("M,N,K", [(854, 1400, 3032), (1988, 896, 2808), (494, 1536, 2056)])
 def test_gemm_long_k_with_odd_pitches(cuda_device, M, N, K):
-    """Operands whose rows begin within a 32-byte sector, behind 32 K blocks and more: other tiles are chosen for them."""
+    """Operands whose rows begin within a 32-byte sector, behind 32 K blocks and more, in every layout."""
     from gpt_from_scratch_b200.ops.gemm import gemm_bf16
     g = torch.Generator(device="cuda").manual_seed(M)
     for a_mn, b_mn in ((False, False), (False, True), (True, True), (True, False)):
