@@ -1281,7 +1281,7 @@ __global__ void cast_qkv_kernel(const CastArgs a, __nv_bfloat16* __restrict__ ds
 constexpr int DVEC_ROWS = 4;
 template <bool F16>
 __global__ void __launch_bounds__(256)
-attn_dvec_kernel(const void* __restrict__ dO_, const void* __restrict__ O_, float* __restrict__ dvec,
+attn_dvec_kernel(const void* dO_, const void* O_, float* __restrict__ dvec,
                  __nv_bfloat16* __restrict__ dO_bf16, int S, int S_pad, int B, int nh, int D, long long do_ss,
                  long long do_bs, long long do_hs, long long o_ss, long long o_bs, long long o_hs, int s_fastest) {
   pdl_wait();

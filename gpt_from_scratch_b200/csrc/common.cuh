@@ -485,6 +485,9 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_addr) {
 // kernel of the stream has completed and its writes are visible (a no-op for a normal launch);
 // nothing before it may touch global memory that another kernel writes or reads. pdl_trigger():
 // this CTA no longer objects to the next kernel's CTAs being scheduled on SMs that become free.
+// Inputs that a kernel ahead may still be writing are plain pointers, not `const __restrict__`: that would promise that nobody writes
+// them while the kernel lives, which it does from before the wait, and the compiler may then use the read-only path
+// for them and move their loads ahead of the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Registers per thread of the calling warpgroup from here on (all four warps call it).

@@ -69,9 +69,8 @@ struct DropResidual {
 };
 template <int NORM_MAXV, bool DROP>
 __global__ void __launch_bounds__(NORM_WARPS * 32)
-rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                   __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int rows, int H, float eps,
-                   const DropResidual dr) {
+rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* __restrict__ y,
+                   float* __restrict__ rstd_out, int rows, int H, float eps, const DropResidual dr) {
   pdl_wait();       // launched programmatically: the preceding kernel's output is complete from here on
   pdl_trigger();
   const int lane = threadIdx.x & 31;
@@ -155,9 +154,9 @@ constexpr int NB_WARPS = 8;
 // pass and its dw partial sums in registers; shared memory is only used once at the end.
 template <int NV>
 __global__ void __launch_bounds__(NB_WARPS * 32, NV <= 4 ? 2 : 1)
-rmsnorm_bwd_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                       const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
-                       const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+rmsnorm_bwd_reg_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                       const __nv_bfloat16* w, const float* rstd,
+                       const __nv_bfloat16* dres, __nv_bfloat16* __restrict__ dx,
                        float* __restrict__ dw_partial, int rows, int H, int rows_per_cta) {
   extern __shared__ float red[];  // [warps][H]
   pdl_wait();
@@ -269,9 +268,9 @@ struct NormBwdShape {
 // DROP: dmask = dropout's gradient of the (rounded) dx, for the branch whose output was dropped
 template <int NV, bool DROP>
 __global__ void __launch_bounds__(NormBwdShape<NV>::WARPS * 32, 2)
-rmsnorm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
-                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+rmsnorm_bwd_ring_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                        const __nv_bfloat16* w, const float* rstd,
+                        const __nv_bfloat16* dres, __nv_bfloat16* __restrict__ dx,
                         float* __restrict__ dw_partial, int rows, int H, int rows_per_cta, uint32_t* status,
                         __nv_bfloat16* __restrict__ dmask, const Dropout drop) {
   constexpr int WARPS = NormBwdShape<NV>::WARPS, SLOTS = NormBwdShape<NV>::SLOTS;
@@ -410,9 +409,9 @@ rmsnorm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
 
 // Generic path (any H that is a multiple of 8): partial sums live in shared memory.
 __global__ void __launch_bounds__(NB_WARPS * 32)
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
-                   const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+rmsnorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                   const __nv_bfloat16* w, const float* rstd,
+                   const __nv_bfloat16* dres, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ dw_partial, int rows, int H, int rows_per_cta) {
   extern __shared__ float red[];  // [warps][H]
   pdl_wait();
@@ -507,7 +506,7 @@ __global__ void rmsnorm_dw_reduce_multi_kernel(const __grid_constant__ DwReduceB
   pdl_wait();
   pdl_trigger();
   const int l = blockIdx.y;
-  const float* __restrict__ partial = b.partial[l];
+  const float* partial = b.partial[l];
   __nv_bfloat16* __restrict__ dw = b.dw[l];
   const int parts = b.parts[l];
   const int i = blockIdx.x * 32 + threadIdx.x;
@@ -563,7 +562,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 // Dropout fused with the residual add (the reference's `residual + dropout(x)`,
 // core/transformer_layer.py:97,103); the native passes have it in the RMSNorm kernels.
 // ---------------------------------------------------------------------------
-__global__ void dropout_residual_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
+__global__ void dropout_residual_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual,
                                         __nv_bfloat16* __restrict__ out, long long nvec, Dropout drop, int backward) {
   pdl_wait();
   pdl_trigger();
@@ -634,7 +633,7 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const 
 // Embedding forward: out[s - s0, b, :] = W[id - v0] if v0 <= id < v1 else 0, ids are [B, S].
 // One warp per output row.
 // ---------------------------------------------------------------------------
-__global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ W,
+__global__ void embedding_fwd_kernel(const long long* ids, const __nv_bfloat16* W,
                                      __nv_bfloat16* __restrict__ out, int B, int S, int H, int v0, int v1, int s0,
                                      int s_count) {
   pdl_wait();

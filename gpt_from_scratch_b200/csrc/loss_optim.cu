@@ -32,7 +32,7 @@ constexpr int CE_THREADS = 256;
 
 // Target id of logits row `row` (rows are [S, B]): from a [S, B] array (tb = 0) or straight from the
 // caller's [B, S] labels (tb = B), which saves the transposing copy.
-__device__ __forceinline__ long long target_of(const long long* __restrict__ target, int row, int M, int tb) {
+__device__ __forceinline__ long long target_of(const long long* target, int row, int M, int tb) {
   return tb == 0 ? target[row] : target[static_cast<size_t>(row % tb) * (M / tb) + row / tb];
 }
 
@@ -40,7 +40,7 @@ __device__ __forceinline__ long long target_of(const long long* __restrict__ tar
 // single pass. stats[row] = {local max, sum exp(z - max), z[target] or 0 if the target
 // id is outside [v0, v0+Vp)}. With single_rank != 0 also writes lse and loss.
 __global__ void __launch_bounds__(CE_THREADS)
-ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
+ce_fwd_kernel(const __nv_bfloat16* logits, const long long* target,
               float* __restrict__ stats, float* __restrict__ lse, float* __restrict__ loss, int Vp, long ld, int v0,
               int single_rank, int tb, long long* __restrict__ rows_target) {
   pdl_wait();
@@ -105,8 +105,8 @@ __device__ __forceinline__ void ce_merge(float& gm, float& gs, float2 ms) {
   gm = nm;
 }
 __global__ void __launch_bounds__(32 * CE_PW)
-ce_from_partials_kernel(const float2* __restrict__ partials, const __nv_bfloat16* __restrict__ logits,
-                        const long long* __restrict__ target, float* __restrict__ stats, float* __restrict__ lse,
+ce_from_partials_kernel(const float2* partials, const __nv_bfloat16* logits,
+                        const long long* target, float* __restrict__ stats, float* __restrict__ lse,
                         float* __restrict__ loss, int parts, int M, int Vp, long ld, int v0, int single_rank, int tb,
                         long long* __restrict__ rows_target) {
   __shared__ float2 part_res[CE_PW][32];
@@ -171,8 +171,8 @@ __global__ void ce_combine_kernel(const float* __restrict__ stats_all, float* __
 // null). Grid: x covers the vectors of a row, y strides over rows. target is in row order: finding a row's id in
 // [B, S] labels here (a division per row for eight values) made the kernel issue-bound, 612 instead of 533 us at
 // 16384 x 50304, so the forward kernels note the ids they look up.
-__global__ void ce_bwd_kernel(__nv_bfloat16* __restrict__ logits, const float* __restrict__ lse,
-                              const long long* __restrict__ target, const float* __restrict__ grad_rows, float grad_all,
+__global__ void ce_bwd_kernel(__nv_bfloat16* __restrict__ logits, const float* lse,
+                              const long long* target, const float* grad_rows, float grad_all,
                               int M, int Vp, long ld, int v0) {
   pdl_wait();
   pdl_trigger();
@@ -226,7 +226,7 @@ constexpr int SUMSQ_MAX_BLOCKS = 1024;
 // SUMSQ_MAX_BLOCKS floats followed by one uint32 ticket that must start at zero
 // (the kernel resets it).
 __global__ void __launch_bounds__(SUMSQ_THREADS)
-sumsq_bf16_kernel(const __nv_bfloat16* __restrict__ x, long long n, float* __restrict__ out,
+sumsq_bf16_kernel(const __nv_bfloat16* x, long long n, float* __restrict__ out,
                   float* __restrict__ scratch) {
   pdl_wait();
   pdl_trigger();
@@ -284,16 +284,15 @@ sumsq_bf16_kernel(const __nv_bfloat16* __restrict__ x, long long n, float* __res
 // g <- grad * grad_scale * clip_coef (clip_coef from the device scalar *sumsq, which holds the
 // squared norm of grad * grad_scale... see launcher), then torch.optim.AdamW's update on the fp32
 // master value, and the bf16 cast of the new value into the parameter buffer.
-__global__ void adamw_kernel(const __nv_bfloat16* __restrict__ grad, float* __restrict__ master,
+__global__ void adamw_kernel(const __nv_bfloat16* grad, float* __restrict__ master,
                              float* __restrict__ exp_avg, float* __restrict__ exp_avg_sq,
-                             __nv_bfloat16* __restrict__ param_out, long long n, const float* __restrict__ sumsq,
+                             __nv_bfloat16* __restrict__ param_out, long long n, const float* sumsq,
                              float* __restrict__ norm_out, AdamArgs a) {
   pdl_wait();
   pdl_trigger();
   float coef = a.grad_scale;
   if (sumsq != nullptr) {
-    // (not through the read-only path: the kernel before this one writes it)
-    const float norm = sqrtf(*reinterpret_cast<const volatile float*>(sumsq)) * a.grad_scale;
+    const float norm = sqrtf(*sumsq) * a.grad_scale;
     if (norm_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *norm_out = norm;
     if (a.clip > 0.f && norm > a.clip) coef *= a.clip / (norm + 1e-6f);
   }
@@ -343,7 +342,7 @@ __global__ void adamw_kernel(const __nv_bfloat16* __restrict__ grad, float* __re
 }
 
 // Mean of n floats by one CTA, in a fixed order.
-__global__ void __launch_bounds__(1024) mean_f32_kernel(const float* __restrict__ x, float* __restrict__ out, int n) {
+__global__ void __launch_bounds__(1024) mean_f32_kernel(const float* x, float* __restrict__ out, int n) {
   __shared__ float sm[32];
   pdl_wait();
   pdl_trigger();
